@@ -63,6 +63,43 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(ptr); }
 };
 
+// Device blocks kept between the calls of one context.  A call that needs large
+// working arrays for its own duration (the eigensolver's arenas, the purification
+// module's matrices) takes blocks here and gives them back at its end, instead of
+// a cudaMalloc and a cudaFree (which waits for the device) per array and call.
+// Blocks are handed out by best fit; their users run on the context's stream or on
+// side streams ordered after it, so a block given back may be taken again at once.
+// The blocks kept unused are bounded (1/16 of the device's memory per context) and
+// freed by ptbgpu_finalize, by trim(), or when any allocation of the library on any
+// context of the process finds no memory (trim_all()).
+class WorkPool {
+public:
+    WorkPool();
+    ~WorkPool();
+    void* take(size_t nbytes, size_t* got);
+    void give(void* ptr, size_t nbytes);
+    void trim();
+    static void trim_all();
+
+private:
+    struct Impl;
+    std::unique_ptr<Impl> im_;
+};
+
+// A call's working array out of its context's pool (given back on destruction).
+struct WorkBuf {
+    std::shared_ptr<WorkPool> pool;
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    WorkBuf() = default;
+    WorkBuf(const WorkBuf&) = delete;
+    WorkBuf& operator=(const WorkBuf&) = delete;
+    ~WorkBuf() { release(); }
+    void reserve(ptbgpu_ctx* c, size_t nbytes);
+    void release();
+    template <class T> T* as() const { return static_cast<T*>(ptr); }
+};
+
 // Device-side error word written by kernels whose bounded waits give up.
 struct DeviceFlags {
     int timeout;      // nonzero: a bounded wait expired (value = site id)
@@ -89,6 +126,8 @@ struct ptbgpu_ctx {
     void* pinned = nullptr;              // small pinned staging area (4 KB)
     // trace-correcting purification state (device)
     void* sp2_state = nullptr;
+    // working blocks kept between calls (shared with the arrays that hold blocks)
+    std::shared_ptr<ptb::WorkPool> work = std::make_shared<ptb::WorkPool>();
     // submatrix method between its phases (plan, prepare, nel, finish): kept
     // until the next plan or the context's end; its destructor frees its buffers
     std::shared_ptr<void> sm_plan;

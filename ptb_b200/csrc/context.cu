@@ -1,5 +1,7 @@
 // Context lifecycle, error plumbing and scratch buffers of libptbgpu.
+#include <algorithm>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -19,6 +21,11 @@ void DevBuf::reserve(size_t nbytes) {
     release();
     nbytes = (nbytes + 255) & ~size_t(255);
     cudaError_t e = cudaMalloc(&ptr, nbytes);
+    if (e == cudaErrorMemoryAllocation) {   // the blocks kept between calls make room
+        (void)cudaGetLastError();
+        WorkPool::trim_all();
+        e = cudaMalloc(&ptr, nbytes);
+    }
     if (e != cudaSuccess) {
         ptr = nullptr;
         bytes = 0;
@@ -32,6 +39,145 @@ void DevBuf::release() {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
+}
+
+// Free blocks of one context; every pool of the process is in the registry so
+// that an allocation that fails on one context can have the others' unused blocks
+// freed.  The registry's lock is taken before a pool's.
+struct WorkPool::Impl {
+    struct Block {
+        void* ptr;
+        size_t bytes;
+    };
+    std::mutex mu;
+    std::vector<Block> free_blocks;   // in the order they were given back
+    size_t kept = 0;
+    size_t limit = 0;                 // bytes kept unused at most (set at the first block)
+};
+
+namespace {
+
+struct PoolRegistry {
+    std::mutex mu;
+    std::vector<WorkPool*> pools;
+};
+PoolRegistry& pool_registry() {
+    static PoolRegistry* r = new PoolRegistry();   // outlives the contexts of late destructors
+    return *r;
+}
+
+// Sizes are rounded up to eighths of a power of two, so that calls on systems of
+// about the same size find each other's blocks.
+size_t work_class(size_t nbytes) {
+    size_t step = 256;
+    while (step * 16 < nbytes) step *= 2;
+    return (nbytes + step - 1) / step * step;
+}
+
+}  // namespace
+
+WorkPool::WorkPool() : im_(new Impl()) {
+    PoolRegistry& r = pool_registry();
+    std::lock_guard<std::mutex> lock(r.mu);
+    r.pools.push_back(this);
+}
+
+WorkPool::~WorkPool() {
+    PoolRegistry& r = pool_registry();
+    {
+        std::lock_guard<std::mutex> lock(r.mu);
+        r.pools.erase(std::remove(r.pools.begin(), r.pools.end(), this), r.pools.end());
+    }
+    trim();
+}
+
+void WorkPool::trim() {
+    std::vector<Impl::Block> gone;
+    {
+        std::lock_guard<std::mutex> lock(im_->mu);
+        gone.swap(im_->free_blocks);
+        im_->kept = 0;
+    }
+    for (const Impl::Block& b : gone) cudaFree(b.ptr);
+}
+
+void WorkPool::trim_all() {
+    PoolRegistry& r = pool_registry();
+    std::lock_guard<std::mutex> lock(r.mu);
+    for (WorkPool* p : r.pools) p->trim();
+}
+
+void* WorkPool::take(size_t nbytes, size_t* got) {
+    const size_t want = work_class(std::max<size_t>(nbytes, 1));
+    {
+        std::lock_guard<std::mutex> lock(im_->mu);
+        size_t best = im_->free_blocks.size();
+        for (size_t i = 0; i < im_->free_blocks.size(); ++i) {
+            const size_t b = im_->free_blocks[i].bytes;
+            if (b >= want && b <= want + want / 2 &&
+                (best == im_->free_blocks.size() || b < im_->free_blocks[best].bytes))
+                best = i;
+        }
+        if (best < im_->free_blocks.size()) {
+            const Impl::Block b = im_->free_blocks[best];
+            im_->free_blocks.erase(im_->free_blocks.begin() + best);
+            im_->kept -= b.bytes;
+            *got = b.bytes;
+            return b.ptr;
+        }
+        if (im_->limit == 0) {
+            size_t free_b = 0, total_b = 0;
+            if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) im_->limit = total_b / 16;
+        }
+    }
+    void* ptr = nullptr;
+    cudaError_t e = cudaMalloc(&ptr, want);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        trim_all();
+        e = cudaMalloc(&ptr, want);
+    }
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        fail(PTBGPU_ENOMEM, "cudaMalloc(%zu) failed: %s", want, cudaGetErrorString(e));
+    }
+    *got = want;
+    return ptr;
+}
+
+void WorkPool::give(void* ptr, size_t nbytes) {
+    std::vector<Impl::Block> gone;
+    {
+        std::lock_guard<std::mutex> lock(im_->mu);
+        if (nbytes > im_->limit) {
+            gone.push_back({ptr, nbytes});
+        } else {
+            // the oldest blocks make room: sizes that no call asks for any more go first
+            size_t drop = 0;
+            while (im_->kept + nbytes > im_->limit) {
+                im_->kept -= im_->free_blocks[drop].bytes;
+                gone.push_back(im_->free_blocks[drop++]);
+            }
+            im_->free_blocks.erase(im_->free_blocks.begin(), im_->free_blocks.begin() + drop);
+            im_->free_blocks.push_back({ptr, nbytes});
+            im_->kept += nbytes;
+        }
+    }
+    for (const Impl::Block& b : gone) cudaFree(b.ptr);
+}
+
+void WorkBuf::reserve(ptbgpu_ctx* c, size_t nbytes) {
+    if (ptr && nbytes <= bytes) return;
+    release();
+    ptr = c->work->take(nbytes, &bytes);
+    pool = c->work;
+}
+
+void WorkBuf::release() {
+    if (ptr) pool->give(ptr, bytes);
+    ptr = nullptr;
+    bytes = 0;
+    pool.reset();
 }
 
 int64_t& launch_counter() {
@@ -119,6 +265,7 @@ int ptbgpu_finalize(ptbgpu_ctx* c) {
     c->sm_side.reset();
     for (ptbgpu_ctx* w : c->workers) ptbgpu_finalize(w);
     c->workers.clear();
+    c->work->trim();
     for (auto& b : c->bufs) b.release();
     if (c->flags) cudaFree(c->flags);
     if (c->info_dev) cudaFree(c->info_dev);

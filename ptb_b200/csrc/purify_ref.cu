@@ -118,17 +118,14 @@ struct Ctx {
     int64_t n;
     Thr thr;
     int prl;
-    DevBuf scratch[8];
+    WorkBuf scratch[8];
     double* m[8];
     double gemm_flops = 0.0;   // 2n^3 per DGEMM issued (eigensolves not counted)
     Ctx(ptbgpu_ctx* cc, int64_t nn, int p) : c(cc), n(nn), thr(thresholds(nn)), prl(p) {
         for (int k = 0; k < 8; ++k) {
-            scratch[k].reserve(sizeof(double) * nn * nn);
+            scratch[k].reserve(cc, sizeof(double) * nn * nn);
             m[k] = scratch[k].as<double>();
         }
-    }
-    ~Ctx() {
-        for (auto& b : scratch) b.release();
     }
     // The module's products on the int8 tensor cores (8 slices, FP64 class);
     // beyond the exact int32 range of the slice sums (n > 16643) cuBLAS DGEMM.
@@ -143,10 +140,10 @@ struct Ctx {
         gemm_flops += 2.0 * (double)n * (double)n * (double)n;
     }
     static constexpr int kSlices = 8;
-    DevBuf loopdev;
+    WorkBuf loopdev;
     LoopGraph sign_loop, mcw_loop;
     LoopDev* ld() {
-        loopdev.reserve(sizeof(LoopDev));
+        loopdev.reserve(c, sizeof(LoopDev));
         return loopdev.as<LoopDev>();
     }
     // Captures body() into a WHILE node's body graph followed by the decision
@@ -267,8 +264,8 @@ void transformation(Ctx& x, const ptbgpu_pur_settings& pur, const double* S, dou
     // eigendecomposition of S: X = V D V^T with D = 1/w or 1/sqrt(w)
     double* V = x.m[4];
     copy_mat(s, n, n, S, n, V);
-    DevBuf w;
-    w.reserve(sizeof(double) * n);
+    WorkBuf w;
+    w.reserve(x.c, sizeof(double) * n);
     dsyevd(x.c, n, n, V, w.as<double>());
     std::vector<double> hw(n);
     PTB_CUDA(cudaMemcpy(hw.data(), w.ptr, sizeof(double) * n, cudaMemcpyDeviceToHost));
@@ -442,9 +439,9 @@ void sign_diag(Ctx& x, const ptbgpu_pur_settings& pur, double& chempot, const do
     double* V = x.m[4];
     double* tmp = x.m[5];
     copy_mat(s, n, n, guess, n, V);
-    DevBuf w, cs;
-    w.reserve(sizeof(double) * n);
-    cs.reserve(sizeof(double) * n);
+    WorkBuf w, cs;
+    w.reserve(x.c, sizeof(double) * n);
+    cs.reserve(x.c, sizeof(double) * n);
     dsyevd(x.c, n, n, V, w.as<double>());
     k_colsq<<<g1(n), 256, 0, s>>>(n, V, cs.as<double>());
     count_launch();

@@ -2728,16 +2728,15 @@ struct EigBatch {
     int G = 1;                    // CTAs per cluster of the large-submatrix solver
     int nsmall = 0, nlarge = 0;
     std::vector<EigProb> hp;
-    DevBuf probs, order, order_l, counter, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Xa, Ka, status, tstage;
+    WorkBuf probs, order, order_l, counter, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Xa, Ka, status, tstage;
     int prl = 0;
     const char* what = "submatrix";   // the problems' name in error messages
     cudaStream_t side = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     ~EigBatch() {
+        // the arrays go back to the context's pool: nothing on the side stream may
+        // still use them (work on the context's stream is ordered before their next use)
         if (side) cudaStreamSynchronize(side);
-        for (DevBuf* b : {&probs, &order, &order_l, &counter, &Ca, &La, &Za, &Qa, &Va, &Da, &Ea, &Ta, &Wa, &Ba, &Xa,
-                          &Ka, &status, &tstage})
-            b->release();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (side) cudaStreamDestroy(side);
@@ -2909,13 +2908,13 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
     const int np = eb->nprob;
     eb->nsmall = (int)ord_s.size();
     eb->nlarge = (int)ord_l.size();
-    eb->probs.reserve(sizeof(EigProb) * np);
-    for (DevBuf* b : {&eb->Ca, &eb->La, &eb->Za, &eb->Qa, &eb->Va}) b->reserve(sizeof(double) * asz);
-    for (DevBuf* b : {&eb->Da, &eb->Ea, &eb->Ta, &eb->Wa}) b->reserve(sizeof(double) * vsz);
-    eb->Ba.reserve(sizeof(double) * std::max<int64_t>(bsz, 1));
-    eb->Xa.reserve(sizeof(double) * std::max<int64_t>(xsz, 2));
-    eb->Ka.reserve(sizeof(double) * std::max<int64_t>(ksz, 2));
-    eb->status.reserve(sizeof(int) * np);
+    eb->probs.reserve(c, sizeof(EigProb) * np);
+    for (WorkBuf* b : {&eb->Ca, &eb->La, &eb->Za, &eb->Qa, &eb->Va}) b->reserve(c, sizeof(double) * asz);
+    for (WorkBuf* b : {&eb->Da, &eb->Ea, &eb->Ta, &eb->Wa}) b->reserve(c, sizeof(double) * vsz);
+    eb->Ba.reserve(c, sizeof(double) * std::max<int64_t>(bsz, 1));
+    eb->Xa.reserve(c, sizeof(double) * std::max<int64_t>(xsz, 2));
+    eb->Ka.reserve(c, sizeof(double) * std::max<int64_t>(ksz, 2));
+    eb->status.reserve(c, sizeof(int) * np);
     PTB_CUDA(cudaMemcpyAsync(eb->probs.ptr, eb->hp.data(), sizeof(EigProb) * np, cudaMemcpyHostToDevice, s));
     PTB_CUDA(cudaMemsetAsync(eb->status.ptr, 0, sizeof(int) * np, s));
     const EigProb* dp = eb->probs.as<EigProb>();
@@ -2925,9 +2924,9 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
     auto by_size = [&](int a, int b) { return eb->hp[a].m > eb->hp[b].m; };
     std::stable_sort(ord_s.begin(), ord_s.end(), by_size);
     std::stable_sort(ord_l.begin(), ord_l.end(), by_size);
-    eb->order.reserve(sizeof(int) * std::max<size_t>(ord_s.size(), 1));
-    eb->order_l.reserve(sizeof(int) * std::max<size_t>(ord_l.size(), 1));
-    eb->counter.reserve(sizeof(int));
+    eb->order.reserve(c, sizeof(int) * std::max<size_t>(ord_s.size(), 1));
+    eb->order_l.reserve(c, sizeof(int) * std::max<size_t>(ord_l.size(), 1));
+    eb->counter.reserve(c, sizeof(int));
     if (!ord_s.empty())
         PTB_CUDA(cudaMemcpyAsync(eb->order.ptr, ord_s.data(), sizeof(int) * ord_s.size(), cudaMemcpyHostToDevice, s));
     if (!ord_l.empty())
@@ -2941,7 +2940,7 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
         PTB_CUDA(cudaEventCreateWithFlags(&eb->ev1, cudaEventDisableTiming));
         unsigned long long* dts = nullptr;
         if (prl >= 2) {
-            eb->tstage.reserve(sizeof(unsigned long long) * kLgStride * np);
+            eb->tstage.reserve(c, sizeof(unsigned long long) * kLgStride * np);
             PTB_CUDA(cudaMemsetAsync(eb->tstage.ptr, 0, sizeof(unsigned long long) * kLgStride * np, s));
             dts = eb->tstage.as<unsigned long long>();
         }
@@ -3089,16 +3088,16 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
     const int64_t mm = (int64_t)m * m;
     const int per = (m + G - 1) / G;
     const LgLayout lay = lg_layout(m, G);
-    for (DevBuf* b : {&eb.Ca, &eb.La, &eb.Za}) b->reserve(sizeof(double) * mm);
-    eb.Qa.reserve(sizeof(double) * std::max<int64_t>(mm, (int64_t)G * lg_wy_stride(per) + 2));
-    eb.Va.reserve(sizeof(double) * std::max<int64_t>(mm, (int64_t)G * NB * NB + 2));
-    for (DevBuf* b : {&eb.Da, &eb.Ea, &eb.Ta, &eb.Wa}) b->reserve(sizeof(double) * n);
-    eb.Ka.reserve(sizeof(double) * std::max<int64_t>(t_panels(m) * NB * NB, 2));
-    eb.Xa.reserve(sizeof(double) * lay.total);
-    eb.Ba.reserve(sizeof(double) * 2);
-    eb.probs.reserve(sizeof(EigProb));
-    eb.status.reserve(sizeof(int) * 4);
-    eb.order.reserve(sizeof(int) * n);   // the identity row map
+    for (WorkBuf* b : {&eb.Ca, &eb.La, &eb.Za}) b->reserve(c, sizeof(double) * mm);
+    eb.Qa.reserve(c, sizeof(double) * std::max<int64_t>(mm, (int64_t)G * lg_wy_stride(per) + 2));
+    eb.Va.reserve(c, sizeof(double) * std::max<int64_t>(mm, (int64_t)G * NB * NB + 2));
+    for (WorkBuf* b : {&eb.Da, &eb.Ea, &eb.Ta, &eb.Wa}) b->reserve(c, sizeof(double) * n);
+    eb.Ka.reserve(c, sizeof(double) * std::max<int64_t>(t_panels(m) * NB * NB, 2));
+    eb.Xa.reserve(c, sizeof(double) * lay.total);
+    eb.Ba.reserve(c, sizeof(double) * 2);
+    eb.probs.reserve(c, sizeof(EigProb));
+    eb.status.reserve(c, sizeof(int) * 4);
+    eb.order.reserve(c, sizeof(int) * n);   // the identity row map
     std::vector<int> ident(n);
     for (int i = 0; i < m; ++i) ident[i] = i;
     PTB_CUDA(cudaMemcpyAsync(eb.order.ptr, ident.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
@@ -3122,7 +3121,7 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
         const int* order = eb.order.as<int>() + 0;   // identity map: order[0] = 0
         unsigned long long* ts = nullptr;
         if (stages) {
-            eb.tstage.reserve(sizeof(unsigned long long) * kLgStride);
+            eb.tstage.reserve(c, sizeof(unsigned long long) * kLgStride);
             PTB_CUDA(cudaMemsetAsync(eb.tstage.ptr, 0, sizeof(unsigned long long) * kLgStride, s));
             ts = eb.tstage.as<unsigned long long>();
         }
@@ -3154,22 +3153,14 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
 
 void eig_full_upper(ptbgpu_ctx* c, int64_t n, double* A, double* B, double* w) {
     cudaStream_t s = c->stream;
-    DevBuf h, b, u;
-    struct Rel {
-        DevBuf *x, *y, *z;
-        ~Rel() {
-            x->release();
-            y->release();
-            z->release();
-        }
-    } rel{&h, &b, &u};
-    h.reserve(sizeof(double) * n * n);
-    u.reserve(sizeof(double) * n * n);
+    WorkBuf h, b, u;
+    h.reserve(c, sizeof(double) * n * n);
+    u.reserve(c, sizeof(double) * n * n);
     const int grid = (int)std::min<int64_t>((n * n + 255) / 256, 148 * 16);
     k_sym_from_upper<<<grid, 256, 0, s>>>(n, A, h.as<double>());
     count_launch();
     if (B) {
-        b.reserve(sizeof(double) * n * n);
+        b.reserve(c, sizeof(double) * n * n);
         k_sym_from_upper<<<grid, 256, 0, s>>>(n, B, b.as<double>());
         count_launch();
     }
@@ -3230,17 +3221,14 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
         (m > kEigBatchMax ? large : small).push_back(k);
     }
     struct Bufs {
-        DevBuf h, sm, pk, maps, e, dummy;
-        ~Bufs() {
-            for (DevBuf* b : {&h, &sm, &pk, &maps, &e, &dummy}) b->release();
-        }
+        WorkBuf h, sm, pk, maps, e, dummy;
     } b;
-    b.h.reserve(sizeof(double) * hsz);
-    b.sm.reserve(sizeof(double) * hsz);
-    b.pk.reserve(sizeof(double) * std::max<int64_t>(2 * pkoff[ninst], 1));
-    b.maps.reserve(sizeof(int) * nsum);
-    b.e.reserve(sizeof(double) * nsum);
-    b.dummy.reserve(64);
+    b.h.reserve(c, sizeof(double) * hsz);
+    b.sm.reserve(c, sizeof(double) * hsz);
+    b.pk.reserve(c, sizeof(double) * std::max<int64_t>(2 * pkoff[ninst], 1));
+    b.maps.reserve(c, sizeof(int) * nsum);
+    b.e.reserve(c, sizeof(double) * nsum);
+    b.dummy.reserve(c, 64);
     std::vector<int> maps((size_t)nsum);
     for (const EigProbHost& q : pr)
         for (int i = 0; i < q.m; ++i) maps[q.moff + i] = i;
@@ -3301,10 +3289,7 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
 void sygv_batched_entry(ptbgpu_ctx* c, int64_t np, const int64_t* dims, const double* H, const double* S,
                         const int64_t* nown, const int64_t* owned, double mu, double* e, double* fe, double* Pcols) {
     struct Bufs {
-        DevBuf h, s, maps, own, ipos, e, fe, p;
-        ~Bufs() {
-            for (DevBuf* b : {&h, &s, &maps, &own, &ipos, &e, &fe, &p}) b->release();
-        }
+        WorkBuf h, s, maps, own, ipos, e, fe, p;
     } b;
     cudaStream_t st = c->stream;
     std::vector<EigProbHost> probs;
@@ -3340,13 +3325,13 @@ void sygv_batched_entry(ptbgpu_ctx* c, int64_t np, const int64_t* dims, const do
         osum += nown[k];
         psz += (int64_t)m * nown[k];
     }
-    b.h.reserve(sizeof(double) * hsz);
-    b.s.reserve(sizeof(double) * hsz);
-    b.maps.reserve(sizeof(int) * nsum);
-    b.own.reserve(sizeof(int) * osum);
-    b.ipos.reserve(sizeof(int) * nsum);
-    b.e.reserve(sizeof(double) * nsum);
-    b.fe.reserve(sizeof(double) * nsum);
+    b.h.reserve(c, sizeof(double) * hsz);
+    b.s.reserve(c, sizeof(double) * hsz);
+    b.maps.reserve(c, sizeof(int) * nsum);
+    b.own.reserve(c, sizeof(int) * osum);
+    b.ipos.reserve(c, sizeof(int) * nsum);
+    b.e.reserve(c, sizeof(double) * nsum);
+    b.fe.reserve(c, sizeof(double) * nsum);
     PTB_CUDA(cudaMemcpyAsync(b.h.ptr, H, sizeof(double) * hsz, cudaMemcpyHostToDevice, st));
     PTB_CUDA(cudaMemcpyAsync(b.s.ptr, S, sizeof(double) * hsz, cudaMemcpyHostToDevice, st));
     PTB_CUDA(cudaMemcpyAsync(b.maps.ptr, maps.data(), sizeof(int) * nsum, cudaMemcpyHostToDevice, st));
@@ -3359,7 +3344,7 @@ void sygv_batched_entry(ptbgpu_ctx* c, int64_t np, const int64_t* dims, const do
     PTB_CUDA(cudaMemcpyAsync(e, b.e.ptr, sizeof(double) * nsum, cudaMemcpyDeviceToHost, st));
     PTB_CUDA(cudaMemcpyAsync(fe, b.fe.ptr, sizeof(double) * nsum, cudaMemcpyDeviceToHost, st));
     if (Pcols) {
-        b.p.reserve(sizeof(double) * psz);
+        b.p.reserve(c, sizeof(double) * psz);
         eig_batch_final(c, *eb, mu, 0, b.maps.as<int>(), b.own.as<int>(), nullptr, b.p.as<double>());
         PTB_CUDA(cudaMemcpyAsync(Pcols, b.p.ptr, sizeof(double) * psz, cudaMemcpyDeviceToHost, st));
     }

@@ -573,7 +573,14 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     PTB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t other = 6 * fplane + 4 * plane + (size_t)(64 << 20);
     int slots = (int)std::min<int64_t>(maxit + 1, kMaxIt + 1);
-    if (free_b > other) slots = (int)std::min<size_t>(slots, (free_b - other) * 6 / 10 / (tp * plane));
+    auto fit = [&] {
+        return free_b > other ? (int)std::min<size_t>(maxit + 1, (free_b - other) * 6 / 10 / (tp * plane)) : slots;
+    };
+    if (free_b <= other || fit() < slots) {   // the blocks kept between calls make room
+        WorkPool::trim_all();
+        PTB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    }
+    slots = std::min(slots, fit());
     PTB_CHECK(slots >= std::min(8, maxit + 1), PTBGPU_ENOMEM,
               "not enough device memory for the purification trajectory");
     DevBuf& btraj = c->buf(B_TRAJ);

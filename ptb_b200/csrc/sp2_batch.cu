@@ -958,6 +958,7 @@ void tc_purify_grouped(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
     std::iota(idx.begin(), idx.end(), 0);
     std::stable_sort(idx.begin(), idx.end(), [&](int64_t a, int64_t b) { return ndim[a] > ndim[b]; });
     size_t free_b = 0, total_b = 0;
+    WorkPool::trim_all();   // the budget counts the blocks kept between calls as free
     PTB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const double budget = 0.6 * (double)free_b;
     std::vector<Chunk> chunks;

@@ -1237,8 +1237,8 @@ void sm_density_device(ptbgpu_ctx* c, int64_t n, int64_t nelref, const double* d
     sm_prepare(c, pl, all);
     const auto t2 = clk::now();
     cudaStream_t s = c->stream;
-    DevBuf bmu;
-    bmu.reserve(sizeof(MuResult));
+    WorkBuf bmu;
+    bmu.reserve(c, sizeof(MuResult));
     const double tol_mu = (double)1e-3f, tol_nel = (double)1e-5f;
     k_mu_bisect<<<1, 1024, 0, s>>>(pl.total, c->buf(B_MISC0).as<double>(), c->buf(B_MISC1).as<double>(),
                                    (double)nelref, tol_mu, tol_nel, bmu.as<MuResult>());
@@ -1247,7 +1247,6 @@ void sm_density_device(ptbgpu_ctx* c, int64_t n, int64_t nelref, const double* d
     MuResult mr;
     PTB_CUDA(cudaMemcpyAsync(&mr, bmu.ptr, sizeof(MuResult), cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
-    bmu.release();
     for (int it = 0; it < mr.iters; ++it)
         log_line(prl, 1, " muiter %d mu %.15g %.15g of %lld", it + 1, mr.trace_mu[it], mr.trace_nel[it],
                  (long long)nelref);
