@@ -351,247 +351,7 @@ __device__ int stage_potrf(const EigProb& p, double* __restrict__ La, const Stag
     return 0;
 }
 
-// X <- L^-1 X (L lower, m x m; X m x m), blocked by 32 rows.
-__device__ void trsm_left_lower(const double* __restrict__ L, double* __restrict__ X, int m, double* sA, double* sB,
-                                double* sD) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i0 = 0; i0 < m; i0 += NB) {
-        const int nb = min(NB, m - i0), i1 = i0 + nb;
-        for (int t = tid; t < NB * NB; t += kT) {
-            const int i = t % NB, j = t / NB;
-            sD[i + j * (NB + 1)] = (i < nb && j < nb) ? L[(int64_t)(i0 + i) + (int64_t)(i0 + j) * m] : 0.0;
-        }
-        __syncthreads();
-        // diagonal block: warp per column of X, lanes over its rows
-        for (int j = warp; j < m; j += kT / 32) {
-            double x = (lane < nb) ? X[(int64_t)(i0 + lane) + (int64_t)j * m] : 0.0;
-            for (int k = 0; k < nb; ++k) {
-                if (lane == k) x /= sD[k + k * (NB + 1)];
-                const double xk = __shfl_sync(0xffffffffu, x, k);
-                if (lane > k && lane < nb) x -= sD[lane + k * (NB + 1)] * xk;
-            }
-            if (lane < nb) X[(int64_t)(i0 + lane) + (int64_t)j * m] = x;
-        }
-        __syncthreads();
-        for (int c0 = 0; c0 < m; c0 += TS)
-            for (int r0 = i1; r0 < m; r0 += TS)
-                tile_update<false, false>(X, m, r0, c0, min(TS, m - r0), min(TS, m - c0), L + (int64_t)i0 * m, m,
-                                          X + i0, m, nb, sA, sB);
-    }
-}
-
-// C <- L^-1 H_k L^-T: C <- L^-1 C, transpose, C <- L^-1 C, then the lower
-// triangle copied to the upper one (exactly symmetric).
-__device__ void stage_reduce(const EigProb& p, const double* __restrict__ La, double* __restrict__ Ca,
-                             const StageSmem& sh) {
-    double* sA = sh.sA;
-    double* sB = sh.sB;
-    double* sD = sh.sD;
-    const int m = p.m;
-    const double* L = La + p.aoff;
-    double* C = Ca + p.aoff;
-    trsm_left_lower(L, C, m, sA, sB, sD);
-    __syncthreads();
-    for (int64_t t = threadIdx.x; t < (int64_t)m * m; t += kT) {
-        const int i = (int)(t % m), j = (int)(t / m);
-        if (i > j) {
-            const double a = C[i + (int64_t)j * m], b = C[j + (int64_t)i * m];
-            C[i + (int64_t)j * m] = b;
-            C[j + (int64_t)i * m] = a;
-        }
-    }
-    __syncthreads();
-    trsm_left_lower(L, C, m, sA, sB, sD);
-    __syncthreads();
-    for (int64_t t = threadIdx.x; t < (int64_t)m * m; t += kT) {
-        const int i = (int)(t % m), j = (int)(t / m);
-        if (i > j) C[j + (int64_t)i * m] = C[i + (int64_t)j * m];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Householder tridiagonalisation of C (lower).  Iteration j applies the
-// previous reflector's rank-2 update to column j, forms reflector j from it
-// (LAPACK's dlarfg convention: beta = -sign(alpha) |x|, tau = (beta - alpha) /
-// beta, v = x / (alpha - beta) with v_{j+1} = 1), and in one pass over the
-// trailing block applies the previous update and accumulates p = A v for the
-// new reflector; w = tau p - (tau^2/2)(p.v) v.  The trailing block is read and
-// written once per column.  Output: d (m), e (m-1), tau, and v_j in C's column
-// j below the subdiagonal.
-constexpr int kSyRows = (kEigBatchMax + kT - 1) / kT;   // rows per thread
-constexpr int kSyChunk = 8;                              // columns per batch of loads
-
-__device__ void stage_sytrd(const EigProb& p, double* __restrict__ Ca, double* __restrict__ Da,
-                            double* __restrict__ Ea, double* __restrict__ Ta, const StageSmem& sh) {
-    double* vc = reinterpret_cast<double*>(sh.uni);
-    double* wc = vc + sh.M;
-    double* vn = wc + sh.M;
-    double* red = sh.dsc + 2;
-    double& sh_tau = sh.dsc[0];
-    double& sh_alpha = sh.dsc[1];
-    const int m = p.m;
-    double* A = Ca + p.aoff;
-    double* d = Da + p.voff;
-    double* e = Ea + p.voff;
-    double* tau = Ta + p.voff;
-    const int tid = threadIdx.x;
-    if (m == 1) {
-        if (tid == 0) {
-            d[0] = A[0];
-            tau[0] = 0.0;
-        }
-        return;
-    }
-    for (int r = tid; r < m; r += kT) {
-        vc[r] = 0.0;
-        wc[r] = 0.0;
-    }
-    __syncthreads();
-    for (int j = 0; j <= m - 2; ++j) {
-        // (1) column j (rows >= j) gets the previous reflector's update
-        const double vj = vc[j], wj = wc[j];
-        for (int r = j + tid; r < m; r += kT) {
-            double a = A[r + (int64_t)j * m];
-            a -= vc[r] * wj + wc[r] * vj;
-            A[r + (int64_t)j * m] = a;
-            vn[r] = a;
-        }
-        __syncthreads();
-        if (j == m - 2) {
-            if (tid == 0) {
-                d[m - 2] = vn[m - 2];
-                e[m - 2] = vn[m - 1];
-                double a = A[(m - 1) + (int64_t)(m - 1) * m];
-                a -= 2.0 * vc[m - 1] * wc[m - 1];
-                A[(m - 1) + (int64_t)(m - 1) * m] = a;
-                d[m - 1] = a;
-                tau[m - 2] = 0.0;
-                tau[m - 1] = 0.0;
-            }
-            break;
-        }
-        // (2) reflector of x = column j, rows j+1..m-1
-        double part = 0.0;
-        for (int r = j + 2 + tid; r < m; r += kT) part += vn[r] * vn[r];
-        const double xn2 = cta_sum(part, red);
-        if (tid == 0) {
-            const double alpha = vn[j + 1];
-            d[j] = vn[j];
-            double t, beta;
-            if (xn2 == 0.0) {
-                t = 0.0;
-                beta = alpha;
-            } else {
-                beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-                t = (beta - alpha) / beta;
-            }
-            e[j] = beta;
-            tau[j] = t;
-            sh_tau = t;
-            sh_alpha = (t == 0.0) ? 0.0 : 1.0 / (alpha - beta);
-            A[(j + 1) + (int64_t)j * m] = beta;
-        }
-        __syncthreads();
-        const double t = sh_tau, sc = sh_alpha;
-        for (int r = j + 1 + tid; r < m; r += kT) {
-            double v;
-            if (r == j + 1) v = 1.0;
-            else v = (t == 0.0) ? 0.0 : vn[r] * sc;
-            vn[r] = v;
-            if (r >= j + 2) A[r + (int64_t)j * m] = v;
-        }
-        __syncthreads();
-        // (3) trailing block [j+1, m)^2: previous update + p = A v
-        const int r0 = j + 1;
-        double acc[kSyRows], vr[kSyRows], wr[kSyRows];
-#pragma unroll
-        for (int q = 0; q < kSyRows; ++q) {
-            const int r = r0 + tid + q * kT;
-            acc[q] = 0.0;
-            vr[q] = (r < m) ? vc[r] : 0.0;
-            wr[q] = (r < m) ? wc[r] : 0.0;
-        }
-        // columns in chunks of kSyChunk: every load of a chunk is issued before
-        // its stores, so the pass streams instead of waiting on each element;
-        // threads without a row in the trailing block skip the pass, and while
-        // the block has at most kT rows each thread carries one row only
-        const bool has_row = r0 + tid < m;
-        if (m - r0 <= kT) {
-            double* colbase = A + r0 + tid;
-            for (int k0 = has_row ? r0 : m; k0 < m; k0 += kSyChunk) {
-                double a1[kSyChunk];
-#pragma unroll
-                for (int u = 0; u < kSyChunk; ++u) {
-                    const int k = k0 + u;
-                    a1[u] = (k < m) ? colbase[(int64_t)k * m] : 0.0;
-                }
-#pragma unroll
-                for (int u = 0; u < kSyChunk; ++u) {
-                    const int k = k0 + u;
-                    if (k < m) {
-                        const double x = a1[u] - (vr[0] * wc[k] + wr[0] * vc[k]);
-                        colbase[(int64_t)k * m] = x;
-                        acc[0] = fma(x, vn[k], acc[0]);
-                    }
-                }
-            }
-        } else
-        for (int k0 = has_row ? r0 : m; k0 < m; k0 += kSyChunk) {
-            double a[kSyChunk][kSyRows];
-#pragma unroll
-            for (int u = 0; u < kSyChunk; ++u) {
-                const int k = k0 + u;
-#pragma unroll
-                for (int q = 0; q < kSyRows; ++q) {
-                    const int r = r0 + tid + q * kT;
-                    a[u][q] = (k < m && r < m) ? A[r + (int64_t)k * m] : 0.0;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kSyChunk; ++u) {
-                const int k = k0 + u;
-                if (k < m) {
-                    const double vk = vc[k], wk = wc[k], nk = vn[k];
-#pragma unroll
-                    for (int q = 0; q < kSyRows; ++q) {
-                        const int r = r0 + tid + q * kT;
-                        if (r < m) {
-                            const double x = a[u][q] - (vr[q] * wk + wr[q] * vk);
-                            A[r + (int64_t)k * m] = x;
-                            acc[q] = fma(x, nk, acc[q]);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        // (4) w = tau p - (tau/2)(tau p . v) v
-        double pv = 0.0;
-#pragma unroll
-        for (int q = 0; q < kSyRows; ++q) {
-            const int r = r0 + tid + q * kT;
-            if (r < m) {
-                acc[q] *= t;
-                pv += acc[q] * vn[r];
-            }
-        }
-        const double ptv = cta_sum(pv, red);
-        const double half = 0.5 * t * ptv;
-#pragma unroll
-        for (int q = 0; q < kSyRows; ++q) {
-            const int r = r0 + tid + q * kT;
-            if (r < m) {
-                wc[r] = acc[q] - half * vn[r];
-                vc[r] = vn[r];
-            }
-        }
-        if (tid == 0) {
-            vc[j] = 0.0;
-            wc[j] = 0.0;
-        }
-        __syncthreads();
-    }
-}
+#include "eig_trd.cuh"
 
 // ---------------------------------------------------------------------------
 // C[crow + r0 + i, col(c0 + j)] = sum_k A(i, kx(k)) B(kxb(k), j) on one TS x TS
@@ -1427,12 +1187,12 @@ __device__ void stage_density(const EigProb& p, const double* __restrict__ Ca, c
 }
 
 // ---------------------------------------------------------------------------
-// One persistent launch for every submatrix of the step: each CTA takes the
-// next submatrix (largest first) from a device counter and runs all stages on
-// it - gather, Cholesky, reduction, tridiagonalisation, divide and conquer,
-// owned rows and fe - so the uneven sizes balance over the SMs without a
-// launch per stage or per size bucket.  status[pi]: 0, the order of a
-// non-positive pivot of S_k, or kStNoConv.
+// The stages of the problems up to kEigBatchMax, a launch each over the whole
+// batch, every stage with its own split: one CTA per problem where a stage is a
+// chain (Cholesky, tridiagonalisation, divide and conquer), one CTA per 64-column
+// block where it is not (the two triangular solves of the reduction), largest
+// problems first.  status[pi]: 0, the order of a non-positive pivot of S_k, or
+// kStNoConv; a problem that failed is skipped by the later stages.
 __host__ __device__ constexpr size_t stage_smem_bytes(int M) {
     return sizeof(double) * (2 * kStageOp + NB * (NB + 1)) + dc_smem_bytes(M) + sizeof(int) * 16 +
            sizeof(double) * (2 + kT / 32) + 16;
@@ -1451,9 +1211,71 @@ __device__ StageSmem stage_smem(unsigned char* base, int M) {
     return sh;
 }
 
-__global__ void __launch_bounds__(kT, 1) k_eig_fused(
+// Gather and Cholesky, one problem per CTA.
+__global__ void __launch_bounds__(kT, 1) k_eig_chol(const EigProb* __restrict__ probs, const int* __restrict__ order,
+                                                    const int* __restrict__ maps, const double* __restrict__ H,
+                                                    const double* __restrict__ S, double* __restrict__ Xa,
+                                                    double* __restrict__ La, int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const StageSmem sh = stage_smem(smraw, 2);
+    const int pi = order[blockIdx.x];
+    const EigProb p = probs[pi];
+    stage_gather(p, maps, H, S, Xa, La);
+    __syncthreads();
+    const int st = stage_potrf(p, La, sh);
+    if (threadIdx.x == 0) status[pi] = st;
+}
+
+// X <- L^-1 X on one 64-column block of X per CTA (tasks: problem, block).
+constexpr size_t kTrsmSmem = sizeof(double) * (2 * kStageOp + TS * (TS + 1));
+__global__ void __launch_bounds__(kT, 2) k_eig_trsm(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
+                                                    const double* __restrict__ La, double* __restrict__ Xa,
+                                                    const int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double* sA = reinterpret_cast<double*>(smraw);
+    const int2 t = tasks[blockIdx.x];
+    if (status[t.x] != kStOk) return;
+    const EigProb p = probs[t.x];
+    trsm_cols(true, La + p.aoff, p.m, Xa + p.aoff, p.m, t.y * TS, min(p.m, (t.y + 1) * TS), sA + 2 * kStageOp, sA,
+              sA + kStageOp);
+}
+
+// Y = X^T, one 64-column block of X per CTA, through 64 x 65 shared tiles.
+__global__ void __launch_bounds__(256) k_eig_transpose(const EigProb* __restrict__ probs,
+                                                       const int2* __restrict__ tasks, const double* __restrict__ Xa,
+                                                       double* __restrict__ Ya, const int* __restrict__ status) {
+    __shared__ double tile[TS][TS + 1];
+    const int2 t = tasks[blockIdx.x];
+    if (status[t.x] != kStOk) return;
+    const EigProb p = probs[t.x];
+    const int m = p.m, c0 = t.y * TS, tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+    const double* X = Xa + p.aoff;
+    double* Y = Ya + p.aoff;
+    for (int r0 = 0; r0 < m; r0 += TS) {
+        for (int c = ty; c < TS; c += 4)
+            if (r0 + tx < m && c0 + c < m) tile[c][tx] = X[r0 + tx + (int64_t)(c0 + c) * m];
+        __syncthreads();
+        for (int r = ty; r < TS; r += 4)
+            if (r0 + r < m && c0 + tx < m) Y[c0 + tx + (int64_t)(r0 + r) * m] = tile[tx][r];
+        __syncthreads();
+    }
+}
+
+// Tridiagonalisation, one problem per CTA.
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) k_eig_trd(const EigProb* __restrict__ probs,
+                                                          const int* __restrict__ order, double* __restrict__ Ca,
+                                                          double* __restrict__ Da, double* __restrict__ Ea,
+                                                          double* __restrict__ Ta, const int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int pi = order[blockIdx.x];
+    if (status[pi] != kStOk) return;
+    stage_trd<NT>(probs[pi], Ca, Da, Ea, Ta, reinterpret_cast<double*>(smraw));
+}
+
+// Divide and conquer, then the owned rows and fe (mode 0) or the density (mode 2).
+__global__ void __launch_bounds__(kT, 1) k_eig_vectors(
     const EigProb* __restrict__ probs, const int* __restrict__ order, int np, int* __restrict__ counter, int M,
-    const int* __restrict__ maps, const double* __restrict__ H, const double* __restrict__ S,
     double* __restrict__ Ca, double* __restrict__ La, double* __restrict__ Za, double* __restrict__ Qa,
     double* __restrict__ Va, double* __restrict__ Da, double* __restrict__ Ea, double* __restrict__ Ta,
     double* __restrict__ Wa, double* __restrict__ Ba, double* __restrict__ Ka, const int* __restrict__ own_cols,
@@ -1469,30 +1291,22 @@ __global__ void __launch_bounds__(kT, 1) k_eig_fused(
         __syncthreads();
         if (q >= np) break;
         const int pi = order[q];
+        if (status[pi] != kStOk) continue;
         const EigProb p = probs[pi];
-        stage_gather(p, maps, H, S, Ca, La);
-        __syncthreads();
-        int st = stage_potrf(p, La, sh);
-        __syncthreads();
-        if (st == kStOk) {
-            stage_reduce(p, La, Ca, sh);
+        if (!stage_dc(p, Da, Ea, Wa, Za, Qa, Va, sh)) {
+            if (tid == 0) status[pi] = kStNoConv;
             __syncthreads();
-            stage_sytrd(p, Ca, Da, Ea, Ta, sh);
-            __syncthreads();
-            if (!stage_dc(p, Da, Ea, Wa, Za, Qa, Va, sh)) st = kStNoConv;
-            __syncthreads();
-            if (st == kStOk) {
-                if (p.m >= kWyMmaMin)
-                    build_T(Ca + p.aoff, p.m, Ta + p.voff, Ka + p.koff, 0, 1, Va + p.aoff, sh.sD, sh.sA, sh.sB);
-                if (p.mode == 2) {
-                    for (int j = threadIdx.x; j < p.m; j += kT) e_out[p.eoff + j] = Wa[p.voff + j];
-                    stage_density(p, Ca, La, Ta, Za, Qa, Va, Ka, Ba, sh);
-                } else {
-                    stage_rows(p, Ca, La, Ta, Wa, Za, own_cols, ipos, Ba, Qa, Va, Ka, e_out, fe_out, sh);
-                }
-            }
+            continue;
         }
-        if (tid == 0) status[pi] = st;
+        __syncthreads();
+        if (p.m >= kWyMmaMin)
+            build_T(Ca + p.aoff, p.m, Ta + p.voff, Ka + p.koff, 0, 1, Va + p.aoff, sh.sD, sh.sA, sh.sB);
+        if (p.mode == 2) {
+            for (int j = threadIdx.x; j < p.m; j += kT) e_out[p.eoff + j] = Wa[p.voff + j];
+            stage_density(p, Ca, La, Ta, Za, Qa, Va, Ka, Ba, sh);
+        } else {
+            stage_rows(p, Ca, La, Ta, Wa, Za, own_cols, ipos, Ba, Qa, Va, Ka, e_out, fe_out, sh);
+        }
         __syncthreads();
     }
 }
@@ -2728,7 +2542,7 @@ struct EigBatch {
     int G = 1;                    // CTAs per cluster of the large-submatrix solver
     int nsmall = 0, nlarge = 0;
     std::vector<EigProb> hp;
-    WorkBuf probs, order, order_l, counter, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Xa, Ka, status, tstage;
+    WorkBuf probs, order, order_l, counter, tasks, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Xa, Ka, status, tstage;
     int prl = 0;
     const char* what = "submatrix";   // the problems' name in error messages
     cudaStream_t side = nullptr;
@@ -2747,8 +2561,13 @@ namespace {
 
 void eig_setup_attrs() {
     static const bool done = [] {
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        PTB_CUDA(cudaFuncSetAttribute(k_eig_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)stage_smem_bytes(kEigBatchMax)));
+        PTB_CUDA(cudaFuncSetAttribute(k_eig_chol, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)stage_smem_bytes(2)));
+        PTB_CUDA(cudaFuncSetAttribute(k_eig_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
+        PTB_CUDA(cudaFuncSetAttribute(k_eig_trd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kTrdCap512));
+        PTB_CUDA(cudaFuncSetAttribute(k_eig_trd<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kTrdCap256));
         PTB_CUDA(cudaFuncSetAttribute(k_eig_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)lg_smem_bytes(kLargeMax)));
         PTB_CUDA(cudaFuncSetAttribute(k_eig_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -2959,15 +2778,39 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
     }
     if (eb->nsmall > 0) {
         int Msmall = 0;
-        for (int q : ord_s) Msmall = std::max(Msmall, eb->hp[q].m);
+        std::vector<int2> tasks;
+        int n512 = 0;   // problems of the one-CTA-per-SM tridiagonalisation
+        for (int q : ord_s) {
+            const int m = eb->hp[q].m;
+            Msmall = std::max(Msmall, m);
+            for (int cb = 0; cb * TS < m; ++cb) tasks.push_back(make_int2(q, cb));
+            if (m > kTrdMax256) ++n512;
+        }
+        const int nsm = c->num_sms > 0 ? c->num_sms : 148;
+        // two CTAs per SM only pay where the small orders fill the SMs
+        if (eb->nsmall - n512 <= nsm) n512 = eb->nsmall;
+        eb->tasks.reserve(c, sizeof(int2) * tasks.size());
+        PTB_CUDA(cudaMemcpyAsync(eb->tasks.ptr, tasks.data(), sizeof(int2) * tasks.size(), cudaMemcpyHostToDevice, s));
+        const int2* dt = eb->tasks.as<int2>();
+        const int* ord = eb->order.as<int>();
+        const unsigned nt = (unsigned)tasks.size();
+        double *Ca = eb->Ca.as<double>(), *La = eb->La.as<double>(), *Qa = eb->Qa.as<double>();
+        double *Da = eb->Da.as<double>(), *Ea = eb->Ea.as<double>(), *Ta = eb->Ta.as<double>();
+        k_eig_chol<<<eb->nsmall, kT, stage_smem_bytes(2), s>>>(dp, ord, d_maps, H, S, Qa, La, dst);
+        k_eig_trsm<<<nt, kT, kTrsmSmem, s>>>(dp, dt, La, Qa, dst);
+        k_eig_transpose<<<nt, 256, 0, s>>>(dp, dt, Qa, Ca, dst);
+        k_eig_trsm<<<nt, kT, kTrsmSmem, s>>>(dp, dt, La, Ca, dst);
+        if (n512 > 0)
+            k_eig_trd<512><<<n512, 512, sizeof(double) * kTrdCap512, s>>>(dp, ord, Ca, Da, Ea, Ta, dst);
+        if (n512 < eb->nsmall)
+            k_eig_trd<256><<<eb->nsmall - n512, 256, sizeof(double) * kTrdCap256, s>>>(dp, ord + n512, Ca, Da, Ea, Ta,
+                                                                                       dst);
         const int Ms = (Msmall + 1) & ~1;   // staging sized for the largest small problem
-        const int grid = std::min(eb->nsmall, c->num_sms > 0 ? c->num_sms : 148);
-        k_eig_fused<<<grid, kT, stage_smem_bytes(Ms), s>>>(
-            dp, eb->order.as<int>(), eb->nsmall, eb->counter.as<int>(), Ms, d_maps, H, S, eb->Ca.as<double>(),
-            eb->La.as<double>(), eb->Za.as<double>(), eb->Qa.as<double>(), eb->Va.as<double>(), eb->Da.as<double>(),
-            eb->Ea.as<double>(), eb->Ta.as<double>(), eb->Wa.as<double>(), eb->Ba.as<double>(), eb->Ka.as<double>(),
-            d_own_cols, d_ipos, d_e, d_fe, dst);
-        count_launch();
+        const int grid = std::min(eb->nsmall, nsm);
+        k_eig_vectors<<<grid, kT, stage_smem_bytes(Ms), s>>>(
+            dp, ord, eb->nsmall, eb->counter.as<int>(), Ms, Ca, La, eb->Za.as<double>(), Qa, eb->Va.as<double>(), Da,
+            Ea, Ta, eb->Wa.as<double>(), eb->Ba.as<double>(), eb->Ka.as<double>(), d_own_cols, d_ipos, d_e, d_fe, dst);
+        count_launch(6 + (n512 > 0 && n512 < eb->nsmall));
         PTB_CUDA(cudaGetLastError());
     }
     if (eb->nlarge > 0 && join) PTB_CUDA(cudaStreamWaitEvent(s, eb->ev1, 0));
