@@ -133,6 +133,8 @@ struct ptbgpu_ctx {
     std::shared_ptr<void> sm_plan;
     // side streams and handles of the submatrix method's large eigensolves
     std::shared_ptr<void> sm_side;
+    // streams and events of the eigensolver's side launches
+    std::shared_ptr<void> eig_streams;
     // device tile lists of the int8-sliced FP64 products of the module code
     std::shared_ptr<void> oz_tile_cache;
     // worker contexts of the multi-instance batch (same device, own streams and buffers)

@@ -263,6 +263,7 @@ int ptbgpu_finalize(ptbgpu_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->sm_plan.reset();
     c->sm_side.reset();
+    c->eig_streams.reset();
     for (ptbgpu_ctx* w : c->workers) ptbgpu_finalize(w);
     c->workers.clear();
     c->work->trim();

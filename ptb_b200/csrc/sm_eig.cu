@@ -1,5 +1,5 @@
-// Batched FP64 generalized eigensolver of the submatrix method, one CTA per
-// submatrix.
+// Batched FP64 generalized eigensolver: the submatrix method's pencils, the
+// many-molecule densities and single dense problems.
 //
 // The reference solves H_k U = S_k U diag(e) with LAPACK dsygvd per submatrix
 // (la_sygvd, source/sm.f90:296-299), forms S_k U for the electron-count
@@ -8,15 +8,22 @@
 // (source/sm.f90:343-362).  Only these quantities leave the solver, and all of
 // them are reached without forming U:
 //
-//   S_k = L L^T                      Cholesky, blocked (k_eig_potrf)
+//   S_k = L L^T                      Cholesky, blocked
 //   C   = L^-1 H_k L^-T              two blocked triangular solves
 //   C   = Q T Q^T                    Householder tridiagonalisation, lower,
-//                                    Q = H_0 H_1 ... H_{m-3} (k_eig_sytrd)
-//   T   = Z diag(e) Z^T              divide and conquer (k_eig_dc)
-//   U   = L^-T Q Z                   never formed:
+//                                    Q = H_0 H_1 ... H_{m-3}
+//   T   = Z diag(e) Z^T              divide and conquer (eig_dc.cuh)
+//   U   = L^-T Q Z                   never formed (eig_vec.cuh):
 //     rows c of U    = (L^-T)[c,:] Q Z,  rows c of S U = L[c,:] Q Z  for the
-//     owned columns c (k_eig_rows), so fe_j = sum_c (SU)[c,j] U[c,j];
-//     P_k[:,c] = U (occ o U[c,:]^T) = L^-T (Q (Z w)) (k_eig_final).
+//     owned columns c, so fe_j = sum_c (SU)[c,j] U[c,j];
+//     P_k[:,c] = U (occ o U[c,:]^T) = L^-T (Q (Z w)).
+//
+// Every stage is a launch (or a few) over all problems of the batch, with its own
+// split: one CTA or one thread-block cluster per problem where the stage is a chain
+// (Cholesky, tridiagonalisation), one CTA per 64-column block, panel, tile or chunk of
+// roots where it is not, largest problems first.  A batch of uneven problems then
+// costs its total work over the SMs in all stages but those two, where one CTA or
+// cluster per problem for everything cost the largest problem's whole chain.
 //
 // Each step's quantities are summed in a fixed order, so results do not depend
 // on scheduling.
@@ -48,7 +55,7 @@ constexpr int kStNoConv = -1;     // a leaf's QL sweeps exhausted
 struct EigProb {
     int k, m, nown;
     int kind;             // 0: H U = S U e; 1: standard problem (S not read, L = I)
-    int mode;             // 0: eigenvalues, fe, owned rows; 2: density 2 U_occ U_occ^T (m x m at boff)
+    int mode;             // 0: eigenvalues, fe, owned rows; 1: all vectors; 2: density U_occ U_occ^T (m x m at boff)
     int nocc;             // mode 2: occupied eigenvectors (the lowest)
     int64_t moff, eoff, o0;
     int64_t gbase, gld;   // the problem's H / S: element (i, j) at gbase + map(i) + map(j) gld
@@ -58,6 +65,7 @@ struct EigProb {
     int64_t boff;     // owned-row arena (4 nown x m)
     int64_t xoff;     // cluster solver scratch (orders above kEigBatchMax)
     int64_t koff;     // T of the compact WY panels (t_panels(m) x NB^2)
+    int topm;         // index of the divide and conquer's last merge (-1: one leaf)
 };
 
 // ---------------------------------------------------------------------------
@@ -241,17 +249,22 @@ __device__ double warp_sum(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// Shared memory of the stages, carved from one dynamic buffer: the tile
-// staging (sA, sB), the diagonal block of the blocked factorisations (sD), a
-// union region (the tridiagonalisation's vectors or the divide and conquer's
-// per-element arrays, M = the largest order of the batch) and a few scalars.
+// Shared memory of the one-CTA Cholesky: the tile staging (sA, sB) and the diagonal
+// block (sD).
 struct StageSmem {
     double *sA, *sB, *sD;
-    unsigned char* uni;
-    int* ints;      // 16
-    double* dsc;    // 2 + kT / 32
-    int M;
+    int* ints;
 };
+constexpr size_t kCholSmem = sizeof(double) * (2 * kStageOp + NB * (NB + 1)) + sizeof(int) * 16;
+__device__ StageSmem stage_smem(unsigned char* base) {
+    StageSmem sh;
+    double* d = reinterpret_cast<double*>(base);
+    sh.sA = d;
+    sh.sB = d + kStageOp;
+    sh.sD = d + 2 * kStageOp;
+    sh.ints = reinterpret_cast<int*>(d + 2 * kStageOp + NB * (NB + 1));
+    return sh;
+}
 
 // ---------------------------------------------------------------------------
 // Gather H_k, S_k (source/sm.f90:240-246) into the C and L arenas.
@@ -363,550 +376,9 @@ __device__ void tile_gemm(double* __restrict__ C, int64_t ldc, int crow, const i
     tile_mma<AT, BT, MMA_SET, false>(C, ldc, crow, ccol, r0, c0, mr, nc, A, lda, kx, B, ldb, kxb, K, sA, sB);
 }
 
-// ---------------------------------------------------------------------------
-// Divide and conquer for the tridiagonal eigenproblem T = Z diag(w) Z^T
-// (Cuppen's split T = diag(T1, T2) + |beta| u u^T, u = e_last + sign(beta)
-// e_first; Gu and Eisenstat's recomputed z for orthogonal eigenvectors), one
-// CTA per problem.  Leaves of at most 32 rows are solved by a warp with the
-// implicit QL iteration (every lane runs the same scalar iteration and applies
-// each rotation to its own row of the leaf's Z); the merges run bottom-up over
-// a balanced tree, one at a time with the whole CTA:
-//   z = [last row of Z1, sign(beta) first row of Z2] / sqrt 2, rho = 2|beta|;
-//   sort the block eigenvalues (merge of two sorted lists);
-//   deflate: rho |z_j| <= tol -> eigenpair (d_j, q_j); two close d's -> a Givens
-//   rotation zeroes one z entry (LAPACK's dlaed2 rules, tol = 8 eps max(|d|, rho));
-//   secular roots lambda_i = d_org + tau in (d_i, d_i+1), each step modelling the
-//   left and right sums by one pole each;
-//   zhat_j^2 = (lambda_j - d_j) prod_{i != j} (lambda_i - d_j)/(d_i - d_j) / rho;
-//   v_i = (zhat_j / (d_j - lambda_i))_j normalised; Z_new = Q v in two GEMMs
-//   (rows of block 1 against the columns that touch it, rows of block 2 likewise).
-// Output: w ascending, Z in the Z arena (column-major, ld m).
-constexpr int kDcLeaf = 32;
-
-struct DcSmem {
-    // per-element arrays of the merge (kEigBatchMax each)
-    double *D, *Ds, *zs, *dk, *zk, *tau, *zh, *val;
-    int *perm, *org, *sec, *dl, *rank, *cls, *ktop, *kbot;
-    int2* rpair;
-    double2* rcs;
-};
-
-// Per-element arrays of capacity M (a multiple of 2, so every block stays
-// 16-byte aligned).
-__device__ DcSmem dc_smem(unsigned char* base, int M) {
-    DcSmem s;
-    double* d = reinterpret_cast<double*>(base);
-    s.D = d;
-    s.Ds = d + M;
-    s.zs = d + 2 * M;
-    s.dk = d + 3 * M;
-    s.zk = d + 4 * M;
-    s.tau = d + 5 * M;
-    s.zh = d + 6 * M;
-    s.val = d + 7 * M;
-    s.rcs = reinterpret_cast<double2*>(d + 8 * M);
-    int* ip = reinterpret_cast<int*>(s.rcs + M);
-    s.perm = ip;
-    s.org = ip + M;
-    s.sec = ip + 2 * M;
-    s.dl = ip + 3 * M;
-    s.rank = ip + 4 * M;
-    s.cls = ip + 5 * M;
-    s.ktop = ip + 6 * M;
-    s.kbot = ip + 7 * M;
-    s.rpair = reinterpret_cast<int2*>(ip + 8 * M);
-    return s;
-}
-__host__ __device__ constexpr size_t dc_smem_bytes(int M) {
-    return (sizeof(double) * 8 + sizeof(double2) + sizeof(int) * 8 + sizeof(int2)) * (size_t)M;
-}
-
-// Leaf: implicit QL on d[0..s), e[0..s-1) with Z = I accumulated.  Every
-// lane runs the same scalar iteration on its own copies of d and e and rotates
-// its own row z of Z (lane r holds row r), so no lane reads another's data.
-__device__ bool dc_leaf(int s, double* d, double* e, double* z, int lane) {
-    const double eps = 2.220446049250313e-16;
-    for (int c = 0; c < kDcLeaf; ++c) z[c] = (c == lane) ? 1.0 : 0.0;
-    for (int l = 0; l < s; ++l) {
-        int iter = 0;
-        for (;;) {
-            int mm = l;
-            for (; mm < s - 1; ++mm)
-                if (fabs(e[mm]) <= eps * (fabs(d[mm]) + fabs(d[mm + 1]))) break;
-            if (mm == l) break;
-            if (++iter > kQlMaxIter) return false;
-            double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-            double r = hypot(g, 1.0);
-            g = d[mm] - d[l] + e[l] / (g + copysign(r, g));
-            double sn = 1.0, c = 1.0, pp = 0.0;
-            bool underflow = false;
-            for (int i = mm - 1; i >= l; --i) {
-                const double f = sn * e[i], b = c * e[i];
-                r = hypot(f, g);
-                e[i + 1] = r;
-                if (r == 0.0) {
-                    d[i + 1] -= pp;
-                    e[mm] = 0.0;
-                    underflow = true;
-                    break;
-                }
-                sn = f / r;
-                c = g / r;
-                g = d[i + 1] - pp;
-                r = (d[i] - g) * sn + 2.0 * c * b;
-                pp = sn * r;
-                d[i + 1] = g + pp;
-                g = c * r - b;
-                const double zi = z[i], zi1 = z[i + 1];
-                z[i + 1] = sn * zi + c * zi1;
-                z[i] = c * zi - sn * zi1;
-            }
-            if (underflow) continue;
-            d[l] -= pp;
-            e[l] = g;
-            e[mm] = 0.0;
-        }
-    }
-    return true;
-}
-
-// Root i of 1 + rho sum_t z_t^2 / (dk_t - lambda) = 0 (dk ascending, k roots):
-// returns tau with lambda = dk[*org] + tau.
-__device__ double dc_secular(int k, const double* dk, const double* zk, double rho, int i, int* org_out) {
-    const double eps = 2.220446049250313e-16;
-    int org;
-    double lo, hi;
-    if (i < k - 1) {
-        const double mid = 0.5 * (dk[i + 1] - dk[i]);
-        double f = 1.0;
-        for (int t = 0; t < k; ++t) f += rho * zk[t] * zk[t] / ((dk[t] - dk[i]) - mid);
-        if (f >= 0.0) {
-            org = i;
-            lo = 0.0;
-            hi = mid;
-        } else {
-            org = i + 1;
-            lo = -mid;
-            hi = 0.0;
-        }
-    } else {
-        double z2 = 0.0;
-        for (int t = 0; t < k; ++t) z2 += zk[t] * zk[t];
-        org = i;
-        lo = 0.0;
-        hi = rho * z2;
-    }
-    const double dorg = dk[org];
-    const double a = dk[i] - dorg;
-    const double b = (i < k - 1) ? dk[i + 1] - dorg : 0.0;
-    double tau = 0.5 * (lo + hi);
-    for (int it = 0; it < 100; ++it) {
-        double psi = 0.0, phi = 0.0, dpsi = 0.0, dphi = 0.0;
-        for (int t = 0; t < k; ++t) {
-            const double den = (dk[t] - dorg) - tau;
-            const double q = rho * zk[t] * zk[t] / den;
-            if (t <= i) {
-                psi += q;
-                dpsi += q / den;
-            } else {
-                phi += q;
-                dphi += q / den;
-            }
-        }
-        const double f = 1.0 + psi + phi;
-        if (f > 0.0) hi = tau;
-        else if (f < 0.0) lo = tau;
-        else break;
-        if (fabs(f) <= 16.0 * eps * (1.0 + fabs(psi) + fabs(phi))) break;
-        const double B = dpsi * (a - tau) * (a - tau);
-        const double A = psi - B / (a - tau);
-        double nt;
-        if (i < k - 1) {
-            const double E = dphi * (b - tau) * (b - tau);
-            const double Cc = phi - E / (b - tau);
-            const double c0 = 1.0 + A + Cc;
-            const double qb = -(c0 * (a + b) + B + E);
-            const double qc = c0 * a * b + B * b + E * a;
-            if (c0 == 0.0) {
-                nt = -qc / qb;
-            } else {
-                const double disc = fmax(qb * qb - 4.0 * c0 * qc, 0.0);
-                const double r1 = (-qb - copysign(sqrt(disc), qb)) / (2.0 * c0);
-                const double r2 = (r1 != 0.0) ? qc / (c0 * r1) : r1;
-                nt = (lo < r1 && r1 < hi) ? r1 : r2;
-            }
-        } else {
-            const double c0 = 1.0 + A + phi;
-            nt = (c0 != 0.0) ? a + B / c0 : 0.5 * (lo + hi);
-        }
-        if (!(lo < nt && nt < hi)) nt = 0.5 * (lo + hi);
-        if (fabs(nt - tau) <= 2.0 * eps * fabs(nt)) {
-            tau = nt;
-            break;
-        }
-        tau = nt;
-    }
-    *org_out = org;
-    return tau;
-}
-
-__device__ bool stage_dc(const EigProb& p, const double* __restrict__ Da, const double* __restrict__ Ea,
-                         double* __restrict__ Wa, double* __restrict__ Za, double* __restrict__ Qa,
-                         double* __restrict__ Va, const StageSmem& sh) {
-    double* sA = sh.sA;
-    double* sB = sh.sB;
-    int& s_k = sh.ints[1];
-    int& s_nd = sh.ints[2];
-    int& s_nrot = sh.ints[3];
-    int& s_ntop = sh.ints[4];
-    int& s_nbot = sh.ints[5];
-    int& s_fail = sh.ints[6];
-    const int m = p.m;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double* Z = Za + p.aoff;
-    double* Qp = Qa + p.aoff;
-    double* V = Va + p.aoff;
-    const double* eo = Ea + p.voff;
-    DcSmem S = dc_smem(sh.uni, sh.M);
-    int L = 0;
-    while (((m + (1 << L) - 1) >> L) > kDcLeaf) ++L;
-    const int nleaf = 1 << L;
-    for (int i = tid; i < m; i += kT) S.D[i] = Da[p.voff + i];
-    if (tid == 0) s_fail = 0;
-    __syncthreads();
-    if (tid == 0)
-        for (int q = 1; q < nleaf; ++q) {
-            const int pos = (int)(((int64_t)q * m) >> L);
-            const double ab = fabs(eo[pos - 1]);
-            S.D[pos - 1] -= ab;
-            S.D[pos] -= ab;
-        }
-    __syncthreads();
-    // leaves: a warp each
-    for (int q = warp; q < nleaf; q += kT / 32) {
-        const int lo = (int)(((int64_t)q * m) >> L), hi = (int)(((int64_t)(q + 1) * m) >> L), s = hi - lo;
-        double dl[kDcLeaf], el[kDcLeaf], zl[kDcLeaf];
-        for (int i = 0; i < kDcLeaf; ++i) {
-            dl[i] = (i < s) ? S.D[lo + i] : 0.0;
-            el[i] = (i < s - 1) ? eo[lo + i] : 0.0;
-        }
-        const bool ok = dc_leaf(s, dl, el, zl, lane);
-        if (!ok && lane == 0) s_fail = 1;
-        // eigenvalues ascending (ties by index) and the columns in that order
-        int rk = 0;
-        if (lane < s) {
-            const double x = dl[lane];
-            for (int c = 0; c < s; ++c) rk += (dl[c] < x || (dl[c] == x && c < lane)) ? 1 : 0;
-        }
-        for (int c = 0; c < s; ++c) {
-            const int rc = __shfl_sync(0xffffffffu, rk, c);
-            if (lane < s) Z[(int64_t)(lo + lane) + (int64_t)(lo + rc) * m] = zl[c];
-        }
-        __syncwarp();
-        if (lane < s) S.D[lo + rk] = dl[lane];
-        __syncwarp();
-    }
-    __syncthreads();
-    if (s_fail) return false;
-    const double eps = 2.220446049250313e-16;
-    for (int lev = L - 1; lev >= 0; --lev) {
-        for (int q = 0; q < (1 << lev); ++q) {
-            const int lo = (int)(((int64_t)q * m) >> lev), hi = (int)(((int64_t)(q + 1) * m) >> lev);
-            const int mid = (int)(((int64_t)(2 * q + 1) * m) >> (lev + 1));
-            const int n1 = mid - lo, n2 = hi - mid, n = n1 + n2;
-            const double beta = eo[mid - 1];
-            const double rho = 2.0 * fabs(beta);
-            const double sgn = beta >= 0.0 ? 1.0 : -1.0;
-            const double rs2 = 0.70710678118654752440;
-            // (a) merged order of the two sorted blocks
-            for (int j = tid; j < n; j += kT) {
-                int r;
-                if (j < n1) {
-                    const double x = S.D[lo + j];
-                    int a = 0, b = n2;
-                    while (a < b) {
-                        const int c = (a + b) >> 1;
-                        if (S.D[mid + c] < x) a = c + 1;
-                        else b = c;
-                    }
-                    r = j + a;
-                } else {
-                    const double x = S.D[mid + j - n1];
-                    int a = 0, b = n1;
-                    while (a < b) {
-                        const int c = (a + b) >> 1;
-                        if (S.D[lo + c] <= x) a = c + 1;
-                        else b = c;
-                    }
-                    r = (j - n1) + a;
-                }
-                S.perm[r] = j;
-            }
-            __syncthreads();
-            // (b) sorted d, z and column classes; (c) Q with the block columns in that order
-            for (int r = tid; r < n; r += kT) {
-                const int j = S.perm[r];
-                if (j < n1) {
-                    S.Ds[r] = S.D[lo + j];
-                    S.zs[r] = Z[(int64_t)(mid - 1) + (int64_t)(lo + j) * m] * rs2;
-                    S.cls[r] = 1;
-                } else {
-                    S.Ds[r] = S.D[mid + j - n1];
-                    S.zs[r] = sgn * Z[(int64_t)mid + (int64_t)(mid + j - n1) * m] * rs2;
-                    S.cls[r] = 2;
-                }
-            }
-            for (int64_t t = tid; t < (int64_t)n * n; t += kT) {
-                const int i = (int)(t % n), r = (int)(t / n);
-                const int j = S.perm[r];
-                double v = 0.0;
-                if (j < n1) {
-                    if (i < n1) v = Z[(int64_t)(lo + i) + (int64_t)(lo + j) * m];
-                } else if (i >= n1) {
-                    v = Z[(int64_t)(lo + i) + (int64_t)(mid + j - n1) * m];
-                }
-                Qp[t] = v;
-            }
-            __syncthreads();
-            // (d) deflation (one thread, in sorted order)
-            if (tid == 0) {
-                double dmax = 0.0;
-                for (int r = 0; r < n; ++r) dmax = fmax(dmax, fabs(S.Ds[r]));
-                const double tol = 8.0 * eps * fmax(dmax, rho);
-                int k = 0, nd = 0, nrot = 0, pj = -1;
-                for (int r = 0; r < n; ++r) {
-                    if (rho * fabs(S.zs[r]) <= tol) {
-                        S.dl[nd++] = r;
-                        continue;
-                    }
-                    if (pj < 0) {
-                        pj = r;
-                        continue;
-                    }
-                    double sn = S.zs[pj], c = S.zs[r];
-                    const double t = hypot(c, sn);
-                    const double dd = S.Ds[r] - S.Ds[pj];
-                    c /= t;
-                    sn = -sn / t;
-                    if (fabs(dd * c * sn) <= tol) {
-                        S.zs[r] = t;
-                        S.zs[pj] = 0.0;
-                        S.rpair[nrot] = make_int2(pj, r);
-                        S.rcs[nrot] = make_double2(c, sn);
-                        ++nrot;
-                        const double t2 = S.Ds[pj] * c * c + S.Ds[r] * sn * sn;
-                        S.Ds[r] = S.Ds[pj] * sn * sn + S.Ds[r] * c * c;
-                        S.Ds[pj] = t2;
-                        S.cls[r] |= S.cls[pj];
-                        S.dl[nd++] = pj;
-                        pj = r;
-                    } else {
-                        S.sec[k++] = pj;
-                        pj = r;
-                    }
-                }
-                if (pj >= 0) S.sec[k++] = pj;
-                // secular columns that touch block 1 / block 2 (the K lists of the two GEMMs)
-                int nt = 0, nb = 0;
-                for (int t = 0; t < k; ++t) {
-                    const int c = S.cls[S.sec[t]];
-                    if (c & 1) S.ktop[nt++] = t;
-                    if (c & 2) S.kbot[nb++] = t;
-                }
-                s_k = k;
-                s_nd = nd;
-                s_nrot = nrot;
-                s_ntop = nt;
-                s_nbot = nb;
-            }
-            __syncthreads();
-            const int k = s_k, nd = s_nd, nrot = s_nrot;
-            // (e) deflation rotations on the columns of Q (thread per row)
-            if (nrot > 0)
-                for (int i = tid; i < n; i += kT)
-                    for (int q2 = 0; q2 < nrot; ++q2) {
-                        const int2 pr = S.rpair[q2];
-                        const double2 cs = S.rcs[q2];
-                        const double a = Qp[i + (int64_t)pr.x * n], b = Qp[i + (int64_t)pr.y * n];
-                        Qp[i + (int64_t)pr.x * n] = cs.x * a + cs.y * b;
-                        Qp[i + (int64_t)pr.y * n] = -cs.y * a + cs.x * b;
-                    }
-            for (int t = tid; t < k; t += kT) {
-                S.dk[t] = S.Ds[S.sec[t]];
-                S.zk[t] = S.zs[S.sec[t]];
-            }
-            __syncthreads();
-            // (f) secular roots
-            for (int i = tid; i < k; i += kT) S.tau[i] = dc_secular(k, S.dk, S.zk, rho, i, &S.org[i]);
-            __syncthreads();
-            // (g) recomputed z
-            for (int j = tid; j < k; j += kT) {
-                const double dj = S.dk[j];
-                double w = (S.dk[S.org[j]] - dj) + S.tau[j];
-                for (int i = 0; i < k; ++i) {
-                    if (i == j) continue;
-                    w *= ((S.dk[S.org[i]] - dj) + S.tau[i]) / (S.dk[i] - dj);
-                }
-                S.zh[j] = copysign(sqrt(fmax(w / rho, 0.0)), S.zk[j]);
-            }
-            __syncthreads();
-            // (h) eigenvectors of the rank-one problem (columns of V, k x k) and the new eigenvalues
-            for (int i = tid; i < k; i += kT) {
-                const double dorg = S.dk[S.org[i]], ti = S.tau[i];
-                double nrm = 0.0;
-                for (int j = 0; j < k; ++j) {
-                    const double v = S.zh[j] / ((S.dk[j] - dorg) - ti);
-                    nrm = fma(v, v, nrm);
-                }
-                const double sc = 1.0 / sqrt(nrm);
-                for (int j = 0; j < k; ++j) V[j + (int64_t)i * k] = sc * (S.zh[j] / ((S.dk[j] - dorg) - ti));
-                S.val[i] = dorg + ti;
-            }
-            for (int q2 = tid; q2 < nd; q2 += kT) S.val[k + q2] = S.Ds[S.dl[q2]];
-            __syncthreads();
-            // (i) positions of the n new eigenvalues in ascending order
-            for (int a = tid; a < n; a += kT) {
-                const double x = S.val[a];
-                int r = 0;
-                for (int b2 = 0; b2 < n; ++b2) r += (S.val[b2] < x || (S.val[b2] == x && b2 < a)) ? 1 : 0;
-                S.rank[a] = lo + r;
-            }
-            __syncthreads();
-            // (j) Z block = Q [V | deflated columns]: block-1 rows against the columns
-            // touching block 1, block-2 rows against those touching block 2
-            // gathered K lists: columns of Q (sec[ktop[t]]) against rows ktop[t] of V
-            for (int t = tid; t < s_ntop; t += kT) S.perm[t] = S.sec[S.ktop[t]];
-            __syncthreads();
-            // rows of block 1: Z[lo + r, rank[c]] = sum_t Q[r, sec[ktop[t]]] V[ktop[t], c]
-            for (int c0 = 0; c0 < k; c0 += TS)
-                for (int r0 = 0; r0 < n1; r0 += TS)
-                    tile_gemm<false>(Z, m, lo, S.rank, r0, c0, min(TS, n1 - r0), min(TS, k - c0), Qp, n, S.perm, V, k,
-                                     S.ktop, s_ntop, sA, sB);
-            __syncthreads();
-            for (int t = tid; t < s_nbot; t += kT) S.perm[t] = S.sec[S.kbot[t]];
-            __syncthreads();
-            // rows of block 2 against the columns that touch block 2
-            for (int c0 = 0; c0 < k; c0 += TS)
-                for (int r0 = n1; r0 < n; r0 += TS)
-                    tile_gemm<false>(Z, m, lo, S.rank, r0, c0, min(TS, n - r0), min(TS, k - c0), Qp, n, S.perm, V, k,
-                                     S.kbot, s_nbot, sA, sB);
-            // deflated columns: copies of Q's columns
-            for (int64_t t = tid; t < (int64_t)nd * n; t += kT) {
-                const int i = (int)(t % n), q2 = (int)(t / n);
-                Z[(int64_t)(lo + i) + (int64_t)S.rank[k + q2] * m] = Qp[i + (int64_t)S.dl[q2] * n];
-            }
-            for (int a = tid; a < n; a += kT) S.D[S.rank[a]] = S.val[a];
-            __syncthreads();
-        }
-    }
-    for (int i = tid; i < m; i += kT) Wa[p.voff + i] = S.D[i];
-    return true;
-}
-
-// ---------------------------------------------------------------------------
-// Q = H_0 H_1 ... H_{m-3} applied to nv vectors x_t of length m (x_t at
-// X + t m): trans -> x <- Q^T x (panels of 32 reflectors in order), else
-// x <- Q x (panels in reverse).  A panel's reflectors act together as
-// I - V T V^T (compact WY: T upper triangular, T_qq = tau_q,
-// T[0:q, q] = -tau_q T[0:q, 0:q] V[:, 0:q]^T v_q), so each panel costs three
-// small products and a handful of barriers instead of two barriers per
-// reflector.  v_j: 1 at j+1, C[r + j m] for r >= j+2, zero above.
-struct WySmem {
-    double* G;   // NB x (NB+1): Gram V^T V, then T
-    double* Xs;  // NB x kWyChunk: V^T x, then T(^T) V^T x
-};
-constexpr int kWyChunk = 64;
 static_assert(TS * NB % kT == 0, "tile staging divides over the CTA");
-static_assert(NB * (NB + 1) <= kStageOp && NB * kWyChunk <= kStageOp, "WY scratch fits the tile staging");
-
-__device__ __forceinline__ double wy_v(const double* C, int m, int j, int r) {
-    return (r == j + 1) ? 1.0 : (r > j + 1 ? C[r + (int64_t)j * m] : 0.0);
-}
-
-__device__ void wy_apply(const double* __restrict__ C, int m, const double* __restrict__ tau, double* X, int nv,
-                         bool trans, WySmem sm) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nref = m - 2;   // reflectors 0..m-3
-    if (nref <= 0) return;
-    const int npan = (nref + NB - 1) / NB;
-    for (int pp = 0; pp < npan; ++pp) {
-        const int pan = trans ? pp : npan - 1 - pp;
-        const int j0 = pan * NB, nb = min(NB, nref - j0);
-        // Gram of the panel's vectors (rows j0+1 .. m-1): a warp per pair, lanes
-        // over the rows (coalesced), fixed-order sums
-        for (int q = warp; q < NB * NB; q += kT / 32) {
-            const int a = q % NB, b = q / NB;
-            double g = 0.0;
-            if (a < nb && b < nb && a <= b) {
-                for (int r = j0 + 1 + b + lane; r < m; r += 32)
-                    g = fma(wy_v(C, m, j0 + a, r), wy_v(C, m, j0 + b, r), g);
-                g = warp_sum(g);
-            }
-            if (lane == 0) sm.G[a + b * (NB + 1)] = g;
-        }
-        __syncthreads();
-        // T in place of the Gram's upper triangle (one warp, column by column)
-        if (warp == 0) {
-            for (int b = 0; b < nb; ++b) {
-                const double tb = tau[j0 + b];
-                // T[a][b] = -tb * sum_{a <= c < b} T[a][c] G[c][b] for a < b (lane a)
-                double acc = 0.0;
-                if (lane < b)
-                    for (int c2 = lane; c2 < b; ++c2) acc = fma(sm.G[lane + c2 * (NB + 1)], sm.G[c2 + b * (NB + 1)], acc);
-                __syncwarp();
-                if (lane < b) sm.G[lane + b * (NB + 1)] = -tb * acc;
-                if (lane == b) sm.G[b + b * (NB + 1)] = tb;
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        for (int t0 = 0; t0 < nv; t0 += kWyChunk) {
-            const int nc = min(kWyChunk, nv - t0);
-            // Xs = V^T x: a warp per (reflector, vector), lanes over the rows
-            for (int q = warp; q < NB * nc; q += kT / 32) {
-                const int a = q % NB, t = q / NB;
-                double g = 0.0;
-                if (a < nb) {
-                    const double* x = X + (int64_t)(t0 + t) * m;
-                    for (int r = j0 + 1 + a + lane; r < m; r += 32) g = fma(wy_v(C, m, j0 + a, r), x[r], g);
-                    g = warp_sum(g);
-                }
-                if (lane == 0) sm.Xs[a + t * NB] = g;
-            }
-            __syncthreads();
-            // Xs <- T Xs or T^T Xs (thread per column t, in registers)
-            for (int t = tid; t < nc; t += kT) {
-                double xv[NB], yv[NB];
-                for (int a = 0; a < NB; ++a) xv[a] = sm.Xs[a + t * NB];
-                for (int a = 0; a < NB; ++a) {
-                    double y = 0.0;
-                    if (a < nb) {
-                        if (trans) {   // (T^T x)_a = sum_{c <= a} T[c][a] x_c
-                            for (int c2 = 0; c2 <= a; ++c2) y = fma(sm.G[c2 + a * (NB + 1)], xv[c2], y);
-                        } else {       // (T x)_a = sum_{c >= a} T[a][c] x_c
-                            for (int c2 = a; c2 < nb; ++c2) y = fma(sm.G[a + c2 * (NB + 1)], xv[c2], y);
-                        }
-                    }
-                    yv[a] = y;
-                }
-                for (int a = 0; a < NB; ++a) sm.Xs[a + t * NB] = yv[a];
-            }
-            __syncthreads();
-            // x <- x - V Xs
-            for (int64_t q = tid; q < (int64_t)nc * (m - j0 - 1); q += kT) {
-                const int t = (int)(q / (m - j0 - 1)), r = j0 + 1 + (int)(q % (m - j0 - 1));
-                double s = 0.0;
-                for (int a = 0; a < nb; ++a) s = fma(wy_v(C, m, j0 + a, r), sm.Xs[a + t * NB], s);
-                X[(int64_t)(t0 + t) * m + r] -= s;
-            }
-            __syncthreads();
-        }
-    }
-}
 
 // ---------------------------------------------------------------------------
-constexpr int kWyMmaMin = 64;   // orders from which the reflectors are applied as tile products
-
 __host__ __device__ constexpr int64_t t_panels(int m) { return m > 2 ? (m - 2 + NB - 1) / NB : 0; }
 
 // T of the compact WY form I - V T V^T of every panel of NB reflectors of
@@ -1061,163 +533,19 @@ __device__ void trsm_cols(bool lower, const double* __restrict__ L, int m, doubl
     }
 }
 
-// ---------------------------------------------------------------------------
-// Owned rows of S U and U, fe and the eigenpairs.  R holds 2 nown rows of
-// length m (row-major, i.e. the column-major m x 2nown matrix R^T): rows
-// t < nown are L[c_t,:] -> (S U)[c_t,:], rows nown + t are (L^-T)[c_t,:] ->
-// U[c_t,:].  The final product with Z goes into the third block G (R Z).
-__device__ void stage_rows(const EigProb& p, const double* __restrict__ Ca, const double* __restrict__ La,
-                           const double* __restrict__ Ta, const double* __restrict__ Wa,
-                           const double* __restrict__ Za, const int* __restrict__ own_cols,
-                           const int* __restrict__ ipos, double* __restrict__ Ba, double* __restrict__ Qa,
-                           double* __restrict__ Va, const double* __restrict__ Ka, double* __restrict__ e_out,
-                           double* __restrict__ fe_out, const StageSmem& sh) {
-    double* sA = sh.sA;
-    double* sB = sh.sB;
-    const int m = p.m, no = p.nown, nb2 = 2 * no;
-    const double* C = Ca + p.aoff;
-    const double* L = La + p.aoff;
-    const double* Z = Za + p.aoff;
-    const double* tau = Ta + p.voff;
-    double* R = Ba + p.boff;                     // 2 nown rows
-    double* R2 = R + (int64_t)no * m;
-    double* G = R + (int64_t)nb2 * m;            // 2 nown rows of R Z
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = kT / 32;
-    for (int t = 0; t < no; ++t) {
-        const int ct = ipos[own_cols[p.o0 + t]];
-        for (int r = tid; r < m; r += kT) {
-            R[(int64_t)t * m + r] = (r <= ct) ? L[ct + (int64_t)r * m] : 0.0;
-            R2[(int64_t)t * m + r] = (r == ct) ? 1.0 : 0.0;
-        }
-    }
-    __syncthreads();
-    // rows of L^-T: x_t = L^-1 e_{c_t}; blocked on the tensor cores when the
-    // divide and conquer's (now free) arrays hold a 64 x 65 diagonal block
-    if (dc_smem_bytes(sh.M) >= sizeof(double) * TS * (TS + 1)) {
-        trsm_cols(true, L, m, R2, m, 0, no, reinterpret_cast<double*>(sh.uni), sA, sB);
-    } else {
-        for (int i0 = 0; i0 < m; i0 += NB) {
-            const int nb = min(NB, m - i0), i1 = i0 + nb;
-            for (int t = warp; t < no; t += nwarp) {
-                double* x = R2 + (int64_t)t * m;
-                double xv = (lane < nb) ? x[i0 + lane] : 0.0;
-                for (int k = 0; k < nb; ++k) {
-                    if (lane == k) xv /= L[(i0 + k) + (int64_t)(i0 + k) * m];
-                    const double xk = __shfl_sync(0xffffffffu, xv, k);
-                    if (lane > k && lane < nb) xv -= L[(i0 + lane) + (int64_t)(i0 + k) * m] * xk;
-                }
-                if (lane < nb) x[i0 + lane] = xv;
-            }
-            __syncthreads();
-            for (int64_t q = tid; q < (int64_t)no * (m - i1); q += kT) {
-                const int t = (int)(q / (m - i1)), r = i1 + (int)(q % (m - i1));
-                double* x = R2 + (int64_t)t * m;
-                double s = 0.0;
-                for (int k = 0; k < nb; ++k) s = fma(L[r + (int64_t)(i0 + k) * m], x[i0 + k], s);
-                x[r] -= s;
-            }
-            __syncthreads();
-        }
-    }
-    // R <- R Q: each row x becomes Q^T x (from order 64 as tile products with the
-    // panels' T, the divide and conquer's Q and V arenas as scratch)
-    if (m >= kWyMmaMin) wy_apply_t(C, m, Ka + p.koff, R, nb2, true, Qa + p.aoff, Va + p.aoff, sA, sB);
-    else wy_apply(C, m, tau, R, nb2, true, WySmem{sA, sB});
-    __syncthreads();
-    // G^T = Z^T R^T (m x 2nown, column-major = G row-major)
-    for (int c0 = 0; c0 < nb2; c0 += TS)
-        for (int r0 = 0; r0 < m; r0 += TS)
-            tile_gemm<true>(G, m, 0, nullptr, r0, c0, min(TS, m - r0), min(TS, nb2 - c0), Z, m, nullptr, R, m, nullptr, m,
-                            sA, sB);
-    __syncthreads();
-    const double* G2 = G + (int64_t)no * m;
-    for (int j = tid; j < m; j += kT) {
-        double f = 0.0;
-        for (int t = 0; t < no; ++t) f = fma(G[(int64_t)t * m + j], G2[(int64_t)t * m + j], f);
-        e_out[p.eoff + j] = Wa[p.voff + j];
-        fe_out[p.eoff + j] = f;
-    }
-}
+#include "eig_dc.cuh"
+#include "eig_vec.cuh"
 
 // ---------------------------------------------------------------------------
-// Density of one system on one CTA (mode 2): U = L^-T Q Z in place of Z (Q as
-// WY tile products, L^-T by blocked back substitution, or one warp per column
-// when the divide and conquer's arrays are too small for the 64 x 65 block),
-// then the upper tiles of U_occ U_occ^T (K = nocc, the lowest eigenvectors:
-// the divide and conquer leaves them ascending) into Ba + boff; the factor 2
-// is applied when packing.
-__device__ void stage_density(const EigProb& p, const double* __restrict__ Ca, const double* __restrict__ La,
-                              const double* __restrict__ Ta, double* __restrict__ Za, double* __restrict__ Qa,
-                              double* __restrict__ Va, const double* __restrict__ Ka, double* __restrict__ Ba,
-                              const StageSmem& sh) {
-    const int m = p.m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int no = p.nocc;   // only the occupied eigenvectors enter P
-    const double* C = Ca + p.aoff;
-    const double* L = La + p.aoff;
-    double* U = Za + p.aoff;
-    if (no == 0) return;
-    if (m >= kWyMmaMin) wy_apply_t(C, m, Ka + p.koff, U, no, false, Qa + p.aoff, Va + p.aoff, sh.sA, sh.sB);
-    else wy_apply(C, m, Ta + p.voff, U, no, false, WySmem{sh.sA, sh.sB});
-    __syncthreads();
-    if (p.kind == 0) {
-        if (dc_smem_bytes(sh.M) >= sizeof(double) * TS * (TS + 1)) {
-            trsm_cols(false, L, m, U, m, 0, no, reinterpret_cast<double*>(sh.uni), sh.sA, sh.sB);
-        } else {
-            for (int t = warp; t < no; t += kT / 32) {
-                double* w = U + (int64_t)t * m;
-                for (int i = m - 1; i >= 0; --i) {
-                    const double* li = L + (int64_t)i * m;
-                    double sum = 0.0;
-                    for (int k = i + 1 + lane; k < m; k += 32) sum = fma(li[k], w[k], sum);
-                    sum = warp_sum(sum);
-                    if (lane == 0) w[i] = (w[i] - sum) / li[i];
-                    __syncwarp();
-                }
-            }
-        }
-    }
-    __syncthreads();
-    double* P = Ba + p.boff;
-    const int nt = (m + TS - 1) / TS;
-    for (int cb = 0; cb < nt; ++cb)
-        for (int rb = 0; rb <= cb; ++rb)
-            tile_mma<false, true, MMA_SET, false>(P, m, 0, nullptr, rb * TS, cb * TS, min(TS, m - rb * TS),
-                                                  min(TS, m - cb * TS), U, m, nullptr, U, m, nullptr, p.nocc, sh.sA,
-                                                  sh.sB);
-}
-
-// ---------------------------------------------------------------------------
-// The stages of the problems up to kEigBatchMax, a launch each over the whole
-// batch, every stage with its own split: one CTA per problem where a stage is a
-// chain (Cholesky, tridiagonalisation, divide and conquer), one CTA per 64-column
-// block where it is not (the two triangular solves of the reduction), largest
-// problems first.  status[pi]: 0, the order of a non-positive pivot of S_k, or
-// kStNoConv; a problem that failed is skipped by the later stages.
-__host__ __device__ constexpr size_t stage_smem_bytes(int M) {
-    return sizeof(double) * (2 * kStageOp + NB * (NB + 1)) + dc_smem_bytes(M) + sizeof(int) * 16 +
-           sizeof(double) * (2 + kT / 32) + 16;
-}
-
-__device__ StageSmem stage_smem(unsigned char* base, int M) {
-    StageSmem sh;
-    double* d = reinterpret_cast<double*>(base);
-    sh.sA = d;
-    sh.sB = d + kStageOp;
-    sh.sD = d + 2 * kStageOp;
-    sh.uni = reinterpret_cast<unsigned char*>(d + 2 * kStageOp + NB * (NB + 1));
-    sh.ints = reinterpret_cast<int*>(sh.uni + dc_smem_bytes(M));
-    sh.dsc = reinterpret_cast<double*>(sh.ints + 16);
-    sh.M = M;
-    return sh;
-}
-
+// status[pi]: 0, the order of a non-positive pivot of S_k, or kStNoConv; a problem
+// that failed is skipped by the later stages.
 // Gather and Cholesky, one problem per CTA.
 __global__ void __launch_bounds__(kT, 1) k_eig_chol(const EigProb* __restrict__ probs, const int* __restrict__ order,
                                                     const int* __restrict__ maps, const double* __restrict__ H,
                                                     const double* __restrict__ S, double* __restrict__ Xa,
                                                     double* __restrict__ La, int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const StageSmem sh = stage_smem(smraw, 2);
+    const StageSmem sh = stage_smem(smraw);
     const int pi = order[blockIdx.x];
     const EigProb p = probs[pi];
     stage_gather(p, maps, H, S, Xa, La);
@@ -1274,121 +602,14 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_eig_trd(const EigProb* __restr
 }
 
 // Divide and conquer, then the owned rows and fe (mode 0) or the density (mode 2).
-__global__ void __launch_bounds__(kT, 1) k_eig_vectors(
-    const EigProb* __restrict__ probs, const int* __restrict__ order, int np, int* __restrict__ counter, int M,
-    double* __restrict__ Ca, double* __restrict__ La, double* __restrict__ Za, double* __restrict__ Qa,
-    double* __restrict__ Va, double* __restrict__ Da, double* __restrict__ Ea, double* __restrict__ Ta,
-    double* __restrict__ Wa, double* __restrict__ Ba, double* __restrict__ Ka, const int* __restrict__ own_cols,
-    const int* __restrict__ ipos, double* __restrict__ e_out, double* __restrict__ fe_out,
-    int* __restrict__ status) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const StageSmem sh = stage_smem(smraw, M);
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) sh.ints[15] = atomicAdd(counter, 1);
-        __syncthreads();
-        const int q = sh.ints[15];
-        __syncthreads();
-        if (q >= np) break;
-        const int pi = order[q];
-        if (status[pi] != kStOk) continue;
-        const EigProb p = probs[pi];
-        if (!stage_dc(p, Da, Ea, Wa, Za, Qa, Va, sh)) {
-            if (tid == 0) status[pi] = kStNoConv;
-            __syncthreads();
-            continue;
-        }
-        __syncthreads();
-        if (p.m >= kWyMmaMin)
-            build_T(Ca + p.aoff, p.m, Ta + p.voff, Ka + p.koff, 0, 1, Va + p.aoff, sh.sD, sh.sA, sh.sB);
-        if (p.mode == 2) {
-            for (int j = threadIdx.x; j < p.m; j += kT) e_out[p.eoff + j] = Wa[p.voff + j];
-            stage_density(p, Ca, La, Ta, Za, Qa, Va, Ka, Ba, sh);
-        } else {
-            stage_rows(p, Ca, La, Ta, Wa, Za, own_cols, ipos, Ba, Qa, Va, Ka, e_out, fe_out, sh);
-        }
-        __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Owned columns of P_k at mu: w_t = occ o U[c_t,:]^T, w <- Z w, w <- Q w
-// (reflectors in reverse), w <- L^-T w; scattered into the packed result,
-// rows map(i) <= c_t of column c_t (or written dense).
-// Shared memory of the final-column kernels: tile staging, a 64 x 65 diagonal
-// block of L and the panel's T.
-constexpr size_t kFinalSmem = sizeof(double) * (2 * kStageOp + TS * (TS + 1) + NB * (NB + 1));
-
-__global__ void __launch_bounds__(kT) k_eig_final(const EigProb* __restrict__ probs, const int* __restrict__ order,
-                                                  const double* __restrict__ Ca,
-                                                  const double* __restrict__ La, const double* __restrict__ Ta,
-                                                  const double* __restrict__ Wa, const double* __restrict__ Za,
-                                                  double* __restrict__ Qa, double* __restrict__ Va,
-                                                  const double* __restrict__ Ka,
-                                                  const int* __restrict__ maps, const int* __restrict__ own_cols,
-                                                  double* __restrict__ Ba, double mu, double* __restrict__ Ppk,
-                                                  double* __restrict__ Pdense) {
-    extern __shared__ __align__(16) unsigned char smf[];
-    double* sA = reinterpret_cast<double*>(smf);
-    double* sB = sA + kStageOp;
-    double* sD = sB + kStageOp;
-    double* sT = sD + TS * (TS + 1);
-    const EigProb p = probs[order[blockIdx.x]];
-    const int m = p.m, no = p.nown;
-    const double* C = Ca + p.aoff;
-    const double* L = La + p.aoff;
-    const double* Z = Za + p.aoff;
-    const double* tau = Ta + p.voff;
-    const double* ev = Wa + p.voff;
-    double* W0 = Ba + p.boff;                       // (S U) rows block: free after the prepare step
-    const double* U2 = Ba + p.boff + 3 * (int64_t)no * m;   // U[c_t, :] (second half of G)
-    double* W = Ba + p.boff + (int64_t)no * m;      // m x nown, column-major
-    const int tid = threadIdx.x;
-    for (int64_t q = tid; q < (int64_t)no * m; q += kT) {
-        const int j = (int)(q % m);
-        const double e = ev[j];
-        const double occ = e < mu ? 2.0 : (e == mu ? 1.0 : 0.0);
-        W0[q] = occ * U2[q];
-    }
-    __syncthreads();
-    // W = Z W0
-    for (int c0 = 0; c0 < no; c0 += TS)
-        for (int r0 = 0; r0 < m; r0 += TS)
-            tile_gemm<false>(W, m, 0, nullptr, r0, c0, min(TS, m - r0), min(TS, no - c0), Z, m, nullptr, W0, m, nullptr, m,
-                             sA, sB);
-    __syncthreads();
-    // Q W (from order 64 as tile products, the divide and conquer's arenas as scratch)
-    if (m >= kWyMmaMin) wy_apply_t(C, m, Ka + p.koff, W, no, false, Qa + p.aoff, Va + p.aoff, sA, sB);
-    else wy_apply(C, m, tau, W, no, false, WySmem{sA, sB});
-    __syncthreads();
-    // L^-T W: blocked back substitution
-    trsm_cols(false, L, m, W, m, 0, no, sD, sA, sB);
-    if (Pdense) {
-        for (int64_t q = tid; q < (int64_t)no * m; q += kT) Pdense[p.poff + q] = W[q];
-        return;
-    }
-    const int* mp = maps + p.moff;
-    for (int64_t q = tid; q < (int64_t)no * m; q += kT) {
-        const int t = (int)(q / m), i = (int)(q % m);
-        const int64_t cgl = own_cols[p.o0 + t];
-        const int64_t gi = mp[i];
-        if (gi <= cgl) Ppk[cgl * (cgl + 1) / 2 + gi] = W[q];
-    }
-}
-
-
 // ===========================================================================
-// Submatrices above kEigBatchMax (the k-means columns of large boxes): the
-// same stages on a thread-block cluster of G CTAs per submatrix, one cluster
-// barrier (barrier.cluster) between dependent steps and every intermediate in
-// global memory (L2-resident for the vectors and panels).
-//   gather       columns split over the CTAs
+// Cholesky and tridiagonalisation of problems above kEigBatchMax (and of single
+// dense problems): G CTAs per problem, a thread-block cluster or a cooperative grid,
+// one barrier between dependent steps and the intermediates in global memory
+// (L2-resident for the vectors and panels).
 //   Cholesky     32-wide panels: the diagonal block factored by every CTA (same
 //                data, same arithmetic, same result), panel rows and lower
 //                trailing tiles split over the CTAs
-//   reduction    C = L^-1 H L^-T: left-looking triangular solves over 64-row
-//                blocks, each CTA owning 64-column blocks of C (no barrier
-//                inside a solve)
 //   tridiag.     blocked Householder with lazy updates (LAPACK's latrd
 //                scheme): per column the panel's earlier reflectors update that
 //                column, the reflector is formed, and y = A v runs over the
@@ -1398,40 +619,11 @@ __global__ void __launch_bounds__(kT) k_eig_final(const EigProb* __restrict__ pr
 //                after 32 columns the trailing block gets A -= V W^T + W V^T.
 //                Rows are owned in 32-row chunks, partial sums go through
 //                per-CTA slots summed in CTA order, so results do not depend on
-//                scheduling.  Two cluster barriers per column.
-//   D&C          leaves and the lower merges one CTA each, merges with fewer
-//                problems than CTAs by the whole cluster
-//   owned rows   vectors split over the CTAs, then one tiled product with Z
+//                scheduling.  Two barriers per column.
 // ===========================================================================
 constexpr int kLargeMax = kEigLargeMax;   // largest order the cluster solver takes (its vectors live in shared memory)
 constexpr int kRedW = 2 * NB + 4;         // per-CTA partial sums of the tridiagonalisation
 constexpr int kRedVAv = 2 * NB + 1;       // slot of the partial v^T A v
-constexpr int kLgStages = 6;              // stage timestamps per problem: start, Cholesky, reduction, tridiag., D&C, rows
-constexpr int kLgSub = 7;                 // tridiagonalisation phase times per problem (ns, summed over its columns)
-constexpr int kLgStride = kLgStages + kLgSub;
-
-// Phase clock of one thread (rank 0, thread 0 of a cluster when stage times are
-// requested): lap(q) adds the time since the previous lap to acc[q].
-struct PhaseClock {
-    unsigned long long* acc;
-    unsigned long long t;
-    __device__ __forceinline__ static unsigned long long now() {
-        unsigned long long v;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
-        return v;
-    }
-    __device__ __forceinline__ void start() {
-        if (acc) t = now();
-    }
-    __device__ __forceinline__ void lap(int q) {
-        if (acc) {
-            const unsigned long long n = now();
-            acc[q] += n - t;
-            t = n;
-        }
-    }
-};
-
 // Software barrier over the CTAs of a cooperative launch (all resident):
 // bar[0] counts arrivals, bar[1] is the generation.  The wait is bounded: after
 // kGridSpin polls the CTA records the failure in *err and goes on, and every
@@ -1478,7 +670,7 @@ struct Grp {
 
 // Per-problem scratch of a cluster solve (offsets in doubles from p.xoff).
 struct LgLayout {
-    int64_t rowp, colp, red, V, W, dc, scal, total;
+    int64_t rowp, colp, red, V, W, total;
 };
 constexpr int kSegW = 64;    // columns of one A v work unit of the tridiagonalisation
 constexpr int kAvGrp = 8;    // columns whose loads are issued together in the A v units
@@ -1495,11 +687,6 @@ __host__ __device__ inline LgLayout lg_layout(int m, int G) {
     o += (int64_t)m * NB;
     L.W = o;
     o += (int64_t)m * NB;
-    o = (o + 1) & ~int64_t(1);
-    L.dc = o;
-    o += (int64_t)((dc_smem_bytes((m + 1) & ~1) + 15) / 16) * 2;
-    L.scal = o;
-    o += ((int64_t)m + 64) / 2 + 2;   // 8 ints per merge of the widest level (at most m / 16 merges)
     L.total = (o + 1) & ~int64_t(1);
     return L;
 }
@@ -1551,17 +738,16 @@ __device__ __forceinline__ void tri_decode(int64_t idx, int& rb, int& cb) {
     cb = (int)(idx - (int64_t)r * (r + 1) / 2);
 }
 
+// H_k into X, S_k into L (generalized problems), columns split over the CTAs.
 __device__ void lg_gather(const Grp& g, const EigProb& p, const int* __restrict__ maps, const double* __restrict__ H,
-                          const double* __restrict__ S, double* __restrict__ Ca, double* __restrict__ La) {
+                          const double* __restrict__ S, double* __restrict__ X, double* __restrict__ L) {
     const int m = p.m;
     const int* mp = maps + p.moff;
-    double* C = Ca + p.aoff;
-    double* L = La + p.aoff;
     for (int j = g.rank; j < m; j += g.size) {
         const int64_t gj = p.gbase + (int64_t)mp[j] * p.gld;
         for (int i = threadIdx.x; i < m; i += kT) {
             const int64_t q = (int64_t)mp[i] + gj;
-            C[i + (int64_t)j * m] = H[q];
+            X[i + (int64_t)j * m] = H[q];
             if (p.kind == 0) L[i + (int64_t)j * m] = S[q];
         }
     }
@@ -1650,68 +836,6 @@ __device__ int lg_potrf(const Grp& g, int m, double* __restrict__ L, const LgSme
 // left-looking over 64-row blocks, X_i -= L[i, <i] X[<i] as one tile product,
 // then the diagonal block's forward substitution (warp per column, two rows per
 // lane).  The column blocks are independent, so no cluster barrier is needed.
-__device__ void lg_trsm_cols(const Grp& g, const double* __restrict__ L, double* X, int m, const LgSmem& sh) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double* sD = sh.sD;   // sD[i + j*(TS+1)]
-    const int ncb = (m + TS - 1) / TS;
-    for (int cb = g.rank; cb < ncb; cb += g.size) {
-        const int c0 = cb * TS, nc = min(TS, m - c0);
-        for (int i0 = 0; i0 < m; i0 += TS) {
-            const int mr = min(TS, m - i0);
-            if (i0 > 0)
-                tile_mma<false, false, MMA_SUB, false>(X, m, 0, nullptr, i0, c0, mr, nc, L, m, nullptr, X, m, nullptr,
-                                                       i0, sh.sA, sh.sB);
-            for (int t = tid; t < TS * TS; t += kT) {
-                const int i = t % TS, j = t / TS;
-                sD[i + j * (TS + 1)] = (i < mr && j < mr && i >= j) ? L[(int64_t)(i0 + i) + (int64_t)(i0 + j) * m] : 0.0;
-            }
-            __syncthreads();
-            for (int jc = warp; jc < nc; jc += kT / 32) {
-                double* x = X + (int64_t)(c0 + jc) * m + i0;
-                double x0 = lane < mr ? x[lane] : 0.0, x1 = lane + 32 < mr ? x[lane + 32] : 0.0;
-                for (int k = 0; k < mr; ++k) {
-                    double xk;
-                    if (k < 32) {
-                        if (lane == k) x0 /= sD[k + k * (TS + 1)];
-                        xk = __shfl_sync(0xffffffffu, x0, k);
-                    } else {
-                        if (lane == k - 32) x1 /= sD[k + k * (TS + 1)];
-                        xk = __shfl_sync(0xffffffffu, x1, k - 32);
-                    }
-                    if (lane > k && lane < mr) x0 -= sD[lane + k * (TS + 1)] * xk;
-                    if (lane + 32 > k && lane + 32 < mr) x1 -= sD[lane + 32 + k * (TS + 1)] * xk;
-                }
-                if (lane < mr) x[lane] = x0;
-                if (lane + 32 < mr) x[lane + 32] = x1;
-            }
-            __syncthreads();
-        }
-    }
-}
-
-// C <- L^-1 H_k L^-T: C <- L^-1 C, transpose, C <- L^-1 C (only the lower
-// triangle is read afterwards).
-__device__ void lg_reduce(const Grp& g, const EigProb& p, const double* __restrict__ La, double* Ca,
-                          const LgSmem& sh) {
-    const int m = p.m;
-    const double* L = La + p.aoff;
-    double* C = Ca + p.aoff;
-    lg_trsm_cols(g, L, C, m, sh);
-    g.sync();
-    const int64_t mm = (int64_t)m * m;
-    for (int64_t t = (int64_t)g.rank * kT + threadIdx.x; t < mm; t += (int64_t)g.size * kT) {
-        const int i = (int)(t % m), j = (int)(t / m);
-        if (i > j) {
-            const double a = C[i + (int64_t)j * m], b = C[j + (int64_t)i * m];
-            C[i + (int64_t)j * m] = b;
-            C[j + (int64_t)i * m] = a;
-        }
-    }
-    g.sync();
-    lg_trsm_cols(g, L, C, m, sh);
-    g.sync();
-}
-
 // w of reflector jp (column j - 1 of the panel's first column j0 = j - 1 - jp)
 // on this CTA's rows r >= j, from the summed partial products; the reflector
 // itself goes into column j - 1 below its leading 1.  Returns w at row j
@@ -1759,11 +883,8 @@ __device__ void lg_finish_w(const Grp& g, int m, int j, int jp, double* __restri
 }
 
 __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca, double* __restrict__ Da,
-                         double* __restrict__ Ea, double* __restrict__ Ta, double* __restrict__ X, const LgSmem& sh,
-                         unsigned long long* tsub) {
+                         double* __restrict__ Ea, double* __restrict__ Ta, double* __restrict__ X, const LgSmem& sh) {
     const int m = p.m, G = g.size, rk = g.rank;
-    PhaseClock pc{(g.rank == 0 && threadIdx.x == 0) ? tsub : nullptr, 0};
-    pc.start();
     double* A = Ca + p.aoff;
     double* d = Da + p.voff;
     double* e = Ea + p.voff;
@@ -1821,9 +942,7 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                 part = warp_sum(part);
                 if (lane == 0) red[rk * kRedW + ((q < jj) ? 1 + q : 1 + NB + (q - jj))] = part;
             }
-            pc.lap(0);
             g.sync();
-            pc.lap(1);
             // ---- phase B: reflector, then y = A v over the trailing lower tiles
             // (column j below the subdiagonal is read into v while the scale is
             // formed, and scaled in shared memory after the barrier)
@@ -1881,7 +1000,6 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                 const int r = ch * 32 + lane;
                 if (r >= s && r < m) V[r + (int64_t)jj * m] = v[r];
             }
-            pc.lap(2);
             // A v over the trailing lower triangle, one pass: every warp streams
             // its own units (64 rows x kSegW columns of one tile row) without a
             // barrier, lane holding rows I*64 + lane and + 32: the row sums stay
@@ -1943,13 +1061,10 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                     if (r1 < m) rowp[(int64_t)seg * m + r1] = rp1;
                     vav = fma(v0, rp0, fma(v1, rp1, vav));
                 }
-                pc.lap(3);
                 const double part = cta_sum(vav, sh.red);
                 if (tid == 0) red[rk * kRedW + kRedVAv] = part;
             }
-            pc.lap(4);
             g.sync();
-            pc.lap(5);
         }
         // ---- panel end: w of the last column, then the trailing block
         const int j1 = j0 + nb;
@@ -1968,7 +1083,6 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
             }
         }
         g.sync();
-        pc.lap(6);
     }
     if (rk == 0 && tid == 0) {
         d[m - 1] = A[(m - 1) + (int64_t)(m - 1) * m];
@@ -1976,606 +1090,130 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
     }
 }
 
-// ---------------------------------------------------------------------------
-// Divide and conquer on a cluster.  A merge is run by one CTA (Split{0, 1,
-// false}) or by the whole group (Split{rank, G, true}); its per-element
-// arrays sit at offset lo of the problem's arrays, its Q and V blocks at
-// column lo of the Q and V arenas, so merges of one level never overlap.
-struct Split {
-    int part, nparts;
-    bool coop;
-    const Grp* g;
-    __device__ __forceinline__ void sync() const {
-        if (coop) g->sync();
-        else __syncthreads();
-    }
-    __device__ __forceinline__ int first() const { return part * kT + (int)threadIdx.x; }
-    __device__ __forceinline__ int step() const { return nparts * kT; }
-    __device__ __forceinline__ bool lead() const { return part == 0 && threadIdx.x == 0; }
-};
 
-__device__ DcSmem dc_shift(const DcSmem& S, int lo) {
-    DcSmem q = S;
-    q.Ds += lo;
-    q.zs += lo;
-    q.dk += lo;
-    q.zk += lo;
-    q.tau += lo;
-    q.zh += lo;
-    q.val += lo;
-    q.perm += lo;
-    q.org += lo;
-    q.sec += lo;
-    q.dl += lo;
-    q.rank += lo;
-    q.cls += lo;
-    q.ktop += lo;
-    q.kbot += lo;
-    q.rpair += lo;
-    q.rcs += lo;
-    return q;
+// Gather and Cholesky, tridiagonalisation: a cluster per problem (order[]: largest
+// first), or with bar non-null one problem on the whole cooperative grid.
+__device__ __forceinline__ Grp lg_group(unsigned* bar, int* err) {
+    if (bar) return Grp{(int)blockIdx.x, (int)gridDim.x, bar, err};
+    cg::cluster_group cl = cg::this_cluster();
+    return Grp{(int)cl.block_rank(), (int)cl.num_blocks(), nullptr, nullptr};
 }
-
-__device__ void dc_merge(const Split& sp, int m, int lo, int mid, int hi, double beta, const DcSmem& S,
-                         double* __restrict__ Z, double* __restrict__ Qp, double* __restrict__ V, int* sc, double* sA,
-                         double* sB) {
-    const DcSmem Q = dc_shift(S, lo);
-    const int n1 = mid - lo, n2 = hi - mid, n = n1 + n2;
-    const double rho = 2.0 * fabs(beta);
-    const double sgn = beta >= 0.0 ? 1.0 : -1.0;
-    const double rs2 = 0.70710678118654752440;
-    const double eps = 2.220446049250313e-16;
-    const int f0 = sp.first(), st = sp.step();
-    // (a) merged order of the two sorted blocks
-    for (int j = f0; j < n; j += st) {
-        int r;
-        if (j < n1) {
-            const double x = S.D[lo + j];
-            int a = 0, b = n2;
-            while (a < b) {
-                const int c = (a + b) >> 1;
-                if (S.D[mid + c] < x) a = c + 1;
-                else b = c;
-            }
-            r = j + a;
-        } else {
-            const double x = S.D[mid + j - n1];
-            int a = 0, b = n1;
-            while (a < b) {
-                const int c = (a + b) >> 1;
-                if (S.D[lo + c] <= x) a = c + 1;
-                else b = c;
-            }
-            r = (j - n1) + a;
-        }
-        Q.perm[r] = j;
-    }
-    sp.sync();
-    // (b) sorted d, z and column classes; (c) Q with the block columns in that order
-    for (int r = f0; r < n; r += st) {
-        const int j = Q.perm[r];
-        if (j < n1) {
-            Q.Ds[r] = S.D[lo + j];
-            Q.zs[r] = Z[(int64_t)(mid - 1) + (int64_t)(lo + j) * m] * rs2;
-            Q.cls[r] = 1;
-        } else {
-            Q.Ds[r] = S.D[mid + j - n1];
-            Q.zs[r] = sgn * Z[(int64_t)mid + (int64_t)(mid + j - n1) * m] * rs2;
-            Q.cls[r] = 2;
-        }
-    }
-    for (int64_t t = f0; t < (int64_t)n * n; t += st) {
-        const int i = (int)(t % n), r = (int)(t / n);
-        const int j = Q.perm[r];
-        double v = 0.0;
-        if (j < n1) {
-            if (i < n1) v = Z[(int64_t)(lo + i) + (int64_t)(lo + j) * m];
-        } else if (i >= n1) {
-            v = Z[(int64_t)(lo + i) + (int64_t)(mid + j - n1) * m];
-        }
-        Qp[t] = v;
-    }
-    sp.sync();
-    // (d) deflation (one thread, in sorted order)
-    if (sp.lead()) {
-        double dmax = 0.0;
-        for (int r = 0; r < n; ++r) dmax = fmax(dmax, fabs(Q.Ds[r]));
-        const double tol = 8.0 * eps * fmax(dmax, rho);
-        int k = 0, nd = 0, nrot = 0, pj = -1;
-        for (int r = 0; r < n; ++r) {
-            if (rho * fabs(Q.zs[r]) <= tol) {
-                Q.dl[nd++] = r;
-                continue;
-            }
-            if (pj < 0) {
-                pj = r;
-                continue;
-            }
-            double sn = Q.zs[pj], c = Q.zs[r];
-            const double t = hypot(c, sn);
-            const double dd = Q.Ds[r] - Q.Ds[pj];
-            c /= t;
-            sn = -sn / t;
-            if (fabs(dd * c * sn) <= tol) {
-                Q.zs[r] = t;
-                Q.zs[pj] = 0.0;
-                Q.rpair[nrot] = make_int2(pj, r);
-                Q.rcs[nrot] = make_double2(c, sn);
-                ++nrot;
-                const double t2 = Q.Ds[pj] * c * c + Q.Ds[r] * sn * sn;
-                Q.Ds[r] = Q.Ds[pj] * sn * sn + Q.Ds[r] * c * c;
-                Q.Ds[pj] = t2;
-                Q.cls[r] |= Q.cls[pj];
-                Q.dl[nd++] = pj;
-                pj = r;
-            } else {
-                Q.sec[k++] = pj;
-                pj = r;
-            }
-        }
-        if (pj >= 0) Q.sec[k++] = pj;
-        int nt = 0, nb = 0;
-        for (int t = 0; t < k; ++t) {
-            const int c = Q.cls[Q.sec[t]];
-            if (c & 1) Q.ktop[nt++] = t;
-            if (c & 2) Q.kbot[nb++] = t;
-        }
-        sc[0] = k;
-        sc[1] = nd;
-        sc[2] = nrot;
-        sc[3] = nt;
-        sc[4] = nb;
-    }
-    sp.sync();
-    const volatile int* vsc = sc;
-    const int k = vsc[0], nd = vsc[1], nrot = vsc[2], ntop = vsc[3], nbot = vsc[4];
-    // (e) deflation rotations on the columns of Q (thread per row)
-    if (nrot > 0)
-        for (int i = f0; i < n; i += st)
-            for (int q2 = 0; q2 < nrot; ++q2) {
-                const int2 pr = Q.rpair[q2];
-                const double2 cs = Q.rcs[q2];
-                const double a = Qp[i + (int64_t)pr.x * n], b = Qp[i + (int64_t)pr.y * n];
-                Qp[i + (int64_t)pr.x * n] = cs.x * a + cs.y * b;
-                Qp[i + (int64_t)pr.y * n] = -cs.y * a + cs.x * b;
-            }
-    for (int t = f0; t < k; t += st) {
-        Q.dk[t] = Q.Ds[Q.sec[t]];
-        Q.zk[t] = Q.zs[Q.sec[t]];
-    }
-    sp.sync();
-    // (f) secular roots
-    for (int i = f0; i < k; i += st) Q.tau[i] = dc_secular(k, Q.dk, Q.zk, rho, i, &Q.org[i]);
-    sp.sync();
-    // (g) recomputed z
-    for (int j = f0; j < k; j += st) {
-        const double dj = Q.dk[j];
-        double w = (Q.dk[Q.org[j]] - dj) + Q.tau[j];
-        for (int i = 0; i < k; ++i) {
-            if (i == j) continue;
-            w *= ((Q.dk[Q.org[i]] - dj) + Q.tau[i]) / (Q.dk[i] - dj);
-        }
-        Q.zh[j] = copysign(sqrt(fmax(w / rho, 0.0)), Q.zk[j]);
-    }
-    sp.sync();
-    // (h) eigenvectors of the rank-one problem (columns of V, k x k) and the new eigenvalues
-    for (int i = f0; i < k; i += st) {
-        const double dorg = Q.dk[Q.org[i]], ti = Q.tau[i];
-        double nrm = 0.0;
-        for (int j = 0; j < k; ++j) {
-            const double v = Q.zh[j] / ((Q.dk[j] - dorg) - ti);
-            nrm = fma(v, v, nrm);
-        }
-        const double scl = 1.0 / sqrt(nrm);
-        for (int j = 0; j < k; ++j) V[j + (int64_t)i * k] = scl * (Q.zh[j] / ((Q.dk[j] - dorg) - ti));
-        Q.val[i] = dorg + ti;
-    }
-    for (int q2 = f0; q2 < nd; q2 += st) Q.val[k + q2] = Q.Ds[Q.dl[q2]];
-    sp.sync();
-    // (i) positions of the n new eigenvalues in ascending order
-    for (int a = f0; a < n; a += st) {
-        const double x = Q.val[a];
-        int r = 0;
-        for (int b2 = 0; b2 < n; ++b2) r += (Q.val[b2] < x || (Q.val[b2] == x && b2 < a)) ? 1 : 0;
-        Q.rank[a] = lo + r;
-    }
-    for (int t = f0; t < ntop; t += st) Q.perm[t] = Q.sec[Q.ktop[t]];
-    sp.sync();
-    // (j) Z block = Q [V | deflated columns], block-1 rows against the columns touching block 1
-    {
-        const int ntr = (n1 + TS - 1) / TS, ntc = (k + TS - 1) / TS;
-        for (int tt = sp.part; tt < ntr * ntc; tt += sp.nparts) {
-            const int r0 = (tt % ntr) * TS, c0 = (tt / ntr) * TS;
-            tile_gemm<false>(Z, m, lo, Q.rank, r0, c0, min(TS, n1 - r0), min(TS, k - c0), Qp, n, Q.perm, V, k, Q.ktop,
-                             ntop, sA, sB);
-        }
-    }
-    sp.sync();
-    for (int t = f0; t < nbot; t += st) Q.perm[t] = Q.sec[Q.kbot[t]];
-    sp.sync();
-    {
-        const int ntr = (n2 + TS - 1) / TS, ntc = (k + TS - 1) / TS;
-        for (int tt = sp.part; tt < ntr * ntc; tt += sp.nparts) {
-            const int r0 = n1 + (tt % ntr) * TS, c0 = (tt / ntr) * TS;
-            tile_gemm<false>(Z, m, lo, Q.rank, r0, c0, min(TS, n - r0), min(TS, k - c0), Qp, n, Q.perm, V, k, Q.kbot,
-                             nbot, sA, sB);
-        }
-    }
-    for (int64_t t = f0; t < (int64_t)nd * n; t += st) {
-        const int i = (int)(t % n), q2 = (int)(t / n);
-        Z[(int64_t)(lo + i) + (int64_t)Q.rank[k + q2] * m] = Qp[i + (int64_t)Q.dl[q2] * n];
-    }
-    for (int a = f0; a < n; a += st) S.D[Q.rank[a]] = Q.val[a];
-    sp.sync();
-}
-
-__device__ bool lg_dc(const Grp& g, const EigProb& p, const double* __restrict__ Da, const double* __restrict__ Ea,
-                      double* __restrict__ Wa, double* __restrict__ Za, double* __restrict__ Qa,
-                      double* __restrict__ Va, double* __restrict__ X, const LgSmem& sh) {
-    const int m = p.m;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const LgLayout lay = lg_layout(m, g.size);
-    const DcSmem S = dc_smem(reinterpret_cast<unsigned char*>(X + lay.dc), (m + 1) & ~1);
-    int* scal = reinterpret_cast<int*>(X + lay.scal);
-    double* Z = Za + p.aoff;
-    const double* eo = Ea + p.voff;
-    int L = 0;
-    while (((m + (1 << L) - 1) >> L) > kDcLeaf) ++L;
-    const int nleaf = 1 << L;
-    for (int i = g.rank * kT + tid; i < m; i += g.size * kT) S.D[i] = Da[p.voff + i];
-    if (g.rank == 0 && tid == 0) scal[7] = 0;
+__global__ void __launch_bounds__(kT, 1) k_lg_chol(const EigProb* __restrict__ probs, const int* __restrict__ order,
+                                                   const int* __restrict__ maps, const double* __restrict__ H,
+                                                   const double* __restrict__ S, double* __restrict__ Ca,
+                                                   double* __restrict__ Xa, double* __restrict__ La,
+                                                   int* __restrict__ status, unsigned* __restrict__ bar,
+                                                   int* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const LgSmem sh = lg_smem(smraw, 2);
+    const Grp g = lg_group(bar, err);
+    const int pi = order[bar ? 0 : blockIdx.x / g.size];
+    const EigProb p = probs[pi];
+    // a standard problem needs no reduction: its matrix goes where that leaves it
+    lg_gather(g, p, maps, H, S, (p.kind == 0 ? Xa : Ca) + p.aoff, La + p.aoff);
     g.sync();
-    if (g.rank == 0 && tid == 0)
-        for (int q = 1; q < nleaf; ++q) {
-            const int pos = (int)(((int64_t)q * m) >> L);
-            const double ab = fabs(eo[pos - 1]);
-            S.D[pos - 1] -= ab;
-            S.D[pos] -= ab;
-        }
-    g.sync();
-    // leaves: a warp each over the whole cluster, numbered warp-major so that
-    // few leaves still spread over every SM
-    for (int q = warp * g.size + g.rank; q < nleaf; q += g.size * (kT / 32)) {
-        const int lo = (int)(((int64_t)q * m) >> L), hi = (int)(((int64_t)(q + 1) * m) >> L), s = hi - lo;
-        double dl[kDcLeaf], el[kDcLeaf], zl[kDcLeaf];
-        for (int i = 0; i < kDcLeaf; ++i) {
-            dl[i] = (i < s) ? S.D[lo + i] : 0.0;
-            el[i] = (i < s - 1) ? eo[lo + i] : 0.0;
-        }
-        const bool ok = dc_leaf(s, dl, el, zl, lane);
-        if (!ok && lane == 0) atomicExch(&scal[7], 1);
-        int rk = 0;
-        if (lane < s) {
-            const double x = dl[lane];
-            for (int c = 0; c < s; ++c) rk += (dl[c] < x || (dl[c] == x && c < lane)) ? 1 : 0;
-        }
-        for (int c = 0; c < s; ++c) {
-            const int rc = __shfl_sync(0xffffffffu, rk, c);
-            if (lane < s) Z[(int64_t)(lo + lane) + (int64_t)(lo + rc) * m] = zl[c];
-        }
-        __syncwarp();
-        if (lane < s) S.D[lo + rk] = dl[lane];
-        __syncwarp();
-    }
-    g.sync();
-    if (((volatile int*)scal)[7] != 0) return false;
-    for (int lev = L - 1; lev >= 0; --lev) {
-        const int nm = 1 << lev;
-        if (nm >= g.size) {
-            for (int q = g.rank; q < nm; q += g.size) {
-                const int lo = (int)(((int64_t)q * m) >> lev), hi = (int)(((int64_t)(q + 1) * m) >> lev);
-                const int mid = (int)(((int64_t)(2 * q + 1) * m) >> (lev + 1));
-                dc_merge(Split{0, 1, false, &g}, m, lo, mid, hi, eo[mid - 1], S, Z, Qa + p.aoff + (int64_t)lo * m,
-                         Va + p.aoff + (int64_t)lo * m, scal + 8 + 8 * q, sh.sA, sh.sB);
-            }
-        } else {
-            for (int q = 0; q < nm; ++q) {
-                const int lo = (int)(((int64_t)q * m) >> lev), hi = (int)(((int64_t)(q + 1) * m) >> lev);
-                const int mid = (int)(((int64_t)(2 * q + 1) * m) >> (lev + 1));
-                dc_merge(Split{g.rank, g.size, true, &g}, m, lo, mid, hi, eo[mid - 1], S, Z,
-                         Qa + p.aoff + (int64_t)lo * m, Va + p.aoff + (int64_t)lo * m, scal + 8 + 8 * q, sh.sA, sh.sB);
-            }
-        }
-        g.sync();
-    }
-    for (int i = g.rank * kT + tid; i < m; i += g.size * kT) Wa[p.voff + i] = S.D[i];
-    return true;
-}
-
-// Owned rows of S U and U, fe and the eigenpairs on the cluster: CTA rk takes a
-// contiguous range of the 2 nown vectors (L rows, then L^-T rows by forward
-// substitution), applies Q^T to them, and the product with Z is tiled over
-// the cluster.
-// Per-CTA scratch of the tile-product reflectors in the Q arena (free after the
-// divide and conquer): Y and T Y, NB x nv each.
-__host__ __device__ inline int64_t lg_wy_stride(int nv) { return 2 * (int64_t)NB * nv; }
-
-__device__ void lg_rows(const Grp& g, const EigProb& p, const double* __restrict__ Ca,
-                        const double* __restrict__ La, const double* __restrict__ Ta, const double* __restrict__ Wa,
-                        const double* __restrict__ Za, const int* __restrict__ own_cols, const int* __restrict__ ipos,
-                        double* __restrict__ Ba, double* __restrict__ Qa, const double* __restrict__ Ka,
-                        double* __restrict__ e_out, double* __restrict__ fe_out, const LgSmem& sh) {
-    const int m = p.m, no = p.nown, nb2 = 2 * no;
-    const double* C = Ca + p.aoff;
-    const double* L = La + p.aoff;
-    const double* Z = Za + p.aoff;
-    const double* tau = Ta + p.voff;
-    double* R = Ba + p.boff;
-    double* G2 = R + (int64_t)nb2 * m;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = kT / 32;
-    const int per = (nb2 + g.size - 1) / g.size;
-    const int u0 = min(nb2, g.rank * per), u1 = min(nb2, u0 + per);
-    for (int u = u0; u < u1; ++u) {
-        const int t = u < no ? u : u - no;
-        const int ct = ipos[own_cols[p.o0 + t]];
-        double* x = R + (int64_t)u * m;
-        for (int r = tid; r < m; r += kT)
-            x[r] = (u < no) ? ((r <= ct) ? L[ct + (int64_t)r * m] : 0.0) : ((r == ct) ? 1.0 : 0.0);
-    }
-    __syncthreads();
-    const int s0 = max(u0, no);
-    if (s0 < u1) trsm_cols(true, L, m, R + (int64_t)s0 * m, m, 0, u1 - s0, sh.sD, sh.sA, sh.sB);
-    if (u1 > u0) {
-        double* scr = Qa + p.aoff + (int64_t)g.rank * lg_wy_stride(per);
-        wy_apply_t(C, m, Ka + p.koff, R + (int64_t)u0 * m, u1 - u0, true, scr, scr + (int64_t)NB * per, sh.sA,
-                   sh.sB);
-    }
-    g.sync();
-    {
-        const int ntr = (m + TS - 1) / TS, ntc = (nb2 + TS - 1) / TS;
-        for (int tt = g.rank; tt < ntr * ntc; tt += g.size) {
-            const int r0 = (tt % ntr) * TS, c0 = (tt / ntr) * TS;
-            tile_gemm<true>(G2, m, 0, nullptr, r0, c0, min(TS, m - r0), min(TS, nb2 - c0), Z, m, nullptr, R, m,
-                            nullptr, m, sh.sA, sh.sB);
-        }
-    }
-    g.sync();
-    const double* G3 = G2 + (int64_t)no * m;
-    for (int j = g.rank * kT + tid; j < m; j += g.size * kT) {
-        double f = 0.0;
-        for (int t = 0; t < no; ++t) f = fma(G2[(int64_t)t * m + j], G3[(int64_t)t * m + j], f);
-        e_out[p.eoff + j] = Wa[p.voff + j];
-        fe_out[p.eoff + j] = f;
-    }
-}
-
-// Every stage of one problem on a group of CTAs.  mode 0: the submatrix
-// method's eigenvalues, fe weights and owned rows of U (lg_rows); mode 1: all
-// eigenvectors U = L^-T Q Z into Uout (m x m, column-major; L = I for the
-// standard problem) and the eigenvalues into wout (ascending).
-__device__ void eig_group_solve(const Grp& g, int pi, const EigProb& p, const LgSmem& sh, int mode,
-                                const int* __restrict__ maps, const double* __restrict__ H,
-                                const double* __restrict__ S, double* __restrict__ Ca, double* __restrict__ La,
-                                double* __restrict__ Za, double* __restrict__ Qa, double* __restrict__ Va,
-                                double* __restrict__ Da, double* __restrict__ Ea, double* __restrict__ Ta,
-                                double* __restrict__ Wa, double* __restrict__ Ba, double* __restrict__ Ka,
-                                double* __restrict__ Xa, const int* __restrict__ own_cols, const int* __restrict__ ipos,
-                                double* __restrict__ e_out, double* __restrict__ fe_out, double* __restrict__ Uout,
-                                double* __restrict__ wout, int* __restrict__ status,
-                                unsigned long long* __restrict__ tstage) {
-    double* X = Xa + p.xoff;
-    const int m = p.m;
-    // stage boundaries (global timer, ns) for the print-level-2 stage summary
-    auto mark = [&](int q) {
-        if (tstage && g.rank == 0 && threadIdx.x == 0) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            tstage[(int64_t)pi * kLgStride + q] = t;
-        }
-    };
-    mark(0);
-    lg_gather(g, p, maps, H, S, Ca, La);
-    g.sync();
-    int st = kStOk;
-    if (p.kind == 0) st = lg_potrf(g, m, La + p.aoff, sh);
-    g.sync();
-    mark(1);
-    if (st == kStOk) {
-        if (p.kind == 0) lg_reduce(g, p, La, Ca, sh);
-        mark(2);
-        lg_sytrd(g, p, Ca, Da, Ea, Ta, X, sh, tstage ? tstage + (int64_t)pi * kLgStride + kLgStages : nullptr);
-        g.sync();
-        mark(3);
-        if (!lg_dc(g, p, Da, Ea, Wa, Za, Qa, Va, X, sh)) st = kStNoConv;
-        g.sync();
-        mark(4);
-        if (st == kStOk) {
-            build_T(Ca + p.aoff, m, Ta + p.voff, Ka + p.koff, g.rank, g.size, Va + p.aoff + (int64_t)g.rank * NB * NB,
-                    sh.sD, sh.sA, sh.sB);
-            g.sync();
-            if (mode == 0 && p.mode == 2) {
-                // density: U_occ = L^-T Q Z_occ in place of Z's occupied (lowest)
-                // columns (column ranges per CTA), then the upper tiles of
-                // U_occ U_occ^T split over the group
-                const int no = p.nocc;
-                const int per = (no + g.size - 1) / g.size;
-                const int t0 = min(no, g.rank * per), t1 = min(no, t0 + per);
-                double* Uz = Za + p.aoff;
-                if (t1 > t0) {
-                    double* scr = Qa + p.aoff + (int64_t)g.rank * lg_wy_stride(per);
-                    wy_apply_t(Ca + p.aoff, m, Ka + p.koff, Uz + (int64_t)t0 * m, t1 - t0, false, scr,
-                               scr + (int64_t)NB * per, sh.sA, sh.sB);
-                    __syncthreads();
-                    if (p.kind == 0)
-                        trsm_cols(false, La + p.aoff, m, Uz + (int64_t)t0 * m, m, 0, t1 - t0, sh.sD, sh.sA, sh.sB);
-                }
-                for (int j = g.rank * kT + threadIdx.x; j < m; j += g.size * kT) e_out[p.eoff + j] = Wa[p.voff + j];
-                g.sync();
-                const int nt = (m + TS - 1) / TS;
-                const int ntile = nt * (nt + 1) / 2;
-                double* P = Ba + p.boff;
-                for (int idx = g.rank; idx < ntile; idx += g.size) {
-                    int cb, rb;
-                    tri_decode(idx, cb, rb);   // cb >= rb: upper tiles
-                    tile_mma<false, true, MMA_SET, false>(P, m, 0, nullptr, rb * TS, cb * TS, min(TS, m - rb * TS),
-                                                          min(TS, m - cb * TS), Uz, m, nullptr, Uz, m, nullptr, p.nocc,
-                                                          sh.sA, sh.sB);
-                }
-            } else if (mode == 0) {
-                lg_rows(g, p, Ca, La, Ta, Wa, Za, own_cols, ipos, Ba, Qa, Ka, e_out, fe_out, sh);
-            } else {
-                const int per = (m + g.size - 1) / g.size;
-                const int t0 = min(m, g.rank * per), t1 = min(m, t0 + per);
-                for (int64_t q = (int64_t)t0 * m + threadIdx.x; q < (int64_t)t1 * m; q += kT) Uout[q] = Za[p.aoff + q];
-                __syncthreads();
-                if (t1 > t0) {
-                    double* scr = Qa + p.aoff + (int64_t)g.rank * lg_wy_stride(per);
-                    wy_apply_t(Ca + p.aoff, m, Ka + p.koff, Uout + (int64_t)t0 * m, t1 - t0, false, scr,
-                               scr + (int64_t)NB * per, sh.sA, sh.sB);
-                    __syncthreads();
-                    if (p.kind == 0)
-                        trsm_cols(false, La + p.aoff, m, Uout + (int64_t)t0 * m, m, 0, t1 - t0, sh.sD, sh.sA, sh.sB);
-                }
-                for (int j = g.rank * kT + threadIdx.x; j < m; j += g.size * kT) wout[j] = Wa[p.voff + j];
-            }
-        }
-    }
-    mark(5);
+    const int st = p.kind == 0 ? lg_potrf(g, p.m, La + p.aoff, sh) : kStOk;
     if (g.rank == 0 && threadIdx.x == 0) status[pi] = st;
 }
 
-// One cluster per submatrix above kEigBatchMax (order[] largest first).
-__global__ void __launch_bounds__(kT, 1) k_eig_cluster(
-    const EigProb* __restrict__ probs, const int* __restrict__ order, int M, const int* __restrict__ maps,
-    const double* __restrict__ H, const double* __restrict__ S, double* __restrict__ Ca, double* __restrict__ La,
-    double* __restrict__ Za, double* __restrict__ Qa, double* __restrict__ Va, double* __restrict__ Da,
-    double* __restrict__ Ea, double* __restrict__ Ta, double* __restrict__ Wa, double* __restrict__ Ba,
-    double* __restrict__ Ka, double* __restrict__ Xa, const int* __restrict__ own_cols, const int* __restrict__ ipos,
-    double* __restrict__ e_out, double* __restrict__ fe_out, int* __restrict__ status,
-    unsigned long long* __restrict__ tstage, int mode, double* __restrict__ Uout, double* __restrict__ wout) {
+__global__ void __launch_bounds__(kT, 1) k_lg_trd(const EigProb* __restrict__ probs, const int* __restrict__ order,
+                                                  int M, double* __restrict__ Ca, double* __restrict__ Da,
+                                                  double* __restrict__ Ea, double* __restrict__ Ta,
+                                                  double* __restrict__ Xa, const int* __restrict__ status,
+                                                  unsigned* __restrict__ bar, int* __restrict__ err) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const LgSmem sh = lg_smem(smraw, M);
-    cg::cluster_group cl = cg::this_cluster();
-    const Grp g{(int)cl.block_rank(), (int)cl.num_blocks(), nullptr, nullptr};
-    const int pi = order[blockIdx.x / g.size];
+    const Grp g = lg_group(bar, err);
+    const int pi = order[bar ? 0 : blockIdx.x / g.size];
+    if (status[pi] != kStOk) return;
     const EigProb p = probs[pi];
-    eig_group_solve(g, pi, p, sh, mode, maps, H, S, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Ka, Xa, own_cols, ipos,
-                    e_out, fe_out, Uout, wout, status, tstage);
-}
-
-// One problem on the whole grid of a cooperative launch (software barrier).
-__global__ void __launch_bounds__(kT, 1) k_eig_grid(
-    const EigProb* __restrict__ probs, int pi, int M, int mode, const int* __restrict__ maps,
-    const double* __restrict__ H, const double* __restrict__ S, double* __restrict__ Ca, double* __restrict__ La,
-    double* __restrict__ Za, double* __restrict__ Qa, double* __restrict__ Va, double* __restrict__ Da,
-    double* __restrict__ Ea, double* __restrict__ Ta, double* __restrict__ Wa, double* __restrict__ Ba,
-    double* __restrict__ Ka, double* __restrict__ Xa, const int* __restrict__ own_cols, const int* __restrict__ ipos,
-    double* __restrict__ e_out, double* __restrict__ fe_out, double* __restrict__ Uout, double* __restrict__ wout,
-    int* __restrict__ status, unsigned* __restrict__ bar, int* __restrict__ err) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const LgSmem sh = lg_smem(smraw, M);
-    const Grp g{(int)blockIdx.x, (int)gridDim.x, bar, err};
-    const EigProb p = probs[pi];
-    eig_group_solve(g, pi, p, sh, mode, maps, H, S, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Ka, Xa, own_cols, ipos,
-                    e_out, fe_out, Uout, wout, status, nullptr);
-}
-
-// Owned columns of P_k at mu on the cluster (the large-submatrix form of
-// k_eig_final): W0 = occ o U[c,:], W = Z W0 tiled over the cluster, then each
-// CTA takes a contiguous range of the columns for Q w, L^-T w and the scatter.
-__global__ void __launch_bounds__(kT, 1) k_eig_final_cluster(
-    const EigProb* __restrict__ probs, const int* __restrict__ order, const double* __restrict__ Ca,
-    const double* __restrict__ La, const double* __restrict__ Ta, const double* __restrict__ Wa,
-    const double* __restrict__ Za, double* __restrict__ Qa, const double* __restrict__ Ka,
-    const int* __restrict__ maps, const int* __restrict__ own_cols, double* __restrict__ Ba, double mu,
-    double* __restrict__ Ppk, double* __restrict__ Pdense) {
-    extern __shared__ __align__(16) unsigned char smf[];
-    double* sA = reinterpret_cast<double*>(smf);
-    double* sB = sA + kStageOp;
-    double* sD = sB + kStageOp;
-    double* sT = sD + TS * (TS + 1);
-    cg::cluster_group cl = cg::this_cluster();
-    const Grp g{(int)cl.block_rank(), (int)cl.num_blocks(), nullptr, nullptr};
-    const EigProb p = probs[order[blockIdx.x / g.size]];
-    const int m = p.m, no = p.nown;
-    const double* C = Ca + p.aoff;
-    const double* L = La + p.aoff;
-    const double* Z = Za + p.aoff;
-    const double* tau = Ta + p.voff;
-    const double* ev = Wa + p.voff;
-    double* W0 = Ba + p.boff;
-    const double* U2 = Ba + p.boff + 3 * (int64_t)no * m;
-    double* W = Ba + p.boff + (int64_t)no * m;
-    const int tid = threadIdx.x;
-    for (int64_t q = (int64_t)g.rank * kT + tid; q < (int64_t)no * m; q += (int64_t)g.size * kT) {
-        const int j = (int)(q % m);
-        const double e = ev[j];
-        const double occ = e < mu ? 2.0 : (e == mu ? 1.0 : 0.0);
-        W0[q] = occ * U2[q];
-    }
-    g.sync();
-    {
-        const int ntr = (m + TS - 1) / TS, ntc = (no + TS - 1) / TS;
-        for (int tt = g.rank; tt < ntr * ntc; tt += g.size) {
-            const int r0 = (tt % ntr) * TS, c0 = (tt / ntr) * TS;
-            tile_gemm<false>(W, m, 0, nullptr, r0, c0, min(TS, m - r0), min(TS, no - c0), Z, m, nullptr, W0, m,
-                             nullptr, m, sA, sB);
-        }
-    }
-    g.sync();
-    const int per = (no + g.size - 1) / g.size;
-    const int t0 = min(no, g.rank * per), t1 = min(no, t0 + per);
-    if (t1 > t0) {
-        double* scr = Qa + p.aoff + (int64_t)g.rank * lg_wy_stride(per);
-        wy_apply_t(C, m, Ka + p.koff, W + (int64_t)t0 * m, t1 - t0, false, scr, scr + (int64_t)NB * per, sA, sB);
-        __syncthreads();
-        trsm_cols(false, L, m, W + (int64_t)t0 * m, m, 0, t1 - t0, sD, sA, sB);
-    }
-    if (Pdense) {
-        for (int64_t q = (int64_t)t0 * m + tid; q < (int64_t)t1 * m; q += kT) Pdense[p.poff + q] = W[q];
-        return;
-    }
-    const int* mp = maps + p.moff;
-    for (int64_t q = (int64_t)t0 * m + tid; q < (int64_t)t1 * m; q += kT) {
-        const int t = (int)(q / m), i = (int)(q % m);
-        const int64_t cgl = own_cols[p.o0 + t];
-        const int64_t gi = mp[i];
-        if (gi <= cgl) Ppk[cgl * (cgl + 1) / 2 + gi] = W[q];
-    }
+    lg_sytrd(g, p, Ca, Da, Ea, Ta, Xa + p.xoff, sh);
 }
 
 }  // namespace
 
+// Streams and events of a context's eigensolver calls: the large problems' chains run
+// on `side` beside the small ones' on the call's stream.
+struct EigStreams {
+    cudaStream_t side = nullptr, base = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
+    EigStreams() {
+        PTB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        PTB_CUDA(cudaStreamCreateWithFlags(&base, cudaStreamNonBlocking));
+        for (cudaEvent_t* e : {&fork, &join, &done}) PTB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    }
+    ~EigStreams() {
+        for (cudaEvent_t e : {fork, join, done})
+            if (e) cudaEventDestroy(e);
+        for (cudaStream_t s : {side, base})
+            if (s) cudaStreamDestroy(s);
+    }
+};
+
 struct EigBatch {
+    struct Seg {   // a run of a task list
+        size_t off = 0;
+        unsigned n = 0;
+    };
+    struct Level {   // one level of the divide and conquer
+        int m0 = 0, nm = 0;
+        Seg permute, elems, product;
+    };
     int nprob = 0;
-    int maxm = 0;
-    int G = 1;                    // CTAs per cluster of the large-submatrix solver
-    int nsmall = 0, nlarge = 0;
+    int G = 1;                    // CTAs per cluster of the large problems
+    int nsmall = 0, nlarge = 0, n512 = 0, maxlarge = 0;
+    bool grid = false;            // one problem on a cooperative grid
     std::vector<EigProb> hp;
-    WorkBuf probs, order, order_l, counter, tasks, Ca, La, Za, Qa, Va, Da, Ea, Ta, Wa, Ba, Xa, Ka, status, tstage;
+    std::vector<int> order;       // small problems first, each part largest first
+    std::vector<int2> lists;
+    std::vector<DcMerge> merges;
+    std::vector<Level> levels;
+    Seg blocks, leaves, panels, rows, rq, back, density, fblocks, frq, fcols;
+    WorkBuf probs, order_d, lists_d, merges_d, cnt, dc, Ca, La, Za, Qa, Va, Da, Ea, Ta, Ba, Xa, Ka, status;
+    DcArr S{};
+    double* Z = nullptr;          // the Z arena (Za, or the caller's array)
     int prl = 0;
     const char* what = "submatrix";   // the problems' name in error messages
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    std::shared_ptr<EigStreams> st;
+    bool async = false;           // launched on st->base
     ~EigBatch() {
-        // the arrays go back to the context's pool: nothing on the side stream may
+        // the arrays go back to the context's pool: nothing on the side streams may
         // still use them (work on the context's stream is ordered before their next use)
-        if (side) cudaStreamSynchronize(side);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        if (side) cudaStreamDestroy(side);
+        if (st) {
+            cudaStreamSynchronize(st->side);
+            cudaStreamSynchronize(st->base);
+        }
     }
+    const int2* list(const Seg& g) const { return lists_d.as<int2>() + g.off; }
 };
 
 namespace {
 
+template <class K>
+void smem_attr(K kern, size_t bytes) {
+    PTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 void eig_setup_attrs() {
     static const bool done = [] {
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)stage_smem_bytes(kEigBatchMax)));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_chol, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)stage_smem_bytes(2)));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_trd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kTrdCap512));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_trd<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kTrdCap256));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)lg_smem_bytes(kLargeMax)));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_final_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_final_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFinalSmem));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)lg_smem_bytes(kLargeMax)));
-        PTB_CUDA(cudaFuncSetAttribute(k_eig_final, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFinalSmem));
+        smem_attr(k_eig_chol, kCholSmem);
+        smem_attr(k_eig_trsm, kTrsmSmem);
+        smem_attr(k_eig_trd<512>, 8 * kTrdCap512);
+        smem_attr(k_eig_trd<256>, 8 * kTrdCap256);
+        smem_attr(k_lg_chol, lg_smem_bytes(2));
+        smem_attr(k_lg_trd, lg_smem_bytes(kLargeMax));
+        smem_attr(k_dc_product, kTileSmem);
+        smem_attr(k_vec_panels, kWySmem);
+        smem_attr(k_vec_rq, kTileSmem);
+        smem_attr(k_vec_rv, kTileSmem);
+        smem_attr(k_fin_vw, kTileSmem);
+        smem_attr(k_fin_qw, kTileSmem);
+        smem_attr(k_vec_density, kTileSmem);
+        smem_attr(k_vec_rows, kChainSmem);
+        smem_attr(k_vec_back, kChainSmem);
+        smem_attr(k_fin_cols, kChainSmem);
+        PTB_CUDA(cudaFuncSetAttribute(k_lg_chol, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        PTB_CUDA(cudaFuncSetAttribute(k_lg_trd, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         return true;
     }();
     (void)done;
@@ -2595,7 +1233,7 @@ int eig_active_clusters(int G) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, (void*)k_eig_cluster, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&ncl, (void*)k_lg_trd, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -2672,23 +1310,304 @@ void launch_clustered(K kern, int nclusters, int G, size_t smem, cudaStream_t s,
     PTB_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
+
+EigStreams& eig_streams(ptbgpu_ctx* c, EigBatch& eb) {
+    if (!c->eig_streams) c->eig_streams = std::make_shared<EigStreams>();
+    eb.st = std::static_pointer_cast<EigStreams>(c->eig_streams);
+    return *eb.st;
+}
+
+// Arenas, task lists and uploads of a batch (on stream s).  hp holds the problems
+// (k, m, nown, kind, mode, nocc, moff, eoff, o0, gbase, gld); Uout: Z's place for a
+// single problem whose vectors the caller wants.
+void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double* Uout) {
+    eig_setup_attrs();
+    const int np = eb.nprob = (int)eb.hp.size();
+    std::vector<int> large;
+    for (int q = 0; q < np; ++q) (eb.hp[q].m > small_max ? large : eb.order).push_back(q);
+    auto by_size = [&](int a, int b) { return eb.hp[a].m > eb.hp[b].m; };
+    std::stable_sort(eb.order.begin(), eb.order.end(), by_size);
+    std::stable_sort(large.begin(), large.end(), by_size);
+    eb.nsmall = (int)eb.order.size();
+    eb.nlarge = (int)large.size();
+    eb.maxlarge = large.empty() ? 0 : eb.hp[large[0]].m;
+    if (eb.nlarge > 0 && !eb.grid) eb.G = eig_batch_cluster_size(c, eb.nlarge);
+    const int nsm = c->num_sms > 0 ? c->num_sms : 148;
+    for (int q : eb.order) eb.n512 += eb.hp[q].m > kTrdMax256;
+    // two CTAs per SM only pay where the small orders fill the SMs
+    if (eb.nsmall - eb.n512 <= nsm) eb.n512 = eb.nsmall;
+
+    int64_t asz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0;
+    for (int q = 0; q < np; ++q) {
+        EigProb& p = eb.hp[q];
+        p.poff = psz;
+        psz += (int64_t)p.m * p.nown;
+        p.aoff = asz;
+        p.voff = vsz;
+        p.boff = bsz;
+        p.xoff = xsz;
+        p.koff = ksz;
+        p.topm = -1;
+        ksz += t_panels(p.m) * NB * NB;
+        asz += (int64_t)p.m * p.m;
+        vsz += p.m;
+        bsz += p.mode == 2 ? (int64_t)p.m * p.m : 4 * (int64_t)p.nown * p.m;
+        if (p.m > small_max) xsz += lg_layout(p.m, eb.G).total;
+    }
+    // task lists, largest problems first in each
+    std::vector<int> all(large);
+    all.insert(all.end(), eb.order.begin(), eb.order.end());
+    eb.order.insert(eb.order.end(), large.begin(), large.end());
+    auto list = [&](EigBatch::Seg& g, auto&& fill) {
+        g.off = eb.lists.size();
+        fill();
+        g.n = (unsigned)(eb.lists.size() - g.off);
+    };
+    auto put = [&](int a, int b) { eb.lists.push_back(make_int2(a, b)); };
+    auto tiles = [](int n) { return (n + TS - 1) / TS; };
+    list(eb.blocks, [&] {   // 64-column blocks (64-element chunks) of the generalized problems
+        for (int q : all)
+            for (int b = 0; b < tiles(eb.hp[q].m); ++b) put(q, b);
+    });
+    list(eb.leaves, [&] {
+        for (int q : all)
+            for (int b = 0; b < (1 << dc_levels(eb.hp[q].m)); ++b) put(q, b);
+    });
+    list(eb.panels, [&] {
+        for (int q : all)
+            for (int b = 0; b < (int)t_panels(eb.hp[q].m); ++b) put(q, b);
+    });
+    auto grid2 = [&](int q, int nr, int nc) {
+        for (int a = 0; a < nr; ++a)
+            for (int b = 0; b < nc; ++b) put(q, a << 16 | b);
+    };
+    auto vectors = [&](auto&& count) {   // 64-vector blocks of every problem
+        for (int q : all)
+            for (int b = 0; b < tiles(count(eb.hp[q])); ++b) put(q, b);
+    };
+    list(eb.rows, [&] { vectors([](const EigProb& p) { return p.mode == 0 ? 2 * p.nown : 0; }); });
+    list(eb.back, [&] {
+        vectors([](const EigProb& p) { return p.mode == 0 ? 0 : p.mode == 1 ? p.m : p.nocc; });
+    });
+    list(eb.rq, [&] {
+        for (int q : all)
+            if (eb.hp[q].mode == 0) grid2(q, tiles(eb.hp[q].m), tiles(2 * eb.hp[q].nown));
+    });
+    list(eb.frq, [&] {
+        for (int q : all)
+            if (eb.hp[q].mode == 0) grid2(q, tiles(eb.hp[q].m), tiles(eb.hp[q].nown));
+    });
+    list(eb.fcols, [&] { vectors([](const EigProb& p) { return p.mode == 0 ? p.nown : 0; }); });
+    list(eb.density, [&] {
+        for (int q : all)
+            if (eb.hp[q].mode == 2)   // no occupied vectors: tiles of zeros
+                for (int cb = 0; cb < tiles(eb.hp[q].m); ++cb)
+                    for (int rb = 0; rb <= cb; ++rb) put(q, rb << 16 | cb);
+    });
+    list(eb.fblocks, [&] {
+        for (int q : all)
+            if (eb.hp[q].mode == 0)
+                for (int b = 0; b < tiles(eb.hp[q].m); ++b) put(q, b);
+    });
+    int nlev = 0;
+    for (int q : all) nlev = std::max(nlev, dc_levels(eb.hp[q].m));
+    eb.levels.resize(nlev);
+    for (int t = 0; t < nlev; ++t) {
+        EigBatch::Level& lv = eb.levels[t];
+        lv.m0 = (int)eb.merges.size();
+        for (int q : all) {
+            EigProb& p = eb.hp[q];
+            const int lev = dc_levels(p.m) - 1 - t;
+            if (lev < 0) continue;
+            for (int b = 0; b < (1 << lev); ++b) {
+                if (lev == 0) p.topm = (int)eb.merges.size();
+                eb.merges.push_back({q, dc_start(p.m, b, lev), dc_start(p.m, 2 * b + 1, lev + 1), dc_start(p.m, b + 1, lev)});
+            }
+        }
+        lv.nm = (int)eb.merges.size() - lv.m0;
+        auto each = [&](auto&& f) {
+            for (int i = lv.m0; i < lv.m0 + lv.nm; ++i) f(i, eb.merges[i]);
+        };
+        list(lv.permute, [&] {
+            each([&](int i, const DcMerge& g) {
+                for (int b = 0; b * kDcRows < g.hi - g.lo; ++b) put(i, b);
+            });
+        });
+        list(lv.elems, [&] {
+            each([&](int i, const DcMerge& g) {
+                for (int b = 0; b * kDcChunk < g.hi - g.lo; ++b) put(i, b);
+            });
+        });
+        list(lv.product, [&] {
+            each([&](int i, const DcMerge& g) {
+                const EigProb& p = eb.hp[g.pi];
+                if (p.mode == 0 && i == p.topm) return;   // its Q and V are used as they are
+                grid2(i, tiles(g.mid - g.lo) + tiles(g.hi - g.mid), tiles(g.hi - g.lo));
+            });
+        });
+    }
+
+    eb.probs.reserve(c, sizeof(EigProb) * np);
+    eb.order_d.reserve(c, sizeof(int) * np);
+    eb.lists_d.reserve(c, sizeof(int2) * std::max<size_t>(eb.lists.size(), 1));
+    eb.merges_d.reserve(c, sizeof(DcMerge) * std::max<size_t>(eb.merges.size(), 1));
+    eb.cnt.reserve(c, 8 * sizeof(int) * std::max<size_t>(eb.merges.size(), 1));
+    const int64_t vpad = (vsz + 1) & ~int64_t(1);
+    eb.dc.reserve(c, kDcBytes * vpad);
+    eb.S = dc_arrays(eb.dc.ptr, vpad, eb.cnt.as<int>());
+    for (WorkBuf* b : {&eb.Ca, &eb.La, &eb.Qa, &eb.Va}) b->reserve(c, sizeof(double) * asz);
+    if (!Uout) eb.Za.reserve(c, sizeof(double) * asz);
+    eb.Z = Uout ? Uout : eb.Za.as<double>();
+    for (WorkBuf* b : {&eb.Da, &eb.Ea, &eb.Ta}) b->reserve(c, sizeof(double) * vsz);
+    eb.Ba.reserve(c, sizeof(double) * std::max<int64_t>(bsz, 1));
+    eb.Xa.reserve(c, sizeof(double) * std::max<int64_t>(xsz, 2));
+    eb.Ka.reserve(c, sizeof(double) * std::max<int64_t>(ksz, 2));
+    eb.status.reserve(c, sizeof(int) * (np + 3));   // and a grid barrier's count, generation and error
+    PTB_CUDA(cudaMemcpyAsync(eb.probs.ptr, eb.hp.data(), sizeof(EigProb) * np, cudaMemcpyHostToDevice, s));
+    PTB_CUDA(cudaMemcpyAsync(eb.order_d.ptr, eb.order.data(), sizeof(int) * np, cudaMemcpyHostToDevice, s));
+    PTB_CUDA(cudaMemcpyAsync(eb.lists_d.ptr, eb.lists.data(), sizeof(int2) * eb.lists.size(), cudaMemcpyHostToDevice, s));
+    if (!eb.merges.empty())
+        PTB_CUDA(cudaMemcpyAsync(eb.merges_d.ptr, eb.merges.data(), sizeof(DcMerge) * eb.merges.size(),
+                                 cudaMemcpyHostToDevice, s));
+    PTB_CUDA(cudaMemsetAsync(eb.status.ptr, 0, sizeof(int) * (np + 3), s));
+}
+
+// Every stage up to the eigenvalues, fe and owned rows (mode 0), all vectors (mode 1)
+// or the densities (mode 2) on stream s.
+void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const double* S, const int* d_maps,
+             const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe) {
+    const EigProb* dp = eb.probs.as<EigProb>();
+    const int *ord = eb.order_d.as<int>(), *ord_l = ord + eb.nsmall;
+    const DcMerge* mg = eb.merges_d.as<DcMerge>();
+    double *Ca = eb.Ca.as<double>(), *La = eb.La.as<double>(), *Za = eb.Z, *Qa = eb.Qa.as<double>(),
+           *Va = eb.Va.as<double>(), *Da = eb.Da.as<double>(), *Ea = eb.Ea.as<double>(), *Ta = eb.Ta.as<double>(),
+           *Ba = eb.Ba.as<double>(), *Xa = eb.Xa.as<double>(), *Ka = eb.Ka.as<double>();
+    int* st = eb.status.as<int>();
+    const DcArr& D = eb.S;
+    unsigned* bar = eb.grid ? reinterpret_cast<unsigned*>(st + eb.nprob) : nullptr;
+    int* err = eb.grid ? st + eb.nprob + 2 : nullptr;
+    // the large problems' chains beside the small ones', joined before the next stage
+    EigStreams* es = eb.nsmall > 0 && eb.nlarge > 0 ? &eig_streams(c, eb) : nullptr;
+    auto fork = [&]() -> cudaStream_t {
+        if (!es) return s;
+        PTB_CUDA(cudaEventRecord(es->fork, s));
+        PTB_CUDA(cudaStreamWaitEvent(es->side, es->fork, 0));
+        return es->side;
+    };
+    auto join = [&] {
+        if (!es) return;
+        PTB_CUDA(cudaEventRecord(es->join, es->side));
+        PTB_CUDA(cudaStreamWaitEvent(s, es->join, 0));
+    };
+    auto launched = [&](int k = 1) {
+        count_launch(k);
+        PTB_CUDA(cudaGetLastError());
+    };
+    // ---- Cholesky
+    if (eb.nlarge > 0) {
+        const cudaStream_t ls = fork();
+        if (eb.grid) {
+            void* args[] = {&dp, &ord_l, &d_maps, &H, &S, &Ca, &Qa, &La, &st, &bar, &err};
+            PTB_CUDA(cudaLaunchCooperativeKernel((void*)k_lg_chol, dim3(eb.G), dim3(kT), args, lg_smem_bytes(2), ls));
+        } else {
+            launch_clustered(k_lg_chol, eb.nlarge, eb.G, lg_smem_bytes(2), ls, dp, ord_l, d_maps, H, S, Ca, Qa, La, st,
+                             bar, err);
+        }
+        launched();
+    }
+    if (eb.nsmall > 0) {
+        k_eig_chol<<<eb.nsmall, kT, kCholSmem, s>>>(dp, ord, d_maps, H, S, Qa, La, st);
+        launched();
+    }
+    join();
+    // ---- C = L^-1 H L^-T
+    if (eb.hp[0].kind == 0) {
+        const int2* bl = eb.list(eb.blocks);
+        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Qa, st);
+        k_eig_transpose<<<eb.blocks.n, 256, 0, s>>>(dp, bl, Qa, Ca, st);
+        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Ca, st);
+        launched(3);
+    }
+    // ---- tridiagonalisation
+    if (eb.nlarge > 0) {
+        const cudaStream_t ls = fork();
+        int M = (eb.maxlarge + 1) & ~1;
+        if (eb.grid) {
+            void* args[] = {&dp, &ord_l, &M, &Ca, &Da, &Ea, &Ta, &Xa, &st, &bar, &err};
+            PTB_CUDA(cudaLaunchCooperativeKernel((void*)k_lg_trd, dim3(eb.G), dim3(kT), args, lg_smem_bytes(M), ls));
+        } else {
+            launch_clustered(k_lg_trd, eb.nlarge, eb.G, lg_smem_bytes(M), ls, dp, ord_l, M, Ca, Da, Ea, Ta, Xa,
+                             (const int*)st, bar, err);
+        }
+        launched();
+    }
+    if (eb.n512 > 0) {
+        k_eig_trd<512><<<eb.n512, 512, sizeof(double) * kTrdCap512, s>>>(dp, ord, Ca, Da, Ea, Ta, st);
+        launched();
+    }
+    if (eb.n512 < eb.nsmall) {
+        k_eig_trd<256><<<eb.nsmall - eb.n512, 256, sizeof(double) * kTrdCap256, s>>>(dp, ord + eb.n512, Ca, Da, Ea, Ta,
+                                                                                     st);
+        launched();
+    }
+    join();
+    // ---- reflector panels, and the owned rows up to Z
+    if (eb.panels.n) {
+        k_vec_panels<<<eb.panels.n, kT, kWySmem, s>>>(dp, eb.list(eb.panels), Ca, Ta, Ka, st);
+        launched();
+    }
+    if (eb.rows.n) {
+        k_vec_rows<<<eb.rows.n, kT, kChainSmem, s>>>(dp, eb.list(eb.rows), Ca, La, Ka, d_own_cols, d_ipos, Ba, st);
+        launched();
+    }
+    // ---- divide and conquer
+    k_dc_leaves<<<(eb.leaves.n + kLeafWarps - 1) / kLeafWarps, 32 * kLeafWarps, 0, s>>>(
+        dp, eb.list(eb.leaves), (int)eb.leaves.n, Da, Ea, Za, D, st);
+    launched();
+    for (const EigBatch::Level& lv : eb.levels) {
+        const int2* el = eb.list(lv.elems);
+        k_dc_deflate<<<lv.nm, kDeflT, 0, s>>>(dp, mg, lv.m0, Ea, Za, D, st);
+        k_dc_permute<<<lv.permute.n, 256, 0, s>>>(dp, mg, eb.list(lv.permute), Za, Qa, D, st);
+        k_dc_secular<<<lv.elems.n, 256, 0, s>>>(dp, mg, el, Ea, D, st);
+        k_dc_zhat<<<lv.elems.n, 256, 0, s>>>(dp, mg, el, Ea, D, st);
+        k_dc_vectors<<<lv.elems.n, 256, 0, s>>>(dp, mg, el, Va, D, st);
+        launched(5);
+        if (lv.product.n) {
+            k_dc_product<<<lv.product.n, kT, kTileSmem, s>>>(dp, mg, eb.list(lv.product), Za, Qa, Va, D, st);
+            launched();
+        }
+    }
+    // ---- what leaves the solver
+    if (eb.rq.n) {
+        const int2* rq = eb.list(eb.rq);
+        k_vec_rq<<<eb.rq.n, kT, kTileSmem, s>>>(dp, rq, Za, Qa, Va, D, Ba, st);
+        k_vec_rv<<<eb.rq.n, kT, kTileSmem, s>>>(dp, rq, Za, Qa, Va, D, Ba, st);
+        k_vec_fe<<<eb.fblocks.n, 256, 0, s>>>(dp, eb.list(eb.fblocks), Ba, D, d_e, d_fe, st);
+        launched(3);
+    }
+    if (eb.hp[0].mode != 0) {
+        k_vec_values<<<eb.blocks.n, TS, 0, s>>>(dp, eb.list(eb.blocks), D, d_e, st);
+        launched();
+    }
+    if (eb.back.n) {
+        k_vec_back<<<eb.back.n, kT, kChainSmem, s>>>(dp, eb.list(eb.back), Ca, La, Ka, Za, st);
+        launched();
+    }
+    if (eb.density.n) {
+        k_vec_density<<<eb.density.n, kT, kTileSmem, s>>>(dp, eb.list(eb.density), Za, Ba, st);
+        launched();
+    }
+}
+
 }  // namespace
 
 std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const double* H, const double* S,
                                            const std::vector<EigProbHost>& probs, const int* d_maps,
-                                            const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe,
-                                            int prl, double* flops, bool join) {
+                                           const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe,
+                                           int prl, double* flops, bool join) {
     if (probs.empty()) return nullptr;
-    eig_setup_attrs();
-    cudaStream_t s = c->stream;
     auto eb = std::make_shared<EigBatch>();
-    eb->nprob = (int)probs.size();
     eb->prl = prl;
-    int nlarge = 0;
-    for (const EigProbHost& q : probs) nlarge += q.m > kEigBatchMax ? 1 : 0;
-    eb->G = nlarge > 0 ? eig_batch_cluster_size(c, nlarge) : 1;
-    int64_t asz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0;
-    std::vector<int> ord_s, ord_l;
     for (const EigProbHost& q : probs) {
         PTB_CHECK(q.m >= 1 && q.m <= kLargeMax, PTBGPU_EINVAL, "submatrix %d of order %d outside the eigensolver (1..%d)",
                   q.k + 1, q.m, kLargeMax);
@@ -2703,194 +1622,61 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
         p.gld = q.gld < 0 ? n : q.gld;
         p.mode = q.mode;
         p.nocc = q.nocc;
-        p.poff = psz;
-        psz += (int64_t)q.m * q.nown;
-        p.aoff = asz;
-        p.voff = vsz;
-        p.boff = bsz;
-        p.xoff = xsz;
-        p.koff = ksz;
-        ksz += t_panels(q.m) * NB * NB;
-        asz += (int64_t)q.m * q.m;
-        vsz += q.m;
-        bsz += q.mode == 2 ? (int64_t)q.m * q.m : 4 * (int64_t)q.nown * q.m;
-        if (q.m > kEigBatchMax) {
-            xsz += lg_layout(q.m, eb->G).total;
-            ord_l.push_back((int)eb->hp.size());
-        } else {
-            ord_s.push_back((int)eb->hp.size());
-        }
-        eb->maxm = std::max(eb->maxm, q.m);
         eb->hp.push_back(p);
         if (flops) *flops += 7.0 * std::pow((double)q.m, 3);
     }
-    const int np = eb->nprob;
-    eb->nsmall = (int)ord_s.size();
-    eb->nlarge = (int)ord_l.size();
-    eb->probs.reserve(c, sizeof(EigProb) * np);
-    for (WorkBuf* b : {&eb->Ca, &eb->La, &eb->Za, &eb->Qa, &eb->Va}) b->reserve(c, sizeof(double) * asz);
-    for (WorkBuf* b : {&eb->Da, &eb->Ea, &eb->Ta, &eb->Wa}) b->reserve(c, sizeof(double) * vsz);
-    eb->Ba.reserve(c, sizeof(double) * std::max<int64_t>(bsz, 1));
-    eb->Xa.reserve(c, sizeof(double) * std::max<int64_t>(xsz, 2));
-    eb->Ka.reserve(c, sizeof(double) * std::max<int64_t>(ksz, 2));
-    eb->status.reserve(c, sizeof(int) * np);
-    PTB_CUDA(cudaMemcpyAsync(eb->probs.ptr, eb->hp.data(), sizeof(EigProb) * np, cudaMemcpyHostToDevice, s));
-    PTB_CUDA(cudaMemsetAsync(eb->status.ptr, 0, sizeof(int) * np, s));
-    const EigProb* dp = eb->probs.as<EigProb>();
-    int* dst = eb->status.as<int>();
-
-    // largest first, so that the small submatrices fill in around the large ones
-    auto by_size = [&](int a, int b) { return eb->hp[a].m > eb->hp[b].m; };
-    std::stable_sort(ord_s.begin(), ord_s.end(), by_size);
-    std::stable_sort(ord_l.begin(), ord_l.end(), by_size);
-    eb->order.reserve(c, sizeof(int) * std::max<size_t>(ord_s.size(), 1));
-    eb->order_l.reserve(c, sizeof(int) * std::max<size_t>(ord_l.size(), 1));
-    eb->counter.reserve(c, sizeof(int));
-    if (!ord_s.empty())
-        PTB_CUDA(cudaMemcpyAsync(eb->order.ptr, ord_s.data(), sizeof(int) * ord_s.size(), cudaMemcpyHostToDevice, s));
-    if (!ord_l.empty())
-        PTB_CUDA(cudaMemcpyAsync(eb->order_l.ptr, ord_l.data(), sizeof(int) * ord_l.size(), cudaMemcpyHostToDevice, s));
-    PTB_CUDA(cudaMemsetAsync(eb->counter.ptr, 0, sizeof(int), s));
-    // the large submatrices on their clusters (a side stream, launched first so
-    // their clusters find free SMs), the small ones in the persistent launch
-    if (eb->nlarge > 0) {
-        PTB_CUDA(cudaStreamCreateWithFlags(&eb->side, cudaStreamNonBlocking));
-        PTB_CUDA(cudaEventCreateWithFlags(&eb->ev0, cudaEventDisableTiming));
-        PTB_CUDA(cudaEventCreateWithFlags(&eb->ev1, cudaEventDisableTiming));
-        unsigned long long* dts = nullptr;
-        if (prl >= 2) {
-            eb->tstage.reserve(c, sizeof(unsigned long long) * kLgStride * np);
-            PTB_CUDA(cudaMemsetAsync(eb->tstage.ptr, 0, sizeof(unsigned long long) * kLgStride * np, s));
-            dts = eb->tstage.as<unsigned long long>();
-        }
-        PTB_CUDA(cudaEventRecord(eb->ev0, s));
-        PTB_CUDA(cudaStreamWaitEvent(eb->side, eb->ev0, 0));
-        launch_clustered(k_eig_cluster, eb->nlarge, eb->G, lg_smem_bytes(kLargeMax), eb->side, dp,
-                         (const int*)eb->order_l.as<int>(), kLargeMax, d_maps, H, S, eb->Ca.as<double>(),
-                         eb->La.as<double>(), eb->Za.as<double>(), eb->Qa.as<double>(), eb->Va.as<double>(),
-                         eb->Da.as<double>(), eb->Ea.as<double>(), eb->Ta.as<double>(), eb->Wa.as<double>(),
-                         eb->Ba.as<double>(), eb->Ka.as<double>(), eb->Xa.as<double>(), d_own_cols, d_ipos, d_e, d_fe,
-                         dst, dts, 0, (double*)nullptr, (double*)nullptr);
-        count_launch();
-        PTB_CUDA(cudaEventRecord(eb->ev1, eb->side));
-        log_line(prl, 2, " * submatrix cluster eigensolver: %d problems above order %d, clusters of %d CTAs",
-                 eb->nlarge, kEigBatchMax, eb->G);
+    cudaStream_t s = c->stream;
+    if (!join) {
+        // beside what follows on the context's stream
+        EigStreams& es = eig_streams(c, *eb);
+        PTB_CUDA(cudaEventRecord(es.fork, s));
+        PTB_CUDA(cudaStreamWaitEvent(es.base, es.fork, 0));
+        s = es.base;
+        eb->async = true;
     }
-    if (eb->nsmall > 0) {
-        int Msmall = 0;
-        std::vector<int2> tasks;
-        int n512 = 0;   // problems of the one-CTA-per-SM tridiagonalisation
-        for (int q : ord_s) {
-            const int m = eb->hp[q].m;
-            Msmall = std::max(Msmall, m);
-            for (int cb = 0; cb * TS < m; ++cb) tasks.push_back(make_int2(q, cb));
-            if (m > kTrdMax256) ++n512;
-        }
-        const int nsm = c->num_sms > 0 ? c->num_sms : 148;
-        // two CTAs per SM only pay where the small orders fill the SMs
-        if (eb->nsmall - n512 <= nsm) n512 = eb->nsmall;
-        eb->tasks.reserve(c, sizeof(int2) * tasks.size());
-        PTB_CUDA(cudaMemcpyAsync(eb->tasks.ptr, tasks.data(), sizeof(int2) * tasks.size(), cudaMemcpyHostToDevice, s));
-        const int2* dt = eb->tasks.as<int2>();
-        const int* ord = eb->order.as<int>();
-        const unsigned nt = (unsigned)tasks.size();
-        double *Ca = eb->Ca.as<double>(), *La = eb->La.as<double>(), *Qa = eb->Qa.as<double>();
-        double *Da = eb->Da.as<double>(), *Ea = eb->Ea.as<double>(), *Ta = eb->Ta.as<double>();
-        k_eig_chol<<<eb->nsmall, kT, stage_smem_bytes(2), s>>>(dp, ord, d_maps, H, S, Qa, La, dst);
-        k_eig_trsm<<<nt, kT, kTrsmSmem, s>>>(dp, dt, La, Qa, dst);
-        k_eig_transpose<<<nt, 256, 0, s>>>(dp, dt, Qa, Ca, dst);
-        k_eig_trsm<<<nt, kT, kTrsmSmem, s>>>(dp, dt, La, Ca, dst);
-        if (n512 > 0)
-            k_eig_trd<512><<<n512, 512, sizeof(double) * kTrdCap512, s>>>(dp, ord, Ca, Da, Ea, Ta, dst);
-        if (n512 < eb->nsmall)
-            k_eig_trd<256><<<eb->nsmall - n512, 256, sizeof(double) * kTrdCap256, s>>>(dp, ord + n512, Ca, Da, Ea, Ta,
-                                                                                       dst);
-        const int Ms = (Msmall + 1) & ~1;   // staging sized for the largest small problem
-        const int grid = std::min(eb->nsmall, nsm);
-        k_eig_vectors<<<grid, kT, stage_smem_bytes(Ms), s>>>(
-            dp, ord, eb->nsmall, eb->counter.as<int>(), Ms, Ca, La, eb->Za.as<double>(), Qa, eb->Va.as<double>(), Da,
-            Ea, Ta, eb->Wa.as<double>(), eb->Ba.as<double>(), eb->Ka.as<double>(), d_own_cols, d_ipos, d_e, d_fe, dst);
-        count_launch(6 + (n512 > 0 && n512 < eb->nsmall));
-        PTB_CUDA(cudaGetLastError());
-    }
-    if (eb->nlarge > 0 && join) PTB_CUDA(cudaStreamWaitEvent(s, eb->ev1, 0));
+    eig_plan(c, *eb, s, kEigBatchMax, nullptr);
+    log_line(prl, 2, " * eigensolver: %d problems, %d above order %d on clusters of %d CTAs, %zu merge levels", eb->nprob,
+             eb->nlarge, kEigBatchMax, eb->G, eb->levels.size());
+    eig_run(c, *eb, s, H, S, d_maps, d_own_cols, d_ipos, d_e, d_fe);
+    if (eb->async) PTB_CUDA(cudaEventRecord(eb->st->done, s));
     return eb;
 }
 
 void eig_batch_join(ptbgpu_ctx* c, EigBatch& eb) {
-    if (eb.nlarge > 0 && eb.ev1) PTB_CUDA(cudaStreamWaitEvent(c->stream, eb.ev1, 0));
+    if (eb.async) PTB_CUDA(cudaStreamWaitEvent(c->stream, eb.st->done, 0));
 }
 
 void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb) {
     cudaStream_t s = c->stream;
     const int np = eb.nprob;
-    std::vector<int> hst(np);
-    PTB_CUDA(cudaMemcpyAsync(hst.data(), eb.status.ptr, sizeof(int) * np, cudaMemcpyDeviceToHost, s));
+    std::vector<int> hst(np + 3);
+    PTB_CUDA(cudaMemcpyAsync(hst.data(), eb.status.ptr, sizeof(int) * (np + 3), cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
+    PTB_CHECK(hst[np + 2] == 0, PTBGPU_ETIMEOUT, "eigensolver: a grid barrier gave up waiting");
     for (int q = 0; q < np; ++q)
         PTB_CHECK(hst[q] <= 0, PTBGPU_ENOTSPD, "overlap of %s %d not positive definite (leading minor %d)", eb.what,
                   eb.hp[q].k + 1, hst[q]);
     for (int q = 0; q < np; ++q)
         PTB_CHECK(hst[q] == kStOk, PTBGPU_EITER, "tridiagonal eigensolver did not converge on %s %d", eb.what,
                   eb.hp[q].k + 1);
-    if (eb.prl >= 2 && eb.nlarge > 0 && eb.tstage.ptr) {
-        // per stage: summed over the large submatrices and the longest one, then
-        // the span from the first cluster's start to the last one's end
-        std::vector<unsigned long long> ts((size_t)kLgStride * np);
-        PTB_CUDA(cudaMemcpy(ts.data(), eb.tstage.ptr, sizeof(unsigned long long) * ts.size(), cudaMemcpyDeviceToHost));
-        static const char* names[kLgStages - 1] = {"gather + Cholesky", "reduction", "tridiagonalisation",
-                                                   "divide and conquer", "owned rows"};
-        double sum[kLgStages - 1] = {}, mx[kLgStages - 1] = {};
-        unsigned long long t_lo = ~0ull, t_hi = 0;
-        for (int q = 0; q < np; ++q) {
-            if (eb.hp[q].m <= kEigBatchMax) continue;
-            const unsigned long long* t = &ts[(size_t)q * kLgStride];
-            t_lo = std::min(t_lo, t[0]);
-            t_hi = std::max(t_hi, t[kLgStages - 1]);
-            for (int k = 0; k + 1 < kLgStages; ++k) {
-                const double d = (t[k + 1] >= t[k] && t[k] != 0) ? (double)(t[k + 1] - t[k]) * 1e-6 : 0.0;
-                sum[k] += d;
-                mx[k] = std::max(mx[k], d);
-            }
-        }
-        for (int k = 0; k + 1 < kLgStages; ++k)
-            log_line(eb.prl, 2, " * cluster eigensolver %-22s sum %10.3f ms, longest %9.3f ms", names[k], sum[k], mx[k]);
-        static const char* sub[kLgSub] = {"column update", "barrier 1", "reflector", "A v tiles", "A v partials",
-                                          "barrier 2", "panel end"};
-        for (int k = 0; k < kLgSub; ++k) {
-            double t = 0.0;
-            for (int q = 0; q < np; ++q)
-                if (eb.hp[q].m > kEigBatchMax) t += (double)ts[(size_t)q * kLgStride + kLgStages + k] * 1e-6;
-            log_line(eb.prl, 2, " *   tridiagonalisation %-14s sum %10.3f ms", sub[k], t);
-        }
-        log_line(eb.prl, 2, " * cluster eigensolver span %10.3f ms (%d submatrices, clusters of %d)",
-                 t_hi > t_lo ? (double)(t_hi - t_lo) * 1e-6 : 0.0, eb.nlarge, eb.G);
-    }
 }
 
 void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, int64_t n, const int* d_maps, const int* d_own_cols,
                      double* dP, double* dPdense) {
     (void)n;
-    if (eb.nprob == 0) return;
+    if (eb.nprob == 0 || eb.fcols.n == 0) return;
     cudaStream_t s = c->stream;
-    if (eb.nsmall > 0) {
-        eig_setup_attrs();
-        k_eig_final<<<eb.nsmall, kT, kFinalSmem, s>>>(eb.probs.as<EigProb>(), eb.order.as<int>(), eb.Ca.as<double>(),
-                                                      eb.La.as<double>(), eb.Ta.as<double>(), eb.Wa.as<double>(),
-                                                      eb.Za.as<double>(), eb.Qa.as<double>(), eb.Va.as<double>(),
-                                                      eb.Ka.as<double>(), d_maps, d_own_cols, eb.Ba.as<double>(), mu, dP,
-                                                      dPdense);
-        count_launch();
-        PTB_CUDA(cudaGetLastError());
-    }
-    if (eb.nlarge > 0) {
-        launch_clustered(k_eig_final_cluster, eb.nlarge, eb.G, kFinalSmem, s, (const EigProb*)eb.probs.as<EigProb>(),
-                         (const int*)eb.order_l.as<int>(), (const double*)eb.Ca.as<double>(),
-                         (const double*)eb.La.as<double>(), (const double*)eb.Ta.as<double>(),
-                         (const double*)eb.Wa.as<double>(), (const double*)eb.Za.as<double>(), eb.Qa.as<double>(),
-                         (const double*)eb.Ka.as<double>(), d_maps, d_own_cols, eb.Ba.as<double>(), mu, dP, dPdense);
-        count_launch();
-    }
+    const EigProb* dp = eb.probs.as<EigProb>();
+    const double *Za = eb.Z, *Qa = eb.Qa.as<double>(), *Va = eb.Va.as<double>();
+    double* Ba = eb.Ba.as<double>();
+    const int2* fr = eb.list(eb.frq);
+    k_fin_occ<<<eb.fblocks.n, 256, 0, s>>>(dp, eb.list(eb.fblocks), eb.S, Ba, mu);
+    k_fin_vw<<<eb.frq.n, kT, kTileSmem, s>>>(dp, fr, Za, Qa, Va, eb.S, Ba);
+    k_fin_qw<<<eb.frq.n, kT, kTileSmem, s>>>(dp, fr, Za, Qa, Va, eb.S, Ba);
+    k_fin_cols<<<eb.fcols.n, kT, kChainSmem, s>>>(dp, eb.list(eb.fcols), eb.Ca.as<double>(), eb.La.as<double>(),
+                                                  eb.Ka.as<double>(), d_maps, d_own_cols, Ba, dP, dPdense);
+    count_launch(4);
+    PTB_CUDA(cudaGetLastError());
 }
 
 // Matrix with both triangles set from the upper one: out[i + j n] = a[min(i,j) + max(i,j) n].
@@ -2911,81 +1697,31 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
     eig_setup_attrs();
     cudaStream_t s = c->stream;
     const int m = (int)n;
-    int per_sm = 0;
-    PTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eig_grid, kT, lg_smem_bytes(kLargeMax)));
-    PTB_CHECK(per_sm >= 1, PTBGPU_ECUDA, "eigensolver kernel does not fit an SM");
-    const int nsm = c->num_sms > 0 ? c->num_sms : 148;
-    // up to order kGridMin one thread-block cluster (hardware barrier), above it
-    // a cooperative grid of one CTA per kGridRows rows, at most kGridMax CTAs
-    // (the software barrier's latency grows with the CTA count)
-    const bool cluster = m <= kGridMin;
-    int G = cluster ? eig_cluster_size(c) : std::min({nsm * per_sm, kGridMax, std::max(1, m / kGridRows)});
     EigBatch eb;
-    eb.nprob = 1;
-    eb.G = G;
     EigProb p{};
     p.m = m;
     p.kind = S ? 0 : 1;
+    p.mode = 1;
     p.gld = n;
     eb.hp.push_back(p);
-    const int64_t mm = (int64_t)m * m;
-    const int per = (m + G - 1) / G;
-    const LgLayout lay = lg_layout(m, G);
-    for (WorkBuf* b : {&eb.Ca, &eb.La, &eb.Za}) b->reserve(c, sizeof(double) * mm);
-    eb.Qa.reserve(c, sizeof(double) * std::max<int64_t>(mm, (int64_t)G * lg_wy_stride(per) + 2));
-    eb.Va.reserve(c, sizeof(double) * std::max<int64_t>(mm, (int64_t)G * NB * NB + 2));
-    for (WorkBuf* b : {&eb.Da, &eb.Ea, &eb.Ta, &eb.Wa}) b->reserve(c, sizeof(double) * n);
-    eb.Ka.reserve(c, sizeof(double) * std::max<int64_t>(t_panels(m) * NB * NB, 2));
-    eb.Xa.reserve(c, sizeof(double) * lay.total);
-    eb.Ba.reserve(c, sizeof(double) * 2);
-    eb.probs.reserve(c, sizeof(EigProb));
-    eb.status.reserve(c, sizeof(int) * 4);
-    eb.order.reserve(c, sizeof(int) * n);   // the identity row map
+    // up to order kGridMin one thread-block cluster (hardware barrier), above it
+    // a cooperative grid of one CTA per kGridRows rows, at most kGridMax CTAs
+    // (the software barrier's latency grows with the CTA count)
+    eb.grid = m > kGridMin;
+    if (eb.grid) {
+        int per_sm = 0;
+        PTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lg_trd, kT, lg_smem_bytes(kLargeMax)));
+        PTB_CHECK(per_sm >= 1, PTBGPU_ECUDA, "eigensolver kernel does not fit an SM");
+        const int nsm = c->num_sms > 0 ? c->num_sms : 148;
+        eb.G = std::min({nsm * per_sm, kGridMax, std::max(1, m / kGridRows)});
+    }
+    WorkBuf map;   // the identity row map
+    map.reserve(c, sizeof(int) * n);
     std::vector<int> ident(n);
     for (int i = 0; i < m; ++i) ident[i] = i;
-    PTB_CUDA(cudaMemcpyAsync(eb.order.ptr, ident.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
-    PTB_CUDA(cudaMemcpyAsync(eb.probs.ptr, &p, sizeof(EigProb), cudaMemcpyHostToDevice, s));
-    PTB_CUDA(cudaMemsetAsync(eb.status.ptr, 0, sizeof(int) * 4, s));
-    unsigned* bar = reinterpret_cast<unsigned*>(eb.status.as<int>() + 1);   // status, bar[0], bar[1], err
-    int* err = eb.status.as<int>() + 3;
-    const EigProb* dp = eb.probs.as<EigProb>();
-    int pi = 0, M = kLargeMax, mode = 1;
-    const int* maps = eb.order.as<int>();
-    double *Ca = eb.Ca.as<double>(), *La = eb.La.as<double>(), *Za = eb.Za.as<double>(), *Qa = eb.Qa.as<double>(),
-           *Va = eb.Va.as<double>(), *Da = eb.Da.as<double>(), *Ea = eb.Ea.as<double>(), *Ta = eb.Ta.as<double>(),
-           *Wa = eb.Wa.as<double>(), *Ba = eb.Ba.as<double>(), *Ka = eb.Ka.as<double>(), *Xa = eb.Xa.as<double>();
-    const int* own = nullptr;
-    const int* ipos = nullptr;
-    double *e_out = nullptr, *fe_out = nullptr;
-    int* status = eb.status.as<int>();
-    // PTBGPU_EIG_STAGES=1: stage and tridiagonalisation phase times on stderr
-    static const bool stages = getenv("PTBGPU_EIG_STAGES") != nullptr;
-    if (cluster) {
-        const int* order = eb.order.as<int>() + 0;   // identity map: order[0] = 0
-        unsigned long long* ts = nullptr;
-        if (stages) {
-            eb.tstage.reserve(c, sizeof(unsigned long long) * kLgStride);
-            PTB_CUDA(cudaMemsetAsync(eb.tstage.ptr, 0, sizeof(unsigned long long) * kLgStride, s));
-            ts = eb.tstage.as<unsigned long long>();
-        }
-        launch_clustered(k_eig_cluster, 1, G, lg_smem_bytes(kLargeMax), s, dp, order, M, maps, H, S, Ca, La, Za, Qa,
-                         Va, Da, Ea, Ta, Wa, Ba, Ka, Xa, own, ipos, e_out, fe_out, status, ts, mode, U, w);
-        if (stages) {
-            unsigned long long t[kLgStride];
-            PTB_CUDA(cudaMemcpyAsync(t, ts, sizeof(t), cudaMemcpyDeviceToHost, s));
-            PTB_CUDA(cudaStreamSynchronize(s));
-            fprintf(stderr, "eig_full n=%d cluster %d: stages", m, G);
-            for (int k = 0; k + 1 < kLgStages; ++k) fprintf(stderr, " %.3f", (double)(t[k + 1] - t[k]) * 1e-6);
-            fprintf(stderr, " ms; tridiag phases");
-            for (int k = 0; k < kLgSub; ++k) fprintf(stderr, " %.3f", (double)t[kLgStages + k] * 1e-6);
-            fprintf(stderr, " ms\n");
-        }
-    } else {
-        void* args[] = {&dp, &pi, &M, &mode, &maps, &H, &S, &Ca, &La, &Za, &Qa, &Va, &Da, &Ea, &Ta, &Wa, &Ba, &Ka, &Xa,
-                        &own, &ipos, &e_out, &fe_out, &U, &w, &status, &bar, &err};
-        PTB_CUDA(cudaLaunchCooperativeKernel((void*)k_eig_grid, dim3(G), dim3(kT), args, lg_smem_bytes(kLargeMax), s));
-    }
-    count_launch();
+    PTB_CUDA(cudaMemcpyAsync(map.ptr, ident.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    eig_plan(c, eb, s, 0, U);
+    eig_run(c, eb, s, H, S, map.as<int>(), nullptr, nullptr, w, nullptr);
     int hs[4];
     PTB_CUDA(cudaMemcpyAsync(hs, eb.status.ptr, sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
