@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(kT, 2) k_vec_panels(const EigProb* __restrict_
     const int2 tk = tasks[blockIdx.x];
     if (status[tk.x] != kStOk) return;
     const EigProb p = probs[tk.x];
-    build_T(Ca + p.aoff, p.m, Ta + p.voff, Ka + p.koff, tk.y, 1 << 20, Gg, Gg + NB * NB, sA, sB);
+    build_T(Ca + p.coff, p.ldc, p.m, Ta + p.voff, Ka + p.koff, tk.y, 1 << 20, Gg, Gg + NB * NB, sA, sB);
 }
 
 constexpr size_t kChainSmem = sizeof(double) * (2 * kStageOp + TS * (TS + 1) + 2 * NB * TS);
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kT, 2) k_vec_rows(const EigProb* __restrict__ 
     __syncthreads();
     const int s0 = max(u0, no);
     if (s0 < u1) trsm_cols(true, L, m, R + (int64_t)s0 * m, m, 0, u1 - s0, sD, sA, sB);
-    wy_apply_t(Ca + p.aoff, m, Ka + p.koff, R + (int64_t)u0 * m, u1 - u0, true, Y, Y + NB * TS, sA, sB);
+    wy_apply_t(Ca + p.coff, p.ldc, m, Ka + p.koff, R + (int64_t)u0 * m, u1 - u0, true, Y, Y + NB * TS, sA, sB);
 }
 
 // Z = Q V of the top merge is not formed: Q (m x m, at Qa; the leaf's Z of a problem
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kT, 2) k_fin_cols(const EigProb* __restrict__ 
     const EigProb p = probs[tk.x];
     const int m = p.m, t0 = tk.y * TS, nt = min(TS, p.nown - t0);
     double* W = Ba + p.boff + (int64_t)t0 * m;
-    wy_apply_t(Ca + p.aoff, m, Ka + p.koff, W, nt, false, Y, Y + NB * TS, sA, sB);
+    wy_apply_t(Ca + p.coff, p.ldc, m, Ka + p.koff, W, nt, false, Y, Y + NB * TS, sA, sB);
     __syncthreads();
     trsm_cols(false, La + p.aoff, m, W, m, 0, nt, sD, sA, sB);
     if (Pdense) {
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kT, 2) k_vec_back(const EigProb* __restrict__ 
     const EigProb p = probs[tk.x];
     const int m = p.m, nv = p.mode == 2 ? p.nocc : m, t0 = tk.y * TS, nt = min(TS, nv - t0);
     double* U = Za + p.aoff + (int64_t)t0 * m;
-    wy_apply_t(Ca + p.aoff, m, Ka + p.koff, U, nt, false, Y, Y + NB * TS, sA, sB);
+    wy_apply_t(Ca + p.coff, p.ldc, m, Ka + p.koff, U, nt, false, Y, Y + NB * TS, sA, sB);
     __syncthreads();
     if (p.kind == 0) trsm_cols(false, La + p.aoff, m, U, m, 0, nt, sD, sA, sB);
 }

@@ -60,7 +60,9 @@ struct EigProb {
     int64_t moff, eoff, o0;
     int64_t gbase, gld;   // the problem's H / S: element (i, j) at gbase + map(i) + map(j) gld
     int64_t poff;         // dense output of the owned columns of P (m x nown, column-major)
-    int64_t aoff;     // C, L, Z and merge-workspace arenas (m x m, column-major, ld = m)
+    int64_t aoff;     // L, Z and merge-workspace arenas (m x m, column-major, ld = m)
+    int64_t coff;     // C arena (m columns, ld = ldc: a multiple of 16, so that columns start on 128-byte lines)
+    int ldc;
     int64_t voff;     // d, e, tau, eigenvalue arenas (m)
     int64_t boff;     // owned-row arena (4 nown x m)
     int64_t xoff;     // cluster solver scratch (orders above kEigBatchMax)
@@ -388,15 +390,15 @@ __host__ __device__ constexpr int64_t t_panels(int m) { return m > 2 ? (m - 2 + 
 // by one warp.  Tall + p NB^2 holds panel p's T (NB x NB, column-major, zero
 // outside the panel's nb x nb upper triangle).  Gg: NB^2 global scratch;
 // T: NB x (NB+1) shared.
-__device__ void build_T(const double* __restrict__ C, int m, const double* __restrict__ tau, double* __restrict__ Tall,
+__device__ void build_T(const double* __restrict__ C, int64_t ldc, int m, const double* __restrict__ tau, double* __restrict__ Tall,
                         int first, int step, double* Gg, double* T, double* sA, double* sB) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nref = m - 2;
     const int npan = (int)t_panels(m);
     for (int pan = first; pan < npan; pan += step) {
         const int j0 = pan * NB, nb = min(NB, nref - j0), r0 = j0 + 1, len = m - r0;
-        const double* Vb = C + r0 + (int64_t)j0 * m;
-        tile_mma<true, false, MMA_SET, false, true, true>(Gg, NB, 0, nullptr, 0, 0, nb, nb, Vb, m, nullptr, Vb, m,
+        const double* Vb = C + r0 + (int64_t)j0 * ldc;
+        tile_mma<true, false, MMA_SET, false, true, true>(Gg, NB, 0, nullptr, 0, 0, nb, nb, Vb, ldc, nullptr, Vb, ldc,
                                                           nullptr, len, sA, sB);
         for (int q = tid; q < NB * NB; q += kT) {
             const int a = q % NB, b = q / NB;
@@ -430,7 +432,7 @@ __device__ void build_T(const double* __restrict__ C, int m, const double* __res
 // from build_T: Y = V^T X, Y2 = T^T Y (trans: panels in order) or T Y (panels
 // in reverse), X -= V Y2, the reflectors read in place from C.  Y and Y2 are
 // NB x nv global scratch each.
-__device__ void wy_apply_t(const double* __restrict__ C, int m, const double* __restrict__ Tall, double* X, int nv,
+__device__ void wy_apply_t(const double* __restrict__ C, int64_t ldc, int m, const double* __restrict__ Tall, double* X, int nv,
                            bool trans, double* Y, double* Y2, double* sA, double* sB) {
     const int tid = threadIdx.x;
     const int nref = m - 2;
@@ -439,10 +441,10 @@ __device__ void wy_apply_t(const double* __restrict__ C, int m, const double* __
     for (int pp = 0; pp < npan; ++pp) {
         const int pan = trans ? pp : npan - 1 - pp;
         const int j0 = pan * NB, nb = min(NB, nref - j0), r0 = j0 + 1, len = m - r0;
-        const double* Vb = C + r0 + (int64_t)j0 * m;
+        const double* Vb = C + r0 + (int64_t)j0 * ldc;
         const double* Tp = Tall + (int64_t)pan * NB * NB;
         for (int c0 = 0; c0 < nv; c0 += TS)
-            tile_mma<true, false, MMA_SET, false, true, false>(Y, NB, 0, nullptr, 0, c0, nb, min(TS, nv - c0), Vb, m,
+            tile_mma<true, false, MMA_SET, false, true, false>(Y, NB, 0, nullptr, 0, c0, nb, min(TS, nv - c0), Vb, ldc,
                                                                nullptr, X + r0, m, nullptr, len, sA, sB);
         for (int64_t q = tid; q < (int64_t)NB * nv; q += kT) {
             const int a = (int)(q % NB), t = (int)(q / NB);
@@ -461,7 +463,7 @@ __device__ void wy_apply_t(const double* __restrict__ C, int m, const double* __
         for (int c0 = 0; c0 < nv; c0 += TS)
             for (int i0 = 0; i0 < len; i0 += TS)
                 tile_mma<false, false, MMA_SUB, false, true, false>(X + r0, m, 0, nullptr, i0, c0, min(TS, len - i0),
-                                                                    min(TS, nv - c0), Vb, m, nullptr, Y2, NB, nullptr,
+                                                                    min(TS, nv - c0), Vb, ldc, nullptr, Y2, NB, nullptr,
                                                                     nb, sA, sB);
     }
 }
@@ -554,21 +556,22 @@ __global__ void __launch_bounds__(kT, 1) k_eig_chol(const EigProb* __restrict__ 
     if (threadIdx.x == 0) status[pi] = st;
 }
 
-// X <- L^-1 X on one 64-column block of X per CTA (tasks: problem, block).
+// X <- L^-1 X on one 64-column block of X per CTA (tasks: problem, block); in_c: X is
+// the C arena.
 constexpr size_t kTrsmSmem = sizeof(double) * (2 * kStageOp + TS * (TS + 1));
 __global__ void __launch_bounds__(kT, 2) k_eig_trsm(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ La, double* __restrict__ Xa,
-                                                    const int* __restrict__ status) {
+                                                    bool in_c, const int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     const int2 t = tasks[blockIdx.x];
     if (status[t.x] != kStOk) return;
     const EigProb p = probs[t.x];
-    trsm_cols(true, La + p.aoff, p.m, Xa + p.aoff, p.m, t.y * TS, min(p.m, (t.y + 1) * TS), sA + 2 * kStageOp, sA,
-              sA + kStageOp);
+    trsm_cols(true, La + p.aoff, p.m, Xa + (in_c ? p.coff : p.aoff), in_c ? p.ldc : p.m, t.y * TS,
+              min(p.m, (t.y + 1) * TS), sA + 2 * kStageOp, sA, sA + kStageOp);
 }
 
-// Y = X^T, one 64-column block of X per CTA, through 64 x 65 shared tiles.
+// Y = X^T (Y in the C arena), one 64-column block of X per CTA, through 64 x 65 shared tiles.
 __global__ void __launch_bounds__(256) k_eig_transpose(const EigProb* __restrict__ probs,
                                                        const int2* __restrict__ tasks, const double* __restrict__ Xa,
                                                        double* __restrict__ Ya, const int* __restrict__ status) {
@@ -578,13 +581,13 @@ __global__ void __launch_bounds__(256) k_eig_transpose(const EigProb* __restrict
     const EigProb p = probs[t.x];
     const int m = p.m, c0 = t.y * TS, tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
     const double* X = Xa + p.aoff;
-    double* Y = Ya + p.aoff;
+    double* Y = Ya + p.coff;
     for (int r0 = 0; r0 < m; r0 += TS) {
         for (int c = ty; c < TS; c += 4)
             if (r0 + tx < m && c0 + c < m) tile[c][tx] = X[r0 + tx + (int64_t)(c0 + c) * m];
         __syncthreads();
         for (int r = ty; r < TS; r += 4)
-            if (r0 + r < m && c0 + tx < m) Y[c0 + tx + (int64_t)(r0 + r) * m] = tile[tx][r];
+            if (r0 + r < m && c0 + tx < m) Y[c0 + tx + (int64_t)(r0 + r) * p.ldc] = tile[tx][r];
         __syncthreads();
     }
 }
@@ -594,11 +597,12 @@ template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_eig_trd(const EigProb* __restrict__ probs,
                                                           const int* __restrict__ order, double* __restrict__ Ca,
                                                           double* __restrict__ Da, double* __restrict__ Ea,
-                                                          double* __restrict__ Ta, const int* __restrict__ status) {
+                                                          double* __restrict__ Ta, int cap,
+                                                          const int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int pi = order[blockIdx.x];
     if (status[pi] != kStOk) return;
-    stage_trd<NT>(probs[pi], Ca, Da, Ea, Ta, reinterpret_cast<double*>(smraw));
+    stage_trd<NT>(probs[pi], Ca, Da, Ea, Ta, reinterpret_cast<double*>(smraw), cap);
 }
 
 // Divide and conquer, then the owned rows and fe (mode 0) or the density (mode 2).
@@ -740,14 +744,14 @@ __device__ __forceinline__ void tri_decode(int64_t idx, int& rb, int& cb) {
 
 // H_k into X, S_k into L (generalized problems), columns split over the CTAs.
 __device__ void lg_gather(const Grp& g, const EigProb& p, const int* __restrict__ maps, const double* __restrict__ H,
-                          const double* __restrict__ S, double* __restrict__ X, double* __restrict__ L) {
+                          const double* __restrict__ S, double* __restrict__ X, int64_t ldx, double* __restrict__ L) {
     const int m = p.m;
     const int* mp = maps + p.moff;
     for (int j = g.rank; j < m; j += g.size) {
         const int64_t gj = p.gbase + (int64_t)mp[j] * p.gld;
         for (int i = threadIdx.x; i < m; i += kT) {
             const int64_t q = (int64_t)mp[i] + gj;
-            X[i + (int64_t)j * m] = H[q];
+            X[i + (int64_t)j * ldx] = H[q];
             if (p.kind == 0) L[i + (int64_t)j * m] = S[q];
         }
     }
@@ -849,7 +853,7 @@ __device__ __forceinline__ int av_nseg(int I, int cstart) {
 // w of column jp of the panel (the column before j) on this CTA's rows, with the
 // reflector stored into A's column j-1; w_j itself goes to sh.wj[jp], computed
 // by the last warp beside the row loop.  The caller synchronises the CTA.
-__device__ void lg_finish_w(const Grp& g, int m, int j, int jp, double* __restrict__ A, double* __restrict__ V,
+__device__ void lg_finish_w(const Grp& g, int m, int j, int jp, double* __restrict__ A, int64_t lda, double* __restrict__ V,
                             double* __restrict__ W, const double* __restrict__ rowp,
                             const double* __restrict__ colp, const double* __restrict__ red, const LgSmem& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -877,7 +881,7 @@ __device__ void lg_finish_w(const Grp& g, int m, int j, int jp, double* __restri
         const int r = ch * 32 + lane;
         if (r >= j && r < m) {
             W[r + (int64_t)jp * m] = w_at(r);
-            if (r >= j + 1) A[r + (int64_t)(j - 1) * m] = sh.v[r];
+            if (r >= j + 1) A[r + (int64_t)(j - 1) * lda] = sh.v[r];
         }
     }
 }
@@ -885,7 +889,8 @@ __device__ void lg_finish_w(const Grp& g, int m, int j, int jp, double* __restri
 __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca, double* __restrict__ Da,
                          double* __restrict__ Ea, double* __restrict__ Ta, double* __restrict__ X, const LgSmem& sh) {
     const int m = p.m, G = g.size, rk = g.rank;
-    double* A = Ca + p.aoff;
+    double* A = Ca + p.coff;
+    const int64_t lda = p.ldc;
     double* d = Da + p.voff;
     double* e = Ea + p.voff;
     double* tau = Ta + p.voff;
@@ -910,15 +915,15 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                 if (tid < jj - 1) sh.wj[tid] = W[j + (int64_t)tid * m];
                 sh.vj[tid] = V[j + (int64_t)tid * m];
             }
-            if (jj > 0) lg_finish_w(g, m, j, jj - 1, A, V, W, rowp, colp, red, sh);
+            if (jj > 0) lg_finish_w(g, m, j, jj - 1, A, lda, V, W, rowp, colp, red, sh);
             __syncthreads();
             for (int ch = rk + G * warp; ch * 32 < m; ch += G * (kT / 32)) {
                 const int r = ch * 32 + lane;
                 if (r >= j && r < m) {
-                    double a = A[r + (int64_t)j * m];
+                    double a = A[r + (int64_t)j * lda];
                     for (int q = 0; q < jj; ++q)
                         a -= V[r + (int64_t)q * m] * sh.wj[q] + W[r + (int64_t)q * m] * sh.vj[q];
-                    A[r + (int64_t)j * m] = a;
+                    A[r + (int64_t)j * lda] = a;
                     yl[r] = a;
                 }
             }
@@ -958,12 +963,12 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                 wj1 = W[(j + 1) + (int64_t)tid * m];
                 vj1 = V[(j + 1) + (int64_t)tid * m];
             }
-            for (int r = j + 2 + tid; r < m; r += kT) v[r] = A[r + (int64_t)j * m];
+            for (int r = j + 2 + tid; r < m; r += kT) v[r] = A[r + (int64_t)j * lda];
             if (tid == 32) {
                 double xn2 = 0.0;
                 for (int q = 0; q < G; ++q) xn2 += red[q * kRedW + 0];
-                const double alpha = A[(j + 1) + (int64_t)j * m];
-                const double dj = A[j + (int64_t)j * m];
+                const double alpha = A[(j + 1) + (int64_t)j * lda];
+                const double dj = A[j + (int64_t)j * lda];
                 double t, beta;
                 if (xn2 == 0.0) {
                     t = 0.0;
@@ -1037,8 +1042,8 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                             for (int u8 = 0; u8 < kAvGrp; ++u8) {
                                 const int c = cb + g8 + u8;
                                 const bool cok = c < c_hi && c >= s;
-                                a0[u8] = (cok && r0 < m && c <= r0) ? A0[(int64_t)c * m] : 0.0;
-                                a1[u8] = (cok && r1 < m && c <= r1) ? A1[(int64_t)c * m] : 0.0;
+                                a0[u8] = (cok && r0 < m && c <= r0) ? A0[(int64_t)c * lda] : 0.0;
+                                a1[u8] = (cok && r1 < m && c <= r1) ? A1[(int64_t)c * lda] : 0.0;
                             }
 #pragma unroll
                             for (int u8 = 0; u8 < kAvGrp; ++u8) {
@@ -1068,7 +1073,7 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
         }
         // ---- panel end: w of the last column, then the trailing block
         const int j1 = j0 + nb;
-        lg_finish_w(g, m, j1, nb - 1, A, V, W, rowp, colp, red, sh);
+        lg_finish_w(g, m, j1, nb - 1, A, lda, V, W, rowp, colp, red, sh);
         g.sync();
         if (j1 < m) {
             const int nt = (m - j1 + TS - 1) / TS;
@@ -1078,14 +1083,14 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
                 tri_decode(idx, rb, cb);
                 const int r0 = j1 + rb * TS, c0 = j1 + cb * TS;
                 const int mr = min(TS, m - r0), nc = min(TS, m - c0);
-                tile_update<true, true>(A, m, r0, c0, mr, nc, V, m, W, m, nb, sh.sA, sh.sB);
-                tile_update<true, true>(A, m, r0, c0, mr, nc, W, m, V, m, nb, sh.sA, sh.sB);
+                tile_update<true, true>(A, (int)lda, r0, c0, mr, nc, V, m, W, m, nb, sh.sA, sh.sB);
+                tile_update<true, true>(A, (int)lda, r0, c0, mr, nc, W, m, V, m, nb, sh.sA, sh.sB);
             }
         }
         g.sync();
     }
     if (rk == 0 && tid == 0) {
-        d[m - 1] = A[(m - 1) + (int64_t)(m - 1) * m];
+        d[m - 1] = A[(m - 1) + (int64_t)(m - 1) * lda];
         tau[m - 1] = 0.0;
     }
 }
@@ -1110,7 +1115,7 @@ __global__ void __launch_bounds__(kT, 1) k_lg_chol(const EigProb* __restrict__ p
     const int pi = order[bar ? 0 : blockIdx.x / g.size];
     const EigProb p = probs[pi];
     // a standard problem needs no reduction: its matrix goes where that leaves it
-    lg_gather(g, p, maps, H, S, (p.kind == 0 ? Xa : Ca) + p.aoff, La + p.aoff);
+    lg_gather(g, p, maps, H, S, p.kind == 0 ? Xa + p.aoff : Ca + p.coff, p.kind == 0 ? p.m : p.ldc, La + p.aoff);
     g.sync();
     const int st = p.kind == 0 ? lg_potrf(g, p.m, La + p.aoff, sh) : kStOk;
     if (g.rank == 0 && threadIdx.x == 0) status[pi] = st;
@@ -1198,8 +1203,8 @@ void eig_setup_attrs() {
     static const bool done = [] {
         smem_attr(k_eig_chol, kCholSmem);
         smem_attr(k_eig_trsm, kTrsmSmem);
-        smem_attr(k_eig_trd<512>, 8 * kTrdCap512);
-        smem_attr(k_eig_trd<256>, 8 * kTrdCap256);
+        smem_attr(k_eig_trd<512>, 8 * trd_cap(kTrdMax512, 512));
+        smem_attr(k_eig_trd<256>, 8 * trd_cap(kTrdMax256, 256));
         smem_attr(k_lg_chol, lg_smem_bytes(2));
         smem_attr(k_lg_trd, lg_smem_bytes(kLargeMax));
         smem_attr(k_dc_product, kTileSmem);
@@ -1337,12 +1342,15 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     // two CTAs per SM only pay where the small orders fill the SMs
     if (eb.nsmall - eb.n512 <= nsm) eb.n512 = eb.nsmall;
 
-    int64_t asz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0;
+    int64_t asz = 0, csz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0;
     for (int q = 0; q < np; ++q) {
         EigProb& p = eb.hp[q];
         p.poff = psz;
         psz += (int64_t)p.m * p.nown;
         p.aoff = asz;
+        p.coff = csz;
+        p.ldc = (int)round_up(p.m, 16);
+        csz += (int64_t)p.ldc * p.m;
         p.voff = vsz;
         p.boff = bsz;
         p.xoff = xsz;
@@ -1455,7 +1463,8 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     const int64_t vpad = (vsz + 1) & ~int64_t(1);
     eb.dc.reserve(c, kDcBytes * vpad);
     eb.S = dc_arrays(eb.dc.ptr, vpad, eb.cnt.as<int>());
-    for (WorkBuf* b : {&eb.Ca, &eb.La, &eb.Qa, &eb.Va}) b->reserve(c, sizeof(double) * asz);
+    eb.Ca.reserve(c, sizeof(double) * csz);
+    for (WorkBuf* b : {&eb.La, &eb.Qa, &eb.Va}) b->reserve(c, sizeof(double) * asz);
     if (!Uout) eb.Za.reserve(c, sizeof(double) * asz);
     eb.Z = Uout ? Uout : eb.Za.as<double>();
     for (WorkBuf* b : {&eb.Da, &eb.Ea, &eb.Ta}) b->reserve(c, sizeof(double) * vsz);
@@ -1523,9 +1532,9 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
     // ---- C = L^-1 H L^-T
     if (eb.hp[0].kind == 0) {
         const int2* bl = eb.list(eb.blocks);
-        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Qa, st);
+        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Qa, false, st);
         k_eig_transpose<<<eb.blocks.n, 256, 0, s>>>(dp, bl, Qa, Ca, st);
-        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Ca, st);
+        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Ca, true, st);
         launched(3);
     }
     // ---- tridiagonalisation
@@ -1542,12 +1551,13 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         launched();
     }
     if (eb.n512 > 0) {
-        k_eig_trd<512><<<eb.n512, 512, sizeof(double) * kTrdCap512, s>>>(dp, ord, Ca, Da, Ea, Ta, st);
+        const int cap = trd_cap(eb.hp[eb.order[0]].m, 512);
+        k_eig_trd<512><<<eb.n512, 512, sizeof(double) * cap, s>>>(dp, ord, Ca, Da, Ea, Ta, cap, st);
         launched();
     }
     if (eb.n512 < eb.nsmall) {
-        k_eig_trd<256><<<eb.nsmall - eb.n512, 256, sizeof(double) * kTrdCap256, s>>>(dp, ord + eb.n512, Ca, Da, Ea, Ta,
-                                                                                     st);
+        const int cap = trd_cap(eb.hp[eb.order[eb.n512]].m, 256);
+        k_eig_trd<256><<<eb.nsmall - eb.n512, 256, sizeof(double) * cap, s>>>(dp, ord + eb.n512, Ca, Da, Ea, Ta, cap, st);
         launched();
     }
     join();
