@@ -62,6 +62,13 @@ constexpr int kTrdMax256 = 288;   // orders two CTAs per SM take (panels of 8 co
 static_assert(trd_cap(kTrdMax512, 512) > 0, "panel fits one CTA per SM");
 static_assert(trd_cap(kTrdMax256, 256) > 0, "panel fits two CTAs per SM");
 
+// 16-byte load that stays where it is written: ahead of the arithmetic before its use.
+__device__ __forceinline__ double2 ld_ahead(const double* p) {
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0,%1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
 template <int NT>
 __device__ void stage_trd(const EigProb& p, double* __restrict__ Ca, double* __restrict__ Da, double* __restrict__ Ea,
                           double* __restrict__ Ta, double* smem, int cap) {

@@ -366,7 +366,6 @@ __device__ int stage_potrf(const EigProb& p, double* __restrict__ La, const Stag
     return 0;
 }
 
-#include "eig_trd.cuh"
 
 // ---------------------------------------------------------------------------
 // C[crow + r0 + i, col(c0 + j)] = sum_k A(i, kx(k)) B(kxb(k), j) on one TS x TS
@@ -541,6 +540,9 @@ __device__ void trsm_cols(bool lower, const double* __restrict__ L, int m, doubl
 // ---------------------------------------------------------------------------
 // status[pi]: 0, the order of a non-positive pivot of S_k, or kStNoConv; a problem
 // that failed is skipped by the later stages.
+#include "eig_trd.cuh"
+#include "eig_trdc.cuh"
+
 // Gather and Cholesky, one problem per CTA.
 __global__ void __launch_bounds__(kT, 1) k_eig_chol(const EigProb* __restrict__ probs, const int* __restrict__ order,
                                                     const int* __restrict__ maps, const double* __restrict__ H,
@@ -1135,23 +1137,42 @@ __global__ void __launch_bounds__(kT, 1) k_lg_trd(const EigProb* __restrict__ pr
     lg_sytrd(g, p, Ca, Da, Ea, Ta, Xa + p.xoff, sh);
 }
 
+__global__ void __launch_bounds__(kT, 1) k_trd_cluster(const EigProb* __restrict__ probs,
+                                                       const int* __restrict__ order, double* __restrict__ Ca,
+                                                       double* __restrict__ Da, double* __restrict__ Ea,
+                                                       double* __restrict__ Ta, double* __restrict__ Xa, int cap,
+                                                       const int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int pi = order[blockIdx.x / cg::this_cluster().num_blocks()];
+    if (status[pi] != kStOk) return;
+    const EigProb p = probs[pi];
+    stage_trd_cluster<4>(p, Ca, Da, Ea, Ta, Xa + p.xoff, reinterpret_cast<double*>(smraw), cap);
+}
+
 }  // namespace
 
-// Streams and events of a context's eigensolver calls: the large problems' chains run
-// on `side` beside the small ones' on the call's stream.
+// Streams and events of a context's eigensolver calls: launches of one stage with
+// different groups run side by side (side), a whole batch beside the call's stream (base).
 struct EigStreams {
-    cudaStream_t side = nullptr, base = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
+    static constexpr int kPerBatch = 6;            // a batch's side streams at most
+    static constexpr int kSide = 2 * kPerBatch;    // of a batch on the call's stream, and of one on base
+    cudaStream_t side[kSide] = {}, base = nullptr;
+    cudaEvent_t fork[2] = {}, join[kSide] = {}, start = nullptr, done = nullptr;
     EigStreams() {
-        PTB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        for (cudaStream_t& s : side) PTB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         PTB_CUDA(cudaStreamCreateWithFlags(&base, cudaStreamNonBlocking));
-        for (cudaEvent_t* e : {&fork, &join, &done}) PTB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        for (cudaEvent_t& e : join) PTB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        for (cudaEvent_t* e : {&fork[0], &fork[1], &start, &done})
+            PTB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     ~EigStreams() {
-        for (cudaEvent_t e : {fork, join, done})
+        for (cudaEvent_t e : join)
             if (e) cudaEventDestroy(e);
-        for (cudaStream_t s : {side, base})
+        for (cudaEvent_t e : {fork[0], fork[1], start, done})
+            if (e) cudaEventDestroy(e);
+        for (cudaStream_t s : side)
             if (s) cudaStreamDestroy(s);
+        if (base) cudaStreamDestroy(base);
     }
 };
 
@@ -1164,12 +1185,18 @@ struct EigBatch {
         int m0 = 0, nm = 0;
         Seg permute, elems, product;
     };
+    struct Trd {   // problems tridiagonalised by groups of the same kind: order[off, off + n)
+        int G = 0;        // CTAs per problem; 0: k_lg_trd
+        int nt = 512;     // threads per CTA (G == 1)
+        int off = 0, n = 0, cap = 0;
+    };
     int nprob = 0;
-    int G = 1;                    // CTAs per cluster of the large problems
-    int nsmall = 0, nlarge = 0, n512 = 0, maxlarge = 0;
+    int G = 1;                    // CTAs per cluster of the large problems' Cholesky
+    int nsmall = 0, nlarge = 0, maxlarge = 0;
     bool grid = false;            // one problem on a cooperative grid
+    std::vector<Trd> trd;
     std::vector<EigProb> hp;
-    std::vector<int> order;       // small problems first, each part largest first
+    std::vector<int> order;       // small problems first, each part largest first; then by tridiagonalisation group
     std::vector<int2> lists;
     std::vector<DcMerge> merges;
     std::vector<Level> levels;
@@ -1185,7 +1212,7 @@ struct EigBatch {
         // the arrays go back to the context's pool: nothing on the side streams may
         // still use them (work on the context's stream is ordered before their next use)
         if (st) {
-            cudaStreamSynchronize(st->side);
+            for (cudaStream_t x : st->side) cudaStreamSynchronize(x);
             cudaStreamSynchronize(st->base);
         }
     }
@@ -1207,6 +1234,8 @@ void eig_setup_attrs() {
         smem_attr(k_eig_trd<256>, 8 * trd_cap(kTrdMax256, 256));
         smem_attr(k_lg_chol, lg_smem_bytes(2));
         smem_attr(k_lg_trd, lg_smem_bytes(kLargeMax));
+        smem_attr(k_trd_cluster, kTrdCaps[3] - 1024);
+        PTB_CUDA(cudaFuncSetAttribute(k_trd_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         smem_attr(k_dc_product, kTileSmem);
         smem_attr(k_vec_panels, kWySmem);
         smem_attr(k_vec_rq, kTileSmem);
@@ -1245,57 +1274,79 @@ int eig_active_clusters(int G) {
     return ncl;
 }
 
-// CTAs per cluster of the large-submatrix solver for one problem or a few
-// waves of them: 16 when clusters of 16 keep at least 80 % of the SMs busy (one
-// 512-thread CTA each), else 8 on the same rule, else the size among 4 and 2
-// that keeps the most SMs busy; a submatrix's stages shorten with the cluster,
-// and the longest submatrix sets the step.  PTBGPU_EIG_CLUSTER = 1, 2, 4, 8 or
-// 16 overrides it.
-int eig_cluster_size(ptbgpu_ctx* c) {
-    static int cached[64] = {};
-    const int dev = c->device & 63;
-    if (cached[dev]) return cached[dev];
-    int best = 1, best_ctas = 0;
-    if (const char* e = getenv("PTBGPU_EIG_CLUSTER")) {
-        const int v = atoi(e);
-        if (v == 1 || v == 2 || v == 4 || v == 8 || v == 16) best = v;
-    } else {
-        const int nsm = c->num_sms > 0 ? c->num_sms : 148;
-        for (int G : {16, 8, 4, 2}) {
-            const int ncl = eig_active_clusters(G);
-            if (ncl == 0) continue;
-            if (G >= 8 && ncl * G * 5 >= nsm * 4) {
-                best = G;
-                break;
-            }
-            if (ncl * G > best_ctas) {
-                best_ctas = ncl * G;
-                best = G;
-            }
-        }
-    }
-    cached[dev] = best;
-    return best;
+int eig_active_cached(ptbgpu_ctx* c, int G) {
+    static int active[64][5] = {};   // known + 1
+    int& a = active[c->device & 63][G == 16 ? 4 : G == 8 ? 3 : G == 4 ? 2 : G == 2 ? 1 : 0];
+    if (a == 0) a = eig_active_clusters(G) + 1;
+    return a - 1;
 }
 
-// Cluster size for a batch with nlarge problems above kEigBatchMax.  When they
-// need kManyWaves or more waves of the one-problem size, clusters of 2 CTAs
-// take them: four times as many run side by side, each with a quarter of the
-// cross-CTA steps per flop, and the last wave is shorter.  Measured on 174
-// systems of order 1025-3064: 2.7-3.0 s per batch against 3.2-3.6 s with
-// clusters of 8; on 50 submatrices up to 2773 clusters of 8 stay faster
-// (0.64-0.71 s against 1.38 s with 2).
-constexpr int kManyWaves = 6;
-int eig_batch_cluster_size(ptbgpu_ctx* c, int nlarge) {
-    const int G = eig_cluster_size(c);
-    if (getenv("PTBGPU_EIG_CLUSTER") || G <= 2) return G;
-    static int active[64] = {}, active2[64] = {};
-    const int dev = c->device & 63;
-    if (!active[dev]) {
-        active2[dev] = eig_active_clusters(2);
-        active[dev] = std::max(1, eig_active_clusters(G));
+// CTAs of the cluster Cholesky and of the cluster tridiagonalisation for orders beyond
+// the shared-memory one: 16 for one problem, else 8.  PTBGPU_EIG_CLUSTER = 1, 2, 4, 8 or
+// 16 sets them, and the tridiagonalisation's of every order above kEigBatchMax.
+int eig_cluster_forced() {
+    const char* e = getenv("PTBGPU_EIG_CLUSTER");
+    const int v = e ? atoi(e) : 0;
+    return v == 1 || v == 2 || v == 4 || v == 8 || v == 16 ? v : 0;
+}
+int eig_cluster_size(ptbgpu_ctx* c, int nlarge) {
+    if (const int v = eig_cluster_forced()) return v;
+    for (int G : {16, 8, 4, 2})
+        if ((G < 16 || nlarge == 1) && eig_active_cached(c, G) > 0) return G;
+    return 1;
+}
+
+// Clocks of one tridiagonalisation on G CTAs: a chain of short steps per column and the
+// passes over the triangle (fitted to orders 576 on one CTA and 900 to 2100 on 8 and 16).
+double trd_clocks(int m, int G) {
+    const double n = m, n3 = n * n * n;
+    return G == 1 ? 7.0e3 * n + 0.058 * n3 : 14.0e3 * n + 0.05 * n3 / G;
+}
+
+// CTAs for every problem's tridiagonalisation (orders in m): the smallest clusters with
+// which each problem ends within T, for the smallest T in which the SMs can also hold them
+// all.  One problem gets the widest cluster, a batch that fills the SMs one CTA each (or the
+// smallest cluster whose shared memory holds the panel), a batch of uneven problems
+// wider ones for its largest: with 96 problems of 218 to 595 the stage's length is no
+// longer the largest one's on one SM.  0: beyond every cluster's shared memory.
+std::vector<int> trd_groups(ptbgpu_ctx* c, const std::vector<int>& m, int small_max, int forced) {
+    const int nsm = c->num_sms > 0 ? c->num_sms : 148;
+    const int sizes[5] = {1, 2, 4, 8, 16};
+    auto allowed = [&](int mm, int G) {
+        if (G == 1) return mm <= small_max;
+        // (many large triangles side by side are bound by HBM, not by their SMs: mixed
+        // clusters of 2 to 16 took 155 ms on 48 problems up to 2773, 8 for all of them 144)
+        if (mm > small_max && G < 8) return false;
+        if (forced > 1 && mm > small_max && G != forced) return false;
+        return tc_cap(mm, 4, G, kT) > 0 && eig_active_cached(c, G) > 0;
+    };
+    std::vector<int> pick(m.size(), 0);
+    auto fill = [&](double T) {
+        double area = 0.0;
+        bool fits = true;
+        for (size_t i = 0; i < m.size(); ++i) {
+            int best = 0;
+            for (int G : sizes) {
+                if (!allowed(m[i], G)) continue;
+                if (best == 0 || trd_clocks(m[i], G) < trd_clocks(m[i], best)) best = G;
+                if (trd_clocks(m[i], best) <= T) break;
+            }
+            pick[i] = best;
+            if (best == 0) continue;
+            const double t = trd_clocks(m[i], best);
+            area += best * t;
+            fits = fits && t <= T;
+        }
+        return fits && area <= 0.85 * nsm * T;
+    };
+    double lo = 0.0, hi = 1.0e6;
+    while (!fill(hi) && hi < 1.0e13) hi *= 2.0;
+    for (int it = 0; it < 30; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        (fill(mid) ? hi : lo) = mid;
     }
-    return nlarge >= kManyWaves * active[dev] && active2[dev] > 0 ? 2 : G;
+    fill(hi);
+    return pick;
 }
 
 template <class K, class... Args>
@@ -1336,12 +1387,8 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     eb.nsmall = (int)eb.order.size();
     eb.nlarge = (int)large.size();
     eb.maxlarge = large.empty() ? 0 : eb.hp[large[0]].m;
-    if (eb.nlarge > 0 && !eb.grid) eb.G = eig_batch_cluster_size(c, eb.nlarge);
+    if (eb.nlarge > 0 && !eb.grid) eb.G = eig_cluster_size(c, eb.nlarge);
     const int nsm = c->num_sms > 0 ? c->num_sms : 148;
-    for (int q : eb.order) eb.n512 += eb.hp[q].m > kTrdMax256;
-    // two CTAs per SM only pay where the small orders fill the SMs
-    if (eb.nsmall - eb.n512 <= nsm) eb.n512 = eb.nsmall;
-
     int64_t asz = 0, csz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0;
     for (int q = 0; q < np; ++q) {
         EigProb& p = eb.hp[q];
@@ -1350,22 +1397,48 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
         p.aoff = asz;
         p.coff = csz;
         p.ldc = (int)round_up(p.m, 16);
-        csz += (int64_t)p.ldc * p.m;
+        csz += (int64_t)p.ldc * (p.m + kTcPadCols) + kTcPadRows;
         p.voff = vsz;
         p.boff = bsz;
-        p.xoff = xsz;
         p.koff = ksz;
         p.topm = -1;
         ksz += t_panels(p.m) * NB * NB;
         asz += (int64_t)p.m * p.m;
         vsz += p.m;
         bsz += p.mode == 2 ? (int64_t)p.m * p.m : 4 * (int64_t)p.nown * p.m;
-        if (p.m > small_max) xsz += lg_layout(p.m, eb.G).total;
     }
     // task lists, largest problems first in each
     std::vector<int> all(large);
     all.insert(all.end(), eb.order.begin(), eb.order.end());
     eb.order.insert(eb.order.end(), large.begin(), large.end());
+    {
+        std::vector<int> ms, pick;
+        for (int q : all) ms.push_back(eb.hp[q].m);
+        if (eb.grid) pick.assign(ms.size(), 0);
+        else pick = trd_groups(c, ms, kTrdMax512, eig_cluster_forced());
+        // two CTAs per SM only pay where the small orders fill the SMs
+        int n256 = 0;
+        for (size_t i = 0; i < all.size(); ++i) n256 += pick[i] == 1 && ms[i] <= kTrdMax256;
+        auto group = [&](int G, int nt, auto&& mine) {
+            EigBatch::Trd t;
+            t.G = G;
+            t.nt = nt;
+            t.off = (int)eb.order.size();
+            for (size_t i = 0; i < all.size(); ++i) {
+                if (pick[i] != G || !mine(ms[i])) continue;
+                EigProb& p = eb.hp[all[i]];
+                p.xoff = xsz;
+                xsz += G == 0 ? lg_layout(p.m, eb.G).total : G == 1 ? 0 : (int64_t)32 * p.m;
+                if (t.n++ == 0) t.cap = G == 0 ? (p.m + 1) & ~1 : 0;
+                t.cap = std::max(t.cap, G == 0 ? 0 : G == 1 ? trd_cap(p.m, nt) : tc_cap(p.m, 4, G, kT));
+                eb.order.push_back(all[i]);
+            }
+            if (t.n > 0) eb.trd.push_back(t);
+        };
+        for (int G : {0, 16, 8, 4, 2}) group(G, 512, [](int) { return true; });
+        group(1, 512, [&](int m) { return m > kTrdMax256 || n256 <= nsm; });
+        group(1, 256, [&](int m) { return m <= kTrdMax256 && n256 > nsm; });
+    }
     auto list = [&](EigBatch::Seg& g, auto&& fill) {
         g.off = eb.lists.size();
         fill();
@@ -1456,7 +1529,7 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     }
 
     eb.probs.reserve(c, sizeof(EigProb) * np);
-    eb.order_d.reserve(c, sizeof(int) * np);
+    eb.order_d.reserve(c, sizeof(int) * eb.order.size());
     eb.lists_d.reserve(c, sizeof(int2) * std::max<size_t>(eb.lists.size(), 1));
     eb.merges_d.reserve(c, sizeof(DcMerge) * std::max<size_t>(eb.merges.size(), 1));
     eb.cnt.reserve(c, 8 * sizeof(int) * std::max<size_t>(eb.merges.size(), 1));
@@ -1473,7 +1546,7 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     eb.Ka.reserve(c, sizeof(double) * std::max<int64_t>(ksz, 2));
     eb.status.reserve(c, sizeof(int) * (np + 3));   // and a grid barrier's count, generation and error
     PTB_CUDA(cudaMemcpyAsync(eb.probs.ptr, eb.hp.data(), sizeof(EigProb) * np, cudaMemcpyHostToDevice, s));
-    PTB_CUDA(cudaMemcpyAsync(eb.order_d.ptr, eb.order.data(), sizeof(int) * np, cudaMemcpyHostToDevice, s));
+    PTB_CUDA(cudaMemcpyAsync(eb.order_d.ptr, eb.order.data(), sizeof(int) * eb.order.size(), cudaMemcpyHostToDevice, s));
     PTB_CUDA(cudaMemcpyAsync(eb.lists_d.ptr, eb.lists.data(), sizeof(int2) * eb.lists.size(), cudaMemcpyHostToDevice, s));
     if (!eb.merges.empty())
         PTB_CUDA(cudaMemcpyAsync(eb.merges_d.ptr, eb.merges.data(), sizeof(DcMerge) * eb.merges.size(),
@@ -1495,26 +1568,35 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
     const DcArr& D = eb.S;
     unsigned* bar = eb.grid ? reinterpret_cast<unsigned*>(st + eb.nprob) : nullptr;
     int* err = eb.grid ? st + eb.nprob + 2 : nullptr;
-    // the large problems' chains beside the small ones', joined before the next stage
-    EigStreams* es = eb.nsmall > 0 && eb.nlarge > 0 ? &eig_streams(c, eb) : nullptr;
-    auto fork = [&]() -> cudaStream_t {
-        if (!es) return s;
-        PTB_CUDA(cudaEventRecord(es->fork, s));
-        PTB_CUDA(cudaStreamWaitEvent(es->side, es->fork, 0));
-        return es->side;
+    // launches of one stage side by side: the first on s, the others on the side streams,
+    // joined before the next stage
+    const int side0 = eb.async ? EigStreams::kPerBatch : 0;
+    int nside = side0;
+    auto branch = [&](bool first) -> cudaStream_t {
+        if (first) return s;
+        EigStreams& es = eig_streams(c, eb);
+        PTB_CHECK(nside < side0 + EigStreams::kPerBatch, PTBGPU_ECUDA, "eigensolver: more side launches than streams");
+        PTB_CUDA(cudaStreamWaitEvent(es.side[nside], es.fork[eb.async], 0));
+        return es.side[nside++];
+    };
+    auto fork = [&](bool many) {
+        if (many) PTB_CUDA(cudaEventRecord(eig_streams(c, eb).fork[eb.async], s));
     };
     auto join = [&] {
-        if (!es) return;
-        PTB_CUDA(cudaEventRecord(es->join, es->side));
-        PTB_CUDA(cudaStreamWaitEvent(s, es->join, 0));
+        for (int i = side0; i < nside; ++i) {
+            PTB_CUDA(cudaEventRecord(eb.st->join[i], eb.st->side[i]));
+            PTB_CUDA(cudaStreamWaitEvent(s, eb.st->join[i], 0));
+        }
+        nside = side0;
     };
     auto launched = [&](int k = 1) {
         count_launch(k);
         PTB_CUDA(cudaGetLastError());
     };
     // ---- Cholesky
+    fork(eb.nsmall > 0 && eb.nlarge > 0);
     if (eb.nlarge > 0) {
-        const cudaStream_t ls = fork();
+        const cudaStream_t ls = branch(eb.nsmall == 0);
         if (eb.grid) {
             void* args[] = {&dp, &ord_l, &d_maps, &H, &S, &Ca, &Qa, &La, &st, &bar, &err};
             PTB_CUDA(cudaLaunchCooperativeKernel((void*)k_lg_chol, dim3(eb.G), dim3(kT), args, lg_smem_bytes(2), ls));
@@ -1537,27 +1619,27 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Ca, true, st);
         launched(3);
     }
-    // ---- tridiagonalisation
-    if (eb.nlarge > 0) {
-        const cudaStream_t ls = fork();
-        int M = (eb.maxlarge + 1) & ~1;
+    // ---- tridiagonalisation, the widest groups first
+    fork(eb.trd.size() > 1);
+    for (size_t i = 0; i < eb.trd.size(); ++i) {
+        const EigBatch::Trd& t = eb.trd[i];
+        const cudaStream_t ls = branch(i + 1 == eb.trd.size());
+        const int* od = ord + t.off;
+        const size_t sm = sizeof(double) * t.cap;
         if (eb.grid) {
-            void* args[] = {&dp, &ord_l, &M, &Ca, &Da, &Ea, &Ta, &Xa, &st, &bar, &err};
+            int M = t.cap;
+            void* args[] = {&dp, &od, &M, &Ca, &Da, &Ea, &Ta, &Xa, &st, &bar, &err};
             PTB_CUDA(cudaLaunchCooperativeKernel((void*)k_lg_trd, dim3(eb.G), dim3(kT), args, lg_smem_bytes(M), ls));
-        } else {
-            launch_clustered(k_lg_trd, eb.nlarge, eb.G, lg_smem_bytes(M), ls, dp, ord_l, M, Ca, Da, Ea, Ta, Xa,
+        } else if (t.G == 0) {
+            launch_clustered(k_lg_trd, t.n, eb.G, lg_smem_bytes(t.cap), ls, dp, od, t.cap, Ca, Da, Ea, Ta, Xa,
                              (const int*)st, bar, err);
+        } else if (t.G > 1) {
+            launch_clustered(k_trd_cluster, t.n, t.G, sm, ls, dp, od, Ca, Da, Ea, Ta, Xa, t.cap, (const int*)st);
+        } else if (t.nt == 512) {
+            k_eig_trd<512><<<t.n, 512, sm, ls>>>(dp, od, Ca, Da, Ea, Ta, t.cap, st);
+        } else {
+            k_eig_trd<256><<<t.n, 256, sm, ls>>>(dp, od, Ca, Da, Ea, Ta, t.cap, st);
         }
-        launched();
-    }
-    if (eb.n512 > 0) {
-        const int cap = trd_cap(eb.hp[eb.order[0]].m, 512);
-        k_eig_trd<512><<<eb.n512, 512, sizeof(double) * cap, s>>>(dp, ord, Ca, Da, Ea, Ta, cap, st);
-        launched();
-    }
-    if (eb.n512 < eb.nsmall) {
-        const int cap = trd_cap(eb.hp[eb.order[eb.n512]].m, 256);
-        k_eig_trd<256><<<eb.nsmall - eb.n512, 256, sizeof(double) * cap, s>>>(dp, ord + eb.n512, Ca, Da, Ea, Ta, cap, st);
         launched();
     }
     join();
@@ -1639,14 +1721,16 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
     if (!join) {
         // beside what follows on the context's stream
         EigStreams& es = eig_streams(c, *eb);
-        PTB_CUDA(cudaEventRecord(es.fork, s));
-        PTB_CUDA(cudaStreamWaitEvent(es.base, es.fork, 0));
+        PTB_CUDA(cudaEventRecord(es.start, s));
+        PTB_CUDA(cudaStreamWaitEvent(es.base, es.start, 0));
         s = es.base;
         eb->async = true;
     }
     eig_plan(c, *eb, s, kEigBatchMax, nullptr);
-    log_line(prl, 2, " * eigensolver: %d problems, %d above order %d on clusters of %d CTAs, %zu merge levels", eb->nprob,
-             eb->nlarge, kEigBatchMax, eb->G, eb->levels.size());
+    log_line(prl, 2, " * eigensolver: %d problems, %d above order %d, %zu merge levels", eb->nprob, eb->nlarge,
+             kEigBatchMax, eb->levels.size());
+    for (const EigBatch::Trd& t : eb->trd)
+        log_line(prl, 2, " *   tridiagonalisation of %d on %d CTAs of %d threads each", t.n, t.G ? t.G : eb->G, t.nt);
     eig_run(c, *eb, s, H, S, d_maps, d_own_cols, d_ipos, d_e, d_fe);
     if (eb->async) PTB_CUDA(cudaEventRecord(eb->st->done, s));
     return eb;
