@@ -202,10 +202,15 @@ void dgemm_nn(ptbgpu_ctx* c, int64_t n, int64_t ld, double alpha, const double* 
 void dsyrk_sq(ptbgpu_ctx* c, int64_t n, int64_t ld, const double* X, double* C);   // C = X X (X symmetric), full C
 int  dpotrf_lower(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A);              // returns info
 void dtrtri_lower(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A);
-// Device-result forms of frob_dev / has_nan_dev (no host synchronisation): the
-// Frobenius norm into a device double; a NaN sets *flag = 1.
-void frob_to_dev(ptbgpu_ctx* c, int64_t n, int64_t ld, const double* a, double* out);
-void nan_flag_dev(ptbgpu_ctx* c, int64_t count, const double* a, int* flag);
+// Device-result form of frob_dev (no host synchronisation; ld = n): the
+// Frobenius norm into a device double; *nan = 1 if it is a NaN, which it is
+// exactly when the matrix holds one (squares are never negative).
+void frob_to_dev(ptbgpu_ctx* c, int64_t n, const double* a, double* norm, int* nan);
+// out = alpha x + beta y (n x n, ld n; out may be y) and its Frobenius norm, in
+// one pass; the second form leaves the norm on the device.
+double axpby_frob(ptbgpu_ctx* c, int64_t n, double alpha, const double* x, double beta, const double* y, double* out);
+void axpby_frob_to_dev(ptbgpu_ctx* c, int64_t n, double alpha, const double* x, double beta, const double* y,
+                       double* out, double* norm, int* nan);
 void dsyevd(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, double* w);
 int  dsygvd(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, double* B, double* w);
 

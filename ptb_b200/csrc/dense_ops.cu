@@ -199,6 +199,23 @@ __global__ void k_axpby_diag(int64_t n, int64_t ld, double alpha, const double* 
         }
 }
 
+// out = alpha x + beta y (out may be y) and per-block sums of its squares, with
+// k_axpby_diag's arithmetic and k_reduce2d's order: one pass over the matrices
+// in place of an update, a copy, a NaN count and a norm (five launches of about
+// 2.5 us each at order 736).
+__global__ void k_axpby_frob(int64_t n, double alpha, const double* __restrict__ x, double beta, const double* y,
+                             double* out, double* __restrict__ part) {
+    double s = 0.0;
+    for (int64_t j = blockIdx.x; j < n; j += gridDim.x)
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const double v = alpha * x[i + j * n] + beta * y[i + j * n];
+            out[i + j * n] = v;
+            s += v * v;
+        }
+    s = block_sum(s);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+
 // Copy the upper triangle (row i < col j) onto the lower one, 32x32 tiles
 // through shared memory so reads and writes are both coalesced.  blockDim = (32, 8).
 __global__ void k_symmetrize(int64_t n, int64_t ld, double* a) {
@@ -253,9 +270,11 @@ __global__ void k_split3(int64_t count, const float* __restrict__ xf, const __nv
     }
 }
 
+constexpr int kMaxPartials = 148 * 32;   // blocks of a grid-stride kernel, and partials of a reduction
+
 int grid_for(int64_t work, int per = kThreads) {
     int64_t g = (work + per - 1) / per;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(g, 148 * 32));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(g, kMaxPartials));
 }
 
 double host_reduce(ptbgpu_ctx* c, const double* dpart, int nb, bool is_max) {
@@ -337,30 +356,48 @@ double frob_dev(ptbgpu_ctx* c, int64_t n, int64_t ld, const double* a) {
     return std::sqrt(host_reduce(c, p, nb, false));
 }
 
-// Sum of nb partials in index order (as host_reduce), optionally its square
-// root, into a device scalar; or the OR of "sum > 0" into a device flag.
-__global__ void k_sum_partials(const double* __restrict__ p, int nb, double* __restrict__ out, int mode) {
+// Sum of nb partials in index order (as host_reduce), its square root into a
+// device scalar; a NaN sets the flag.  A chain of nb dependent additions by one
+// thread: the others bring the partials into shared memory first, so that the
+// chain waits for an addition (8 clocks) and not for memory (40 -> 5 us for the
+// 736 partials of order 736).
+__global__ void __launch_bounds__(kThreads) k_sum_partials(const double* __restrict__ p, int nb,
+                                                           double* __restrict__ out, int* __restrict__ nan) {
+    __shared__ double sh[kMaxPartials];
+    for (int i = threadIdx.x; i < nb; i += kThreads) sh[i] = p[i];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     double r = 0.0;
-    for (int i = 0; i < nb; ++i) r = r + p[i];
-    if (mode == 0) *out = sqrt(r);
-    else if (mode == 1) *out = r;
-    else if (r > 0.0) *reinterpret_cast<int*>(out) = 1;
+#pragma unroll 16
+    for (int i = 0; i < nb; ++i) r = r + sh[i];
+    *out = sqrt(r);
+    if (r != r) *nan = 1;
 }
 
-void frob_to_dev(ptbgpu_ctx* c, int64_t n, int64_t ld, const double* a, double* out) {
+void frob_to_dev(ptbgpu_ctx* c, int64_t n, const double* a, double* out, int* nan) {
     int nb = grid_for(n, 1);
     double* p = partials(c, nb);
-    k_reduce2d<0><<<nb, kThreads, 0, c->stream>>>(n, ld, a, nullptr, p);
-    k_sum_partials<<<1, 1, 0, c->stream>>>(p, nb, out, 0);
+    k_reduce2d<0><<<nb, kThreads, 0, c->stream>>>(n, n, a, nullptr, p);
+    k_sum_partials<<<1, kThreads, 0, c->stream>>>(p, nb, out, nan);
     count_launch(2);
     PTB_CUDA(cudaGetLastError());
 }
 
-void nan_flag_dev(ptbgpu_ctx* c, int64_t count, const double* a, int* flag) {
-    int nb = grid_for(count);
+double axpby_frob(ptbgpu_ctx* c, int64_t n, double alpha, const double* x, double beta, const double* y, double* out) {
+    int nb = grid_for(n, 1);
     double* p = partials(c, nb);
-    k_reduce1d<2><<<nb, kThreads, 0, c->stream>>>(count, a, nullptr, p);
-    k_sum_partials<<<1, 1, 0, c->stream>>>(p, nb, reinterpret_cast<double*>(flag), 2);
+    k_axpby_frob<<<nb, kThreads, 0, c->stream>>>(n, alpha, x, beta, y, out, p);
+    count_launch();
+    PTB_CUDA(cudaGetLastError());
+    return std::sqrt(host_reduce(c, p, nb, false));
+}
+
+void axpby_frob_to_dev(ptbgpu_ctx* c, int64_t n, double alpha, const double* x, double beta, const double* y,
+                       double* out, double* norm, int* nan) {
+    int nb = grid_for(n, 1);
+    double* p = partials(c, nb);
+    k_axpby_frob<<<nb, kThreads, 0, c->stream>>>(n, alpha, x, beta, y, out, p);
+    k_sum_partials<<<1, kThreads, 0, c->stream>>>(p, nb, norm, nan);
     count_launch(2);
     PTB_CUDA(cudaGetLastError());
 }

@@ -38,6 +38,7 @@ using namespace tc::ptx;
 constexpr int THREADS = 256;
 constexpr int kSmemBudget = 196608;
 constexpr int kTmemCols = 512;
+constexpr int kSms = 148;
 // Dynamic shared memory that keeps a kernel at one resident CTA per SM (more
 // than half of the 227 KB a block may use).  The CTA-pair kernels hold all 512
 // TMEM columns of both SMs of a pair: two pair CTAs resident on the same SMs
@@ -120,6 +121,69 @@ __global__ void k_oz_rowmax(const double* __restrict__ M, int64_t rs, int64_t cs
     }
 }
 
+// The S digits of a fraction that is not below 1 in magnitude or not a number
+// (infinities, and what shares a row with one), byte b = digit S - 1 - b.
+template <int S>
+__device__ __noinline__ uint2 slice_digits_general(double x) {
+    uint32_t w[2] = {0u, 0u};
+#pragma unroll 1
+    for (int p = S - 1; p >= 0; --p) {
+        x *= 128.0;
+        const double q = trunc(x);
+        x -= q;
+        const uint32_t byte = (uint32_t)(uint8_t)(int8_t)(int)q;
+        if (p >= 4) w[1] |= byte << (8 * (p - 4));
+        else w[0] |= byte << (8 * p);
+    }
+    return make_uint2(w[0], w[1]);
+}
+// 28 bits spread into four bytes of 7, each negated for neg = all ones.
+__device__ __forceinline__ uint32_t spread7(uint32_t a, bool neg) {
+    a = (a & 0x3FFFu) | ((a & 0x0FFFC000u) << 2);
+    a = (a & 0x007F007Fu) | ((a & 0x3F803F80u) << 1);
+    return neg ? (0x80808080u - a) ^ 0x80808080u : a;   // no borrow: every byte <= 127
+}
+
+// The S 7-bit slices of eight elements x sc, eight bytes per slice: the base-128
+// digits of the fraction, truncated towards zero, each with the element's sign.
+// trunc(|x| 2^(7S)) holds them all (7S <= 56 bits): one conversion, a spread of
+// the bits into bytes and a byte transpose, about 30 instructions per element
+// in place of S rounds of multiply, truncate, subtract and convert in FP64
+// (k_oz_slice at order 3073: 54 -> 43 us).
+template <int S>
+__device__ __forceinline__ void slice8(const double* v, double sc, uint2 (&out)[S]) {
+    uint32_t o[2][8];   // [elements 0..3, 4..7][byte]
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t lo[4], hi[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double x = v[4 * h + j] * sc;
+            if (fabs(x) < 1.0) {
+                const unsigned long long t = (unsigned long long)(fabs(x) * (double)(1ull << (7 * S)));
+                lo[j] = spread7((uint32_t)t & 0x0FFFFFFFu, x < 0.0);
+                hi[j] = S > 4 ? spread7((uint32_t)(t >> 28), x < 0.0) : 0u;
+            } else {
+                const uint2 d = slice_digits_general<S>(x);
+                lo[j] = d.x;
+                hi[j] = d.y;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const uint32_t* a = q == 0 ? lo : hi;
+            const uint32_t t0 = __byte_perm(a[0], a[1], 0x5140), t1 = __byte_perm(a[2], a[3], 0x5140);
+            const uint32_t t2 = __byte_perm(a[0], a[1], 0x7362), t3 = __byte_perm(a[2], a[3], 0x7362);
+            o[h][4 * q + 0] = __byte_perm(t0, t1, 0x5410);
+            o[h][4 * q + 1] = __byte_perm(t0, t1, 0x7632);
+            o[h][4 * q + 2] = __byte_perm(t2, t3, 0x5410);
+            o[h][4 * q + 3] = __byte_perm(t2, t3, 0x7632);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < S; ++p) out[p] = make_uint2(o[0][S - 1 - p], o[1][S - 1 - p]);
+}
+
 // Slices of a 32-row x 64-column tile; rows/columns beyond n (the padding up
 // to ldp) are written as zero.  e_i: |M(i,k)| < 2^e_i, taken from the
 // exponent field of the row maximum.
@@ -155,24 +219,86 @@ __global__ void k_oz_slice(const double* __restrict__ M, int64_t rs, int64_t cs,
     }
     if (blockIdx.x == 0 && (threadIdx.x & 7) == 0) exps[i] = e;
     const double sc = pow2i(-e);
-    uint32_t w[S][2];
-#pragma unroll
-    for (int p = 0; p < S; ++p) w[p][0] = w[p][1] = 0u;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        double x = t[r][kq + j] * sc;   // |x| < 1
-#pragma unroll
-        for (int p = 0; p < S; ++p) {
-            x *= 128.0;
-            const double q = trunc(x);   // |q| <= 127
-            x -= q;                      // exact: the fraction of x
-            const uint32_t byte = (uint32_t)(uint8_t)(int8_t)(int)q;
-            w[p][j >> 2] |= byte << (8 * (j & 3));
-        }
-    }
+    uint2 q[S];
+    slice8<S>(&t[r][kq], sc, q);
 #pragma unroll
     for (int p = 0; p < S; ++p)
-        *reinterpret_cast<uint2*>(planes + ((int64_t)p * ldp + i) * ldp + k0 + kq) = make_uint2(w[p][0], w[p][1]);
+        *reinterpret_cast<uint2*>(planes + ((int64_t)p * ldp + i) * ldp + k0 + kq) = q[p];
+}
+
+// One or two operands sliced in one launch, kSliceRows rows of one operand per
+// CTA: the rows go to shared memory once, and warp w takes row w from there for
+// its maximum and its slices, so the matrix is read once and no maxima pass,
+// clearing or atomics come before it.  Figures at kSliceRowsMax below.
+//   tile element (row, k) at row * pitch + k + k / 8: a warp reads 32 groups of
+//   8 columns with stride 9 and (columns contiguous in memory) writes 8 rows x 4
+//   columns with row stride 2 mod 16 doubles, both without bank conflicts.
+constexpr int kSliceRows = THREADS / 32;
+constexpr int kSliceAhead = 12;   // loads of a thread in flight
+struct SliceJob {
+    const double* M;
+    int64_t rs, cs;
+    int tri;
+    int8_t* planes;
+    int* exps;
+};
+struct SliceJobs {
+    SliceJob j[2];
+};
+__host__ __device__ constexpr int slice_pitch(int64_t ldp) {
+    return (int)((ldp + ldp / 8 + 13) / 16 * 16 + 2);   // >= ldp + ldp / 8, 2 mod 16
+}
+constexpr int slice_smem(int64_t ldp) { return kSliceRows * slice_pitch(ldp) * (int)sizeof(double); }
+
+template <int S>
+__global__ void __launch_bounds__(THREADS) k_oz_slice_rows(const __grid_constant__ SliceJobs jobs, int64_t n,
+                                                           int64_t ldp) {
+    extern __shared__ double tile[];
+    const SliceJob& jb = jobs.j[blockIdx.y];
+    const int pitch = slice_pitch(ldp);
+    const int64_t i0 = (int64_t)blockIdx.x * kSliceRows;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tri = jb.tri;
+    // lanes along the contiguous index: 32 columns of row w, or 8 rows x 4 columns
+    const bool rowc = jb.cs == 1;
+    const int r = rowc ? w : lane & 7, kq = rowc ? lane : 4 * w + (lane >> 3);
+    const int64_t il = i0 + r;
+    const double* __restrict__ src = jb.M + (il < n ? il : n - 1) * jb.rs;
+    double* trow = tile + r * pitch;
+    for (int k0 = kq; k0 < (int)ldp; k0 += 32 * kSliceAhead) {
+        double v[kSliceAhead];   // loads at clamped positions, so that all are in flight together
+#pragma unroll
+        for (int u = 0; u < kSliceAhead; ++u) {
+            const int64_t k = k0 + 32 * u;
+            v[u] = __ldg(src + (k < n ? k : n - 1) * jb.cs);
+        }
+#pragma unroll
+        for (int u = 0; u < kSliceAhead; ++u) {
+            const int k = k0 + 32 * u;
+            if (k < (int)ldp) trow[k + (k >> 3)] = (il < n && k < n && tri_keep(tri, il, k)) ? v[u] : 0.0;
+        }
+    }
+    __syncthreads();
+    const double* row = tile + w * pitch;
+    double m = 0.0;
+#pragma unroll 8
+    for (int k = lane; k < (int)ldp; k += 32) m = fmax(m, fabs(row[k + (k >> 3)]));
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const int64_t i = i0 + w;
+    int e = 0;
+    if (m > 0.0) {
+        const int fld = (int)((__double_as_longlong(m) >> 52) & 0x7FF);
+        e = fld == 0 ? -1022 : fld - 1022;   // as k_oz_slice
+    }
+    if (lane == 0) jb.exps[i] = e;
+    const double sc = pow2i(-e);
+    for (int g = lane; g < (int)ldp / 8; g += 32) {
+        uint2 q[S];
+        slice8<S>(row + 9 * g, sc, q);
+#pragma unroll
+        for (int p = 0; p < S; ++p)
+            *reinterpret_cast<uint2*>(jb.planes + ((int64_t)p * ldp + i) * ldp + g * 8) = q[p];
+    }
 }
 
 // ---- product ---------------------------------------------------------------
@@ -1398,23 +1524,70 @@ int64_t max_k(int S) { return (int64_t)2147483647 / ((int64_t)S * 127 * 127); }
 int64_t padded(int64_t n) { return round_up(n, BM); }
 bool supported(int64_t n, int S) { return (S == 4 || (S >= 6 && S <= 8)) && padded(n) <= max_k(S); }
 
-void slice(cudaStream_t s, const double* M, int64_t rs, int64_t cs, int64_t n, int tri, const Operand& op,
-           unsigned long long* rowmax) {
-    PTB_CHECK(rs == 1 || cs == 1, PTBGPU_EINVAL, "slicing needs rows or columns contiguous");
-    PTB_CHECK(op.ldp >= n && op.ldp % BM == 0, PTBGPU_EINVAL, "bad slice leading dimension");
-    PTB_CUDA(cudaMemsetAsync(rowmax, 0, sizeof(unsigned long long) * (size_t)op.ldp, s));
-    const dim3 g1((unsigned)((n + 127) / 128), (unsigned)((n + 31) / 32));
-    k_oz_rowmax<<<g1, THREADS, 0, s>>>(M, rs, cs, n, tri, rowmax);
+namespace {
+// Padded orders whose slices k_oz_slice_rows takes.  Both operands of an order-736
+// product in one launch 10.3 us, against 19 us in six (maxima cleared, maxima and
+// slices of each operand).  Per operand the two ways meet near order 1500 (19.8
+// and 19 us); at 2048 the pass through shared memory, with fewer loads in flight,
+// takes 38 us against 27.
+constexpr int64_t kSliceRowsMax = 1536;
+
+template <int S>
+void launch_slice_rows(cudaStream_t s, const SliceJobs& jobs, int count, int64_t n, int64_t ldp) {
+    static const bool attr = [] {   // thread-safe one-time setup
+        PTB_CUDA(cudaFuncSetAttribute(k_oz_slice_rows<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      slice_smem(kSliceRowsMax)));
+        return true;
+    }();
+    (void)attr;
+    k_oz_slice_rows<S><<<dim3((unsigned)(ldp / kSliceRows), (unsigned)count), THREADS, slice_smem(ldp), s>>>(jobs, n,
+                                                                                                          ldp);
     count_launch();
-    const dim3 g2((unsigned)(op.ldp / 64), (unsigned)(op.ldp / 32));
-    switch (op.S) {
-        case 4: k_oz_slice<4><<<g2, THREADS, 0, s>>>(M, rs, cs, n, tri, rowmax, op.planes, op.exps, op.ldp); break;
-        case 6: k_oz_slice<6><<<g2, THREADS, 0, s>>>(M, rs, cs, n, tri, rowmax, op.planes, op.exps, op.ldp); break;
-        case 7: k_oz_slice<7><<<g2, THREADS, 0, s>>>(M, rs, cs, n, tri, rowmax, op.planes, op.exps, op.ldp); break;
-        case 8: k_oz_slice<8><<<g2, THREADS, 0, s>>>(M, rs, cs, n, tri, rowmax, op.planes, op.exps, op.ldp); break;
-        default: PTB_CHECK(false, PTBGPU_EINVAL, "unsupported slice count %d (4, 6, 7 or 8)", op.S);
+}
+
+template <int S>
+void launch_slice(cudaStream_t s, const SliceSrc& a, int64_t n, unsigned long long* rowmax) {
+    const dim3 g((unsigned)(a.op.ldp / 64), (unsigned)(a.op.ldp / 32));
+    k_oz_slice<S><<<g, THREADS, 0, s>>>(a.M, a.rs, a.cs, n, a.tri, rowmax, a.op.planes, a.op.exps, a.op.ldp);
+    count_launch();
+}
+
+template <int S>
+void slice_s(cudaStream_t s, const SliceSrc* src, int count, int64_t n, unsigned long long* rowmax) {
+    const int64_t ldp = src[0].op.ldp;
+    if (ldp <= kSliceRowsMax) {
+        SliceJobs jobs{};
+        for (int k = 0; k < count; ++k)
+            jobs.j[k] = {src[k].M, src[k].rs, src[k].cs, src[k].tri, src[k].op.planes, src[k].op.exps};
+        launch_slice_rows<S>(s, jobs, count, n, ldp);
+        return;
     }
-    count_launch();
+    for (int k = 0; k < count; ++k) {
+        const SliceSrc& a = src[k];
+        PTB_CUDA(cudaMemsetAsync(rowmax, 0, sizeof(unsigned long long) * (size_t)ldp, s));
+        const dim3 g1((unsigned)((n + 127) / 128), (unsigned)((n + 31) / 32));
+        k_oz_rowmax<<<g1, THREADS, 0, s>>>(a.M, a.rs, a.cs, n, a.tri, rowmax);
+        count_launch();
+        launch_slice<S>(s, a, n, rowmax);
+    }
+}
+}  // namespace
+
+void slice(cudaStream_t s, const SliceSrc* src, int count, int64_t n, unsigned long long* rowmax) {
+    PTB_CHECK(count == 1 || count == 2, PTBGPU_EINVAL, "one or two operands are sliced at a time");
+    for (int k = 0; k < count; ++k) {
+        PTB_CHECK(src[k].rs == 1 || src[k].cs == 1, PTBGPU_EINVAL, "slicing needs rows or columns contiguous");
+        PTB_CHECK(src[k].op.ldp >= n && src[k].op.ldp % BM == 0, PTBGPU_EINVAL, "bad slice leading dimension");
+        PTB_CHECK(src[k].op.ldp == src[0].op.ldp && src[k].op.S == src[0].op.S, PTBGPU_EINVAL,
+                  "operands do not match");
+    }
+    switch (src[0].op.S) {
+        case 4: slice_s<4>(s, src, count, n, rowmax); break;
+        case 6: slice_s<6>(s, src, count, n, rowmax); break;
+        case 7: slice_s<7>(s, src, count, n, rowmax); break;
+        case 8: slice_s<8>(s, src, count, n, rowmax); break;
+        default: PTB_CHECK(false, PTBGPU_EINVAL, "unsupported slice count %d (4, 6, 7 or 8)", src[0].op.S);
+    }
     PTB_CUDA(cudaGetLastError());
 }
 
@@ -1424,6 +1597,14 @@ int resolve_variant(int variant, int S, int rb) {
     // with 6, 7 or 8 slices at ndim 4096-11776 (N = 128 MMAs: x1.09-1.22 on one CTA;
     // the pair halves the B loads per SM); they take 32-byte K blocks only
     return S >= 6 && rb != 64 ? V_WPAIR : V_SMEM_A;
+}
+
+int variant_for(int64_t ldp, int S) {
+    // 128 x 64 tiles on one CTA while they fit one wave: a 256 x 128 pair tile then
+    // leaves more than half of the SMs idle (order 736, 8 slices: 72 CTAs 25 us, 36
+    // CTAs 58 us; order 900: 128 CTAs 33 us, 64 CTAs 66 us).  Above one wave the
+    // pair is faster again (order 1100: 162 CTAs 87 us, 90 CTAs 72 us).
+    return (ldp / BM) * (ldp / BN) <= kSms ? V_SMEM_A : resolve_variant(V_DEFAULT, S, 0);
 }
 
 int tile_n(int S, int variant) {

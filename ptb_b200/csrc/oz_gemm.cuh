@@ -60,9 +60,15 @@ bool supported(int64_t n, int S);
 int64_t padded(int64_t n);   // round_up(n, 128)
 
 // Slices of M(i,k) = M[i * rs + k * cs] (rs == 1 or cs == 1), i,k < n, masked by
-// `tri`.  `rowmax` is device scratch of ldp 64-bit words.
-void slice(cudaStream_t s, const double* M, int64_t rs, int64_t cs, int64_t n, int tri, const Operand& op,
-           unsigned long long* rowmax);
+// `tri`, of one or two operands of the same shape.  `rowmax` is device scratch of
+// ldp 64-bit words.
+struct SliceSrc {
+    const double* M;
+    int64_t rs, cs;
+    int tri;
+    Operand op;
+};
+void slice(cudaStream_t s, const SliceSrc* src, int count, int64_t n, unsigned long long* rowmax);
 
 // Kernel variants: A slices re-read from shared memory by every MMA (64-column
 // tiles), or copied once per K step into tensor memory (48-column tiles for 7
@@ -75,6 +81,9 @@ enum Variant : int { V_DEFAULT = 0, V_SMEM_A = 1, V_TMEM_A = 2, V_PAIR = 3, V_WI
 // The variant V_DEFAULT stands for with S slices and rb-byte K blocks (0 = the
 // variant's default); the functions below take resolved variants only.
 int resolve_variant(int variant, int S, int rb);
+// The fastest variant for a whole (not triangular) product of padded order ldp,
+// with its default K blocks.
+int variant_for(int64_t ldp, int S);
 int tile_n(int S, int variant);   // output columns per tile
 
 // Tiles {bi, bj, k0, k1}: 128-row blocks of ldp by bn-column blocks (the last

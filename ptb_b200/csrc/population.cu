@@ -158,9 +158,9 @@ void mlpop2_diag_device(ptbgpu_ctx* c, int64_t n, const double* dPpk, const floa
     ob.exps = beb.as<int>();
     oa.ldp = ob.ldp = ldp;
     oa.S = ob.S = S;
-    oz::slice(s, P, 1, n, n, oz::TRI_NONE, oa, brm.as<unsigned long long>());
-    oz::slice(s, S1, n, 1, n, oz::TRI_NONE, ob, brm.as<unsigned long long>());
-    const int variant = oz::resolve_variant(oz::V_DEFAULT, S, 0);
+    const oz::SliceSrc src[2] = {{P, 1, n, oz::TRI_NONE, oa}, {S1, n, 1, oz::TRI_NONE, ob}};
+    oz::slice(s, src, 2, n, brm.as<unsigned long long>());
+    const int variant = oz::variant_for(ldp, S);
     const std::vector<int4> t = oz::build_tiles(ldp, false, oz::TRI_NONE, oz::TRI_NONE, S, variant);
     DevBuf& bt = c->buf(B_OZT);
     bt.reserve(sizeof(int4) * t.size());

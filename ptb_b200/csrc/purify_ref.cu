@@ -80,14 +80,13 @@ struct LoopDev {
     int pad;
 };
 
-// sign_iterative's rule (source/purification.f90:587): stop when
-// | ||X||_F - ||X_prev||_F | < thrs%normal, at the cycle cap, or on a NaN.
-// McWeeny's rule (source/purification.f90:496) is the same with the norm
-// carried over to the next iteration.
-__global__ void k_loop_decide(cudaGraphConditionalHandle h, LoopDev* d, double thr, long long cycles, int carry) {
+// sign_iterative's rule (source/purification.f90:587) and McWeeny's
+// (source/purification.f90:496): stop when | ||X||_F - ||X_prev||_F | <
+// thrs%normal, at the cycle cap, or on a NaN.
+__global__ void k_loop_decide(cudaGraphConditionalHandle h, LoopDev* d, double thr, long long cycles) {
     d->iters += 1;
     const bool stop = d->nan != 0 || std::fabs(d->norm1 - d->norm0) < thr || d->iters >= cycles;
-    if (!stop && carry) d->norm0 = d->norm1;
+    if (!stop) d->norm0 = d->norm1;
     cudaGraphSetConditional(h, stop ? 0u : 1u);
 }
 
@@ -150,7 +149,7 @@ struct Ctx {
     // kernel; false if the stream could not be captured (then the loop runs
     // eagerly).
     template <class Body>
-    bool build_loop(LoopGraph& lg, Body body, double thr, long long cycles, int carry) {
+    bool build_loop(LoopGraph& lg, Body body, double thr, long long cycles) {
         if (lg.exec) return true;
         if (lg.failed) return false;
         cudaStream_t s = c->stream;
@@ -175,7 +174,7 @@ struct Ctx {
             const double f0 = gemm_flops;
             try {
                 body();
-                k_loop_decide<<<1, 1, 0, s>>>(lg.handle, d, thr, cycles, carry);
+                k_loop_decide<<<1, 1, 0, s>>>(lg.handle, d, thr, cycles);
                 count_launch();
             } catch (...) {
                 ok = false;
@@ -325,37 +324,32 @@ void mcweeny(Ctx& x, const ptbgpu_pur_settings& pur, const double* guess, const 
     double* t3 = x.m[7];
     copy_mat(s, n, n, guess, n, g);
     double norm = x.frob(g);
-    copy_mat(s, n, n, guess, n, P);
-    auto step = [&] {
+    auto products = [&] {
         x.gemm(S, g, t1);
         x.gemm(g, t1, t2);
         x.gemm(t2, t1, t3);
-        copy_mat(s, n, n, t2, n, P);
-        axpby_diag(s, n, n, -2.0, t3, 3.0, P, 0.0);
-    };
+    };   // the new iterate is 3 t2 - 2 t3
     for (int64_t i = 0; i < pur.cycles; ++i) {
-        step();
-        x.nan_check(P, "Error: NaN is encountered during purification");
-        const double np = x.frob(P);
+        products();
+        const double np = axpby_frob(x.c, n, -2.0, t3, 3.0, t2, g);
+        PTB_CHECK(!std::isnan(np), PTBGPU_ENAN, "%s", "Error: NaN is encountered during purification");
         if (std::fabs(np - norm) < x.thr.normal) break;
-        copy_mat(s, n, n, P, n, g);
         norm = np;
         // the remaining iterations as one graph launch (the stop rule on the device)
         if (i + 1 < pur.cycles && graph_loops()) {
             LoopDev* d = x.ld();
             auto body = [&] {
-                step();
-                nan_flag_dev(x.c, n * n, P, &d->nan);
-                frob_to_dev(x.c, n, n, P, &d->norm1);
-                copy_mat(s, n, n, P, n, g);   // the next iteration's input (unused after the last)
+                products();
+                axpby_frob_to_dev(x.c, n, -2.0, t3, 3.0, t2, g, &d->norm1, &d->nan);
             };
-            if (x.build_loop(x.mcw_loop, body, x.thr.normal, (long long)pur.cycles, 1)) {
+            if (x.build_loop(x.mcw_loop, body, x.thr.normal, (long long)pur.cycles)) {
                 const LoopDev r = x.run_loop(x.mcw_loop, LoopDev{norm, 0.0, (long long)(i + 1), 0, 0});
                 PTB_CHECK(r.nan == 0, PTBGPU_ENAN, "%s", "Error: NaN is encountered during purification");
                 break;
             }
         }
     }
+    copy_mat(s, n, n, g, n, P);
     axpby_diag(s, n, n, 0.0, nullptr, 2.0, P, 0.0);
 }
 
@@ -388,37 +382,46 @@ void sign_iterative(Ctx& x, const ptbgpu_pur_settings& pur, const double* guess,
     double* t2 = x.m[6];
     double* t3 = x.m[7];
     copy_mat(s, n, n, guess, n, Y);
-    auto step = [&] {
-        if (pur.type == PTBGPU_TYPE_PADE) {
-            x.gemm(Y, Y, t1);
-            x.gemm(t1, t1, t2);
-            copy_mat(s, n, n, t2, n, t3);
-            axpby_diag(s, n, n, -10.0, t1, 3.0, t3, 15.0);   // 15 I - 10 X^2 + 3 X^4
-            x.gemm(Y, t3, t1, 0.125);
-            copy_mat(s, n, n, t1, n, Y);
-        } else {
-            x.gemm(Y, Y, t1);
-            x.gemm(Y, t1, t2);
-            axpby_diag(s, n, n, -0.5, t2, 1.5, Y, 0.0);      // 0.5 (3X - X^3)
-        }
+    auto pade = [&] {
+        x.gemm(Y, Y, t1);
+        x.gemm(t1, t1, t2);
+        copy_mat(s, n, n, t2, n, t3);
+        axpby_diag(s, n, n, -10.0, t1, 3.0, t3, 15.0);   // 15 I - 10 X^2 + 3 X^4
+        x.gemm(Y, t3, t1, 0.125);
+        copy_mat(s, n, n, t1, n, Y);
     };
+    auto newton_schulz = [&] {   // the new iterate is 0.5 (3X - X^3) = 1.5 Y - 0.5 t2
+        x.gemm(Y, Y, t1);
+        x.gemm(Y, t1, t2);
+    };
+    double norm = x.frob(Y);
     for (int64_t i = 0; i < pur.cycles; ++i) {
-        const double norm = x.frob(Y);
         ++*iters;
-        step();
-        x.nan_check(Y, "Error: NaN is encountered during purification");
-        if (std::fabs(x.frob(Y) - norm) < x.thr.normal) break;
+        double np;
+        if (pur.type == PTBGPU_TYPE_PADE) {
+            pade();
+            np = x.frob(Y);
+        } else {
+            newton_schulz();
+            np = axpby_frob(x.c, n, -0.5, t2, 1.5, Y, Y);
+        }
+        PTB_CHECK(!std::isnan(np), PTBGPU_ENAN, "%s", "Error: NaN is encountered during purification");
+        if (std::fabs(np - norm) < x.thr.normal) break;
+        norm = np;
         // the remaining iterations as one graph launch (the stop rule on the device)
         if (i + 1 < pur.cycles && graph_loops()) {
             LoopDev* d = x.ld();
             auto body = [&] {
-                frob_to_dev(x.c, n, n, Y, &d->norm0);
-                step();
-                nan_flag_dev(x.c, n * n, Y, &d->nan);
-                frob_to_dev(x.c, n, n, Y, &d->norm1);
+                if (pur.type == PTBGPU_TYPE_PADE) {
+                    pade();
+                    frob_to_dev(x.c, n, Y, &d->norm1, &d->nan);
+                } else {
+                    newton_schulz();
+                    axpby_frob_to_dev(x.c, n, -0.5, t2, 1.5, Y, Y, &d->norm1, &d->nan);
+                }
             };
-            if (x.build_loop(x.sign_loop, body, x.thr.normal, (long long)pur.cycles, 0)) {
-                const LoopDev r = x.run_loop(x.sign_loop, LoopDev{0.0, 0.0, (long long)(i + 1), 0, 0});
+            if (x.build_loop(x.sign_loop, body, x.thr.normal, (long long)pur.cycles)) {
+                const LoopDev r = x.run_loop(x.sign_loop, LoopDev{norm, 0.0, (long long)(i + 1), 0, 0});
                 *iters += r.iters - (i + 1);
                 PTB_CHECK(r.nan == 0, PTBGPU_ENAN, "%s", "Error: NaN is encountered during purification");
                 break;

@@ -305,10 +305,14 @@ oz::Operand oz_operand(ptbgpu_ctx* c, int slot, int64_t n, int S) {
     return op;
 }
 
-void oz_slice(ptbgpu_ctx* c, const double* M, int64_t rs, int64_t cs, int64_t n, int tri, const oz::Operand& op) {
+void oz_slice(ptbgpu_ctx* c, const oz::SliceSrc* src, int count, int64_t n) {
     DevBuf& br = c->buf(B_OZR);
-    br.reserve(sizeof(unsigned long long) * (size_t)op.ldp);
-    oz::slice(c->stream, M, rs, cs, n, tri, op, br.as<unsigned long long>());
+    br.reserve(sizeof(unsigned long long) * (size_t)src[0].op.ldp);
+    oz::slice(c->stream, src, count, n, br.as<unsigned long long>());
+}
+void oz_slice(ptbgpu_ctx* c, const double* M, int64_t rs, int64_t cs, int64_t n, int tri, const oz::Operand& op) {
+    const oz::SliceSrc src{M, rs, cs, tri, op};
+    oz_slice(c, &src, 1, n);
 }
 
 // One product over a freshly uploaded tile list, bracketed by CUDA events.
@@ -1135,7 +1139,7 @@ void oz_dgemm(ptbgpu_ctx* c, int64_t n, double alpha, const double* A, bool ta, 
     if (!c->oz_tile_cache) c->oz_tile_cache = std::make_shared<OzTileCache>();
     OzTileCache& tc = *static_cast<OzTileCache*>(c->oz_tile_cache.get());
     const oz::Operand opA = oz_operand(c, 0, n, S), opB = oz_operand(c, 1, n, S);
-    const int variant = oz::resolve_variant(oz::V_DEFAULT, S, 0);
+    const int variant = oz::variant_for(opA.ldp, S);
     auto key = std::make_pair(n, S);
     auto it = tc.lists.find(key);
     if (it == tc.lists.end()) {
@@ -1149,9 +1153,10 @@ void oz_dgemm(ptbgpu_ctx* c, int64_t n, double alpha, const double* A, bool ta, 
     }
     c->oz_ops += it->second.ops;
     // rows i of op(A): A(i,k) = A[i + k n], A^T(i,k) = A[k + i n]
-    oz_slice(c, A, ta ? n : 1, ta ? 1 : n, n, oz::TRI_NONE, opA);
     // rows j of op(B)^T, i.e. op(B)(k, j): B[k + j n], or B^T: B[j + k n]
-    oz_slice(c, B, tb ? 1 : n, tb ? n : 1, n, oz::TRI_NONE, opB);
+    const oz::SliceSrc src[2] = {{A, ta ? n : 1, ta ? 1 : n, oz::TRI_NONE, opA},
+                                 {B, tb ? 1 : n, tb ? n : 1, oz::TRI_NONE, opB}};
+    oz_slice(c, src, 2, n);
     oz::OzEpi ep;
     ep.n = n;
     ep.alpha = alpha;
