@@ -7,7 +7,7 @@
 // or the triangular solve, (problem, tile) where it is a product.
 
 // T of one panel of reflectors per CTA (tasks: problem, panel).
-constexpr size_t kWySmem = sizeof(double) * (2 * kStageOp + NB * NB + NB * (NB + 1));
+constexpr size_t kWySmem = sizeof(double) * (2 * kStageOp + TS * TS + TS * kTld);
 __global__ void __launch_bounds__(kT, 2) k_vec_panels(const EigProb* __restrict__ probs,
                                                       const int2* __restrict__ tasks, const double* __restrict__ Ca,
                                                       const double* __restrict__ Ta, double* __restrict__ Ka,
@@ -15,43 +15,44 @@ __global__ void __launch_bounds__(kT, 2) k_vec_panels(const EigProb* __restrict_
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     double* sB = sA + kStageOp;
-    double* Gg = sB + kStageOp;
+    double* G = sB + kStageOp;
     const int2 tk = tasks[blockIdx.x];
     if (status[tk.x] != kStOk) return;
     const EigProb p = probs[tk.x];
-    build_T(Ca + p.coff, p.ldc, p.m, Ta + p.voff, Ka + p.koff, tk.y, 1 << 20, Gg, Gg + NB * NB, sA, sB);
+    build_T(Ca + p.coff, p.ldc, p.m, Ta + p.voff, Ka + p.koff + (int64_t)tk.y * TS * TS, tk.y, G, G + TS * TS, sA, sB);
 }
 
-constexpr size_t kChainSmem = sizeof(double) * (2 * kStageOp + TS * (TS + 1) + 2 * NB * TS);
+constexpr size_t kChainSmem = sizeof(double) * (2 * kStageOp + TS * TS + TS * kY2ld);
 
 // Rows of L (S U) and of L^-T (U) for the owned columns, times Q: block u of the 2 nown
 // vectors (the rows of L first).
 __global__ void __launch_bounds__(kT, 2) k_vec_rows(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ Ca, const double* __restrict__ La,
-                                                    const double* __restrict__ Ka, const int* __restrict__ own_cols,
+                                                    const double* __restrict__ Ia, const double* __restrict__ Ka, const int* __restrict__ own_cols,
                                                     const int* __restrict__ ipos, double* __restrict__ Ba,
                                                     const int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     double* sB = sA + kStageOp;
-    double* sD = sB + kStageOp;
-    double* Y = sD + TS * (TS + 1);
+    double* Y = sB + kStageOp;
     const int2 tk = tasks[blockIdx.x];
     if (status[tk.x] != kStOk) return;
     const EigProb p = probs[tk.x];
     const int m = p.m, no = p.nown, u0 = tk.y * TS, u1 = min(2 * no, u0 + TS);
     const double* L = La + p.aoff;
     double* R = Ba + p.boff;
+    int top = m;   // L^-1 e_c is zero above row c
     for (int u = u0; u < u1; ++u) {
         const int ct = ipos[own_cols[p.o0 + (u < no ? u : u - no)]];
+        if (u >= no) top = min(top, ct);
         double* x = R + (int64_t)u * m;
         for (int r = threadIdx.x; r < m; r += kT)
             x[r] = (u < no) ? ((r <= ct) ? L[ct + (int64_t)r * m] : 0.0) : ((r == ct) ? 1.0 : 0.0);
     }
     __syncthreads();
     const int s0 = max(u0, no);
-    if (s0 < u1) trsm_cols(true, L, m, R + (int64_t)s0 * m, m, 0, u1 - s0, sD, sA, sB);
-    wy_apply_t(Ca + p.coff, p.ldc, m, Ka + p.koff, R + (int64_t)u0 * m, u1 - u0, true, Y, Y + NB * TS, sA, sB);
+    if (s0 < u1) trsm_cols(true, L, m, Ia + p.ioff, R + (int64_t)s0 * m, m, u1 - s0, sA, sB, top);
+    wy_apply(Ca + p.coff, p.ldc, m, Ka + p.koff, R + (int64_t)u0 * m, u1 - u0, true, Y, Y + TS * TS, sA, sB);
 }
 
 // Z = Q V of the top merge is not formed: Q (m x m, at Qa; the leaf's Z of a problem
@@ -184,21 +185,20 @@ __global__ void __launch_bounds__(kT, 2) k_fin_qw(const EigProb* __restrict__ pr
 
 __global__ void __launch_bounds__(kT, 2) k_fin_cols(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ Ca, const double* __restrict__ La,
-                                                    const double* __restrict__ Ka, const int* __restrict__ maps,
+                                                    const double* __restrict__ Ia, const double* __restrict__ Ka, const int* __restrict__ maps,
                                                     const int* __restrict__ own_cols, double* __restrict__ Ba,
                                                     double* __restrict__ Ppk, double* __restrict__ Pdense) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     double* sB = sA + kStageOp;
-    double* sD = sB + kStageOp;
-    double* Y = sD + TS * (TS + 1);
+    double* Y = sB + kStageOp;
     const int2 tk = tasks[blockIdx.x];
     const EigProb p = probs[tk.x];
     const int m = p.m, t0 = tk.y * TS, nt = min(TS, p.nown - t0);
     double* W = Ba + p.boff + (int64_t)t0 * m;
-    wy_apply_t(Ca + p.coff, p.ldc, m, Ka + p.koff, W, nt, false, Y, Y + NB * TS, sA, sB);
+    wy_apply(Ca + p.coff, p.ldc, m, Ka + p.koff, W, nt, false, Y, Y + TS * TS, sA, sB);
     __syncthreads();
-    trsm_cols(false, La + p.aoff, m, W, m, 0, nt, sD, sA, sB);
+    trsm_cols(false, La + p.aoff, m, Ia + p.ioff, W, m, nt, sA, sB);
     if (Pdense) {
         for (int64_t q = threadIdx.x; q < (int64_t)nt * m; q += kT) Pdense[p.poff + (int64_t)t0 * m + q] = W[q];
         return;
@@ -218,21 +218,20 @@ __global__ void __launch_bounds__(kT, 2) k_fin_cols(const EigProb* __restrict__ 
 // nocc lowest for a density)
 __global__ void __launch_bounds__(kT, 2) k_vec_back(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ Ca, const double* __restrict__ La,
-                                                    const double* __restrict__ Ka, double* __restrict__ Za,
+                                                    const double* __restrict__ Ia, const double* __restrict__ Ka, double* __restrict__ Za,
                                                     const int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     double* sB = sA + kStageOp;
-    double* sD = sB + kStageOp;
-    double* Y = sD + TS * (TS + 1);
+    double* Y = sB + kStageOp;
     const int2 tk = tasks[blockIdx.x];
     if (status[tk.x] != kStOk) return;
     const EigProb p = probs[tk.x];
     const int m = p.m, nv = p.mode == 2 ? p.nocc : m, t0 = tk.y * TS, nt = min(TS, nv - t0);
     double* U = Za + p.aoff + (int64_t)t0 * m;
-    wy_apply_t(Ca + p.coff, p.ldc, m, Ka + p.koff, U, nt, false, Y, Y + NB * TS, sA, sB);
+    wy_apply(Ca + p.coff, p.ldc, m, Ka + p.koff, U, nt, false, Y, Y + TS * TS, sA, sB);
     __syncthreads();
-    if (p.kind == 0) trsm_cols(false, La + p.aoff, m, U, m, 0, nt, sD, sA, sB);
+    if (p.kind == 0) trsm_cols(false, La + p.aoff, m, Ia + p.ioff, U, m, nt, sA, sB);
 }
 
 // Upper tiles of U_occ U_occ^T (tasks: problem, row tile << 16 | column tile); the

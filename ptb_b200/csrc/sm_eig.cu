@@ -66,7 +66,8 @@ struct EigProb {
     int64_t voff;     // d, e, tau, eigenvalue arenas (m)
     int64_t boff;     // owned-row arena (4 nown x m)
     int64_t xoff;     // cluster solver scratch (orders above kEigBatchMax)
-    int64_t koff;     // T of the compact WY panels (t_panels(m) x NB^2)
+    int64_t koff;     // T of the compact WY panels (t_panels(m) x TS^2)
+    int64_t ioff;     // inverses of the diagonal blocks of L (TS^2 per 64 rows)
     int topm;         // index of the divide and conquer's last merge (-1: one leaf)
 };
 
@@ -380,156 +381,209 @@ __device__ void tile_gemm(double* __restrict__ C, int64_t ldc, int crow, const i
 static_assert(TS * NB % kT == 0, "tile staging divides over the CTA");
 
 // ---------------------------------------------------------------------------
-__host__ __device__ constexpr int64_t t_panels(int m) { return m > 2 ? (m - 2 + NB - 1) / NB : 0; }
+// Compact WY panels of Q = H_0 ... H_{m-3}: TS reflectors each, so that V^T X fills
+// the rows of a tile product and X - V Y2 has a K range of two chunks.
+__host__ __device__ constexpr int64_t t_panels(int m) { return m > 2 ? (m - 2 + TS - 1) / TS : 0; }
+constexpr int kTld = TS + 1;
 
-// T of the compact WY form I - V T V^T of every panel of NB reflectors of
-// Q = H_0 ... H_{m-3} (panels p = first, first + step, ...): the panel's
-// Gram V^T V as one tile product reading the reflectors in place, then T
-// column by column (T_bb = tau_b, T[0:b, b] = -tau_b T[0:b, 0:b] G[0:b, b])
-// by one warp.  Tall + p NB^2 holds panel p's T (NB x NB, column-major, zero
-// outside the panel's nb x nb upper triangle).  Gg: NB^2 global scratch;
-// T: NB x (NB+1) shared.
-__device__ void build_T(const double* __restrict__ C, int64_t ldc, int m, const double* __restrict__ tau, double* __restrict__ Tall,
-                        int first, int step, double* Gg, double* T, double* sA, double* sB) {
+// T of the compact WY form I - V T V^T of panel `pan`: the panel's Gram V^T V as one
+// tile product reading the reflectors in place, the two halves' T column by column
+// (T_bb = tau_b, T[0:b, b] = -tau_b T[0:b, 0:b] G[0:b, b]) by one warp each, and
+// between them T12 = -T11 G12 T22.  Tp: TS x TS, column-major, zero outside the
+// panel's nb x nb upper triangle.  G: TS x TS, T: TS x kTld shared.
+__device__ void build_T(const double* __restrict__ C, int64_t ldc, int m, const double* __restrict__ tau,
+                        double* __restrict__ Tp, int pan, double* G, double* T, double* sA, double* sB) {
+    static_assert(TS == 64 && NB == 32, "a panel is two halves of one warp's width");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nref = m - 2;
-    const int npan = (int)t_panels(m);
-    for (int pan = first; pan < npan; pan += step) {
-        const int j0 = pan * NB, nb = min(NB, nref - j0), r0 = j0 + 1, len = m - r0;
-        const double* Vb = C + r0 + (int64_t)j0 * ldc;
-        tile_mma<true, false, MMA_SET, false, true, true>(Gg, NB, 0, nullptr, 0, 0, nb, nb, Vb, ldc, nullptr, Vb, ldc,
-                                                          nullptr, len, sA, sB);
-        for (int q = tid; q < NB * NB; q += kT) {
-            const int a = q % NB, b = q / NB;
-            T[a + b * (NB + 1)] = (a <= b && b < nb) ? Gg[a + b * NB] : 0.0;
+    const int j0 = pan * TS, nb = min(TS, m - 2 - j0), r0 = j0 + 1, len = m - r0;
+    const double* Vb = C + r0 + (int64_t)j0 * ldc;
+    tile_mma<true, false, MMA_SET, false, true, true>(G, TS, 0, nullptr, 0, 0, nb, nb, Vb, ldc, nullptr, Vb, ldc,
+                                                      nullptr, len, sA, sB);
+    for (int q = tid; q < TS * TS; q += kT) {
+        const int a = q % TS, b = q / TS;
+        T[a + b * kTld] = (a <= b && b < nb) ? G[a + b * TS] : 0.0;
+    }
+    __syncthreads();
+    if (warp < 2) {
+        double* Th = T + warp * NB * (kTld + 1);
+        const int nh = min(NB, nb - warp * NB);
+        for (int b = 0; b < nh; ++b) {
+            const double tb = tau[j0 + warp * NB + b];
+            double acc = 0.0;
+            if (lane < b)
+                for (int c2 = lane; c2 < b; ++c2) acc = fma(Th[lane + c2 * kTld], Th[c2 + b * kTld], acc);
+            __syncwarp();
+            if (lane < b) Th[lane + b * kTld] = -tb * acc;
+            if (lane == b) Th[b + b * kTld] = tb;
+            __syncwarp();
         }
+    }
+    __syncthreads();
+    // W = G12 T22 (in G), then T12 = -T11 W
+    for (int q = tid; q < NB * NB; q += kT) {
+        const int a = q % NB, b = q / NB;
+        double w = 0.0;
+        for (int k = 0; k <= b; ++k) w = fma(T[a + (NB + k) * kTld], T[NB + k + (NB + b) * kTld], w);
+        G[a + b * NB] = w;
+    }
+    __syncthreads();
+    for (int q = tid; q < NB * NB; q += kT) {
+        const int a = q % NB, b = q / NB;
+        double w = 0.0;
+        for (int k = a; k < NB; ++k) w = fma(T[a + k * kTld], G[k + b * NB], w);
+        T[a + (NB + b) * kTld] = -w;
+    }
+    __syncthreads();
+    for (int q = tid; q < TS * TS; q += kT) Tp[q] = T[q % TS + (q / TS) * kTld];
+}
+
+// X (len x nv, nv <= TS) -= V Y2 with the panel's reflectors V (nb of them, read in
+// place) and Y2 (TS x nv, in shared memory with column stride kY2ld = 4 mod 16, the
+// layout of a B fragment): Y2 stays where it is, each 64-row tile of V goes through
+// sA once, and the next tile's V and this tile's X are on their way to registers
+// while a tile is multiplied.
+constexpr int kY2ld = TS + 4;
+__device__ void wy_update(const double* __restrict__ Vb, int64_t ldv, int nb, double* X, int64_t ldx, int len, int nv,
+                          const double* Y2, double* sA) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int wr = (warp & 3) * 16, wc = (warp >> 2) * 16;
+    constexpr int kPer = TS * TS / kT;
+    const int vi = tid % TS, vk = tid / TS;   // row and first reflector of this thread's loads
+    double va[kPer];
+    auto fetch = [&](int i0) {
+        const int row = i0 + vi;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int k = vk + q * (kT / TS);
+            va[q] = (k < nb && row < len) ? (row == k ? 1.0 : row > k ? Vb[row + (int64_t)k * ldv] : 0.0) : 0.0;
+        }
+    };
+    fetch(0);
+    const int ksteps = (nb + 3) >> 2;
+    for (int i0 = 0; i0 < len; i0 += TS) {
+        const int mr = min(TS, len - i0);
+        double cv[2][2][2], acc[2][2][2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = wr + 8 * a + g, j = wc + 8 * b + 2 * t4 + h;
+                    cv[a][b][h] = (i < mr && j < nv) ? X[i0 + i + (int64_t)j * ldx] : 0.0;
+                    acc[a][b][h] = 0.0;
+                }
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) sA[(vk + q * (kT / TS)) * kY2ld + vi] = va[q];
         __syncthreads();
-        if (warp == 0) {
-            for (int b = 0; b < nb; ++b) {
-                const double tb = tau[j0 + b];
-                double acc = 0.0;
-                if (lane < b)
-                    for (int c2 = lane; c2 < b; ++c2) acc = fma(T[lane + c2 * (NB + 1)], T[c2 + b * (NB + 1)], acc);
-                __syncwarp();
-                if (lane < b) T[lane + b * (NB + 1)] = -tb * acc;
-                if (lane == b) T[b + b * (NB + 1)] = tb;
-                __syncwarp();
-            }
+        if (i0 + TS < len) fetch(i0 + TS);
+        for (int ks = 0; ks < ksteps; ++ks) {
+            const int k = ks * 4 + t4;
+            const double a0 = sA[k * kY2ld + wr + g], a1 = sA[k * kY2ld + wr + 8 + g];
+            const double b0 = Y2[(wc + g) * kY2ld + k], b1 = Y2[(wc + 8 + g) * kY2ld + k];
+            dmma(acc[0][0][0], acc[0][0][1], a0, b0);
+            dmma(acc[0][1][0], acc[0][1][1], a0, b1);
+            dmma(acc[1][0][0], acc[1][0][1], a1, b0);
+            dmma(acc[1][1][0], acc[1][1][1], a1, b1);
         }
-        __syncthreads();
-        double* Tp = Tall + (int64_t)pan * NB * NB;
-        for (int q = tid; q < NB * NB; q += kT) {
-            const int a = q % NB, b = q / NB;
-            Tp[q] = (a < nb && b < nb) ? T[a + b * (NB + 1)] : 0.0;
-        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = wr + 8 * a + g, j = wc + 8 * b + 2 * t4 + h;
+                    if (i < mr && j < nv) X[i0 + i + (int64_t)j * ldx] = cv[a][b][h] - acc[a][b][h];
+                }
         __syncthreads();
     }
 }
 
-// Q = H_0 ... H_{m-3} applied to nv vectors (X, ld m) on the FP64 tensor
-// cores, a panel of NB reflectors at a time as I - V T V^T with the panels' T
-// from build_T: Y = V^T X, Y2 = T^T Y (trans: panels in order) or T Y (panels
-// in reverse), X -= V Y2, the reflectors read in place from C.  Y and Y2 are
-// NB x nv global scratch each.
-__device__ void wy_apply_t(const double* __restrict__ C, int64_t ldc, int m, const double* __restrict__ Tall, double* X, int nv,
-                           bool trans, double* Y, double* Y2, double* sA, double* sB) {
-    const int tid = threadIdx.x;
-    const int nref = m - 2;
+// Q = H_0 ... H_{m-3} applied to nv <= TS vectors (X, ld m) on the FP64 tensor cores,
+// a panel at a time as I - V T V^T with the panels' T from build_T: Y = V^T X,
+// Y2 = T^T Y (trans: panels in order) or T Y (panels in reverse), X -= V Y2.  Y: TS x
+// TS, Y2: TS x kY2ld shared.  Bound by the FP64 tensor pipe with two CTAs per SM
+// (a chunk of V^T X 3.9k clocks each, 3.45k of them multiplying) and by the chain of
+// chunks with one.
+__device__ void wy_apply(const double* __restrict__ C, int64_t ldc, int m, const double* __restrict__ Tall, double* X,
+                         int nv, bool trans, double* Y, double* Y2, double* sA, double* sB) {
     const int npan = (int)t_panels(m);
-    if (npan == 0 || nv <= 0) return;
+    if (nv <= 0) return;
     for (int pp = 0; pp < npan; ++pp) {
         const int pan = trans ? pp : npan - 1 - pp;
-        const int j0 = pan * NB, nb = min(NB, nref - j0), r0 = j0 + 1, len = m - r0;
+        const int j0 = pan * TS, nb = min(TS, m - 2 - j0), r0 = j0 + 1, len = m - r0;
         const double* Vb = C + r0 + (int64_t)j0 * ldc;
-        const double* Tp = Tall + (int64_t)pan * NB * NB;
-        for (int c0 = 0; c0 < nv; c0 += TS)
-            tile_mma<true, false, MMA_SET, false, true, false>(Y, NB, 0, nullptr, 0, c0, nb, min(TS, nv - c0), Vb, ldc,
-                                                               nullptr, X + r0, m, nullptr, len, sA, sB);
-        for (int64_t q = tid; q < (int64_t)NB * nv; q += kT) {
-            const int a = (int)(q % NB), t = (int)(q / NB);
-            const double* yc = Y + (int64_t)t * NB;
-            double y = 0.0;
-            if (a < nb) {
-                if (trans) {
-                    for (int c2 = 0; c2 <= a; ++c2) y = fma(Tp[c2 + a * NB], yc[c2], y);
-                } else {
-                    for (int c2 = a; c2 < nb; ++c2) y = fma(Tp[a + c2 * NB], yc[c2], y);
-                }
-            }
-            Y2[q] = y;
-        }
-        __syncthreads();
-        for (int c0 = 0; c0 < nv; c0 += TS)
-            for (int i0 = 0; i0 < len; i0 += TS)
-                tile_mma<false, false, MMA_SUB, false, true, false>(X + r0, m, 0, nullptr, i0, c0, min(TS, len - i0),
-                                                                    min(TS, nv - c0), Vb, ldc, nullptr, Y2, NB, nullptr,
-                                                                    nb, sA, sB);
+        const double* Tp = Tall + (int64_t)pan * TS * TS;
+        tile_mma<true, false, MMA_SET, false, true, false>(Y, TS, 0, nullptr, 0, 0, nb, nv, Vb, ldc, nullptr, X + r0, m,
+                                                           nullptr, len, sA, sB);
+        if (trans)
+            tile_mma<true, false, MMA_SET, false>(Y2, kY2ld, 0, nullptr, 0, 0, TS, nv, Tp, TS, nullptr, Y, TS, nullptr,
+                                                  nb, sA, sB);
+        else
+            tile_mma<false, false, MMA_SET, false>(Y2, kY2ld, 0, nullptr, 0, 0, TS, nv, Tp, TS, nullptr, Y, TS, nullptr,
+                                                   nb, sA, sB);
+        wy_update(Vb, ldc, nb, X + r0, m, len, nv, Y2, sA);
     }
 }
 
-// X <- L^-1 X (lower = true) or X <- L^-T X (lower = false) for the columns
-// [c_begin, c_end) of X (ld ldx), L lower (ld m): over 64-row blocks (from the
-// top, or from the bottom for L^-T), the earlier blocks' contribution as one
-// tile product per 64-column block, then the diagonal block's substitution
-// (warp per column, two rows per lane).  One CTA; sD holds TS x (TS+1).
-__device__ void trsm_cols(bool lower, const double* __restrict__ L, int m, double* X, int64_t ldx, int c_begin,
-                          int c_end, double* sD, double* sA, double* sB) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nrb = (m + TS - 1) / TS;
-    for (int c0 = c_begin; c0 < c_end; c0 += TS) {
-        const int nc = min(TS, c_end - c0);
-        for (int q = 0; q < nrb; ++q) {
-            const int rb = lower ? q : nrb - 1 - q;
-            const int i0 = rb * TS, mr = min(TS, m - i0), i1 = i0 + mr;
-            if (lower) {
-                if (i0 > 0)
-                    tile_mma<false, false, MMA_SUB, false>(X, ldx, 0, nullptr, i0, c0, mr, nc, L, m, nullptr, X, ldx,
-                                                           nullptr, i0, sA, sB);
-            } else if (i1 < m) {
-                // (L^T)[i, k] = L[k, i] for k >= i1
-                tile_mma<true, false, MMA_SUB, false>(X, ldx, 0, nullptr, i0, c0, mr, nc, L + i1, m, nullptr, X + i1,
+// Inverse of one TS x TS diagonal block of L (mr rows of it are L's, sD holds them
+// with sR the reciprocals of the diagonal) by substitution on kSubCols identity columns
+// per warp: mr steps of shuffle, multiply and fused multiply-add, whose latency the
+// columns share.
+constexpr int kSubCols = TS / (kT / 32);
+__device__ void diag_inverse(const double* __restrict__ sD, const double* __restrict__ sR, int mr,
+                             double* __restrict__ Inv) {
+    const int lane = threadIdx.x & 31, jc = (threadIdx.x >> 5) * kSubCols;
+    double x0[kSubCols], x1[kSubCols];
+#pragma unroll
+    for (int c = 0; c < kSubCols; ++c) {
+        x0[c] = (lane == jc + c && lane < mr) ? 1.0 : 0.0;
+        x1[c] = (lane + 32 == jc + c && lane + 32 < mr) ? 1.0 : 0.0;
+    }
+    for (int k = 0; k < mr; ++k) {
+        const double r = sR[k], l0 = sD[lane + k * (TS + 1)], l1 = sD[lane + 32 + k * (TS + 1)];
+        const int kl = k & 31;
+#pragma unroll
+        for (int c = 0; c < kSubCols; ++c) {
+            const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0[c] : x1[c], kl) * r;
+            x0[c] = lane == k ? xk : lane > k ? fma(-l0, xk, x0[c]) : x0[c];
+            x1[c] = lane + 32 == k ? xk : lane + 32 > k ? fma(-l1, xk, x1[c]) : x1[c];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < kSubCols; ++c) {
+        Inv[lane + (jc + c) * TS] = x0[c];
+        Inv[lane + 32 + (jc + c) * TS] = x1[c];
+    }
+}
+
+// X <- L^-1 X (lower = true) or X <- L^-T X (lower = false) for the nc <= TS columns of
+// X (ld ldx), L lower (ld m): over 64-row blocks (from the top, or from the bottom
+// for L^-T), the earlier blocks' contribution as one tile product, then the
+// diagonal block's inverse (Inv: TS x TS per block) as another.  One CTA.  X is zero
+// above row `top` (lower): the blocks before it are skipped.
+//   With a substitution in place of the inverse, a block took 60k clocks besides its
+// products of 3.7k per chunk (two CTAs per SM); the inverse takes 8k.
+__device__ void trsm_cols(bool lower, const double* __restrict__ L, int m, const double* __restrict__ Inv, double* X,
+                          int64_t ldx, int nc, double* sA, double* sB, int top = 0) {
+    const int nrb = (m + TS - 1) / TS, q0 = top / TS, k0 = q0 * TS;
+    for (int q = q0; q < nrb; ++q) {
+        const int rb = lower ? q : nrb - 1 - q + q0;
+        const int i0 = rb * TS, mr = min(TS, m - i0), i1 = i0 + mr;
+        const double* Ib = Inv + (int64_t)rb * TS * TS;
+        if (lower) {
+            if (i0 > k0)
+                tile_mma<false, false, MMA_SUB, false>(X, ldx, 0, nullptr, i0, 0, mr, nc, L + (int64_t)k0 * m, m, nullptr,
+                                                       X + k0, ldx, nullptr, i0 - k0, sA, sB);
+            tile_mma<false, false, MMA_SET, false>(X, ldx, i0, nullptr, 0, 0, mr, nc, Ib, TS, nullptr, X + i0, ldx,
+                                                   nullptr, mr, sA, sB);
+        } else {
+            if (i1 < m)   // (L^T)[i, k] = L[k, i] for k >= i1
+                tile_mma<true, false, MMA_SUB, false>(X, ldx, 0, nullptr, i0, 0, mr, nc, L + i1, m, nullptr, X + i1,
                                                       ldx, nullptr, m - i1, sA, sB);
-            }
-            for (int t = tid; t < TS * TS; t += kT) {
-                const int i = t % TS, j = t / TS;
-                sD[i + j * (TS + 1)] = (i < mr && j < mr && i >= j) ? L[(int64_t)(i0 + i) + (int64_t)(i0 + j) * m] : 0.0;
-            }
-            __syncthreads();
-            for (int jc = warp; jc < nc; jc += kT / 32) {
-                double* x = X + (int64_t)(c0 + jc) * ldx + i0;
-                double x0 = lane < mr ? x[lane] : 0.0, x1 = lane + 32 < mr ? x[lane + 32] : 0.0;
-                if (lower) {
-                    for (int k = 0; k < mr; ++k) {
-                        double xk;
-                        if (k < 32) {
-                            if (lane == k) x0 /= sD[k + k * (TS + 1)];
-                            xk = __shfl_sync(0xffffffffu, x0, k);
-                        } else {
-                            if (lane == k - 32) x1 /= sD[k + k * (TS + 1)];
-                            xk = __shfl_sync(0xffffffffu, x1, k - 32);
-                        }
-                        if (lane > k && lane < mr) x0 -= sD[lane + k * (TS + 1)] * xk;
-                        if (lane + 32 > k && lane + 32 < mr) x1 -= sD[lane + 32 + k * (TS + 1)] * xk;
-                    }
-                } else {
-                    // L_bb^T x = b: back substitution, (L^T)[i, k] = sD[k + i (TS+1)] for k > i
-                    for (int k = mr - 1; k >= 0; --k) {
-                        double xk;
-                        if (k < 32) {
-                            if (lane == k) x0 /= sD[k + k * (TS + 1)];
-                            xk = __shfl_sync(0xffffffffu, x0, k);
-                        } else {
-                            if (lane == k - 32) x1 /= sD[k + k * (TS + 1)];
-                            xk = __shfl_sync(0xffffffffu, x1, k - 32);
-                        }
-                        if (lane < k) x0 -= sD[k + lane * (TS + 1)] * xk;
-                        if (lane + 32 < k) x1 -= sD[k + (lane + 32) * (TS + 1)] * xk;
-                    }
-                }
-                if (lane < mr) x[lane] = x0;
-                if (lane + 32 < mr) x[lane + 32] = x1;
-            }
-            __syncthreads();
+            tile_mma<true, false, MMA_SET, false>(X, ldx, i0, nullptr, 0, 0, mr, nc, Ib, TS, nullptr, X + i0, ldx,
+                                                  nullptr, mr, sA, sB);
         }
     }
 }
@@ -558,19 +612,40 @@ __global__ void __launch_bounds__(kT, 1) k_eig_chol(const EigProb* __restrict__ 
     if (threadIdx.x == 0) status[pi] = st;
 }
 
+// Inverses of the 64 x 64 diagonal blocks of L, one per CTA (tasks: problem, block).
+__global__ void __launch_bounds__(kT, 2) k_eig_dinv(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
+                                                    const double* __restrict__ La, double* __restrict__ Ia,
+                                                    const int* __restrict__ status) {
+    __shared__ double sD[TS * (TS + 1)], sR[TS];
+    const int2 t = tasks[blockIdx.x];
+    if (status[t.x] != kStOk) return;
+    const EigProb p = probs[t.x];
+    const int m = p.m, i0 = t.y * TS, mr = min(TS, m - i0);
+    const double* L = La + p.aoff + i0 + (int64_t)i0 * m;
+    for (int q = threadIdx.x; q < TS * TS; q += kT) {
+        const int i = q % TS, j = q / TS;
+        const double v = (i < mr && j < mr && i >= j) ? L[i + (int64_t)j * m] : 0.0;
+        sD[i + j * (TS + 1)] = v;
+        if (i == j) sR[i] = i < mr ? 1.0 / v : 0.0;
+    }
+    __syncthreads();
+    diag_inverse(sD, sR, mr, Ia + p.ioff + (int64_t)t.y * TS * TS);
+}
+
 // X <- L^-1 X on one 64-column block of X per CTA (tasks: problem, block); in_c: X is
 // the C arena.
-constexpr size_t kTrsmSmem = sizeof(double) * (2 * kStageOp + TS * (TS + 1));
 __global__ void __launch_bounds__(kT, 2) k_eig_trsm(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
-                                                    const double* __restrict__ La, double* __restrict__ Xa,
-                                                    bool in_c, const int* __restrict__ status) {
+                                                    const double* __restrict__ La, const double* __restrict__ Ia,
+                                                    double* __restrict__ Xa, bool in_c,
+                                                    const int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     const int2 t = tasks[blockIdx.x];
     if (status[t.x] != kStOk) return;
     const EigProb p = probs[t.x];
-    trsm_cols(true, La + p.aoff, p.m, Xa + (in_c ? p.coff : p.aoff), in_c ? p.ldc : p.m, t.y * TS,
-              min(p.m, (t.y + 1) * TS), sA + 2 * kStageOp, sA, sA + kStageOp);
+    const int c0 = t.y * TS, ld = in_c ? p.ldc : p.m;
+    trsm_cols(true, La + p.aoff, p.m, Ia + p.ioff, Xa + (in_c ? p.coff : p.aoff) + (int64_t)c0 * ld, ld,
+              min(TS, p.m - c0), sA, sA + kStageOp);
 }
 
 // Y = X^T (Y in the C arena), one 64-column block of X per CTA, through 64 x 65 shared tiles.
@@ -1201,7 +1276,7 @@ struct EigBatch {
     std::vector<DcMerge> merges;
     std::vector<Level> levels;
     Seg blocks, leaves, panels, rows, rq, back, density, fblocks, frq, fcols;
-    WorkBuf probs, order_d, lists_d, merges_d, cnt, dc, Ca, La, Za, Qa, Va, Da, Ea, Ta, Ba, Xa, Ka, status;
+    WorkBuf probs, order_d, lists_d, merges_d, cnt, dc, Ca, La, Za, Qa, Va, Da, Ea, Ta, Ba, Xa, Ka, Ia, status;
     DcArr S{};
     double* Z = nullptr;          // the Z arena (Za, or the caller's array)
     int prl = 0;
@@ -1229,7 +1304,7 @@ void smem_attr(K kern, size_t bytes) {
 void eig_setup_attrs() {
     static const bool done = [] {
         smem_attr(k_eig_chol, kCholSmem);
-        smem_attr(k_eig_trsm, kTrsmSmem);
+        smem_attr(k_eig_trsm, kTileSmem);
         smem_attr(k_eig_trd<512>, 8 * trd_cap(kTrdMax512, 512));
         smem_attr(k_eig_trd<256>, 8 * trd_cap(kTrdMax256, 256));
         smem_attr(k_lg_chol, lg_smem_bytes(2));
@@ -1389,7 +1464,7 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     eb.maxlarge = large.empty() ? 0 : eb.hp[large[0]].m;
     if (eb.nlarge > 0 && !eb.grid) eb.G = eig_cluster_size(c, eb.nlarge);
     const int nsm = c->num_sms > 0 ? c->num_sms : 148;
-    int64_t asz = 0, csz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0;
+    int64_t asz = 0, csz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0, isz = 0;
     for (int q = 0; q < np; ++q) {
         EigProb& p = eb.hp[q];
         p.poff = psz;
@@ -1401,8 +1476,10 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
         p.voff = vsz;
         p.boff = bsz;
         p.koff = ksz;
+        p.ioff = isz;
         p.topm = -1;
-        ksz += t_panels(p.m) * NB * NB;
+        ksz += t_panels(p.m) * TS * TS;
+        isz += (int64_t)((p.m + TS - 1) / TS) * TS * TS;
         asz += (int64_t)p.m * p.m;
         vsz += p.m;
         bsz += p.mode == 2 ? (int64_t)p.m * p.m : 4 * (int64_t)p.nown * p.m;
@@ -1544,6 +1621,7 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     eb.Ba.reserve(c, sizeof(double) * std::max<int64_t>(bsz, 1));
     eb.Xa.reserve(c, sizeof(double) * std::max<int64_t>(xsz, 2));
     eb.Ka.reserve(c, sizeof(double) * std::max<int64_t>(ksz, 2));
+    eb.Ia.reserve(c, sizeof(double) * std::max<int64_t>(isz, 2));
     eb.status.reserve(c, sizeof(int) * (np + 3));   // and a grid barrier's count, generation and error
     PTB_CUDA(cudaMemcpyAsync(eb.probs.ptr, eb.hp.data(), sizeof(EigProb) * np, cudaMemcpyHostToDevice, s));
     PTB_CUDA(cudaMemcpyAsync(eb.order_d.ptr, eb.order.data(), sizeof(int) * eb.order.size(), cudaMemcpyHostToDevice, s));
@@ -1563,7 +1641,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
     const DcMerge* mg = eb.merges_d.as<DcMerge>();
     double *Ca = eb.Ca.as<double>(), *La = eb.La.as<double>(), *Za = eb.Z, *Qa = eb.Qa.as<double>(),
            *Va = eb.Va.as<double>(), *Da = eb.Da.as<double>(), *Ea = eb.Ea.as<double>(), *Ta = eb.Ta.as<double>(),
-           *Ba = eb.Ba.as<double>(), *Xa = eb.Xa.as<double>(), *Ka = eb.Ka.as<double>();
+           *Ba = eb.Ba.as<double>(), *Xa = eb.Xa.as<double>(), *Ka = eb.Ka.as<double>(), *Ia = eb.Ia.as<double>();
     int* st = eb.status.as<int>();
     const DcArr& D = eb.S;
     unsigned* bar = eb.grid ? reinterpret_cast<unsigned*>(st + eb.nprob) : nullptr;
@@ -1614,10 +1692,11 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
     // ---- C = L^-1 H L^-T
     if (eb.hp[0].kind == 0) {
         const int2* bl = eb.list(eb.blocks);
-        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Qa, false, st);
+        k_eig_dinv<<<eb.blocks.n, kT, 0, s>>>(dp, bl, La, Ia, st);
+        k_eig_trsm<<<eb.blocks.n, kT, kTileSmem, s>>>(dp, bl, La, Ia, Qa, false, st);
         k_eig_transpose<<<eb.blocks.n, 256, 0, s>>>(dp, bl, Qa, Ca, st);
-        k_eig_trsm<<<eb.blocks.n, kT, kTrsmSmem, s>>>(dp, bl, La, Ca, true, st);
-        launched(3);
+        k_eig_trsm<<<eb.blocks.n, kT, kTileSmem, s>>>(dp, bl, La, Ia, Ca, true, st);
+        launched(4);
     }
     // ---- tridiagonalisation, the widest groups first
     fork(eb.trd.size() > 1);
@@ -1649,7 +1728,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         launched();
     }
     if (eb.rows.n) {
-        k_vec_rows<<<eb.rows.n, kT, kChainSmem, s>>>(dp, eb.list(eb.rows), Ca, La, Ka, d_own_cols, d_ipos, Ba, st);
+        k_vec_rows<<<eb.rows.n, kT, kChainSmem, s>>>(dp, eb.list(eb.rows), Ca, La, Ia, Ka, d_own_cols, d_ipos, Ba, st);
         launched();
     }
     // ---- divide and conquer
@@ -1682,7 +1761,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         launched();
     }
     if (eb.back.n) {
-        k_vec_back<<<eb.back.n, kT, kChainSmem, s>>>(dp, eb.list(eb.back), Ca, La, Ka, Za, st);
+        k_vec_back<<<eb.back.n, kT, kChainSmem, s>>>(dp, eb.list(eb.back), Ca, La, Ia, Ka, Za, st);
         launched();
     }
     if (eb.density.n) {
@@ -1768,7 +1847,7 @@ void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, int64_t n, const in
     k_fin_vw<<<eb.frq.n, kT, kTileSmem, s>>>(dp, fr, Za, Qa, Va, eb.S, Ba);
     k_fin_qw<<<eb.frq.n, kT, kTileSmem, s>>>(dp, fr, Za, Qa, Va, eb.S, Ba);
     k_fin_cols<<<eb.fcols.n, kT, kChainSmem, s>>>(dp, eb.list(eb.fcols), eb.Ca.as<double>(), eb.La.as<double>(),
-                                                  eb.Ka.as<double>(), d_maps, d_own_cols, Ba, dP, dPdense);
+                                                  eb.Ia.as<double>(), eb.Ka.as<double>(), d_maps, d_own_cols, Ba, dP, dPdense);
     count_launch(4);
     PTB_CUDA(cudaGetLastError());
 }
