@@ -9,7 +9,8 @@
 // them are reached without forming U:
 //
 //   S_k = L L^T                      Cholesky, blocked
-//   C   = L^-1 H_k L^-T              two blocked triangular solves
+//   C   = L^-1 H_k L^-T              two blocked triangular solves, the second for the
+//                                    lower triangle only
 //   C   = Q T Q^T                    Householder tridiagonalisation, lower,
 //                                    Q = H_0 H_1 ... H_{m-3}
 //   T   = Z diag(e) Z^T              divide and conquer (eig_dc.cuh)
@@ -19,10 +20,10 @@
 //     P_k[:,c] = U (occ o U[c,:]^T) = L^-T (Q (Z w)).
 //
 // Every stage is a launch (or a few) over all problems of the batch, with its own
-// split: one CTA or one thread-block cluster per problem where the stage is a chain
-// (Cholesky, tridiagonalisation), one CTA per 64-column block, panel, tile or chunk of
-// roots where it is not, largest problems first.  A batch of uneven problems then
-// costs its total work over the SMs in all stages but those two, where one CTA or
+// split: one CTA or one thread-block cluster per problem where the stage is a chain over
+// the whole problem (tridiagonalisation), one CTA per 64-row block, panel, tile or chunk
+// of roots where it is not, largest problems first.  A batch of uneven problems then
+// costs its total work over the SMs in all stages but that one, where one CTA or
 // cluster per problem for everything cost the largest problem's whole chain.
 //
 // Each step's quantities are summed in a fixed order, so results do not depend
@@ -65,7 +66,7 @@ struct EigProb {
     int ldc;
     int64_t voff;     // d, e, tau, eigenvalue arenas (m)
     int64_t boff;     // owned-row arena (4 nown x m)
-    int64_t xoff;     // cluster solver scratch (orders above kEigBatchMax)
+    int64_t xoff;     // scratch of the cluster and grid tridiagonalisations
     int64_t koff;     // T of the compact WY panels (t_panels(m) x TS^2)
     int64_t ioff;     // inverses of the diagonal blocks of L (TS^2 per 64 rows)
     int topm;         // index of the divide and conquer's last merge (-1: one leaf)
@@ -252,123 +253,6 @@ __device__ double warp_sum(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// Shared memory of the one-CTA Cholesky: the tile staging (sA, sB) and the diagonal
-// block (sD).
-struct StageSmem {
-    double *sA, *sB, *sD;
-    int* ints;
-};
-constexpr size_t kCholSmem = sizeof(double) * (2 * kStageOp + NB * (NB + 1)) + sizeof(int) * 16;
-__device__ StageSmem stage_smem(unsigned char* base) {
-    StageSmem sh;
-    double* d = reinterpret_cast<double*>(base);
-    sh.sA = d;
-    sh.sB = d + kStageOp;
-    sh.sD = d + 2 * kStageOp;
-    sh.ints = reinterpret_cast<int*>(d + 2 * kStageOp + NB * (NB + 1));
-    return sh;
-}
-
-// ---------------------------------------------------------------------------
-// Gather H_k, S_k (source/sm.f90:240-246) into the C and L arenas.
-__device__ void stage_gather(const EigProb& p, const int* __restrict__ maps, const double* __restrict__ H,
-                             const double* __restrict__ S, double* __restrict__ Ca, double* __restrict__ La) {
-    const int m = p.m;
-    const int* mp = maps + p.moff;
-    double* C = Ca + p.aoff;
-    double* L = La + p.aoff;
-    for (int j = 0; j < m; ++j) {
-        const int64_t gj = p.gbase + (int64_t)mp[j] * p.gld;
-        for (int i = threadIdx.x; i < m; i += kT) {
-            const int64_t g = (int64_t)mp[i] + gj;
-            C[i + (int64_t)j * m] = H[g];
-            L[i + (int64_t)j * m] = S[g];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// S_k = L L^T in place (lower), right-looking with 32-wide panels; the strict
-// upper triangle is zeroed.  Returns the order of the first non-positive
-// pivot (0: positive definite).
-__device__ int stage_potrf(const EigProb& p, double* __restrict__ La, const StageSmem& sh) {
-    double* sA = sh.sA;
-    double* sB = sh.sB;
-    double* sD = sh.sD;   // sD[i + j*(NB+1)]
-    int& fail = sh.ints[0];
-    const int m = p.m;
-    double* L = La + p.aoff;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) fail = 0;
-    __syncthreads();
-    for (int kb = 0; kb < m; kb += NB) {
-        const int nb = min(NB, m - kb);
-        for (int t = tid; t < NB * NB; t += kT) {
-            const int i = t % NB, j = t / NB;
-            sD[i + j * (NB + 1)] = (i < nb && j < nb) ? L[(int64_t)(kb + i) + (int64_t)(kb + j) * m] : 0.0;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            for (int jj = 0; jj < nb; ++jj) {
-                if (lane == jj) {
-                    const double piv = sD[jj + jj * (NB + 1)];
-                    if (!(piv > 0.0)) fail = kb + jj + 1;
-                    else sD[jj + jj * (NB + 1)] = sqrt(piv);
-                }
-                __syncwarp();
-                if (fail) break;
-                const double djj = sD[jj + jj * (NB + 1)];
-                if (lane > jj && lane < nb) sD[lane + jj * (NB + 1)] /= djj;
-                __syncwarp();
-                if (lane > jj && lane < nb) {
-                    const double lij = sD[lane + jj * (NB + 1)];
-                    for (int k = jj + 1; k <= lane; ++k) sD[lane + k * (NB + 1)] -= lij * sD[k + jj * (NB + 1)];
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        if (fail) break;
-        for (int t = tid; t < nb * nb; t += kT) {
-            const int i = t % nb, j = t / nb;
-            if (i >= j) L[(int64_t)(kb + i) + (int64_t)(kb + j) * m] = sD[i + j * (NB + 1)];
-        }
-        // panel: rows below solve x L11^T = a
-        for (int r = kb + nb + tid; r < m; r += kT) {
-            double x[NB];
-#pragma unroll
-            for (int j = 0; j < NB; ++j) x[j] = (j < nb) ? L[(int64_t)r + (int64_t)(kb + j) * m] : 0.0;
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                if (j < nb) {
-                    double v = x[j];
-                    for (int k = 0; k < j; ++k) v -= x[k] * sD[j + k * (NB + 1)];
-                    x[j] = v / sD[j + j * (NB + 1)];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < NB; ++j)
-                if (j < nb) L[(int64_t)r + (int64_t)(kb + j) * m] = x[j];
-        }
-        __syncthreads();
-        // trailing update of the lower triangle: A22 -= L21 L21^T
-        const int t0 = kb + nb;
-        for (int c0 = t0; c0 < m; c0 += TS)
-            for (int r0 = c0; r0 < m; r0 += TS)
-                tile_update<true, true>(L, m, r0, c0, min(TS, m - r0), min(TS, m - c0), L + (int64_t)kb * m, m,
-                                        L + (int64_t)kb * m, m, nb, sA, sB);
-    }
-    __syncthreads();
-    const int f = fail;
-    __syncthreads();
-    if (f) return f;
-    for (int j = 1; j < m; ++j)
-        for (int i = tid; i < j; i += kT) L[(int64_t)i + (int64_t)j * m] = 0.0;
-    return 0;
-}
-
-
-// ---------------------------------------------------------------------------
 // C[crow + r0 + i, col(c0 + j)] = sum_k A(i, kx(k)) B(kxb(k), j) on one TS x TS
 // output tile (tile_mma, MMA_SET).
 template <bool AT, bool BT = false>
@@ -527,37 +411,6 @@ __device__ void wy_apply(const double* __restrict__ C, int64_t ldc, int m, const
     }
 }
 
-// Inverse of one TS x TS diagonal block of L (mr rows of it are L's, sD holds them
-// with sR the reciprocals of the diagonal) by substitution on kSubCols identity columns
-// per warp: mr steps of shuffle, multiply and fused multiply-add, whose latency the
-// columns share.
-constexpr int kSubCols = TS / (kT / 32);
-__device__ void diag_inverse(const double* __restrict__ sD, const double* __restrict__ sR, int mr,
-                             double* __restrict__ Inv) {
-    const int lane = threadIdx.x & 31, jc = (threadIdx.x >> 5) * kSubCols;
-    double x0[kSubCols], x1[kSubCols];
-#pragma unroll
-    for (int c = 0; c < kSubCols; ++c) {
-        x0[c] = (lane == jc + c && lane < mr) ? 1.0 : 0.0;
-        x1[c] = (lane + 32 == jc + c && lane + 32 < mr) ? 1.0 : 0.0;
-    }
-    for (int k = 0; k < mr; ++k) {
-        const double r = sR[k], l0 = sD[lane + k * (TS + 1)], l1 = sD[lane + 32 + k * (TS + 1)];
-        const int kl = k & 31;
-#pragma unroll
-        for (int c = 0; c < kSubCols; ++c) {
-            const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0[c] : x1[c], kl) * r;
-            x0[c] = lane == k ? xk : lane > k ? fma(-l0, xk, x0[c]) : x0[c];
-            x1[c] = lane + 32 == k ? xk : lane + 32 > k ? fma(-l1, xk, x1[c]) : x1[c];
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < kSubCols; ++c) {
-        Inv[lane + (jc + c) * TS] = x0[c];
-        Inv[lane + 32 + (jc + c) * TS] = x1[c];
-    }
-}
-
 // X <- L^-1 X (lower = true) or X <- L^-T X (lower = false) for the nc <= TS columns of
 // X (ld ldx), L lower (ld m): over 64-row blocks (from the top, or from the bottom
 // for L^-T), the earlier blocks' contribution as one tile product, then the
@@ -597,76 +450,171 @@ __device__ void trsm_cols(bool lower, const double* __restrict__ L, int m, const
 #include "eig_trd.cuh"
 #include "eig_trdc.cuh"
 
-// Gather and Cholesky, one problem per CTA.
-__global__ void __launch_bounds__(kT, 1) k_eig_chol(const EigProb* __restrict__ probs, const int* __restrict__ order,
-                                                    const int* __restrict__ maps, const double* __restrict__ H,
-                                                    const double* __restrict__ S, double* __restrict__ Xa,
-                                                    double* __restrict__ La, int* __restrict__ status) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const StageSmem sh = stage_smem(smraw);
-    const int pi = order[blockIdx.x];
-    const EigProb p = probs[pi];
-    stage_gather(p, maps, H, S, Xa, La);
-    __syncthreads();
-    const int st = stage_potrf(p, La, sh);
-    if (threadIdx.x == 0) status[pi] = st;
+// ---- gather, Cholesky and reduction: stages over the 64-row (or 64-column) blocks
+// of every problem (tasks: problem, block)
+
+// H_k, S_k (source/sm.f90:240-246) into the X and L arenas, 64 columns per CTA; of S the
+// lower triangle, zeros above it.  A standard problem needs no reduction: its matrix
+// goes where that leaves it.
+__global__ void __launch_bounds__(kT, 2) k_eig_gather(const EigProb* __restrict__ probs,
+                                                      const int2* __restrict__ tasks, const int* __restrict__ maps,
+                                                      const double* __restrict__ H, const double* __restrict__ S,
+                                                      double* __restrict__ Ca, double* __restrict__ Xa,
+                                                      double* __restrict__ La) {
+    const int2 t = tasks[blockIdx.x];
+    const EigProb p = probs[t.x];
+    const int m = p.m;
+    const int* mp = maps + p.moff;
+    double* X = p.kind == 0 ? Xa + p.aoff : Ca + p.coff;
+    const int64_t ldx = p.kind == 0 ? m : p.ldc;
+    double* L = La + p.aoff;
+    for (int j = t.y * TS; j < min(m, (t.y + 1) * TS); ++j) {
+        const int64_t gj = p.gbase + (int64_t)mp[j] * p.gld;
+        for (int i = threadIdx.x; i < m; i += kT) {
+            const int64_t q = (int64_t)mp[i] + gj;
+            X[i + (int64_t)j * ldx] = H[q];
+            if (p.kind == 0) L[i + (int64_t)j * m] = i >= j ? S[q] : 0.0;
+        }
+    }
 }
 
-// Inverses of the 64 x 64 diagonal blocks of L, one per CTA (tasks: problem, block).
-__global__ void __launch_bounds__(kT, 2) k_eig_dinv(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
-                                                    const double* __restrict__ La, double* __restrict__ Ia,
-                                                    const int* __restrict__ status) {
-    __shared__ double sD[TS * (TS + 1)], sR[TS];
-    const int2 t = tasks[blockIdx.x];
-    if (status[t.x] != kStOk) return;
-    const EigProb p = probs[t.x];
-    const int m = p.m, i0 = t.y * TS, mr = min(TS, m - i0);
-    const double* L = La + p.aoff + i0 + (int64_t)i0 * m;
-    for (int q = threadIdx.x; q < TS * TS; q += kT) {
-        const int i = q % TS, j = q / TS;
-        const double v = (i < mr && j < mr && i >= j) ? L[i + (int64_t)j * m] : 0.0;
-        sD[i + j * (TS + 1)] = v;
-        if (i == j) sR[i] = i < mr ? 1.0 / v : 0.0;
+// Factor and inverse of one TS x TS diagonal block (its first mr rows at L, ld m; the
+// rest counts as the identity), by elimination on [A | I]: thread (i, g) holds row i,
+// columns g, g + 8, ... of both in registers, and a step broadcasts column k of A and
+// row k of the right half through shared memory (two buffers, one barrier a step).
+// With A = (unit lower) D (unit lower)^T: L = lower sqrt(D), L^-1 = D^-1/2 lower^-1.
+// Bound by the chain of TS steps of a barrier, a division and the
+// updates (48k clocks).  Returns
+// the first non-positive pivot's position (1-based; 0: none), the same on every thread.
+__device__ int diag_factor(double* __restrict__ L, int m, int mr, double* __restrict__ Inv) {
+    constexpr int NG = kT / TS, NQ = TS / NG;
+    __shared__ double colb[2][TS], rowb[2][TS], piv[TS];
+    const int i = threadIdx.x % TS, g = threadIdx.x / TS;
+    double a[NQ], e[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int c = g + NG * q;
+        a[q] = (i < mr && c <= i) ? L[i + (int64_t)c * m] : (i == c ? 1.0 : 0.0);
+        e[q] = i == c ? 1.0 : 0.0;
+    }
+    int bad = 0;
+#pragma unroll
+    for (int kq = 0; kq < NQ; ++kq) {
+#pragma unroll 1
+        for (int kg = 0; kg < NG; ++kg) {
+            const int k = kq * NG + kg;
+            double* cb = colb[k & 1];
+            double* rb = rowb[k & 1];
+            if (g == kg) cb[i] = a[kq];
+            if (i == k) {
+#pragma unroll
+                for (int q = 0; q <= kq; ++q) rb[g + NG * q] = e[q];
+            }
+            __syncthreads();
+            const double pk = cb[k];
+            if (!(pk > 0.0) && bad == 0) bad = k + 1;
+            if (threadIdx.x == 0) piv[k] = pk;
+            const double r = 1.0 / pk, f = i > k ? cb[i] * r : 0.0;
+#pragma unroll
+            for (int q = 0; q <= kq; ++q) e[q] = fma(-f, rb[g + NG * q], e[q]);
+            a[kq] = fma(g > kg ? -f : 0.0, cb[g + NG * kq], a[kq]);
+#pragma unroll
+            for (int q = kq + 1; q < NQ; ++q) a[q] = fma(-f, cb[g + NG * q], a[q]);
+        }
     }
     __syncthreads();
-    diag_inverse(sD, sR, mr, Ia + p.ioff + (int64_t)t.y * TS * TS);
+    if (bad) return bad;
+    const double si = sqrt(piv[i]);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int c = g + NG * q;
+        if (i < mr && c < mr) L[i + (int64_t)c * m] = i > c ? a[q] / sqrt(piv[c]) : i == c ? si : 0.0;
+        Inv[i + c * TS] = (i < mr && c <= i) ? e[q] / si : 0.0;
+    }
+    return 0;
 }
 
-// X <- L^-1 X on one 64-column block of X per CTA (tasks: problem, block); in_c: X is
-// the C arena.
+// Block column j of the Cholesky factor, left-looking: every 64 x 64 tile of the column
+// gets the earlier columns' contribution as one product, the CTA of the diagonal tile
+// goes on to factor and invert it; then the tiles below are multiplied by the
+// inverse's transpose (k_chol_scale).  Two launches per block column over the whole
+// batch.  One CTA (order <= 800) or cluster per problem, with 32-wide panels and
+// rank-32 updates, took 2.3 ms against 0.8 for 32 H2O and 28 ms against 11.4
+// for 512-H2O clusters (orders to 2773).
+__global__ void __launch_bounds__(kT, 2) k_chol_column(const EigProb* __restrict__ probs,
+                                                       const int2* __restrict__ tasks, int j, double* __restrict__ La,
+                                                       double* __restrict__ Ia, int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double* sA = reinterpret_cast<double*>(smraw);
+    const int2 t = tasks[blockIdx.x];
+    if (t.y < j || status[t.x] != kStOk) return;
+    const EigProb p = probs[t.x];
+    const int m = p.m, i0 = t.y * TS, j0 = j * TS, mr = min(TS, m - i0), nc = min(TS, m - j0);
+    double* L = La + p.aoff;
+    if (j > 0)
+        tile_mma<false, true, MMA_SUB, false>(L, m, 0, nullptr, i0, j0, mr, nc, L, m, nullptr, L, m, nullptr, j0, sA,
+                                              sA + kStageOp);
+    if (t.y == j) {
+        const int f = diag_factor(L + i0 + (int64_t)i0 * m, m, mr, Ia + p.ioff + (int64_t)j * TS * TS);
+        if (f != 0 && threadIdx.x == 0) status[t.x] = i0 + f;
+    }
+}
+
+__global__ void __launch_bounds__(kT, 2) k_chol_scale(const EigProb* __restrict__ probs,
+                                                      const int2* __restrict__ tasks, int j, double* __restrict__ La,
+                                                      const double* __restrict__ Ia, const int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double* sA = reinterpret_cast<double*>(smraw);
+    const int2 t = tasks[blockIdx.x];
+    if (t.y <= j || status[t.x] != kStOk) return;
+    const EigProb p = probs[t.x];
+    const int m = p.m, i0 = t.y * TS;
+    double* Lj = La + p.aoff + (int64_t)j * TS * m;
+    tile_mma<false, true, MMA_SET, false>(Lj, m, 0, nullptr, i0, 0, min(TS, m - i0), TS, Lj, m, nullptr,
+                                          Ia + p.ioff + (int64_t)j * TS * TS, TS, nullptr, TS, sA, sA + kStageOp);
+}
+
+// X <- L^-1 X on one 64-column block of X per CTA.
 __global__ void __launch_bounds__(kT, 2) k_eig_trsm(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ La, const double* __restrict__ Ia,
-                                                    double* __restrict__ Xa, bool in_c,
-                                                    const int* __restrict__ status) {
+                                                    double* __restrict__ Xa, const int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double* sA = reinterpret_cast<double*>(smraw);
     const int2 t = tasks[blockIdx.x];
     if (status[t.x] != kStOk) return;
     const EigProb p = probs[t.x];
-    const int c0 = t.y * TS, ld = in_c ? p.ldc : p.m;
-    trsm_cols(true, La + p.aoff, p.m, Ia + p.ioff, Xa + (in_c ? p.coff : p.aoff) + (int64_t)c0 * ld, ld,
-              min(TS, p.m - c0), sA, sA + kStageOp);
+    const int m = p.m, c0 = t.y * TS;
+    trsm_cols(true, La + p.aoff, m, Ia + p.ioff, Xa + p.aoff + (int64_t)c0 * m, m, min(TS, m - c0), sA, sA + kStageOp);
 }
 
-// Y = X^T (Y in the C arena), one 64-column block of X per CTA, through 64 x 65 shared tiles.
-__global__ void __launch_bounds__(256) k_eig_transpose(const EigProb* __restrict__ probs,
-                                                       const int2* __restrict__ tasks, const double* __restrict__ Xa,
-                                                       double* __restrict__ Ya, const int* __restrict__ status) {
-    __shared__ double tile[TS][TS + 1];
+// Row block i of the lower triangle of A = X L^-T into the C arena (zeros above it), one
+// per CTA, the last and longest rows of a problem first: block column j as X_ij less
+// one product with the row's earlier blocks, times the transpose of the diagonal block's
+// inverse.  A third of the products of a solve over whole columns, and no transposed
+// copy (14.8 -> 5.7 ms for 512-H2O clusters).
+__global__ void __launch_bounds__(kT, 2) k_eig_rsolve(const EigProb* __restrict__ probs,
+                                                      const int2* __restrict__ tasks, const double* __restrict__ La,
+                                                      const double* __restrict__ Ia, double* __restrict__ Xa,
+                                                      double* __restrict__ Ca, const int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double *sA = reinterpret_cast<double*>(smraw), *sB = sA + kStageOp;
     const int2 t = tasks[blockIdx.x];
     if (status[t.x] != kStOk) return;
     const EigProb p = probs[t.x];
-    const int m = p.m, c0 = t.y * TS, tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-    const double* X = Xa + p.aoff;
-    double* Y = Ya + p.coff;
-    for (int r0 = 0; r0 < m; r0 += TS) {
-        for (int c = ty; c < TS; c += 4)
-            if (r0 + tx < m && c0 + c < m) tile[c][tx] = X[r0 + tx + (int64_t)(c0 + c) * m];
-        __syncthreads();
-        for (int r = ty; r < TS; r += 4)
-            if (r0 + r < m && c0 + tx < m) Y[c0 + tx + (int64_t)(r0 + r) * p.ldc] = tile[tx][r];
-        __syncthreads();
+    const int m = p.m, i = (m + TS - 1) / TS - 1 - t.y, i0 = i * TS, mr = min(TS, m - i0);
+    const double* L = La + p.aoff;
+    double *X = Xa + p.aoff, *C = Ca + p.coff;
+    for (int j = 0; j <= i; ++j) {
+        const int j0 = j * TS, nc = min(TS, m - j0);
+        if (j > 0)
+            tile_mma<false, true, MMA_SUB, false>(X, m, 0, nullptr, i0, j0, mr, nc, C, p.ldc, nullptr, L, m, nullptr, j0,
+                                                  sA, sB);
+        tile_mma<false, true, MMA_SET, false>(C + (int64_t)j0 * p.ldc, p.ldc, 0, nullptr, i0, 0, mr, nc,
+                                              X + (int64_t)j0 * m, m, nullptr, Ia + p.ioff + (int64_t)j * TS * TS, TS,
+                                              nullptr, nc, sA, sB);
     }
+    for (int c = i0 + mr + threadIdx.x / TS; c < m; c += kT / TS)
+        if (threadIdx.x % TS < mr) C[i0 + threadIdx.x % TS + (int64_t)c * p.ldc] = 0.0;
 }
 
 // Tridiagonalisation, one problem per CTA.
@@ -682,15 +630,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_eig_trd(const EigProb* __restr
     stage_trd<NT>(probs[pi], Ca, Da, Ea, Ta, reinterpret_cast<double*>(smraw), cap);
 }
 
-// Divide and conquer, then the owned rows and fe (mode 0) or the density (mode 2).
 // ===========================================================================
-// Cholesky and tridiagonalisation of problems above kEigBatchMax (and of single
-// dense problems): G CTAs per problem, a thread-block cluster or a cooperative grid,
-// one barrier between dependent steps and the intermediates in global memory
-// (L2-resident for the vectors and panels).
-//   Cholesky     32-wide panels: the diagonal block factored by every CTA (same
-//                data, same arithmetic, same result), panel rows and lower
-//                trailing tiles split over the CTAs
+// Tridiagonalisation of orders that no cluster's shared memory holds, and of single
+// dense problems above kGridMin: G CTAs per problem, a thread-block cluster or a
+// cooperative grid, one barrier between dependent steps and the intermediates in
+// global memory (L2-resident for the vectors and panels).
 //   tridiag.     blocked Householder with lazy updates (LAPACK's latrd
 //                scheme): per column the panel's earlier reflectors update that
 //                column, the reflector is formed, and y = A v runs over the
@@ -702,7 +646,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_eig_trd(const EigProb* __restr
 //                per-CTA slots summed in CTA order, so results do not depend on
 //                scheduling.  Two barriers per column.
 // ===========================================================================
-constexpr int kLargeMax = kEigLargeMax;   // largest order the cluster solver takes (its vectors live in shared memory)
+constexpr int kLargeMax = kEigLargeMax;   // largest order it takes (its vectors live in shared memory)
 constexpr int kRedW = 2 * NB + 4;         // per-CTA partial sums of the tridiagonalisation
 constexpr int kRedVAv = 2 * NB + 1;       // slot of the partial v^T A v
 // Software barrier over the CTAs of a cooperative launch (all resident):
@@ -819,104 +763,6 @@ __device__ __forceinline__ void tri_decode(int64_t idx, int& rb, int& cb) {
     cb = (int)(idx - (int64_t)r * (r + 1) / 2);
 }
 
-// H_k into X, S_k into L (generalized problems), columns split over the CTAs.
-__device__ void lg_gather(const Grp& g, const EigProb& p, const int* __restrict__ maps, const double* __restrict__ H,
-                          const double* __restrict__ S, double* __restrict__ X, int64_t ldx, double* __restrict__ L) {
-    const int m = p.m;
-    const int* mp = maps + p.moff;
-    for (int j = g.rank; j < m; j += g.size) {
-        const int64_t gj = p.gbase + (int64_t)mp[j] * p.gld;
-        for (int i = threadIdx.x; i < m; i += kT) {
-            const int64_t q = (int64_t)mp[i] + gj;
-            X[i + (int64_t)j * ldx] = H[q];
-            if (p.kind == 0) L[i + (int64_t)j * m] = S[q];
-        }
-    }
-}
-
-// S_k = L L^T (lower) on the cluster; returns the order of the first
-// non-positive pivot (0: positive definite), the same on every CTA.
-__device__ int lg_potrf(const Grp& g, int m, double* __restrict__ L, const LgSmem& sh) {
-    double* sD = sh.sD;   // sD[i + j*(NB+1)]
-    int& fail = sh.ints[0];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) fail = 0;
-    __syncthreads();
-    for (int kb = 0; kb < m; kb += NB) {
-        const int nb = min(NB, m - kb);
-        for (int t = tid; t < NB * NB; t += kT) {
-            const int i = t % NB, j = t / NB;
-            sD[i + j * (NB + 1)] = (i < nb && j < nb) ? L[(int64_t)(kb + i) + (int64_t)(kb + j) * m] : 0.0;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            for (int jj = 0; jj < nb; ++jj) {
-                if (lane == jj) {
-                    const double piv = sD[jj + jj * (NB + 1)];
-                    if (!(piv > 0.0)) fail = kb + jj + 1;
-                    else sD[jj + jj * (NB + 1)] = sqrt(piv);
-                }
-                __syncwarp();
-                if (fail) break;
-                const double djj = sD[jj + jj * (NB + 1)];
-                if (lane > jj && lane < nb) sD[lane + jj * (NB + 1)] /= djj;
-                __syncwarp();
-                if (lane > jj && lane < nb) {
-                    const double lij = sD[lane + jj * (NB + 1)];
-                    for (int k = jj + 1; k <= lane; ++k) sD[lane + k * (NB + 1)] -= lij * sD[k + jj * (NB + 1)];
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        if (fail) break;   // every CTA factored the same block: the same decision everywhere
-        if (g.rank == 0)
-            for (int t = tid; t < nb * nb; t += kT) {
-                const int i = t % nb, j = t / nb;
-                if (i >= j) L[(int64_t)(kb + i) + (int64_t)(kb + j) * m] = sD[i + j * (NB + 1)];
-            }
-        for (int r = kb + nb + g.rank * kT + tid; r < m; r += g.size * kT) {
-            double x[NB];
-#pragma unroll
-            for (int j = 0; j < NB; ++j) x[j] = (j < nb) ? L[(int64_t)r + (int64_t)(kb + j) * m] : 0.0;
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                if (j < nb) {
-                    double v = x[j];
-                    for (int k = 0; k < j; ++k) v -= x[k] * sD[j + k * (NB + 1)];
-                    x[j] = v / sD[j + j * (NB + 1)];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < NB; ++j)
-                if (j < nb) L[(int64_t)r + (int64_t)(kb + j) * m] = x[j];
-        }
-        g.sync();
-        const int t0 = kb + nb;
-        const int nt = (m - t0 + TS - 1) / TS;
-        const int64_t ntile = (int64_t)nt * (nt + 1) / 2;
-        for (int64_t idx = g.rank; idx < ntile; idx += g.size) {
-            int rb, cb;
-            tri_decode(idx, rb, cb);
-            const int r0 = t0 + rb * TS, c0 = t0 + cb * TS;
-            tile_update<true, true>(L, m, r0, c0, min(TS, m - r0), min(TS, m - c0), L + (int64_t)kb * m, m,
-                                    L + (int64_t)kb * m, m, nb, sh.sA, sh.sB);
-        }
-        g.sync();
-    }
-    __syncthreads();
-    const int f = fail;
-    __syncthreads();
-    if (f) return f;
-    for (int j = 1 + g.rank; j < m; j += g.size)
-        for (int i = tid; i < j; i += kT) L[(int64_t)i + (int64_t)j * m] = 0.0;
-    return 0;
-}
-
-// X <- L^-1 X for the 64-column blocks cb = rank, rank + G, ... of X (m x m):
-// left-looking over 64-row blocks, X_i -= L[i, <i] X[<i] as one tile product,
-// then the diagonal block's forward substitution (warp per column, two rows per
-// lane).  The column blocks are independent, so no cluster barrier is needed.
 // w of reflector jp (column j - 1 of the panel's first column j0 = j - 1 - jp)
 // on this CTA's rows r >= j, from the summed partial products; the reflector
 // itself goes into column j - 1 below its leading 1.  Returns w at row j
@@ -1180,24 +1026,6 @@ __device__ __forceinline__ Grp lg_group(unsigned* bar, int* err) {
     cg::cluster_group cl = cg::this_cluster();
     return Grp{(int)cl.block_rank(), (int)cl.num_blocks(), nullptr, nullptr};
 }
-__global__ void __launch_bounds__(kT, 1) k_lg_chol(const EigProb* __restrict__ probs, const int* __restrict__ order,
-                                                   const int* __restrict__ maps, const double* __restrict__ H,
-                                                   const double* __restrict__ S, double* __restrict__ Ca,
-                                                   double* __restrict__ Xa, double* __restrict__ La,
-                                                   int* __restrict__ status, unsigned* __restrict__ bar,
-                                                   int* __restrict__ err) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const LgSmem sh = lg_smem(smraw, 2);
-    const Grp g = lg_group(bar, err);
-    const int pi = order[bar ? 0 : blockIdx.x / g.size];
-    const EigProb p = probs[pi];
-    // a standard problem needs no reduction: its matrix goes where that leaves it
-    lg_gather(g, p, maps, H, S, p.kind == 0 ? Xa + p.aoff : Ca + p.coff, p.kind == 0 ? p.m : p.ldc, La + p.aoff);
-    g.sync();
-    const int st = p.kind == 0 ? lg_potrf(g, p.m, La + p.aoff, sh) : kStOk;
-    if (g.rank == 0 && threadIdx.x == 0) status[pi] = st;
-}
-
 __global__ void __launch_bounds__(kT, 1) k_lg_trd(const EigProb* __restrict__ probs, const int* __restrict__ order,
                                                   int M, double* __restrict__ Ca, double* __restrict__ Da,
                                                   double* __restrict__ Ea, double* __restrict__ Ta,
@@ -1275,6 +1103,9 @@ struct EigBatch {
     std::vector<int2> lists;
     std::vector<DcMerge> merges;
     std::vector<Level> levels;
+    bool timed = false;   // stage times wanted (PTBGPU_EIG_STAGES)
+    std::vector<std::pair<const char*, cudaEvent_t>> marks;   // what ended, and when
+    std::vector<unsigned> deep;   // tasks of `blocks` that block column j of the Cholesky factor launches
     Seg blocks, leaves, panels, rows, rq, back, density, fblocks, frq, fcols;
     WorkBuf probs, order_d, lists_d, merges_d, cnt, dc, Ca, La, Za, Qa, Va, Da, Ea, Ta, Ba, Xa, Ka, Ia, status;
     DcArr S{};
@@ -1303,11 +1134,12 @@ void smem_attr(K kern, size_t bytes) {
 
 void eig_setup_attrs() {
     static const bool done = [] {
-        smem_attr(k_eig_chol, kCholSmem);
+        smem_attr(k_chol_column, kTileSmem);
+        smem_attr(k_chol_scale, kTileSmem);
+        smem_attr(k_eig_rsolve, kTileSmem);
         smem_attr(k_eig_trsm, kTileSmem);
         smem_attr(k_eig_trd<512>, 8 * trd_cap(kTrdMax512, 512));
         smem_attr(k_eig_trd<256>, 8 * trd_cap(kTrdMax256, 256));
-        smem_attr(k_lg_chol, lg_smem_bytes(2));
         smem_attr(k_lg_trd, lg_smem_bytes(kLargeMax));
         smem_attr(k_trd_cluster, kTrdCaps[3] - 1024);
         PTB_CUDA(cudaFuncSetAttribute(k_trd_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -1321,7 +1153,6 @@ void eig_setup_attrs() {
         smem_attr(k_vec_rows, kChainSmem);
         smem_attr(k_vec_back, kChainSmem);
         smem_attr(k_fin_cols, kChainSmem);
-        PTB_CUDA(cudaFuncSetAttribute(k_lg_chol, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         PTB_CUDA(cudaFuncSetAttribute(k_lg_trd, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         return true;
     }();
@@ -1356,9 +1187,9 @@ int eig_active_cached(ptbgpu_ctx* c, int G) {
     return a - 1;
 }
 
-// CTAs of the cluster Cholesky and of the cluster tridiagonalisation for orders beyond
-// the shared-memory one: 16 for one problem, else 8.  PTBGPU_EIG_CLUSTER = 1, 2, 4, 8 or
-// 16 sets them, and the tridiagonalisation's of every order above kEigBatchMax.
+// CTAs of the cluster tridiagonalisation for orders beyond the shared-memory one: 16
+// for one problem, else 8.  PTBGPU_EIG_CLUSTER = 1, 2, 4, 8 or 16 sets them, and those
+// of every order above kEigBatchMax.
 int eig_cluster_forced() {
     const char* e = getenv("PTBGPU_EIG_CLUSTER");
     const int v = e ? atoi(e) : 0;
@@ -1526,6 +1357,13 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     list(eb.blocks, [&] {   // 64-column blocks (64-element chunks) of the generalized problems
         for (int q : all)
             for (int b = 0; b < tiles(eb.hp[q].m); ++b) put(q, b);
+        // deep[j]: the leading tasks that hold every problem of more than j blocks
+        eb.deep.clear();
+        for (size_t i = eb.blocks.off; i < eb.lists.size(); ++i) {
+            const size_t nb = (size_t)tiles(eb.hp[eb.lists[i].x].m);
+            if (eb.deep.size() < nb) eb.deep.resize(nb);
+            for (size_t j = 0; j < nb; ++j) eb.deep[j] = (unsigned)(i - eb.blocks.off + 1);
+        }
     });
     list(eb.leaves, [&] {
         for (int q : all)
@@ -1637,7 +1475,7 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
 void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const double* S, const int* d_maps,
              const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe) {
     const EigProb* dp = eb.probs.as<EigProb>();
-    const int *ord = eb.order_d.as<int>(), *ord_l = ord + eb.nsmall;
+    const int* ord = eb.order_d.as<int>();
     const DcMerge* mg = eb.merges_d.as<DcMerge>();
     double *Ca = eb.Ca.as<double>(), *La = eb.La.as<double>(), *Za = eb.Z, *Qa = eb.Qa.as<double>(),
            *Va = eb.Va.as<double>(), *Da = eb.Da.as<double>(), *Ea = eb.Ea.as<double>(), *Ta = eb.Ta.as<double>(),
@@ -1671,33 +1509,30 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         count_launch(k);
         PTB_CUDA(cudaGetLastError());
     };
-    // ---- Cholesky
-    fork(eb.nsmall > 0 && eb.nlarge > 0);
-    if (eb.nlarge > 0) {
-        const cudaStream_t ls = branch(eb.nsmall == 0);
-        if (eb.grid) {
-            void* args[] = {&dp, &ord_l, &d_maps, &H, &S, &Ca, &Qa, &La, &st, &bar, &err};
-            PTB_CUDA(cudaLaunchCooperativeKernel((void*)k_lg_chol, dim3(eb.G), dim3(kT), args, lg_smem_bytes(2), ls));
-        } else {
-            launch_clustered(k_lg_chol, eb.nlarge, eb.G, lg_smem_bytes(2), ls, dp, ord_l, d_maps, H, S, Ca, Qa, La, st,
-                             bar, err);
-        }
-        launched();
-    }
-    if (eb.nsmall > 0) {
-        k_eig_chol<<<eb.nsmall, kT, kCholSmem, s>>>(dp, ord, d_maps, H, S, Qa, La, st);
-        launched();
-    }
-    join();
-    // ---- C = L^-1 H L^-T
+    auto mark = [&](const char* what) {
+        if (!eb.timed) return;
+        eb.marks.push_back({what, c->take_event()});
+        PTB_CUDA(cudaEventRecord(eb.marks.back().second, s));
+    };
+    mark("");
+    // ---- Cholesky and C = L^-1 H L^-T (lower triangle)
+    const int2* bl = eb.list(eb.blocks);
+    k_eig_gather<<<eb.blocks.n, kT, 0, s>>>(dp, bl, d_maps, H, S, Ca, Qa, La);
+    launched();
     if (eb.hp[0].kind == 0) {
-        const int2* bl = eb.list(eb.blocks);
-        k_eig_dinv<<<eb.blocks.n, kT, 0, s>>>(dp, bl, La, Ia, st);
-        k_eig_trsm<<<eb.blocks.n, kT, kTileSmem, s>>>(dp, bl, La, Ia, Qa, false, st);
-        k_eig_transpose<<<eb.blocks.n, 256, 0, s>>>(dp, bl, Qa, Ca, st);
-        k_eig_trsm<<<eb.blocks.n, kT, kTileSmem, s>>>(dp, bl, La, Ia, Ca, true, st);
-        launched(4);
+        for (size_t j = 0; j < eb.deep.size(); ++j) {
+            k_chol_column<<<eb.deep[j], kT, kTileSmem, s>>>(dp, bl, (int)j, La, Ia, st);
+            launched();
+            if (j + 1 == eb.deep.size()) break;
+            k_chol_scale<<<eb.deep[j + 1], kT, kTileSmem, s>>>(dp, bl, (int)j, La, Ia, st);
+            launched();
+        }
+        mark("Cholesky");
+        k_eig_trsm<<<eb.blocks.n, kT, kTileSmem, s>>>(dp, bl, La, Ia, Qa, st);
+        k_eig_rsolve<<<eb.blocks.n, kT, kTileSmem, s>>>(dp, bl, La, Ia, Qa, Ca, st);
+        launched(2);
     }
+    mark("reduction");
     // ---- tridiagonalisation, the widest groups first
     fork(eb.trd.size() > 1);
     for (size_t i = 0; i < eb.trd.size(); ++i) {
@@ -1722,6 +1557,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         launched();
     }
     join();
+    mark("tridiagonalisation");
     // ---- reflector panels, and the owned rows up to Z
     if (eb.panels.n) {
         k_vec_panels<<<eb.panels.n, kT, kWySmem, s>>>(dp, eb.list(eb.panels), Ca, Ta, Ka, st);
@@ -1731,6 +1567,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         k_vec_rows<<<eb.rows.n, kT, kChainSmem, s>>>(dp, eb.list(eb.rows), Ca, La, Ia, Ka, d_own_cols, d_ipos, Ba, st);
         launched();
     }
+    mark("panels");
     // ---- divide and conquer
     k_dc_leaves<<<(eb.leaves.n + kLeafWarps - 1) / kLeafWarps, 32 * kLeafWarps, 0, s>>>(
         dp, eb.list(eb.leaves), (int)eb.leaves.n, Da, Ea, Za, D, st);
@@ -1748,6 +1585,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
             launched();
         }
     }
+    mark("divide and conquer");
     // ---- what leaves the solver
     if (eb.rq.n) {
         const int2* rq = eb.list(eb.rq);
@@ -1768,6 +1606,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
         k_vec_density<<<eb.density.n, kT, kTileSmem, s>>>(dp, eb.list(eb.density), Za, Ba, st);
         launched();
     }
+    mark("vectors");
 }
 
 }  // namespace
@@ -1893,11 +1732,23 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
     std::vector<int> ident(n);
     for (int i = 0; i < m; ++i) ident[i] = i;
     PTB_CUDA(cudaMemcpyAsync(map.ptr, ident.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    // PTBGPU_EIG_STAGES=1: stage times on stderr
+    static const bool stages = getenv("PTBGPU_EIG_STAGES") != nullptr;
+    eb.timed = stages;
     eig_plan(c, eb, s, 0, U);
     eig_run(c, eb, s, H, S, map.as<int>(), nullptr, nullptr, w, nullptr);
     int hs[4];
     PTB_CUDA(cudaMemcpyAsync(hs, eb.status.ptr, sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
+    if (!eb.marks.empty()) {
+        fprintf(stderr, "eig_full n=%d:", m);
+        for (size_t i = 1; i < eb.marks.size(); ++i) {
+            float ms = 0.f;
+            PTB_CUDA(cudaEventElapsedTime(&ms, eb.marks[i - 1].second, eb.marks[i].second));
+            fprintf(stderr, " %s %.3f", eb.marks[i].first, ms);
+        }
+        fprintf(stderr, " ms\n");
+    }
     PTB_CHECK(hs[3] == 0, PTBGPU_ETIMEOUT, "eigensolver: a grid barrier gave up waiting");
     PTB_CHECK(hs[0] <= 0, PTBGPU_ENOTSPD, "overlap matrix not positive definite (leading minor %d)", hs[0]);
     PTB_CHECK(hs[0] == kStOk, PTBGPU_EITER, "tridiagonal eigensolver did not converge");

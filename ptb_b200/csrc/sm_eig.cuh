@@ -8,12 +8,12 @@
 
 namespace ptb {
 
-// Largest submatrix the batched solver takes (its per-problem shared-memory
-// vectors are sized for it); larger ones go to the side-stream path.
+// Largest order whose tridiagonalisation may run on one CTA (its vectors fill the
+// shared memory); larger ones take a thread-block cluster.  Problems above it go up and
+// start before the rest of a batch does.
 constexpr int kEigBatchMax = 800;
-// Largest submatrix the library's eigensolver takes at all: orders above
-// kEigBatchMax run on a thread-block cluster each, whose tridiagonalisation
-// keeps two vectors of this length in shared memory.
+// Largest submatrix the library's eigensolver takes at all: the tridiagonalisation of
+// the largest orders keeps two vectors of this length in shared memory.
 constexpr int kEigLargeMax = 12032;
 
 // One submatrix as the host plan describes it.
@@ -42,8 +42,8 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
                                            const std::vector<EigProbHost>& probs, const int* d_maps,
                                            const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe,
                                            int prl, double* flops, bool join = true);
-// With join = false the launch's side stream (the clusters of the problems
-// above kEigBatchMax) is not waited for on the context's stream; this does it.
+// With join = false the batch runs on a stream of its own, which the context's stream
+// does not wait for; this does it.
 void eig_batch_join(ptbgpu_ctx* c, EigBatch& eb);
 void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb);
 
@@ -54,7 +54,7 @@ void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, int64_t n, const in
                      const int* d_own_cols, double* dP, double* dPdense = nullptr);
 
 // All eigenpairs of a dense problem on the device with the same solver on the
-// whole GPU (one cooperative launch): H U = S U diag(w) (S null: the standard
+// whole GPU, in the same stages: H U = S U diag(w) (S null: the standard
 // problem), H and S full symmetric (n x n, ld n; only the lower triangles are
 // read), w ascending, U column-major with U^T S U = I.  Orders up to
 // kEigLargeMax.
@@ -63,7 +63,7 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
 // triangles read): A (and B) n x n, ld n; A is overwritten by the eigenvectors.
 void eig_full_upper(ptbgpu_ctx* c, int64_t n, double* A, double* B, double* w);
 
-// The density step of many independent systems in one launch of the
+// The density step of many independent systems as one batch of the
 // eigensolver (ptbgpu_eig_density_batch): Hpk / Spk / Ppk host packed arrays
 // per system, P_k = 2 sum_{i < nel_k/2} u_i u_i^T of H_k U = S_k U e after the
 // filter; stats per system (may be null).

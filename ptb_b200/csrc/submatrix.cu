@@ -893,7 +893,7 @@ void sm_prepare(ptbgpu_ctx* c, SmPlan& pl, const std::vector<int>& ids) {
         t_last = now;
     };
 
-    constexpr int kBatchMax = kEigBatchMax;
+    constexpr int kBatchMax = 1024;   // the cuSOLVER comparison's batched routines take these
     std::vector<Prob> small, large;
     int64_t eoff = 0;
     for (int k : ids) {
@@ -907,10 +907,9 @@ void sm_prepare(ptbgpu_ctx* c, SmPlan& pl, const std::vector<int>& ids) {
     DevBuf& bfe = c->buf(B_MISC1);
     be.reserve(sizeof(double) * std::max<int64_t>(eoff, 1));
     bfe.reserve(sizeof(double) * std::max<int64_t>(eoff, 1));
-    // every submatrix through the library's eigensolver: up to kEigBatchMax one
-    // CTA each in a persistent launch, above it one thread-block cluster each;
+    // every submatrix up to kEigLargeMax through the library's eigensolver;
     // PTBGPU_SM_EIG=library sends them through cuSOLVER instead (batched routines
-    // in tuned size buckets, dsygvd above kEigBatchMax; kept for comparison)
+    // in tuned size buckets, dsygvd above kBatchMax; kept for comparison)
     static const bool use_library = [] {
         const char* v = getenv("PTBGPU_SM_EIG");
         return v != nullptr && std::string(v) == "library";
@@ -924,7 +923,7 @@ void sm_prepare(ptbgpu_ctx* c, SmPlan& pl, const std::vector<int>& ids) {
             own_probs.push_back(
                 {p.k, p.m, (int)(pl.own_off[p.k + 1] - pl.own_off[p.k]), p.moff, p.eoff, pl.own_off[p.k]});
         small.clear();
-        // above kEigBatchMax: one thread-block cluster per submatrix, up to kEigLargeMax
+        // the eigensolver takes orders up to kEigLargeMax
         std::vector<Prob> rest;
         for (const Prob& p : large) {
             if (p.m <= kEigLargeMax)
