@@ -195,14 +195,13 @@ int ptbgpu_tc_purify_batch(ptbgpu_ctx* ctx, int64_t ninst, const int64_t* ndim, 
                            const double* const* Hpk, const double* const* Spk, double* const* Ppk,
                            int64_t workers, const ptbgpu_opts* opts, ptbgpu_stats* st, double* wall_ms);
 
-/* The density step of many independent systems in one launch of the library's
+/* The density step of many independent systems as one batch of the library's
  * FP64 eigensolver: per system the filtered generalized eigenproblem
  * H_k U = S_k U e and P_k = 2 sum_{i < nel_k/2} u_i u_i^T (the dense projector
  * at T = 0, i.e. the reference's solve2, source/pgtb.f90:1066-1170, without the
- * Fermi smearing), P_k formed in the same launch; nel_k must be even (closed
- * shell: an odd count is EINVAL).  Systems up to order 1024 run
- * one CTA each in a persistent launch (largest first), larger ones (up to 12032)
- * one thread-block cluster each, beside them.  opts->filter is applied to H and
+ * Fermi smearing), P_k formed in the same batch; nel_k must be even (closed
+ * shell: an odd count is EINVAL).  Systems of orders up to 12032; every stage of the
+ * solver is launched over all of them.  opts->filter is applied to H and
  * S (filter_matrix_sym).  Per-system stats carry flops; wall_ms the host time of
  * the call.  ENOTSPD names the first system whose S is not positive definite. */
 int ptbgpu_eig_density_batch(ptbgpu_ctx* ctx, int64_t ninst, const int64_t* ndim, const int64_t* nel,
@@ -321,7 +320,8 @@ int ptbgpu_symsq_bf16x3(ptbgpu_ctx* ctx, int64_t n, const double* X, float* C);
 int ptbgpu_symsq_bf16x6(ptbgpu_ctx* ctx, int64_t n, const double* X, float* C);
 /* Either split with an explicit kernel: planes 2 or 3; kblock 32 or 64 (one CTA,
  * that K block), 1032 or 1064 (two planes only: the CTA-pair cta_group::2
- * kernel with K block 32 or 64), or 0 (the autotuned choice). */
+ * kernel with K block 32 or 64), 2064 (two planes only: 128 x 128 tiles), or 0
+ * (the autotuned choice). */
 int ptbgpu_symsq_split(ptbgpu_ctx* ctx, int64_t n, int64_t planes, int64_t kblock, const double* X, float* C,
                        double* ms);   /* ms (may be NULL): device time of the product launch(es) */
 /* C = A * B for n x n FP64 row-major host matrices, on the int8 tensor cores
@@ -353,8 +353,7 @@ int ptbgpu_oz_gemm(ptbgpu_ctx* ctx, int64_t n, int64_t slices, int64_t kblock, i
 /* The batched FP64 generalized eigensolver of the submatrix method on dense
  * host problems (kernel-level entry for tests and measurements; it replaces the
  * per-submatrix la_sygvd and the S_k U product of source/sm.f90:296-310).
- * Orders up to 1024 run one CTA per problem in a persistent launch, larger ones
- * one thread-block cluster per problem.  nprob problems of orders dims[k]
+ * Every stage is launched over all problems of the call.  nprob problems of orders dims[k]
  * (1..10240): H and S hold their column-major dims[k]^2 blocks one after
  * another; owned holds nown[k] (0-based, local) owned indices per problem, one
  * list after another.  Out: e and fe (sum of dims each, per problem in the

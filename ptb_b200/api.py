@@ -443,7 +443,7 @@ class Context:
         return Ps, [Stats.from_c(st[i]) for i in range(n)], wall.value
 
     def eig_density_batch(self, systems, opts: Options | None = None):
-        """The density step of many independent systems in one launch of the
+        """The density step of many independent systems as one batch of the
         FP64 eigensolver (ptbgpu_eig_density_batch): `systems` a sequence of
         (ndim, nel, H, S) packed; P = 2 sum of the nel/2 lowest generalized
         eigenvectors' outer products (opts.filter applied to H and S).  Returns
@@ -545,7 +545,8 @@ class Context:
 
     def symsq_split(self, X: np.ndarray, planes: int, kblock: int, timed: bool = False):
         """C = X X with an explicit plane count (2 or 3) and kernel: K block 32 /
-        64 (one CTA), 1032 / 1064 (CTA pair, two planes), 0 = tuned.  timed:
+        64 (one CTA), 1032 / 1064 (CTA pair, two planes), 2064 (128 x 128
+        tiles, two planes), 0 = tuned.  timed:
         returns (C, device milliseconds of the product launches)."""
         ms = C.c_double(0.0)
         out = self._symsq(X, lambda h, n, x, o: self._lib.ptbgpu_symsq_split(h, n, planes, kblock, x, o,

@@ -381,8 +381,8 @@ int ptbgpu_symsq_bf16x6(ptbgpu_ctx* c, int64_t n, const double* X, float* C) {
 int ptbgpu_symsq_split(ptbgpu_ctx* c, int64_t n, int64_t planes, int64_t kblock, const double* X, float* C,
                        double* ms) {
     return guarded(c, [&] {
-        // kblock: 0 tuned, 32 / 64 one CTA, 1032 / 1064 CTA pair (two planes only)
-        const bool pair = kblock == tc::kPairKernel + 32 || kblock == tc::kPairKernel + 64;
+        // kblock: 0 tuned, 32 / 64 one CTA, 1032 / 1064 CTA pair, 2064 128 x 128 tiles (two planes only)
+        const bool pair = kblock == tc::kPairKernel + 32 || kblock == tc::kPairKernel + 64 || kblock == tc::kNarrowKernel;
         PTB_CHECK(n > 0 && X && C && (planes == 2 || planes == 3) &&
                       (kblock == 0 || kblock == 32 || kblock == 64 || (pair && planes == 2)),
                   PTBGPU_EINVAL, "bad arguments");

@@ -601,7 +601,10 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     // tiles and per-tile stats
     std::vector<int2> up = tc::make_tiles(ldp, true, 256);
     std::vector<int2> up3 = tc::make_tiles(ldp, true, 128);
-    std::vector<int2> all = tc::make_tiles(ldp, false, 256);
+    std::vector<int2> all3 = tc::make_tiles(ldp, false, 128);
+    // 128 x 128 tiles where one wave takes them
+    const bool narrow_up = tc::narrow_fits(up3.size()), narrow_all = tc::narrow_fits(all3.size());
+    std::vector<int2> all = narrow_all ? std::move(all3) : tc::make_tiles(ldp, false, 256);
     std::vector<int2> pup = tc::make_pair_tiles(ldp, true);     // CTA-pair kernel tiles
     std::vector<int2> pall = tc::make_pair_tiles(ldp, false);
     DevBuf& bt = c->buf(B_TILES);
@@ -656,6 +659,10 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     auto three_planes = [&](int k) { return split3_iters < 0 ? false : (split3_iters == 0 || k < split3_iters); };
     int launched = 0;
     const size_t timed0 = c->timed.size();   // pass-1 step timings start here
+    auto general = [&](const void* const* a, const void* const* b, const tc::EpiParams& e) {
+        timed_product(c, tc::EPI_FULL, 2, ldp, a, b, split3, tiles_all, (int)all.size(), e,
+                      narrow_all ? tc::kNarrowKernel : 0, pairs_all, npall);
+    };
     SP2State* hs = (SP2State*)c->pinned;   // only the 8-int header is read back while iterating
     for (int k = 0; k < cap; ++k) {
         ep.xcur = xf[k & 1];
@@ -666,7 +673,8 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
         const void* pl[3] = {traj(k, 0), traj(k, 1), traj(k, 2)};
         const bool three = three_planes(k);
         const int ntl = three ? timed_product(c, tc::EPI_SP2, 3, ldp, pl, pl, split6, tiles_up3, n6, ep)
-                              : timed_product(c, tc::EPI_SP2, 2, ldp, pl, pl, split3, tiles_up, n3, ep, 0, pairs_up,
+                              : timed_product(c, tc::EPI_SP2, 2, ldp, pl, pl, split3, narrow_up ? tiles_up3 : tiles_up,
+                                              narrow_up ? n6 : n3, ep, narrow_up ? tc::kNarrowKernel : 0, pairs_up,
                                               npup);
         k_decide<<<1, 256, 0, s>>>(state, stats, ntl, N, tol_abs, e_asym, e_stag, cap);
         count_launch();
@@ -694,7 +702,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     // executed tcgen05 flops (all tiles of every launch that ran, every product of the split)
     double tc_exec = 0.0;
     for (int k = 0; k < K; ++k)
-        tc_exec += three_planes(k) ? 2.0 * 6 * 128 * 128 * (double)ldp * n6 : 2.0 * 3 * 128 * 256 * (double)ldp * n3;
+        tc_exec += three_planes(k) ? 2.0 * 6 * 128 * 128 * (double)ldp * n6 : (narrow_up ? 2.0 * 3 * 128 * 128 * (double)ldp * n6 : 2.0 * 3 * 128 * 256 * (double)ldp * n3);
     const double tc_exec_full = 2.0 * 3 * (double)ldp * ldp * ldp;   // one general bf16x3 product
     for (int k = 0; k <= K && prl >= 2; ++k)
         log_line(prl, 2, " SP2 (bf16x3) iter %3d  trX %.10f  err %.3e  %s", k, H.trX[k], H.err[k],
@@ -848,7 +856,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
         epf.out = wf;
         const void* pc[2] = {chi, clo};
         const void* pp[2] = {phi, plo};
-        timed_product(c, tc::EPI_FULL, 2, ldp, pc, pp, split3, tiles_all, (int)all.size(), epf, 0, pairs_all, npall);
+        general(pc, pp, epf);
         // The planes hold C^T (column-major C read row-major), so wf = C^T P~ = -C P~.
         // A1 = C P~ - P~ C = -(wf + wf^T) and X1_0 = -A1 / (e_max - e_min) = (wf + wf^T) * scale.
         const unsigned nbp = (unsigned)(ldp / 32);
@@ -869,7 +877,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
             const int a = k & 1, b = a ^ 1;
             const void* p0[2] = {traj_hi(k), traj_lo(k)};
             const void* p1[2] = {x1hi[a], x1lo[a]};
-            timed_product(c, tc::EPI_FULL, 2, ldp, p0, p1, split3, tiles_all, (int)all.size(), epf, 0, pairs_all, npall);
+            general(p0, p1, epf);
             const bool sq = H.sq[k] != 0;
             k_sym_update<<<dim3(nbp, nbp), dim3(32, 8), 0, s>>>(ldp, wf, x1f[a], sq ? 1.0f : -1.0f,
                                                                 sq ? 0.0f : 2.0f, x1f[b], x1hi[b], x1lo[b]);
@@ -886,14 +894,14 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
             const int a = K & 1, b = a ^ 1;
             const void* pp2[2] = {phi, plo};
             const void* px[2] = {x1hi[a], x1lo[a]};
-            timed_product(c, tc::EPI_FULL, 2, ldp, pp2, px, split3, tiles_all, (int)all.size(), epf, 0, pairs_all, npall);   // W
+            general(pp2, px, epf);   // W
             k_split2<<<grid1(ldp * ldp / 256), 256, 0, s>>>(ldp * ldp, wf, x1hi[b], x1lo[b]);
             count_launch();
             PTB_CUDA(cudaGetLastError());
             tc::EpiParams epv = epf;
             epv.out = x1f[b];
             const void* pw[2] = {x1hi[b], x1lo[b]};
-            timed_product(c, tc::EPI_FULL, 2, ldp, pw, pp2, split3, tiles_all, (int)all.size(), epv, 0, pairs_all, npall);  // W P~
+            general(pw, pp2, epv);  // W P~
             k_sym_update<<<dim3(nbp, nbp), dim3(32, 8), 0, s>>>(ldp, wf, x1f[b], 1.0f, -2.0f, x1f[a], x1hi[a],
                                                                 x1lo[a]);
             count_launch();
@@ -906,12 +914,12 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
             const void* px1[2] = {x1hi[a], x1lo[a]};
             tc::EpiParams epy = epf;
             epy.out = x1f[b];
-            timed_product(c, tc::EPI_FULL, 2, ldp, px1, px1, split3, tiles_all, (int)all.size(), epy, 0, pairs_all, npall);   // Y
+            general(px1, px1, epy);   // Y
             k_split2<<<grid1(ldp * ldp / 256), 256, 0, s>>>(ldp * ldp, x1f[b], x1hi[b], x1lo[b]);
             count_launch();
             PTB_CUDA(cudaGetLastError());
             const void* py[2] = {x1hi[b], x1lo[b]};
-            timed_product(c, tc::EPI_FULL, 2, ldp, pp2, py, split3, tiles_all, (int)all.size(), epf, 0, pairs_all, npall);    // W2
+            general(pp2, py, epf);    // W2
             k_add_f32<<<grid1(ldp * ldp / 256), 256, 0, s>>>(ldp * ldp, x1f[a], x1f[b]);              // Y + X1
             count_launch();
             PTB_CUDA(cudaGetLastError());
@@ -1054,7 +1062,7 @@ void symsq_entry(ptbgpu_ctx* c, int64_t n, int np, int kblock, const double* hX,
     // planes of the FP32-rounded X: hi, mid = bf16(x - hi), lo = bf16(x - hi - mid)
     d2f_split(s, n, ldp, bx.as<double>(), xf, hi, mid);
     d2f_split3(s, ldp, xf, hi, mid, lo);
-    std::vector<int2> all = tc::make_tiles(ldp, false, np == 2 ? 256 : 128);
+    std::vector<int2> all = tc::make_tiles(ldp, false, np == 2 && kblock != tc::kNarrowKernel ? 256 : 128);
     std::vector<int2> pall = np == 2 ? tc::make_pair_tiles(ldp, false) : std::vector<int2>();
     DevBuf& bt = c->buf(B_TILES);
     bt.reserve(sizeof(int2) * (all.size() + pall.size()));

@@ -131,13 +131,16 @@ __device__ __forceinline__ void tc_epilogue(const EpiParams& ep, uint32_t tmem, 
                 uint4* ho = reinterpret_cast<uint4*>(ep.hi + r * ld + cbase);
                 uint4* mo = reinterpret_cast<uint4*>(ep.lo + r * ld + cbase);
                 uint4* lo = w3 ? reinterpret_cast<uint4*>(ep.lo2 + r * ld + cbase) : nullptr;
+                // X is only needed for 2X - X^2: skip its read on the square branch.  The chunk's
+                // eight reads go out together, before any store that could alias them holds
+                // them back
+                float4 xc[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) xc[q] = square ? make_float4(0.f, 0.f, 0.f, 0.f) : xin[q];
 #pragma unroll
                 for (int j8 = 0; j8 < 4; ++j8) {
                     float val[8];
-                    // X is only needed for 2X - X^2: skip its read on the square branch
-                    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float4 x0 = square ? zero4 : xin[2 * j8];
-                    const float4 x1 = square ? zero4 : xin[2 * j8 + 1];
+                    const float4 x0 = xc[2 * j8], x1 = xc[2 * j8 + 1];
                     const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
                     __align__(16) __nv_bfloat16 hh[8], mm[8], ll[8];
 #pragma unroll
@@ -577,11 +580,13 @@ void launch_pair(cudaStream_t s, const TmaPlanes& maps, const ProdList& prods, c
 }
 
 template <int EPI>
-void launch_epi(cudaStream_t s, int np, int kb, bool pair, const TmaPlanes& maps, const ProdList& prods,
+void launch_epi(cudaStream_t s, int np, int kb, bool pair, bool narrow, const TmaPlanes& maps, const ProdList& prods,
                 const int2* tiles, int ntiles, int nk, const EpiParams& ep) {
     if (pair) {
         if (kb == 64) launch_pair<EPI, 64>(s, maps, prods, tiles, ntiles, nk, ep);
         else launch_pair<EPI, 32>(s, maps, prods, tiles, ntiles, nk, ep);
+    } else if (narrow) {
+        launch_t<EPI, 128, 2, 64>(s, maps, prods, tiles, ntiles, nk, ep);
     } else if (np == 2) {
         if (kb == 64) launch_t<EPI, 256, 2, 64>(s, maps, prods, tiles, ntiles, nk, ep);
         else launch_t<EPI, 256, 2, 32>(s, maps, prods, tiles, ntiles, nk, ep);
@@ -616,12 +621,14 @@ int launch_product(cudaStream_t s, int epi, int np, long long ld, const void* co
               "stacked planes: rows must be a multiple of ld and the epilogue told so");
     PTB_CHECK(np == 2 || np == 3, PTBGPU_EINVAL, "unsupported plane count %d", np);
     PTB_CHECK(kblock == 0 || kblock == 32 || kblock == 64 || kblock == kPairKernel + 32 ||
-                  kblock == kPairKernel + 64,
+                  kblock == kPairKernel + 64 || kblock == kNarrowKernel,
               PTBGPU_EINVAL, "bad kernel choice %d", kblock);
-    PTB_CHECK(kblock < kPairKernel || (np == 2 && pairs_dev != nullptr), PTBGPU_EINVAL,
+    const bool narrow = kblock == kNarrowKernel;
+    PTB_CHECK(!narrow || np == 2, PTBGPU_EINVAL, "the 128-column kernel takes two planes");
+    PTB_CHECK(narrow || kblock < kPairKernel || (np == 2 && pairs_dev != nullptr), PTBGPU_EINVAL,
               "the CTA-pair kernel needs two planes and pair tiles");
     PTB_CHECK(ld % 256 == 0, PTBGPU_EINVAL, "leading dimension must be a multiple of 256");
-    const int bn = np == 2 ? 256 : 128;
+    const int bn = np == 2 && !narrow ? 256 : 128;
     PTB_CHECK(prods.n >= 1 && prods.n <= 6, PTBGPU_EINVAL, "1 to 6 plane products (got %d)", prods.n);
     for (int p = 0; p < prods.n; ++p)
         PTB_CHECK(prods.a[p] >= 0 && prods.a[p] < np && prods.b[p] >= 0 && prods.b[p] < np, PTBGPU_EINVAL,
@@ -630,8 +637,8 @@ int launch_product(cudaStream_t s, int epi, int np, long long ld, const void* co
               "the SP2 epilogue writes at least two planes");
     // returns the number of per-CTA stats partials the launch writes
     auto run = [&](int choice) {
-        const bool pair = choice >= kPairKernel;
-        const int kb = pair ? choice - kPairKernel : choice;
+        const bool pair = choice >= kPairKernel && !narrow;
+        const int kb = narrow ? 64 : pair ? choice - kPairKernel : choice;
         TmaPlanes maps;
         for (int p = 0; p < np; ++p) {
             encode_plane(&maps.a[p], a[p], ld, rows, BM, kb);
@@ -640,13 +647,13 @@ int launch_product(cudaStream_t s, int epi, int np, long long ld, const void* co
         const int nk = (int)(ld / kb);
         const int2* t = pair ? pairs_dev : tiles_dev;
         const int nt = pair ? npairs : ntiles;
-        if (epi == EPI_SP2) launch_epi<EPI_SP2>(s, np, kb, pair, maps, prods, t, nt, nk, ep);
-        else launch_epi<EPI_FULL>(s, np, kb, pair, maps, prods, t, nt, nk, ep);
+        if (epi == EPI_SP2) launch_epi<EPI_SP2>(s, np, kb, pair, narrow, maps, prods, t, nt, nk, ep);
+        else launch_epi<EPI_FULL>(s, np, kb, pair, narrow, maps, prods, t, nt, nk, ep);
         PTB_CUDA(cudaGetLastError());
         return pair ? 2 * npairs : ntiles;
     };
     if (kblock == 0) kblock = tuned_kblock(epi, np, ld, rows);
-    if (kblock != 0 && (kblock < kPairKernel || pairs_dev)) return run(kblock);
+    if (kblock != 0 && (narrow || kblock < kPairKernel || pairs_dev)) return run(kblock);
     std::vector<int> cand = {64, 32};
     if (np == 2 && pairs_dev) {
         cand.push_back(kPairKernel + 64);

@@ -14,6 +14,15 @@ enum : int { EPI_FULL = 0, EPI_SP2 = 1 };
 // Kernel choice codes: K block 64 or 32 for the one-CTA kernel, and
 // kPairKernel + K block for the CTA-pair (cta_group::2, 256 x 256) kernel.
 constexpr int kPairKernel = 1000;
+// Two planes on 128 x 128 tiles (one CTA each, K block 64), for products whose
+// tiles fit one wave.  The accumulation order over K and the plane products is
+// that of every other kernel: the results are the same bits.
+constexpr int kNarrowKernel = 2064;
+// Whether they do, with `tiles` tiles of 128 x 128: 256 x 256 tiles on CTA pairs
+// then occupy less than half of the 148 SMs for twice the time (order 1495, padded
+// to 1536: the symmetric product 42 CTAs 73 us, 78 narrow ones 58; the general one
+// 72 CTAs 43 us, 144 narrow ones 38).
+inline bool narrow_fits(size_t tiles) { return tiles <= 148; }
 
 // Tensor maps of up to three A-role and three B-role bf16 planes (64-byte aligned).
 struct TmaPlanes {
@@ -51,7 +60,7 @@ int tile_n();
 std::vector<int2> make_tiles(long long ld, bool upper_only, int bn);
 std::vector<int2> make_pair_tiles(long long ld, bool upper_only);
 // kblock: 64 / 32 (one CTA), kPairKernel + 64 / + 32 (CTA pair, needs two
-// planes and pairs_dev), or 0 = the autotuned choice for this shape (every
+// planes and pairs_dev), kNarrowKernel (two planes, tiles_dev of 128 x 128), or 0 = the autotuned choice for this shape (every
 // candidate is timed on its first launch).  Returns the number of per-CTA
 // stats partials written (EPI_SP2 reduces that many).
 // rows: rows of every plane (0 = ld; a multiple of ld for stacked systems).
