@@ -201,7 +201,6 @@ void dgemm_nn(ptbgpu_ctx* c, int64_t n, int64_t ld, double alpha, const double* 
               double beta, double* C);
 void dsyrk_sq(ptbgpu_ctx* c, int64_t n, int64_t ld, const double* X, double* C);   // C = X X (X symmetric), full C
 int  dpotrf_lower(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A);              // returns info
-void dtrtri_lower(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A);
 // Device-result form of frob_dev (no host synchronisation; ld = n): the
 // Frobenius norm into a device double; *nan = 1 if it is a NaN, which it is
 // exactly when the matrix holds one (squares are never negative).

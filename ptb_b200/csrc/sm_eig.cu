@@ -82,13 +82,14 @@ struct EigProb {
 //   A(i, k) = AT ? A[kg + (r0+i) lda] : A[(r0+i) + kg lda],   kg = kx ? kx[k] : k
 //   B(k, j) = BT ? B[(c0+j) + kg ldb] : B[kg + (c0+j) ldb],   kg = kxb ? kxb[k] : k
 //   MMA_SET: C[crow + r0 + i, col] = sum_k A(i,k) B(k,j); MMA_SUB: C[...] -= sum;
+//   MMA_ADD: C[...] += sum; MMA_NEG: C[...] = -sum;
 //   col = ccol ? ccol[c0+j] : c0+j; LOWER: only r0+i >= c0+j is written.
 // Staged layouts keep both the stores (contiguous global runs) and the
 // fragment reads free of bank conflicts: the operand whose global run is along
 // the tile edge is stored k-major with row stride 68, the other edge-major with
 // stride 36 (both = 4 mod 16 doubles).
 constexpr int kStageOp = 2304;   // doubles of one staged operand chunk (max of 32 x 68 and 64 x 36)
-enum { MMA_SET = 0, MMA_SUB = 1 };
+enum { MMA_SET = 0, MMA_SUB = 1, MMA_ADD = 2, MMA_NEG = 3 };
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -199,7 +200,7 @@ __device__ void tile_mma(double* __restrict__ C, int64_t ldc, int crow, const in
                 const int i = wr + 8 * a + g, j = wc + 8 * b + 2 * t4 + h;
                 const bool ok = i < mr && j < nc && !(LOWER && r0 + i < c0 + j);
                 cv[a][b][h] = 0.0;
-                if (MODE == MMA_SUB && ok) {
+                if ((MODE == MMA_SUB || MODE == MMA_ADD) && ok) {
                     const int64_t col = ccol ? ccol[c0 + j] : (c0 + j);
                     cv[a][b][h] = C[(int64_t)(crow + r0 + i) + col * ldc];
                 }
@@ -215,7 +216,10 @@ __device__ void tile_mma(double* __restrict__ C, int64_t ldc, int crow, const in
                 if (ok) {
                     const int64_t col = ccol ? ccol[c0 + j] : (c0 + j);
                     C[(int64_t)(crow + r0 + i) + col * ldc] =
-                        (MODE == MMA_SUB) ? cv[a][b][h] - acc[a][b][h] : acc[a][b][h];
+                        MODE == MMA_SUB   ? cv[a][b][h] - acc[a][b][h]
+                        : MODE == MMA_ADD ? cv[a][b][h] + acc[a][b][h]
+                        : MODE == MMA_NEG ? -acc[a][b][h]
+                                          : acc[a][b][h];
                 }
             }
     __syncthreads();
@@ -1052,6 +1056,86 @@ __global__ void __launch_bounds__(kT, 1) k_trd_cluster(const EigProb* __restrict
     stage_trd_cluster<4>(p, Ca, Da, Ea, Ta, Xa + p.xoff, reinterpret_cast<double*>(smraw), cap);
 }
 
+// ---- inverse of a lower triangle, in place (the strict upper triangle is not read)
+
+// Inverse of one TS x TS diagonal block (mr rows of it are L's), by elimination on the
+// identity as in diag_factor: into its place and, with zeros above the diagonal, into Inv.
+__global__ void __launch_bounds__(kT, 1) k_tri_diag(int64_t n, int64_t ld, double* __restrict__ A,
+                                                    double* __restrict__ Ia) {
+    constexpr int NG = kT / TS, NQ = TS / NG;
+    __shared__ double sL[TS * (TS + 1)], rowb[2][TS];
+    const int i = threadIdx.x % TS, g = threadIdx.x / TS;
+    const int64_t i0 = (int64_t)blockIdx.x * TS;
+    const int mr = (int)min((int64_t)TS, n - i0);
+    double* L = A + i0 + i0 * ld;
+    double* Inv = Ia + (int64_t)blockIdx.x * TS * TS;
+    double e[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int c = g + NG * q;
+        sL[i + c * (TS + 1)] = (i < mr && c <= i) ? L[i + c * ld] : (i == c ? 1.0 : 0.0);
+        e[q] = i == c ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    const double dinv = 1.0 / sL[i + i * (TS + 1)];
+    for (int k = 0; k < TS; ++k) {
+        double* rb = rowb[k & 1];
+        if (i == k) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                e[q] *= dinv;
+                rb[g + NG * q] = e[q];
+            }
+        }
+        __syncthreads();
+        const double f = i > k ? sL[i + k * (TS + 1)] : 0.0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) e[q] = fma(-f, rb[g + NG * q], e[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int c = g + NG * q;
+        const bool in = i < mr && c <= i;
+        if (in) L[i + c * ld] = e[q];
+        Inv[i + c * TS] = in ? e[q] : 0.0;
+    }
+}
+
+// One level: the off-diagonal blocks [r0, r0 + h) x [r0 - h, r0) (r0 = h, 3h, 5h, ...)
+// between inverted diagonal blocks.  FIRST: W = -L21 L11^-1 (h x h per block in Wa);
+// then L21 <- L22^-1 W.  One 64 x 64 tile per CTA, the zero K blocks of the triangles
+// skipped; the diagonal tiles come from Ia, whose upper triangles are zero.
+template <bool FIRST>
+__global__ void __launch_bounds__(kT, 2) k_tri_level(int64_t n, int64_t ld, int h, double* __restrict__ A,
+                                                     const double* __restrict__ Ia, double* __restrict__ Wa) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double *sA = reinterpret_cast<double*>(smraw), *sB = sA + kStageOp;
+    // the longest K ranges first
+    const int rt = FIRST ? blockIdx.y : gridDim.y - 1 - blockIdx.y, ct = blockIdx.x;
+    const int64_t c1 = (int64_t)2 * h * blockIdx.z, r1 = c1 + h;   // of the block's columns and rows
+    const int nr = (int)min((int64_t)h, n - r1);
+    if (rt * TS >= nr) return;
+    const int r0 = rt * TS, c0 = ct * TS, mr = min(TS, nr - r0);
+    double* W = Wa + (int64_t)blockIdx.z * h * h;
+    double* L21 = A + r1 + c1 * ld;
+    if (FIRST) {
+        const double* L11 = A + c1 + c1 * ld;
+        tile_mma<false, false, MMA_NEG, false>(W + (int64_t)c0 * h, h, 0, nullptr, r0, 0, mr, TS, L21 + c0 * ld, ld,
+                                               nullptr, Ia + (c1 / TS + ct) * TS * TS, TS, nullptr, TS, sA, sB);
+        const int k1 = c0 + TS;
+        if (k1 < h)
+            tile_mma<false, false, MMA_SUB, false>(W, h, 0, nullptr, r0, c0, mr, TS, L21 + k1 * ld, ld, nullptr,
+                                                   L11 + k1, ld, nullptr, h - k1, sA, sB);
+    } else {
+        tile_mma<false, false, MMA_SET, false>(L21 + c0 * ld, ld, r0, nullptr, 0, 0, mr, TS,
+                                               Ia + (r1 / TS + rt) * TS * TS, TS, nullptr, W + r0 + (int64_t)c0 * h, h,
+                                               nullptr, mr, sA, sB);
+        if (r0 > 0)
+            tile_mma<false, false, MMA_ADD, false>(L21, ld, 0, nullptr, r0, c0, mr, TS, A + r1 + r1 * ld, ld, nullptr, W,
+                                                   h, nullptr, r0, sA, sB);
+    }
+}
+
 }  // namespace
 
 // Streams and events of a context's eigensolver calls: launches of one stage with
@@ -1135,6 +1219,8 @@ void smem_attr(K kern, size_t bytes) {
 void eig_setup_attrs() {
     static const bool done = [] {
         smem_attr(k_chol_column, kTileSmem);
+        smem_attr(k_tri_level<true>, kTileSmem);
+        smem_attr(k_tri_level<false>, kTileSmem);
         smem_attr(k_chol_scale, kTileSmem);
         smem_attr(k_eig_rsolve, kTileSmem);
         smem_attr(k_eig_trsm, kTileSmem);
@@ -1702,6 +1788,33 @@ __global__ void k_sym_from_upper(int64_t n, const double* __restrict__ a, double
 constexpr int kGridRows = 64;   // rows per CTA of a cooperative-grid solve
 constexpr int kGridMax = 64;    // CTAs of a cooperative-grid solve at most
 constexpr int kGridMin = 4096;  // orders solved by one cluster instead
+
+// By doubling: the 64 x 64 diagonal blocks, then per level every pair of neighbouring
+// inverted blocks, [L11 0; L21 L22]^-1 = [L11^-1 0; -L22^-1 L21 L11^-1  L22^-1], two launches
+// over all tiles of all pairs.  At order 1495 0.25 ms, bound by the chain of levels, against
+// 1.9 for library calls over recursive halves, which followed one another; the four blocks
+// of 2944 of order 11776 3.2 ms against 19.
+void tri_inverse(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A) {
+    if (n <= 0) return;
+    eig_setup_attrs();
+    cudaStream_t s = c->stream;
+    const int64_t nb = (n + TS - 1) / TS;
+    int64_t wsz = 1;
+    for (int64_t h = TS; h < n; h *= 2) wsz = std::max(wsz, (n - h + 2 * h - 1) / (2 * h) * h * h);
+    WorkBuf inv, w;
+    inv.reserve(c, sizeof(double) * nb * TS * TS);
+    w.reserve(c, sizeof(double) * wsz);
+    k_tri_diag<<<(unsigned)nb, kT, 0, s>>>(n, ld, A, inv.as<double>());
+    count_launch();
+    for (int64_t h = TS; h < n; h *= 2) {
+        const dim3 grid((unsigned)(h / TS), (unsigned)((std::min(h, n - h) + TS - 1) / TS),
+                        (unsigned)((n - h + 2 * h - 1) / (2 * h)));
+        k_tri_level<true><<<grid, kT, kTileSmem, s>>>(n, ld, (int)h, A, inv.as<double>(), w.as<double>());
+        k_tri_level<false><<<grid, kT, kTileSmem, s>>>(n, ld, (int)h, A, inv.as<double>(), w.as<double>());
+        count_launch(2);
+    }
+    PTB_CUDA(cudaGetLastError());
+}
 
 void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double* w, double* U) {
     PTB_CHECK(n >= 1 && n <= kLargeMax, PTBGPU_EINVAL, "eigenproblem of order %lld outside the eigensolver (1..%d)",

@@ -63,6 +63,10 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
 // triangles read): A (and B) n x n, ld n; A is overwritten by the eigenvectors.
 void eig_full_upper(ptbgpu_ctx* c, int64_t n, double* A, double* B, double* w);
 
+// In-place inverse of the lower triangle of A (n x n, column-major, leading dimension
+// ld; the strict upper triangle is not referenced).
+void tri_inverse(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A);
+
 // The density step of many independent systems as one batch of the
 // eigensolver (ptbgpu_eig_density_batch): Hpk / Spk / Ppk host packed arrays
 // per system, P_k = 2 sum_{i < nel_k/2} u_i u_i^T of H_k U = S_k U e after the

@@ -40,6 +40,7 @@
 
 #include "common.cuh"
 #include "oz_gemm.cuh"
+#include "sm_eig.cuh"
 #include "sp2_state.cuh"
 #include "tc_gemm.cuh"
 
@@ -388,11 +389,11 @@ Prologue orthogonalise(ptbgpu_ctx* c, int64_t n, const double* dHpk, const doubl
 // halves are equal and at least 2048, the two products of the off-diagonal
 // block run on the int8 tensor cores (S slices, triangular operands masked and
 // their zero K blocks skipped, written in place); smaller or uneven blocks go
-// to the FP64 routine (cuBLAS trmm, cuSOLVER trtri leaves).
+// to the FP64 tensor cores (tri_inverse).
 void trtri_oz(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, int S) {
     const int64_t n1 = (n / 2 + 127) / 128 * 128, n2 = n - n1;
     if (n < 4096 || n1 != n2 || !oz::supported(n1, S)) {
-        dtrtri_lower(c, n, ld, A);
+        tri_inverse(c, n, ld, A);
         return;
     }
     double* L11 = A;
@@ -417,7 +418,7 @@ void trtri_oz(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, int S) {
     oz_product(c, oz::OZ_OUT, opA, opB, false, oz::TRI_LOWER, oz::TRI_NONE, ep);
 }
 
-// The same on the int8 tensor cores: L^-1 by cuSOLVER trtri (in place in B_S,
+// The same on the int8 tensor cores: L^-1 by trtri_oz (in place in B_S,
 // lower triangle), T = L^-1 H (lower-triangular A operand: K blocks past the
 // diagonal are skipped), A = T L^-T (symmetric: upper tiles, mirrored).
 Prologue orthogonalise_oz(ptbgpu_ctx* c, int64_t n, const double* dHpk, const double* dSpk, double filter, int S) {
