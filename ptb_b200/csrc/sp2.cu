@@ -356,7 +356,7 @@ struct Prologue {
     double emin, emax;
 };
 
-// H (packed) -> A = L^-1 H L^-T in B_H; S (packed) -> L in B_S.  Both column-major, ld = n.
+// H (packed) -> A = L^-1 H L^-T in B_H; S (packed) -> L^-1 in B_S.  Both column-major, ld = n.
 Prologue orthogonalise(ptbgpu_ctx* c, int64_t n, const double* dHpk, const double* dSpk, double filter) {
     DevBuf& bh = c->buf(B_H);
     DevBuf& bs = c->buf(B_S);
@@ -370,13 +370,12 @@ Prologue orthogonalise(ptbgpu_ctx* c, int64_t n, const double* dHpk, const doubl
     const int info = dpotrf_lower(c, n, n, S);
     PTB_CHECK(info == 0, PTBGPU_ENOTSPD, "overlap matrix not positive definite (potrf info=%d)", info);
     phase("potrf");
-    const double one = 1.0;
-    PTB_CUBLAS(cublasDtrsm(c->blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT,
-                           (int)n, (int)n, &one, S, (int)n, H, (int)n));
-    PTB_CUBLAS(cublasDtrsm(c->blas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT,
-                           (int)n, (int)n, &one, S, (int)n, H, (int)n));
-    symmetrize_upper(c->stream, n, n, H);
-    phase("2 trsm (A = L^-1 H L^-T)");
+    tri_inverse(c, n, n, S);
+    phase("L^-1");
+    DevBuf& bt = c->buf(B_W0);   // the iteration's scratch
+    bt.reserve(sizeof(double) * n * n);
+    tri_congruence(c, n, S, H, bt.as<double>());
+    phase("A = L^-1 H L^-T");
     Prologue p;
     gershgorin_bounds(c, n, n, H, &p.emin, &p.emax);
     PTB_CHECK(std::isfinite(p.emin) && std::isfinite(p.emax) && p.emax > p.emin, PTBGPU_ENAN,
@@ -497,13 +496,9 @@ void back_transform_oz(ptbgpu_ctx* c, int64_t n, double* X, double* W, double* d
 }
 
 // P = 2 L^-T X L^-1 (X in place, column-major n x n), then packed into dPpk.
-void back_transform(ptbgpu_ctx* c, int64_t n, double* X, double* dPpk) {
-    const double* L = c->buf(B_S).as<double>();
-    const double two = 2.0, one = 1.0;
-    PTB_CUBLAS(cublasDtrsm(c->blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT,
-                           (int)n, (int)n, &two, L, (int)n, X, (int)n));
-    PTB_CUBLAS(cublasDtrsm(c->blas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT,
-                           (int)n, (int)n, &one, L, (int)n, X, (int)n));
+void back_transform(ptbgpu_ctx* c, int64_t n, double* X, double* T, double* dPpk) {
+    tri_back(c, n, c->buf(B_S).as<double>(), X, T);
+    axpby_diag(c->stream, n, n, 0.0, nullptr, 2.0, X, 0.0);
     pack_cols(c->stream, n, n, X, dPpk);
 }
 
@@ -528,7 +523,7 @@ StepInfo fp64_step(ptbgpu_ctx* c, int64_t n, double N, double*& X, double*& W) {
 }
 
 // FP64 trace-correcting purification of A (B_H, overwritten); the back-transform
-// uses L from the cuBLAS prologue (S == 0) or L^-1 from the int8 one (S slices).
+// uses L^-1 from the prologue, with FP64 products (S == 0) or int8 ones (S slices).
 void sp2_fp64(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int maxit, int S, double* dPpk,
               ptbgpu_stats* st, int prl) {
     double* X = c->buf(B_H).as<double>();
@@ -554,7 +549,7 @@ void sp2_fp64(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int ma
     PTB_CHECK(done, PTBGPU_EITER, "trace-correcting purification did not converge in %d iterations", maxit);
     phase("SP2 iterations (FP64 syrk)");
     if (S > 0) back_transform_oz(c, n, X, W, dPpk, S);
-    else back_transform(c, n, X, dPpk);
+    else back_transform(c, n, X, W, dPpk);
     phase("back-transform and pack");
     if (st) {
         st->iterations = it;
@@ -984,7 +979,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
         phase(S > 0 ? "cleanup (int8 FP64 squares)" : "cleanup (FP64 syrk)");
     }
     if (S > 0) back_transform_oz(c, n, X, W, dPpk, S);   // sets tr(PS) directly: full slice count
-    else back_transform(c, n, X, dPpk);
+    else back_transform(c, n, X, W, dPpk);
     phase("back-transform and pack");
     if (st) {
         st->iterations = K + nclean;
