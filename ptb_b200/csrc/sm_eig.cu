@@ -1162,18 +1162,21 @@ struct EigStreams {
     static constexpr int kPerBatch = 6;            // a batch's side streams at most
     static constexpr int kSide = 2 * kPerBatch;    // of a batch on the call's stream, and of one on base
     cudaStream_t side[kSide] = {}, base = nullptr;
-    cudaEvent_t fork[2] = {}, join[kSide] = {}, start = nullptr, done = nullptr;
+    cudaEvent_t fork[2] = {}, join[kSide] = {}, start = nullptr, done[kEigSlots] = {};
     EigStreams() {
         for (cudaStream_t& s : side) PTB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         PTB_CUDA(cudaStreamCreateWithFlags(&base, cudaStreamNonBlocking));
         for (cudaEvent_t& e : join) PTB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        for (cudaEvent_t* e : {&fork[0], &fork[1], &start, &done})
+        for (cudaEvent_t* e : {&fork[0], &fork[1], &start})
             PTB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        for (cudaEvent_t& e : done) PTB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     ~EigStreams() {
         for (cudaEvent_t e : join)
             if (e) cudaEventDestroy(e);
-        for (cudaEvent_t e : {fork[0], fork[1], start, done})
+        for (cudaEvent_t e : {fork[0], fork[1], start})
+            if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : done)
             if (e) cudaEventDestroy(e);
         for (cudaStream_t s : side)
             if (s) cudaStreamDestroy(s);
@@ -1216,6 +1219,7 @@ struct EigBatch {
     const char* what = "submatrix";   // the problems' name in error messages
     std::shared_ptr<EigStreams> st;
     bool async = false;           // launched on st->base
+    int slot = 0;                 // whose done event it records there
     ~EigBatch() {
         // the arrays go back to the context's pool: nothing on the side streams may
         // still use them (work on the context's stream is ordered before their next use)
@@ -1722,7 +1726,7 @@ void eig_run(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, const double* H, const
 std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const double* H, const double* S,
                                            const std::vector<EigProbHost>& probs, const int* d_maps,
                                            const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe,
-                                           int prl, double* flops, bool join) {
+                                           int prl, double* flops, int slot) {
     if (probs.empty()) return nullptr;
     auto eb = std::make_shared<EigBatch>();
     eb->prl = prl;
@@ -1744,26 +1748,30 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
         if (flops) *flops += 7.0 * std::pow((double)q.m, 3);
     }
     cudaStream_t s = c->stream;
-    if (!join) {
-        // beside what follows on the context's stream
-        EigStreams& es = eig_streams(c, *eb);
-        PTB_CUDA(cudaEventRecord(es.start, s));
-        PTB_CUDA(cudaStreamWaitEvent(es.base, es.start, 0));
-        s = es.base;
-        eb->async = true;
-    }
+    // the uploads of the plan on the context's stream: on base they would wait for the
+    // batches before this one, and the host with them
     eig_plan(c, *eb, s, kEigBatchMax, nullptr);
     log_line(prl, 2, " * eigensolver: %d problems, %d above order %d, %zu merge levels", eb->nprob, eb->nlarge,
              kEigBatchMax, eb->levels.size());
     for (const EigBatch::Trd& t : eb->trd)
         log_line(prl, 2, " *   tridiagonalisation of %d on %d CTAs of %d threads each", t.n, t.G ? t.G : eb->G, t.nt);
+    if (slot >= 0) {
+        // beside what follows on the context's stream
+        PTB_CHECK(slot < kEigSlots, PTBGPU_EINVAL, "eigensolver: no such batch slot");
+        EigStreams& es = eig_streams(c, *eb);
+        PTB_CUDA(cudaEventRecord(es.start, s));
+        PTB_CUDA(cudaStreamWaitEvent(es.base, es.start, 0));
+        s = es.base;
+        eb->async = true;
+        eb->slot = slot;
+    }
     eig_run(c, *eb, s, H, S, d_maps, d_own_cols, d_ipos, d_e, d_fe);
-    if (eb->async) PTB_CUDA(cudaEventRecord(eb->st->done, s));
+    if (eb->async) PTB_CUDA(cudaEventRecord(eb->st->done[slot], s));
     return eb;
 }
 
 void eig_batch_join(ptbgpu_ctx* c, EigBatch& eb) {
-    if (eb.async) PTB_CUDA(cudaStreamWaitEvent(c->stream, eb.st->done, 0));
+    if (eb.async) PTB_CUDA(cudaStreamWaitEvent(c->stream, eb.st->done[eb.slot], 0));
 }
 
 void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb) {
@@ -1946,10 +1954,14 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
                        int prl, ptbgpu_stats* st) {
     if (ninst <= 0) return;
     cudaStream_t s = c->stream;
-    // The systems above kEigBatchMax are copied in and launched on their
-    // clusters first; the small ones are copied in while those run, then solved
-    // by the persistent launch beside them, and their results copied out while
-    // the clusters finish.
+    // The systems above kEigBatchMax go first, in up to kEigSlots parts of the input
+    // order, each a batch on a stream of its own: a part is copied in while the one
+    // before it is solved, and copied out while the next is.  The small systems are
+    // copied in after them and solved and copied out beside them.  Parts smaller than
+    // kPartMin systems leave a wave of clusters short (64 systems in four parts 590 ms, in
+    // two 550, in one 659), but two parts pay from kPartMin on: 32 systems 368 -> 336 ms,
+    // 100 862 -> 782, 256 1.79 -> 1.65 s (pageable host arrays, copies inside).
+    constexpr size_t kPartMin = 24;
     std::vector<int64_t> large, small;
     std::vector<int64_t> pkoff((size_t)ninst + 1, 0);
     int64_t hsz = 0, nsum = 0;
@@ -2003,13 +2015,13 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
             unpack_sym(s, m, m, pkS + pkoff[k], b.sm.as<double>() + pr[k].gbase, filter);
         }
     };
-    auto launch = [&](const std::vector<int64_t>& ids, bool join) {
+    auto launch = [&](const std::vector<int64_t>& ids, int slot) {
         std::vector<EigProbHost> probs;
         for (int64_t k : ids) probs.push_back(pr[k]);
         double flops = 0.0;
         auto eb = eig_batch_launch(c, 0, b.h.as<double>(), b.sm.as<double>(), probs, b.maps.as<int>(),
                                    b.dummy.as<int>(), b.dummy.as<int>(), b.e.as<double>(), b.e.as<double>(), prl,
-                                   &flops, join);
+                                   &flops, slot);
         eb->what = "system";
         return eb;
     };
@@ -2023,19 +2035,36 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
             PTB_CUDA(cudaMemcpyAsync(Ppk[k], pkH + pkoff[k], sizeof(double) * np, cudaMemcpyDeviceToHost, s));
         }
     };
-    std::shared_ptr<EigBatch> ebl, ebs;   // declared after b: released (side stream drained) before its buffers
-    upload(large);
-    if (!large.empty()) ebl = launch(large, false);
+    // parts of about equal work (m^3, which the copies follow at a distance)
+    const size_t nparts =
+        large.size() < kPartMin ? 1 : std::min<size_t>(kEigSlots, std::max<size_t>(2, large.size() / kPartMin));
+    std::vector<std::vector<int64_t>> parts;
+    double work = 0.0, done = 0.0;
+    for (int64_t k : large) work += std::pow((double)ndim[k], 3);
+    for (int64_t k : large) {
+        const size_t part = std::min(nparts - 1, (size_t)(done / work * (double)nparts));
+        if (parts.size() <= part) parts.resize(part + 1);
+        parts[part].push_back(k);
+        done += std::pow((double)ndim[k], 3);
+    }
+    // declared after b: released (side streams drained) before its buffers
+    std::vector<std::shared_ptr<EigBatch>> ebl;
+    std::shared_ptr<EigBatch> ebs;
+    for (size_t i = 0; i < parts.size(); ++i) {
+        upload(parts[i]);
+        ebl.push_back(parts[i].empty() ? nullptr : launch(parts[i], (int)i));
+    }
     upload(small);
     if (!small.empty()) {
-        ebs = launch(small, true);
+        ebs = launch(small, -1);
         eig_batch_check(c, *ebs);
         download(*ebs, small);
     }
-    if (ebl) {
-        eig_batch_join(c, *ebl);
-        eig_batch_check(c, *ebl);
-        download(*ebl, large);
+    for (size_t i = 0; i < parts.size(); ++i) {
+        if (!ebl[i]) continue;
+        eig_batch_join(c, *ebl[i]);
+        eig_batch_check(c, *ebl[i]);
+        download(*ebl[i], parts[i]);
     }
     PTB_CUDA(cudaStreamSynchronize(s));
     if (st)

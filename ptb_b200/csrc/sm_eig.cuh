@@ -15,6 +15,8 @@ constexpr int kEigBatchMax = 800;
 // Largest submatrix the library's eigensolver takes at all: the tridiagonalisation of
 // the largest orders keeps two vectors of this length in shared memory.
 constexpr int kEigLargeMax = 12032;
+// Batches that may be on their way beside the context's stream at a time.
+constexpr int kEigSlots = 4;
 
 // One submatrix as the host plan describes it.
 struct EigProbHost {
@@ -41,9 +43,9 @@ struct EigBatch;
 std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const double* H, const double* S,
                                            const std::vector<EigProbHost>& probs, const int* d_maps,
                                            const int* d_own_cols, const int* d_ipos, double* d_e, double* d_fe,
-                                           int prl, double* flops, bool join = true);
-// With join = false the batch runs on a stream of its own, which the context's stream
-// does not wait for; this does it.
+                                           int prl, double* flops, int slot = -1);
+// With a slot (0 .. kEigSlots - 1) the batch runs on a stream beside the context's, after
+// the earlier ones there; the context's stream waits for it here.
 void eig_batch_join(ptbgpu_ctx* c, EigBatch& eb);
 void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb);
 
