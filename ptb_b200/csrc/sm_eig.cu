@@ -483,15 +483,16 @@ __global__ void __launch_bounds__(kT, 2) k_eig_gather(const EigProb* __restrict_
 
 // Factor and inverse of one TS x TS diagonal block (its first mr rows at L, ld m; the
 // rest counts as the identity), by elimination on [A | I]: thread (i, g) holds row i,
-// columns g, g + 8, ... of both in registers, and a step broadcasts column k of A and
-// row k of the right half through shared memory (two buffers, one barrier a step).
+// columns g, g + 8, ... of both in registers, and a step eliminates two columns, which
+// it broadcasts with the two rows of the right half through shared memory (two
+// buffers, one barrier a step).
 // With A = (unit lower) D (unit lower)^T: L = lower sqrt(D), L^-1 = D^-1/2 lower^-1.
-// Bound by the chain of TS steps of a barrier, a division and the
-// updates (48k clocks).  Returns
+// Bound by the chain of TS / 2 steps of a barrier, two divisions and the updates
+// (46k clocks; with one column a step 48k).  Returns
 // the first non-positive pivot's position (1-based; 0: none), the same on every thread.
 __device__ int diag_factor(double* __restrict__ L, int m, int mr, double* __restrict__ Inv) {
     constexpr int NG = kT / TS, NQ = TS / NG;
-    __shared__ double colb[2][TS], rowb[2][TS], piv[TS];
+    __shared__ double colb[2][2][TS], rowb[2][2][TS], piv[TS];
     const int i = threadIdx.x % TS, g = threadIdx.x / TS;
     double a[NQ], e[NQ];
 #pragma unroll
@@ -504,25 +505,39 @@ __device__ int diag_factor(double* __restrict__ L, int m, int mr, double* __rest
 #pragma unroll
     for (int kq = 0; kq < NQ; ++kq) {
 #pragma unroll 1
-        for (int kg = 0; kg < NG; ++kg) {
+        for (int kg = 0; kg < NG; kg += 2) {
             const int k = kq * NG + kg;
-            double* cb = colb[k & 1];
-            double* rb = rowb[k & 1];
-            if (g == kg) cb[i] = a[kq];
-            if (i == k) {
+            double(*cb)[TS] = colb[(kg >> 1) & 1];
+            double(*rb)[TS] = rowb[(kg >> 1) & 1];
+            if (g == kg || g == kg + 1) cb[g - kg][i] = a[kq];
+            if (i == k || i == k + 1) {
 #pragma unroll
-                for (int q = 0; q <= kq; ++q) rb[g + NG * q] = e[q];
+                for (int q = 0; q <= kq; ++q) rb[i - k][g + NG * q] = e[q];
             }
             __syncthreads();
-            const double pk = cb[k];
-            if (!(pk > 0.0) && bad == 0) bad = k + 1;
-            if (threadIdx.x == 0) piv[k] = pk;
-            const double r = 1.0 / pk, f = i > k ? cb[i] * r : 0.0;
+            // the second column after the first one's step: pivot p1, entry y
+            const double p0 = cb[0][k], p10 = cb[0][k + 1], r0 = 1.0 / p0, l = p10 * r0;
+            const double p1 = fma(-l, p10, cb[1][k + 1]), r1 = 1.0 / p1;
+            if (bad == 0) bad = !(p0 > 0.0) ? k + 1 : !(p1 > 0.0) ? k + 2 : 0;
+            if (threadIdx.x == 0) {
+                piv[k] = p0;
+                piv[k + 1] = p1;
+            }
+            const double f0 = i > k ? cb[0][i] * r0 : 0.0;
+            const double y = fma(-f0, p10, cb[1][i]);
+            const double f1 = i > k + 1 ? y * r1 : 0.0, h0 = fma(-f1, l, f0);
 #pragma unroll
-            for (int q = 0; q <= kq; ++q) e[q] = fma(-f, rb[g + NG * q], e[q]);
-            a[kq] = fma(g > kg ? -f : 0.0, cb[g + NG * kq], a[kq]);
+            for (int q = 0; q <= kq; ++q) {
+                const int c = g + NG * q;
+                e[q] = fma(-f1, rb[1][c], fma(-h0, rb[0][c], e[q]));
+            }
+            if (g == kg + 1) a[kq] = y;
+            else if (g > kg + 1) a[kq] = fma(-f1, cb[1][g + NG * kq], fma(-h0, cb[0][g + NG * kq], a[kq]));
 #pragma unroll
-            for (int q = kq + 1; q < NQ; ++q) a[q] = fma(-f, cb[g + NG * q], a[q]);
+            for (int q = kq + 1; q < NQ; ++q) {
+                const int c = g + NG * q;
+                a[q] = fma(-f1, cb[1][c], fma(-h0, cb[0][c], a[q]));
+            }
         }
     }
     __syncthreads();
