@@ -36,7 +36,7 @@ with the chemical-potential search, source/purification.f90) in FP64 on the
 
 --workload lattice256 measures the uneven multi-instance batch instead: 256
 synthetic cubic-lattice systems (20-400 atoms, ndim 166-3064), every system's
-dense projector by the FP64 eigensolver in one launch
+dense projector by the FP64 eigensolver in one batch
 (ptbgpu_eig_density_batch); one step = the whole batch, host buffers in and
 out (value and e2e are the same call).  The trace-correcting purification of
 the same systems (ptbgpu_tc_purify_batch, mixed and FP64, host worker threads)
@@ -432,9 +432,8 @@ def run_sm(args, rank, world, local, pg):
                           + ("" if world == 1 else ", max over ranks")},
         "gpu_launches": int(sum(x.kernel_launches for x in stats)),
         "roofline": {"bound": "fp64", "kernel": "the library's FP64 generalized eigensolver (Cholesky, reduction, "
-                     "tridiagonalisation, divide and conquer, owned rows; DMMA tile products): k_eig_fused, one "
-                     "persistent launch for submatrices of order <= 1024, and k_eig_cluster, one thread-block "
-                     "cluster per larger submatrix, side by side",
+                     "tridiagonalisation, divide and conquer, owned rows; DMMA tile products): each stage launched "
+                     "over all submatrices, k_eig_trd and k_trd_cluster (tridiagonalisation) the longest",
                      "achieved": feig / (ms / 1e3) / 1e12,
                      "peak": 37.0, "unit": "TFLOP/s", "frac": feig / (ms / 1e3) / 1e12 / 37.0, "traffic": None,
                      "peak_kind": "nominal B200 FP64 (no measured FP64 figure on this pool)",
@@ -550,14 +549,14 @@ def run_purify_types(args, rank, world, local, pg):
 
 def run_batch(args, rank, world, local, pg):
     """The multi-instance batch of 256 independent systems.  The timed path is
-    the library's FP64 eigensolver with every system in one launch
-    (ptbgpu_eig_density_batch: one CTA per system up to order 1024, one
-    thread-block cluster per larger system, P formed in the same launch).  On
+    the library's FP64 eigensolver with every system in one batch
+    (ptbgpu_eig_density_batch: every stage launched over all systems, P formed
+    in the same batch).  On
     one GPU the trace-correcting purification of the same systems (mixed
     precision and FP64, host worker streams) and the grouped entry are reported
     beside it.  With N ranks the systems are split size-balanced (decreasing
     ndim^3 to the least-loaded rank, the submatrix shards' rule) and each rank
-    solves its share in one launch: no collective, the batch's time is the
+    solves its share in one batch: no collective, the batch's time is the
     maximum over ranks (strong scaling of the fixed batch)."""
     import torch
 
@@ -636,8 +635,8 @@ def run_batch(args, rank, world, local, pg):
                 "timing": "host wall clock of the whole C call (packed host arrays in and out, copies inside), "
                           "median of the timed calls"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "fp64", "kernel": "k_eig_fused / k_eig_cluster (FP64 generalized eigensolver, DMMA "
-                                                "tile products)",
+        "roofline": {"bound": "fp64", "kernel": "k_trd_cluster and the stages around it (FP64 generalized "
+                                                "eigensolver, DMMA tile products)",
                      "achieved": feig / (ms / 1e3) / 1e12, "peak": 37.0 * world, "unit": "TFLOP/s",
                      "frac": feig / (ms / 1e3) / 1e12 / (37.0 * world), "traffic": None,
                      "peak_kind": "nominal B200 FP64 (no measured FP64 figure on this pool)"

@@ -25,7 +25,9 @@ __global__ void __launch_bounds__(kT, 2) k_vec_panels(const EigProb* __restrict_
 constexpr size_t kChainSmem = sizeof(double) * (2 * kStageOp + TS * TS + TS * kY2ld);
 
 // Rows of L (S U) and of L^-T (U) for the owned columns, times Q: block u of the 2 nown
-// vectors (the rows of L first).
+// vectors (the rows of L first).  A chain of panels per task, so 64 vectors a task rather
+// than a wider tile: the tasks of a batch fill the SMs twice (512-H2O clusters 36 -> 18 ms
+// with the panels and solves of wy_apply and trsm_cols).
 __global__ void __launch_bounds__(kT, 2) k_vec_rows(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ Ca, const double* __restrict__ La,
                                                     const double* __restrict__ Ia, const double* __restrict__ Ka, const int* __restrict__ own_cols,
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(kT, 2) k_fin_cols(const EigProb* __restrict__ 
 }
 
 // ---- eigenvectors U = L^-T Q Z in place of Z, 64 columns per CTA (all of them, or the
-// nocc lowest for a density)
+// nocc lowest for a density): order 1495, 24 CTAs, 6.6 -> 3.6 ms, the chain of K chunks
 __global__ void __launch_bounds__(kT, 2) k_vec_back(const EigProb* __restrict__ probs, const int2* __restrict__ tasks,
                                                     const double* __restrict__ Ca, const double* __restrict__ La,
                                                     const double* __restrict__ Ia, const double* __restrict__ Ka, double* __restrict__ Za,

@@ -1601,9 +1601,9 @@ int resolve_variant(int variant, int S, int rb) {
 
 int variant_for(int64_t ldp, int S) {
     // 128 x 64 tiles on one CTA while they fit one wave: a 256 x 128 pair tile then
-    // leaves more than half of the SMs idle (order 736, 8 slices: 72 CTAs 25 us, 36
-    // CTAs 58 us; order 900: 128 CTAs 33 us, 64 CTAs 66 us).  Above one wave the
-    // pair is faster again (order 1100: 162 CTAs 87 us, 90 CTAs 72 us).
+    // leaves more than half of the SMs idle (one launch between events, 8 slices: order
+    // 736 72 CTAs 49 us, 36 CTAs 84 us; order 900 128 CTAs 57 us, 64 CTAs 90 us).  Above
+    // one wave the pair is faster again (order 1100: 162 CTAs 111 us, 90 CTAs 96 us).
     return (ldp / BM) * (ldp / BN) <= kSms ? V_SMEM_A : resolve_variant(V_DEFAULT, S, 0);
 }
 
