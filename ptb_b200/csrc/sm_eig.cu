@@ -471,9 +471,13 @@ __global__ void __launch_bounds__(kT, 2) k_eig_gather(const EigProb* __restrict_
     double* X = p.kind == 0 ? Xa + p.aoff : Ca + p.coff;
     const int64_t ldx = p.kind == 0 ? m : p.ldc;
     double* L = La + p.aoff;
-    for (int j = t.y * TS; j < min(m, (t.y + 1) * TS); ++j) {
+    // 64 rows x 8 columns at a time: loads of scattered elements, whose latency the eight
+    // columns share (one column at a time 41 us for the 92 rows of 4 H2O)
+    const int tx = threadIdx.x % TS, ty = threadIdx.x / TS;
+    for (int j = t.y * TS + ty; j < min(m, (t.y + 1) * TS); j += kT / TS) {
         const int64_t gj = p.gbase + (int64_t)mp[j] * p.gld;
-        for (int i = threadIdx.x; i < m; i += kT) {
+#pragma unroll 4
+        for (int i = tx; i < m; i += TS) {
             const int64_t q = (int64_t)mp[i] + gj;
             X[i + (int64_t)j * ldx] = H[q];
             if (p.kind == 0) L[i + (int64_t)j * m] = i >= j ? S[q] : 0.0;
@@ -557,7 +561,7 @@ __device__ int diag_factor(double* __restrict__ L, int m, int mr, double* __rest
 // goes on to factor and invert it; then the tiles below are multiplied by the
 // inverse's transpose (k_chol_scale).  Two launches per block column over the whole
 // batch.  One CTA (order <= 800) or cluster per problem, with 32-wide panels and
-// rank-32 updates, took 2.3 ms against 0.8 for 32 H2O and 28 ms against 11.4
+// rank-32 updates, took 2.3 ms against 0.6 for 32 H2O and 28 ms against 10.2
 // for 512-H2O clusters (orders to 2773).
 __global__ void __launch_bounds__(kT, 2) k_chol_column(const EigProb* __restrict__ probs,
                                                        const int2* __restrict__ tasks, int j, double* __restrict__ La,
@@ -1215,7 +1219,7 @@ struct EigBatch {
     };
     int nprob = 0;
     int G = 1;                    // CTAs per cluster of the large problems' Cholesky
-    int nsmall = 0, nlarge = 0, maxlarge = 0;
+    int nsmall = 0, nlarge = 0;
     bool grid = false;            // one problem on a cooperative grid
     std::vector<Trd> trd;
     std::vector<EigProb> hp;
@@ -1419,7 +1423,6 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
     std::stable_sort(large.begin(), large.end(), by_size);
     eb.nsmall = (int)eb.order.size();
     eb.nlarge = (int)large.size();
-    eb.maxlarge = large.empty() ? 0 : eb.hp[large[0]].m;
     if (eb.nlarge > 0 && !eb.grid) eb.G = eig_cluster_size(c, eb.nlarge);
     const int nsm = c->num_sms > 0 ? c->num_sms : 148;
     int64_t asz = 0, csz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0, isz = 0;
