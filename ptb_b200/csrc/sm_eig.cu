@@ -1354,7 +1354,7 @@ std::vector<int> trd_groups(ptbgpu_ctx* c, const std::vector<int>& m, int small_
         // (many large triangles side by side are bound by HBM, not by their SMs: mixed
         // clusters of 2 to 16 took 155 ms on 48 problems up to 2773, 8 for all of them 144)
         if (mm > small_max && G < 8) return false;
-        if (forced > 1 && mm > small_max && G != forced) return false;
+        if (forced > 0 && mm > small_max && G != forced) return false;
         return tc_cap(mm, 4, G, kT) > 0 && eig_active_cached(c, G) > 0;
     };
     std::vector<int> pick(m.size(), 0);
@@ -2009,6 +2009,10 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
         pkoff[k + 1] = pkoff[k] + m * (m + 1) / 2;
         (m > kEigBatchMax ? large : small).push_back(k);
     }
+    struct Drain {   // a failing part leaves no copy into the caller's arrays on its way
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
+    } drain{s};
     struct Bufs {
         WorkBuf h, sm, pk, maps, e, dummy;
     } b;
