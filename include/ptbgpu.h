@@ -200,10 +200,13 @@ int ptbgpu_tc_purify_batch(ptbgpu_ctx* ctx, int64_t ninst, const int64_t* ndim, 
  * H_k U = S_k U e and P_k = 2 sum_{i < nel_k/2} u_i u_i^T (the dense projector
  * at T = 0, i.e. the reference's solve2, source/pgtb.f90:1066-1170, without the
  * Fermi smearing), P_k formed in the same batch; nel_k must be even (closed
- * shell: an odd count is EINVAL).  Systems of orders up to 12032; every stage of the
- * solver is launched over all of them.  opts->filter is applied to H and
- * S (filter_matrix_sym).  Per-system stats carry flops; wall_ms the host time of
- * the call.  ENOTSPD names the first system whose S is not positive definite. */
+ * shell: an odd count is EINVAL).  Systems of orders up to 12032.  Every stage of
+ * the solver is launched over all systems up to order 800, and over all larger ones
+ * or, of 24 and more, over each of up to four parts of them, whose copies run
+ * beside the solves.  opts->filter is applied to H and S (filter_matrix_sym).
+ * Per-system stats carry flops; wall_ms the host time of the call.  ENOTSPD names
+ * the first system whose S is not positive definite; the P_k of parts that had ended
+ * before the failure was seen are written by then. */
 int ptbgpu_eig_density_batch(ptbgpu_ctx* ctx, int64_t ninst, const int64_t* ndim, const int64_t* nel,
                              const double* const* Hpk, const double* const* Spk, double* const* Ppk,
                              const ptbgpu_opts* opts, ptbgpu_stats* st, double* wall_ms);

@@ -1203,6 +1203,16 @@ struct EigStreams {
     }
 };
 
+// A failing problem and its status word (0: none).
+struct EigFault {
+    int k = 0, status = 0;
+    void merge(const EigFault& o) {   // a non-positive pivot goes before a leaf, then the lower problem
+        if (o.status == 0) return;
+        const bool earlier = (o.status > 0) != (status > 0) ? o.status > 0 : o.k < k;
+        if (status == 0 || earlier) *this = o;
+    }
+};
+
 struct EigBatch {
     struct Seg {   // a run of a task list
         size_t off = 0;
@@ -1235,7 +1245,6 @@ struct EigBatch {
     DcArr S{};
     double* Z = nullptr;          // the Z arena (Za, or the caller's array)
     int prl = 0;
-    const char* what = "submatrix";   // the problems' name in error messages
     std::shared_ptr<EigStreams> st;
     bool async = false;           // launched on st->base
     int slot = 0;                 // whose done event it records there
@@ -1792,20 +1801,29 @@ void eig_batch_join(ptbgpu_ctx* c, EigBatch& eb) {
     if (eb.async) PTB_CUDA(cudaStreamWaitEvent(c->stream, eb.st->done[eb.slot], 0));
 }
 
-void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb) {
+// A batch's first failing problem: the lowest one with a non-positive-definite overlap, else
+// the lowest whose leaves did not converge.  Waits for the batch (joined into the
+// context's stream).
+EigFault eig_batch_fault(ptbgpu_ctx* c, EigBatch& eb) {
     cudaStream_t s = c->stream;
     const int np = eb.nprob;
     std::vector<int> hst(np + 3);
     PTB_CUDA(cudaMemcpyAsync(hst.data(), eb.status.ptr, sizeof(int) * (np + 3), cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
     PTB_CHECK(hst[np + 2] == 0, PTBGPU_ETIMEOUT, "eigensolver: a grid barrier gave up waiting");
+    EigFault f;
     for (int q = 0; q < np; ++q)
-        PTB_CHECK(hst[q] <= 0, PTBGPU_ENOTSPD, "overlap of %s %d not positive definite (leading minor %d)", eb.what,
-                  eb.hp[q].k + 1, hst[q]);
-    for (int q = 0; q < np; ++q)
-        PTB_CHECK(hst[q] == kStOk, PTBGPU_EITER, "tridiagonal eigensolver did not converge on %s %d", eb.what,
-                  eb.hp[q].k + 1);
+        if (hst[q] != kStOk) f.merge({eb.hp[q].k, hst[q]});
+    return f;
 }
+
+void eig_fault_raise(const EigFault& f, const char* what) {
+    PTB_CHECK(f.status <= 0, PTBGPU_ENOTSPD, "overlap of %s %d not positive definite (leading minor %d)", what, f.k + 1,
+              f.status);
+    PTB_CHECK(f.status == kStOk, PTBGPU_EITER, "tridiagonal eigensolver did not converge on %s %d", what, f.k + 1);
+}
+
+void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb) { eig_fault_raise(eig_batch_fault(c, eb), "submatrix"); }
 
 void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, int64_t n, const int* d_maps, const int* d_own_cols,
                      double* dP, double* dPdense) {
@@ -2044,7 +2062,6 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
         auto eb = eig_batch_launch(c, 0, b.h.as<double>(), b.sm.as<double>(), probs, b.maps.as<int>(),
                                    b.dummy.as<int>(), b.dummy.as<int>(), b.e.as<double>(), b.e.as<double>(), prl,
                                    &flops, slot);
-        eb->what = "system";
         return eb;
     };
     auto download = [&](EigBatch& eb, const std::vector<int64_t>& ids) {
@@ -2077,17 +2094,19 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
         ebl.push_back(parts[i].empty() ? nullptr : launch(parts[i], (int)i));
     }
     upload(small);
-    if (!small.empty()) {
-        ebs = launch(small, -1);
-        eig_batch_check(c, *ebs);
-        download(*ebs, small);
-    }
-    for (size_t i = 0; i < parts.size(); ++i) {
-        if (!ebl[i]) continue;
-        eig_batch_join(c, *ebl[i]);
-        eig_batch_check(c, *ebl[i]);
-        download(*ebl[i], parts[i]);
-    }
+    if (!small.empty()) ebs = launch(small, -1);
+    // Results are copied out as their batch ends, while the next one is solved; after a
+    // failure the others are waited for only, and the call's first failing system is named.
+    EigFault fault;
+    auto finish = [&](EigBatch& eb, const std::vector<int64_t>& ids) {
+        eig_batch_join(c, eb);
+        fault.merge(eig_batch_fault(c, eb));
+        if (fault.status == kStOk) download(eb, ids);
+    };
+    if (ebs) finish(*ebs, small);
+    for (size_t i = 0; i < parts.size(); ++i)
+        if (ebl[i]) finish(*ebl[i], parts[i]);
+    eig_fault_raise(fault, "system");
     PTB_CUDA(cudaStreamSynchronize(s));
     if (st)
         for (int64_t k = 0; k < ninst; ++k) st[k].flops += 7.0 * std::pow((double)ndim[k], 3);
