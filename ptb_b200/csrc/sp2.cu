@@ -105,7 +105,7 @@ __global__ void k_x0_init(int64_t n, int64_t ldp, const double* __restrict__ A, 
 
 // Reduce the partials of iterate k in a fixed order and decide the next step.
 __global__ void k_decide(SP2State* st, const double* __restrict__ stats, int nparts, double N, double tol_abs,
-                         double e_asym, double e_stag, int maxit) {
+                         double e_asym, int maxit) {
     if (!st->active) return;
     __shared__ double sh[2][256];
     double a = 0.0, b = 0.0;
@@ -124,7 +124,7 @@ __global__ void k_decide(SP2State* st, const double* __restrict__ stats, int npa
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    sp2_decide(st, sh[0][0], sh[1][0], N, tol_abs, e_asym, e_stag, maxit);
+    sp2_decide(st, sh[0][0], sh[1][0], N, tol_abs, e_asym, maxit);
 }
 
 // out(i,j) = alpha (W_ij + W_ji) + beta X_ij over the ldp x ldp FP32 planes
@@ -541,7 +541,7 @@ void sp2_fp64(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int ma
         const double e = std::fabs(s.err);
         hist.push_back(e);
         log_line(prl, 2, " SP2 (fp64) iter %3d  trX %.10f  err %.3e  %s", it, s.trX, s.err, s.sq ? "X^2" : "2X-X^2");
-        if (e < 1e-13 * (double)n || (hist.size() > 2 && e < 1e-2 && e >= hist[hist.size() - 3])) {
+        if (sp2_floor(hist, s.trX, N, (double)n)) {
             done = true;
             break;
         }
@@ -632,14 +632,14 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     const double N = 0.5 * (double)nel;
     // pass 1 runs to its rounding floor: the two-step non-decrease rule ends it
     const double tol_abs = 1e-12 * (double)n;
-    const double e_asym = 0.1, e_stag = 0.01 * (double)n;
+    const double e_asym = 0.1;
     k_x0_init<<<x0_blocks, 256, 0, s>>>(n, ldp, A, pro.emax, scale, xf[0], traj(0, 0), traj(0, 1), traj(0, 2),
                                         stats);
     count_launch();
     PTB_CUDA(cudaGetLastError());
     const int cap = std::min(maxit, slots - 1);
     const int n6 = (int)up3.size(), n3 = (int)up.size();
-    k_decide<<<1, 256, 0, s>>>(state, stats, x0_blocks, N, tol_abs, e_asym, e_stag, cap);
+    k_decide<<<1, 256, 0, s>>>(state, stats, x0_blocks, N, tol_abs, e_asym, cap);
     count_launch();
     PTB_CUDA(cudaGetLastError());
 
@@ -672,7 +672,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
                               : timed_product(c, tc::EPI_SP2, 2, ldp, pl, pl, split3, narrow_up ? tiles_up3 : tiles_up,
                                               narrow_up ? n6 : n3, ep, narrow_up ? tc::kNarrowKernel : 0, pairs_up,
                                               npup);
-        k_decide<<<1, 256, 0, s>>>(state, stats, ntl, N, tol_abs, e_asym, e_stag, cap);
+        k_decide<<<1, 256, 0, s>>>(state, stats, ntl, N, tol_abs, e_asym, cap);
         count_launch();
         PTB_CUDA(cudaGetLastError());
         ++launched;
@@ -690,8 +690,12 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     const SP2State& H = hstate[0];
     phase("pass 1 (tcgen05 bf16 SP2)");
     PTB_CHECK(tmo == 0, PTBGPU_ETIMEOUT, "tensor-core product gave up waiting (site %d)", tmo);
-    PTB_CHECK(H.status == 0, H.status, "pass-1 purification failed (status %d at iterate %d)", H.status, H.next);
-    PTB_CHECK(H.converged, PTBGPU_EITER, "pass-1 purification did not converge in %d iterations", cap);
+    PTB_CHECK(H.status == 0 || H.status == PTBGPU_EITER, H.status, "pass-1 purification failed (status %d at iterate %d)",
+              H.status, H.next);
+    if (!H.converged) {
+        log_line(prl, 1, " pass 1 did not settle in %d iterations: FP64 purification", cap);
+        return false;
+    }
     const int K = H.next;   // index of the final pass-1 iterate
     // steps launched after the decision that ended pass 1 did nothing: drop their timings
     if (timed0 + (size_t)K < c->timed.size()) c->timed.resize(timed0 + (size_t)K);
@@ -715,10 +719,13 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     count_launch();
     PTB_CUDA(cudaGetLastError());
     // SP2 steps in FP64 precision until the idempotency error reaches FP64
-    // rounding or stops falling over two steps (at most 8); returns the steps
-    auto cleanup = [&]() -> int {
+    // rounding or stops falling over two steps (at most 8, counted in nclean); whether
+    // X is a projector onto N states then
+    int nclean = 0;
+    auto cleanup = [&]() -> bool {
         std::vector<double> hist;
-        int nclean = 0;
+        bool settled = false;
+        int steps = 0;
         if (S > 0) {
             // int8-sliced squares, X updated in place (the epilogue reads X(r,c), c >= r,
             // before writing it; the mirrored lower triangle is never read); the error
@@ -735,8 +742,11 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
                 const double err = trX - trX2, e = std::fabs(err);
                 PTB_CHECK(std::isfinite(err), PTBGPU_ENAN, "NaN during purification");
                 hist.push_back(e);
-                log_line(prl, 2, " SP2 (int8 FP64 cleanup) %d  err %.3e", nclean, err);
-                if (e < 1e-13 * (double)n || (hist.size() > 2 && e >= hist[hist.size() - 3]) || nclean >= 8) break;
+                log_line(prl, 2, " SP2 (int8 FP64 cleanup) %d  err %.3e", steps, err);
+                if (sp2_floor(hist, trX, N, (double)n) || steps >= 8) {
+                    settled = sp2_settled(e, trX, N);
+                    break;
+                }
                 const bool sq = std::fabs(trX2 - N) <= std::fabs(2.0 * trX - trX2 - N);
                 // while the iterate is still far from idempotent its square needs no
                 // more than 6 slices (42 bits): the last digits only matter in the
@@ -760,24 +770,27 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
                     trX += hst[2 * t];
                     trX2 += hst[2 * t + 1];
                 }
-                ++nclean;
+                ++steps;
             }
         } else {
-            for (nclean = 1; nclean <= 8; ++nclean) {
+            while (steps < 8) {
                 StepInfo si = fp64_step(c, n, N, X, W);
                 const double e = std::fabs(si.err);
                 hist.push_back(e);
-                log_line(prl, 2, " SP2 (fp64 cleanup) %d  err %.3e", nclean, si.err);
+                ++steps;
+                log_line(prl, 2, " SP2 (fp64 cleanup) %d  err %.3e", steps, si.err);
                 // until the error reaches FP64 rounding or stops falling over two steps: a
                 // single SP2 step squares the deviation on one side of the spectrum but
                 // doubles it on the other, so a small error on entry is not enough
-                if (e < 1e-13 * (double)n || (hist.size() > 2 && e >= hist[hist.size() - 3])) break;
+                settled = sp2_settled(e, si.trX, N);
+                if (sp2_floor(hist, si.trX, N, (double)n)) break;
             }
-            nclean = std::min(nclean, 8);
         }
-        return nclean;
+        nclean += steps;
+        if (!settled) log_line(prl, 1, " cleanup left no projector onto %.0f states: FP64 purification", N);
+        return settled;
     };
-    int nclean = cleanup();
+    if (!cleanup()) return false;
     phase(S > 0 ? "cleanup (int8 FP64 squares)" : "cleanup (FP64 syrk)");
     // algorithmic: every SP2 step is one symmetric square (n^3), pass 1 and cleanup alike
     double flops = (double)K * (double)n * n * n + (double)nclean * (double)n * n * n;
@@ -973,9 +986,12 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
             }
             break;
         }
-        const int more = cleanup();
-        nclean += more;
-        flops += (double)more * (double)n * n * n;
+        const int before = nclean;
+        if (!cleanup()) {
+            if (st) st->refine_rounds = rounds;
+            return false;
+        }
+        flops += (double)(nclean - before) * (double)n * n * n;
         phase(S > 0 ? "cleanup (int8 FP64 squares)" : "cleanup (FP64 syrk)");
     }
     if (S > 0) back_transform_oz(c, n, X, W, dPpk, S);   // sets tr(PS) directly: full slice count

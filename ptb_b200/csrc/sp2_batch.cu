@@ -179,8 +179,7 @@ __global__ void k_x0d(int64_t B, const double* __restrict__ A, const double* __r
 // Block s: reduce its `per` partials in a fixed order and run the decision.
 __global__ void k_decide_g(SP2State* __restrict__ st, const double* __restrict__ stats, int per,
                            const double* __restrict__ N, const double* __restrict__ tol, double e_asym,
-                           const double* __restrict__ e_stag, int maxit, int* __restrict__ active,
-                           int* __restrict__ sq) {
+                           int maxit, int* __restrict__ active, int* __restrict__ sq) {
     const int s = blockIdx.x;
     if (!st[s].active) return;
     double a = 0.0, b = 0.0;
@@ -190,7 +189,7 @@ __global__ void k_decide_g(SP2State* __restrict__ st, const double* __restrict__
     }
     block_sum2(a, b);
     if (threadIdx.x != 0) return;
-    sp2_decide(&st[s], a, b, N[s], tol[s], e_asym, e_stag[s], maxit);
+    sp2_decide(&st[s], a, b, N[s], tol[s], e_asym, maxit);
     active[s] = st[s].active;
     sq[s] = st[s].sq_cur;
 }
@@ -445,7 +444,7 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
         unpack_sym(s, ndim[i], B, dSpk[q], L + q * BB, o->filter);
     }
     // small per-system device arrays in one buffer
-    enum { M_NSYS = 0, M_EMAX, M_SCALE, M_N, M_TOL, M_ESTAG, M_ACTIVE, M_SQ, M_PAR, M_MODE, M_FAC, M_UPD, M_INFO,
+    enum { M_NSYS = 0, M_EMAX, M_SCALE, M_N, M_TOL, M_ACTIVE, M_SQ, M_PAR, M_MODE, M_FAC, M_UPD, M_INFO,
            M_COUNT };
     bM.reserve(64 * (size_t)M_COUNT * (nb + 1) + 16 * (size_t)nb * sizeof(void*));
     auto marr = [&](int k) { return (char*)bM.ptr + (size_t)k * 8 * (nb + 1); };
@@ -454,7 +453,6 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
     double* d_scale = (double*)marr(M_SCALE);
     double* d_N = (double*)marr(M_N);
     double* d_tol = (double*)marr(M_TOL);
-    double* d_estag = (double*)marr(M_ESTAG);
     int* d_active = (int*)marr(M_ACTIVE);
     int* d_sq = (int*)marr(M_SQ);
     int* d_par = (int*)marr(M_PAR);
@@ -528,7 +526,7 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
     std::vector<double> hg(2 * (size_t)nb * ng);
     PTB_CUDA(cudaMemcpyAsync(hg.data(), parts, sizeof(double) * hg.size(), cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
-    std::vector<double> emin(nb), emax(nb), scale(nb), Nv(nb), tol(nb), estag(nb);
+    std::vector<double> emin(nb), emax(nb), scale(nb), Nv(nb), tol(nb);
     for (int q = 0; q < nb; ++q) {
         double lo = INFINITY, hi = -INFINITY;
         for (int b = 0; b < ng; ++b) {
@@ -542,13 +540,11 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
         scale[q] = 1.0 / (hi - lo);
         Nv[q] = 0.5 * (double)nel[ch.ids[q]];
         tol[q] = 1e-12 * (double)nsys[q];
-        estag[q] = 0.01 * (double)nsys[q];
     }
     PTB_CUDA(cudaMemcpyAsync(d_emax, emax.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, s));
     PTB_CUDA(cudaMemcpyAsync(d_scale, scale.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, s));
     PTB_CUDA(cudaMemcpyAsync(d_N, Nv.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, s));
     PTB_CUDA(cudaMemcpyAsync(d_tol, tol.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, s));
-    PTB_CUDA(cudaMemcpyAsync(d_estag, estag.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, s));
     k_pad_diag<<<gpad, kThr, 0, s>>>(B, d_nsys, A, d_emax, 0.0);
     count_launch();
     PTB_CUDA(cudaGetLastError());
@@ -561,9 +557,9 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
     std::vector<int> rounds(nb, 0), nclean(nb, 0);
 
     // FP64 cleanup / FP64 purification on X: SP2 steps with per-system stop rules.
-    // fp64_path: the whole purification (stop e < 1e-13 n, or e < 1e-2 not falling over two
-    // steps, up to maxit); otherwise the cleanup rule (e < 1e-13 n, not falling over two steps,
-    // at most 8 steps).  Only systems with sel[q] take part.
+    // fp64_path: the whole purification (up to maxit steps to the floor); otherwise the
+    // cleanup (at most 8 steps, to a projector).  Only systems with sel[q] take part; one
+    // that does not get there is left to the single-system path (conv[q] = 0).
     auto fp64_steps = [&](const std::vector<int>& sel, bool fp64_path) {
         std::vector<std::vector<double>> hist(nb);
         std::vector<int> done(nb, 0), steps(nb, 0), mode(nb, 0);
@@ -592,11 +588,13 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
                     continue;
                 }
                 hist[q].push_back(e);
-                const auto& h = hist[q];
-                const bool flat = h.size() > 2 && e >= h[h.size() - 3] && (!fp64_path || e < 1e-2);
-                if (e < 1e-13 * (double)nsys[q] || flat || steps[q] >= cap) {
+                const bool floor = sp2_floor(hist[q], trX, Nv[q], (double)nsys[q]);
+                if (floor || steps[q] >= cap) {
                     done[q] = 1;
-                    if (fp64_path && !(e < 1e-13 * (double)nsys[q] || flat)) conv[q] = 0;
+                    if (!(fp64_path ? floor : sp2_settled(e, trX, Nv[q]))) {
+                        conv[q] = 0;
+                        redo[ch.ids[q]] = 1;
+                    }
                     continue;
                 }
                 mode[q] = std::fabs(trX2 - Nv[q]) <= std::fabs(2.0 * trX - trX2 - Nv[q]) ? 1 : 2;
@@ -626,8 +624,6 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
         PTB_CUDA(cudaGetLastError());
         std::fill(conv.begin(), conv.end(), 1);
         fp64_steps(std::vector<int>(nb, 1), true);
-        for (int q = 0; q < nb; ++q)
-            if (!conv[q]) redo[ch.ids[q]] = 1;
     } else {
         // ---- pass 1: stacked tcgen05 SP2 ----
         const int cap = std::min(maxit, slots - 1);
@@ -660,7 +656,7 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
         count_launch();
         PTB_CUDA(cudaGetLastError());
         const double e_asym = 0.1;
-        k_decide_g<<<nb, kThr, 0, s>>>(d_state, parts, nchunk, d_N, d_tol, e_asym, d_estag, cap, d_active, d_sq);
+        k_decide_g<<<nb, kThr, 0, s>>>(d_state, parts, nchunk, d_N, d_tol, e_asym, cap, d_active, d_sq);
         count_launch();
         PTB_CUDA(cudaGetLastError());
         tc::ProdList split3{3, {0, 0, 1}, {0, 1, 0}};
@@ -695,7 +691,7 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
                 per = T1;
             }
             PTB_CUDA(cudaGetLastError());
-            k_decide_g<<<nb, kThr, 0, s>>>(d_state, parts, per, d_N, d_tol, e_asym, d_estag, cap, d_active, d_sq);
+            k_decide_g<<<nb, kThr, 0, s>>>(d_state, parts, per, d_N, d_tol, e_asym, cap, d_active, d_sq);
             count_launch();
             PTB_CUDA(cudaGetLastError());
             if ((k & 3) == 3 || k + 1 == cap) {
@@ -899,6 +895,7 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
             tmark("refinement round");
             if (std::any_of(need.begin(), need.end(), [](int v) { return v != 0; })) {
                 fp64_steps(need, false);
+                for (int q = 0; q < nb; ++q) need[q] = need[q] && conv[q];
                 tmark("cleanup");
             }
         }

@@ -1,0 +1,64 @@
+"""Trace-correcting purification of systems with many states right above a small gap, the
+highest occupied one among them.  On the way X^2 takes all of these down to a few hundredths
+together, with an idempotency error far below one and the trace an electron short; the
+occupied one then doubles its way back.  Every precision and the grouped entry against
+LAPACK's projector, with the tolerances of the mixed step's own tests (1e-6; 1e-9 for
+FP64; the electron count to 1e-8), and an impossible iteration limit refused.
+"""
+import numpy as np
+import pytest
+import scipy.linalg as sl
+
+from oracle import ptb_oracle as O
+from ptb_b200 import PREC_FP64, PREC_MIXED, Options, PtbGpuError, api
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n, near, gap, seed):
+    """n // 4 occupied states, the highest at -gap, `near` empty ones within 8 gaps above."""
+    rng = np.random.default_rng(seed)
+    nocc = n // 4
+    e = np.concatenate([-1.0 - 0.5 * rng.random(nocc - 1), [-gap], 8.0 * gap * rng.random(near),
+                        0.5 + 0.5 * rng.random(n - nocc - near)])
+    Q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    A = rng.standard_normal((n, n))
+    S = A @ A.T / n * 0.5 + 0.5 * np.eye(n)        # condition about 5
+    L = np.linalg.cholesky(S)
+    H = (L @ (Q * e)) @ (L @ Q).T
+    H = 0.5 * (H + H.T)
+    U = sl.eigh(H, S)[1][:, :nocc]
+    return (n, 2 * nocc, O.packsym(H), O.packsym(S)), 2.0 * U @ U.T, S
+
+
+def _check(n, nel, P, ref, S, tol):
+    P = O.blowsym(n, P)
+    assert np.max(np.abs(P - ref)) <= tol
+    assert abs(np.sum(P * S) - nel) <= 1e-8
+
+
+CASES = [(130, 10, 1e-2), (130, 60, 1e-2), (300, 30, 3e-3), (520, 60, 1e-2), (520, 10, 3e-3)]
+
+
+@pytest.mark.parametrize("n,near,gap", CASES)
+@pytest.mark.parametrize("precision,slices,tol", [(PREC_MIXED, 8, 1e-6), (PREC_MIXED, 0, 1e-6), (PREC_FP64, 8, 1e-9)])
+def test_states_close_to_the_gap(ctx, n, near, gap, precision, slices, tol):
+    (n, nel, H, S), ref, Sf = _system(n, near, gap, seed=n + near)
+    P, _ = ctx.tc_purify(n, nel, H, S, Options(filter=0.0, precision=precision, fp64_slices=slices))
+    _check(n, nel, P, ref, Sf, tol)
+
+
+@pytest.mark.parametrize("precision,tol", [(PREC_MIXED, 1e-6), (PREC_FP64, 1e-9)])
+def test_states_close_to_the_gap_grouped(ctx, precision, tol):
+    made = [_system(n, near, gap, seed=n + near) for n, near, gap in CASES]
+    Ps, _, _ = ctx.tc_purify_grouped([m[0] for m in made], Options(filter=0.0, precision=precision))
+    for ((n, nel, _, _), ref, Sf), P in zip(made, Ps):
+        _check(n, nel, P, ref, Sf, tol)
+
+
+@pytest.mark.parametrize("precision", [PREC_MIXED, PREC_FP64])
+def test_too_few_iterations_are_refused(ctx, precision):
+    (n, nel, H, S), _, _ = _system(300, 30, 3e-3, seed=1)
+    with pytest.raises(PtbGpuError) as ei:
+        ctx.tc_purify(n, nel, H, S, Options(filter=0.0, precision=precision, max_iter=40))
+    assert ei.value.code == api.EITER
