@@ -194,6 +194,26 @@ __global__ void k_split2(int64_t count, const float* __restrict__ x, __nv_bfloat
     }
 }
 
+// Per-block partials of ||Y - X||_F^2: X an FP32 plane (ldp), Y FP64 column-major, both
+// symmetric n x n.
+constexpr int kParts = 296;
+__global__ void k_moved(int64_t n, int64_t ldp, const float* __restrict__ x, const double* __restrict__ y,
+                        double* __restrict__ out) {
+    double t = 0.0;
+    for (int64_t j = blockIdx.x; j < n; j += gridDim.x)
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const double d = y[i + j * n] - (double)x[i + j * ldp];
+            t = fma(d, d, t);
+        }
+    __shared__ double sh[8];
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) t += sh[w];
+    out[blockIdx.x] = t;
+}
+
 // y += x over FP32 planes.
 __global__ void k_add_f32(int64_t count, const float* __restrict__ x, float* __restrict__ y) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < count; k += (int64_t)gridDim.x * blockDim.x)
@@ -722,6 +742,15 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     // rounding or stops falling over two steps (at most 8, counted in nclean); whether
     // X is a projector onto N states then
     int nclean = 0;
+    double moved[kParts] = {};   // ||.||_F^2 of the first step, by blocks
+    auto first_step = [&] {
+        DevBuf& bm = c->buf(B_MISC2);
+        bm.reserve(sizeof(double) * 4 * kParts);
+        k_moved<<<kParts, 256, 0, s>>>(n, ldp, xf[K & 1], X, bm.as<double>());
+        count_launch();
+        PTB_CUDA(cudaGetLastError());
+        PTB_CUDA(cudaMemcpyAsync(moved, bm.ptr, sizeof(moved), cudaMemcpyDeviceToHost, s));
+    };
     auto cleanup = [&]() -> bool {
         std::vector<double> hist;
         bool settled = false;
@@ -763,6 +792,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
                 const int nt = oz_product(c, oz::OZ_SYM, opX, opX, true, oz::TRI_NONE, oz::TRI_NONE, es);
                 hst.resize(2 * (size_t)nt);
                 PTB_CUDA(cudaMemcpyAsync(hst.data(), es.stats, sizeof(double) * hst.size(), cudaMemcpyDeviceToHost, s));
+                if (nclean == 0 && steps == 0) first_step();
                 check_timeout(c, "int8 product (cleanup)");
                 trX = 0.0;
                 trX2 = 0.0;
@@ -775,6 +805,7 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
         } else {
             while (steps < 8) {
                 StepInfo si = fp64_step(c, n, N, X, W);
+                if (nclean == 0 && steps == 0) first_step();
                 const double e = std::fabs(si.err);
                 hist.push_back(e);
                 ++steps;
@@ -804,13 +835,18 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
     // factor that grows with the first round's response gain g1 = max|X1| /
     // max|X1_0|.  Measured on water clusters, an alkane chain and cubic-lattice
     // systems (range/gap 25 to 1e4): the next correction stays below kRho1 * g1
-    // of the first one and below max(kRho2 * g1, last ratio) of a later one.
+    // of the first one, or below the share that pass 1 had left unconverged
+    // (kRhoF), and below max(kRho2 * g1, last ratio) of a later one.
     // Another round, after an FP64 cleanup of the corrected X, runs while that
     // predicted error exceeds refine_tol, up to refine_rounds.  If the rounds
     // cannot get there (contraction above 1/2, or the cap reached with the
     // prediction above 10 refine_tol) the caller redoes the purification in FP64.
     int rounds = 0;
     double g1 = 0.0, prev_x1max = 0.0, resid = 0.0, rho = 0.0;
+    PTB_CUDA(cudaStreamSynchronize(s));   // `moved`
+    double frontier = 0.0;
+    for (const double v : moved) frontier += v;
+    frontier = std::sqrt(frontier);
     while (refine) {
         // C = A P~ - P~ A (FP64)
         DevBuf& bw2 = c->buf(B_W2);
@@ -874,7 +910,6 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
         count_launch();
         PTB_CUDA(cudaGetLastError());
         // max |X1_0| (second half of the partials buffer, read with the final ones)
-        constexpr int kParts = 296;
         DevBuf& btau = c->buf(B_MISC2);
         btau.reserve(sizeof(double) * 4 * kParts);
         k_trace_maxabs_f32<<<kParts, 256, 0, s>>>(n, ldp, x1f[0], btau.as<double>() + 2 * kParts);
@@ -968,14 +1003,15 @@ bool sp2_mixed(ptbgpu_ctx* c, int64_t n, int64_t nel, const Prologue& pro, int m
         const double gain = x10max > 0.0 ? x1max / x10max : 0.0;
         if (rounds == 1) {
             g1 = gain;
-            rho = x10max > 0.0 ? std::min(1.0, kRho1 * g1) : 1.0;
+            rho = x10max > 0.0 ? std::min(1.0, std::max(kRho1 * g1, kRhoF * frontier)) : 1.0;
         } else {
             rho = std::min(1.0, std::max(kRho2 * g1, prev_x1max > 0.0 ? x1max / prev_x1max : 1.0));
         }
         prev_x1max = x1max;
         resid = x1max * rho;
-        log_line(prl, 2, " refinement round %d  max|X1| %.3e  max|X1_0| %.3e  gain %.3e  predicted %.3e  tau %.3e",
-                 rounds, x1max, x10max, gain, resid, tau);
+        log_line(prl, 2, " refinement round %d  max|X1| %.3e  max|X1_0| %.3e  gain %.3e  pass 1 left %.3e  predicted %.3e  "
+                 "tau %.3e",
+                 rounds, x1max, x10max, gain, frontier, resid, tau);
         if (!(resid > refine_tol)) break;
         if (rounds >= refine_rounds || std::min(1.0, kRho2 * g1) > 0.5) {
             if (resid > 10.0 * refine_tol) {

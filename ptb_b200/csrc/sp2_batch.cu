@@ -221,6 +221,21 @@ __global__ void k_trfrob(int64_t B, const double* __restrict__ X, double* __rest
     }
 }
 
+// Per-block partials of ||X - x||_F^2 with x as in k_f2d_par: what a step moved.  grid (nchunk, nb).
+__global__ void k_moved_par(int64_t B, const float* __restrict__ x0, const float* __restrict__ x1,
+                            const int* __restrict__ par, const double* __restrict__ X, double* __restrict__ parts) {
+    const int s = blockIdx.y;
+    const int64_t base = (int64_t)s * B * B, nn = B * B;
+    const float* x = par[s] ? x1 : x0;
+    double ss = 0.0, none = 0.0;
+    for (int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; l < nn; l += (int64_t)gridDim.x * blockDim.x) {
+        const double v = X[base + l] - (double)x[base + l];
+        ss += v * v;
+    }
+    block_sum2(ss, none);
+    if (threadIdx.x == 0) parts[(int64_t)s * gridDim.x + blockIdx.x] = ss;
+}
+
 // SP2 update in FP64: mode 1 X = W, 2 X = 2X - W, 0 unchanged.  grid (x, nb).
 __global__ void k_sp2_update(int64_t B, const int* __restrict__ mode, const double* __restrict__ W,
                              double* __restrict__ X) {
@@ -560,7 +575,8 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
     // fp64_path: the whole purification (up to maxit steps to the floor); otherwise the
     // cleanup (at most 8 steps, to a projector).  Only systems with sel[q] take part; one
     // that does not get there is left to the single-system path (conv[q] = 0).
-    auto fp64_steps = [&](const std::vector<int>& sel, bool fp64_path) {
+    // frontier (may be null): the length of every system's first step, from its last pass-1 iterate.
+    auto fp64_steps = [&](const std::vector<int>& sel, bool fp64_path, std::vector<double>* frontier = nullptr) {
         std::vector<std::vector<double>> hist(nb);
         std::vector<int> done(nb, 0), steps(nb, 0), mode(nb, 0);
         std::vector<double> hp(2 * (size_t)nb * nchunk);
@@ -614,6 +630,19 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
             k_sp2_update<<<gE, kThr, 0, s>>>(B, d_mode, W, X);
             count_launch();
             PTB_CUDA(cudaGetLastError());
+            if (frontier && it == 0) {
+                k_moved_par<<<dim3(nchunk, nb), kThr, 0, s>>>(B, xf[0], xf[1], d_par, X, parts);
+                count_launch();
+                PTB_CUDA(cudaGetLastError());
+                std::vector<double> hm((size_t)nb * nchunk);
+                PTB_CUDA(cudaMemcpyAsync(hm.data(), parts, sizeof(double) * hm.size(), cudaMemcpyDeviceToHost, s));
+                PTB_CUDA(cudaStreamSynchronize(s));
+                for (int q = 0; q < nb; ++q) {
+                    double f = 0.0;
+                    for (int b = 0; b < nchunk; ++b) f += hm[(size_t)q * nchunk + b];
+                    (*frontier)[q] = std::sqrt(f);
+                }
+            }
         }
         for (int q = 0; q < nb; ++q) nclean[q] += steps[q];
     };
@@ -722,7 +751,8 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
         k_f2d_par<<<gE, kThr, 0, s>>>(B, xf[0], xf[1], d_par, X);
         count_launch();
         PTB_CUDA(cudaGetLastError());
-        fp64_steps(sel, false);
+        std::vector<double> frontier(nb, 0.0);
+        fp64_steps(sel, false, &frontier);
         tmark("cleanup");
 
         // ---- refinement rounds (stacked) ----
@@ -867,7 +897,7 @@ void run_chunk(ptbgpu_ctx* c, const Chunk& ch, const int64_t* ndim, const int64_
                 double rho;
                 if (rounds[q] == 1) {
                     g1[q] = gain;
-                    rho = x10max > 0.0 ? std::min(1.0, kRho1 * g1[q]) : 1.0;
+                    rho = x10max > 0.0 ? std::min(1.0, std::max(kRho1 * g1[q], kRhoF * frontier[q])) : 1.0;
                 } else {
                     rho = std::min(1.0, std::max(kRho2 * g1[q], prevmax[q] > 0.0 ? x1max / prevmax[q] : 1.0));
                 }

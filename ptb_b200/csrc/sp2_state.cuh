@@ -16,6 +16,14 @@ constexpr int kMaxIt = 255;
 // kRho1 * g of its correction, every later one at most kRho2 * g of its own.
 constexpr double kRho1 = 6.5e-5;
 constexpr double kRho2 = 2.6e-4;
+// What pass 1 had not converged when it ended: the replay gives a state that still is f
+// away from 0 or 1 a share 1 - f of its response.  f <= ||X - X^2||_F of pass 1's last
+// iterate, which is the length of the step that the cleanup takes from it; it can hide
+// below the rounding floor of the trace, to 0.03 (2e-5 to 4e-4 in three of four boxes).
+// The first round left up to 0.9 of this bound of its correction in 1925 water boxes and
+// chains; half of it keeps what is left above 1e-7 to 0.2 % of them and 1.7e-7 (without:
+// 1.9 % and 6.3e-7) and takes a second round in 13 % (6.5 %).
+constexpr double kRhoF = 0.5;
 
 struct SP2State {
     int active;      // 1 while pass 1 runs; product/decision launches are no-ops at 0

@@ -62,3 +62,22 @@ def test_too_few_iterations_are_refused(ctx, precision):
     with pytest.raises(PtbGpuError) as ei:
         ctx.tc_purify(n, nel, H, S, Options(filter=0.0, precision=precision, max_iter=40))
     assert ei.value.code == api.EITER
+
+
+@pytest.mark.parametrize("nmol,seed", [(130, 31), (190, 27)])
+def test_frontier_state_below_the_floor_of_pass_1(ctx, nmol, seed):
+    """Boxes whose pass 1 ends with a frontier state a percent away from 0 or 1, under the
+    rounding noise of the traces: one refinement round leaves more than refine_tol (1e-7, in
+    the orthogonal basis) although its gain predicts half of that.  Against the library's
+    FP64 dense diagonalisation."""
+    from ptb_b200 import synth
+
+    s = synth.water_cluster(nmol, seed=seed)
+    n = s.ndim
+    P, st = ctx.tc_purify(n, s.nel, s.Hvec, s.Svec, Options(filter=1e-5, precision=PREC_MIXED))
+    ref, _, focc, _ = ctx.solve2(1, n, s.nel, 0, s.Hvec, s.Svec, Options(filter=1e-5))
+    assert np.array_equal(np.sort(focc)[::-1][: s.nel // 2], np.full(s.nel // 2, 2.0))
+    L = np.linalg.cholesky(O.blowsym(n, O.filter_matrix_sym(s.Svec, 1e-5)))
+    d = L.T @ O.blowsym(n, P - ref) @ L
+    assert np.max(np.abs(d)) / 2.0 <= 1e-7
+    assert st.refine_rounds >= 2 and st.fp64_fallback == 0
