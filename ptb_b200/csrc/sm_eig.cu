@@ -1117,8 +1117,8 @@ __global__ void __launch_bounds__(kT, 1) k_tri_diag(int64_t n, int64_t ld, doubl
 }
 
 // One level: the off-diagonal blocks [r1, r1 + h) x [r1 - h, r1) (r1 = h, 3h, 5h, ...)
-// between inverted diagonal blocks.  FIRST: W = -L21 L11^-1 (h x h per block in Wa);
-// then L21 <- L22^-1 W.  One 64 x 64 tile per CTA, the zero K blocks of the triangles
+// between inverted diagonal blocks.  FIRST: W = -L21 L11^-1 (nr x h per block in Wa, nr = h
+// but for a short last block); then L21 <- L22^-1 W.  One 64 x 64 tile per CTA, the zero K blocks of the triangles
 // skipped, the longest K ranges first.
 template <bool FIRST>
 __global__ void __launch_bounds__(kT, 2) k_tri_level(int64_t n, int64_t ld, int h, double* __restrict__ A,
@@ -1133,10 +1133,10 @@ __global__ void __launch_bounds__(kT, 2) k_tri_level(int64_t n, int64_t ld, int 
     double* W = Wa + (int64_t)blockIdx.z * h * h;
     double* L21 = A + r1 + c1 * ld;
     if (FIRST)
-        tile_mma<false, false, MMA_NEG, false>(W, h, 0, nullptr, r0, c0, mr, TS, L21 + c0 * ld, ld, nullptr,
+        tile_mma<false, false, MMA_NEG, false>(W, nr, 0, nullptr, r0, c0, mr, TS, L21 + c0 * ld, ld, nullptr,
                                                A + c1 + c0 + c1 * ld, ld, nullptr, h - c0, sA, sB);
     else
-        tile_mma<false, false, MMA_SET, false>(L21, ld, 0, nullptr, r0, c0, mr, TS, A + r1 + r1 * ld, ld, nullptr, W, h,
+        tile_mma<false, false, MMA_SET, false>(L21, ld, 0, nullptr, r0, c0, mr, TS, A + r1 + r1 * ld, ld, nullptr, W, nr,
                                                nullptr, r0 + mr, sA, sB);
 }
 
@@ -1860,22 +1860,20 @@ constexpr int kGridMin = 4096;  // orders solved by one cluster instead
 // over all tiles of all pairs.  At order 1495 0.25 ms, bound by the chain of levels, against
 // 1.9 for library calls over recursive halves, which followed one another; the four blocks
 // of 2944 of order 11776 3.2 ms against 19.
-void tri_inverse(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A) {
+//   W takes h doubles for each of a level's rows below the diagonal blocks, which are at most
+// n - h and at most n / 2: n^2 / 4 in all.
+void tri_inverse(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, double* W) {
     if (n <= 0) return;
     eig_setup_attrs();
     cudaStream_t s = c->stream;
     const int64_t nb = (n + TS - 1) / TS;
-    int64_t wsz = 1;
-    for (int64_t h = TS; h < n; h *= 2) wsz = std::max(wsz, (n - h + 2 * h - 1) / (2 * h) * h * h);
-    WorkBuf w;
-    w.reserve(c, sizeof(double) * wsz);
     k_tri_diag<<<(unsigned)nb, kT, 0, s>>>(n, ld, A);
     count_launch();
     for (int64_t h = TS; h < n; h *= 2) {
         const dim3 grid((unsigned)(h / TS), (unsigned)((std::min(h, n - h) + TS - 1) / TS),
                         (unsigned)((n - h + 2 * h - 1) / (2 * h)));
-        k_tri_level<true><<<grid, kT, kTileSmem, s>>>(n, ld, (int)h, A, w.as<double>());
-        k_tri_level<false><<<grid, kT, kTileSmem, s>>>(n, ld, (int)h, A, w.as<double>());
+        k_tri_level<true><<<grid, kT, kTileSmem, s>>>(n, ld, (int)h, A, W);
+        k_tri_level<false><<<grid, kT, kTileSmem, s>>>(n, ld, (int)h, A, W);
         count_launch(2);
     }
     PTB_CUDA(cudaGetLastError());

@@ -67,8 +67,8 @@ void eig_full_upper(ptbgpu_ctx* c, int64_t n, double* A, double* B, double* w);
 
 // In-place inverse of the lower triangle of A (n x n, column-major, leading dimension
 // ld); of the strict upper triangle only the 64 x 64 diagonal blocks' parts are touched
-// (zeroed).
-void tri_inverse(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A);
+// (zeroed).  W: n^2 / 4 doubles of scratch at most.
+void tri_inverse(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, double* W);
 // With Li from it (ld n) and T as n x n scratch: H <- Li H Li^T (both triangles), and
 // X <- Li^T X Li (X symmetric; the upper triangle of the result).
 void tri_congruence(ptbgpu_ctx* c, int64_t n, const double* Li, double* H, double* T);

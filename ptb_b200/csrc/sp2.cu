@@ -390,10 +390,10 @@ Prologue orthogonalise(ptbgpu_ctx* c, int64_t n, const double* dHpk, const doubl
     const int info = dpotrf_lower(c, n, n, S);
     PTB_CHECK(info == 0, PTBGPU_ENOTSPD, "overlap matrix not positive definite (potrf info=%d)", info);
     phase("potrf");
-    tri_inverse(c, n, n, S);
-    phase("L^-1");
     DevBuf& bt = c->buf(B_W0);   // the iteration's scratch
     bt.reserve(sizeof(double) * n * n);
+    tri_inverse(c, n, n, S, bt.as<double>());
+    phase("L^-1");
     tri_congruence(c, n, S, H, bt.as<double>());
     phase("A = L^-1 H L^-T");
     Prologue p;
@@ -408,18 +408,18 @@ Prologue orthogonalise(ptbgpu_ctx* c, int64_t n, const double* dHpk, const doubl
 // halves are equal and at least 2048, the two products of the off-diagonal
 // block run on the int8 tensor cores (S slices, triangular operands masked and
 // their zero K blocks skipped, written in place); smaller or uneven blocks go
-// to the FP64 tensor cores (tri_inverse).
-void trtri_oz(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, int S) {
+// to the FP64 tensor cores (tri_inverse, with W as its scratch).
+void trtri_oz(ptbgpu_ctx* c, int64_t n, int64_t ld, double* A, double* W, int S) {
     const int64_t n1 = (n / 2 + 127) / 128 * 128, n2 = n - n1;
     if (n < 4096 || n1 != n2 || !oz::supported(n1, S)) {
-        tri_inverse(c, n, ld, A);
+        tri_inverse(c, n, ld, A, W);
         return;
     }
     double* L11 = A;
     double* L21 = A + n1;
     double* L22 = A + n1 + n1 * ld;
-    trtri_oz(c, n1, ld, L11, S);
-    trtri_oz(c, n2, ld, L22, S);
+    trtri_oz(c, n1, ld, L11, W, S);
+    trtri_oz(c, n2, ld, L22, W, S);
     const oz::Operand opA = oz_operand(c, 0, n1, S), opB = oz_operand(c, 1, n1, S);
     oz::OzEpi ep;
     ep.n = n1;
@@ -456,7 +456,7 @@ Prologue orthogonalise_oz(ptbgpu_ctx* c, int64_t n, const double* dHpk, const do
     const int info = dpotrf_lower(c, n, n, L);
     PTB_CHECK(info == 0, PTBGPU_ENOTSPD, "overlap matrix not positive definite (potrf info=%d)", info);
     phase("potrf");
-    trtri_oz(c, n, n, L, S);
+    trtri_oz(c, n, n, L, T, S);
     phase("trtri");
     const oz::Operand opL = oz_operand(c, 0, n, S), op1 = oz_operand(c, 1, n, S);
     oz_slice(c, L, 1, n, n, oz::TRI_LOWER, opL);   // rows of L^-1 (column-major storage)
