@@ -132,6 +132,11 @@ typedef struct {
  * is an unbuilt stub).  One context per device and host thread. */
 int  ptbgpu_init(int device, ptbgpu_ctx** ctx);
 int  ptbgpu_finalize(ptbgpu_ctx* ctx);
+/* Between calls a context keeps working blocks of the eigensolver and the purification
+ * module for the next one (unused ones up to 1/16 of the device's memory).  This gives them,
+ * and those of its worker contexts, back to the device, for an allocation that the
+ * program makes outside the library; plans and results in progress stay valid. */
+int  ptbgpu_trim(ptbgpu_ctx* ctx);
 int  ptbgpu_last_error(const ptbgpu_ctx* ctx, char* buf, size_t len);
 void ptbgpu_default_settings(ptbgpu_pur_settings* s);   /* type-bound defaults, purification_settings.f90:29-86 */
 void ptbgpu_default_opts(ptbgpu_opts* o);

@@ -65,7 +65,7 @@ class _Stats(C.Structure):
                 ("refine_rounds", C.c_int64), ("fp64_fallback", C.c_int64)]
 
 
-EXPORTED = ("ptbgpu_init", "ptbgpu_finalize", "ptbgpu_last_error", "ptbgpu_default_settings",
+EXPORTED = ("ptbgpu_init", "ptbgpu_finalize", "ptbgpu_trim", "ptbgpu_last_error", "ptbgpu_default_settings",
             "ptbgpu_default_opts", "ptbgpu_filter_packed", "ptbgpu_check_density", "ptbgpu_sm_density",
             "ptbgpu_purify", "ptbgpu_tc_purify", "ptbgpu_tc_purify_device", "ptbgpu_tc_purify_batch", "ptbgpu_tc_purify_grouped",
             "ptbgpu_eig_density_batch",
@@ -101,6 +101,7 @@ def load_library():
     i64 = C.c_int64
     lib.ptbgpu_init.argtypes = [C.c_int, P(C.c_void_p)]
     lib.ptbgpu_finalize.argtypes = [C.c_void_p]
+    lib.ptbgpu_trim.argtypes = [C.c_void_p]
     lib.ptbgpu_last_error.argtypes = [C.c_void_p, C.c_char_p, C.c_size_t]
     lib.ptbgpu_default_settings.argtypes = [P(_Settings)]
     lib.ptbgpu_default_settings.restype = None
@@ -272,6 +273,10 @@ class Context:
         if getattr(self, "_h", None):
             self._lib.ptbgpu_finalize(self._h)
             self._h = None
+
+    def trim(self):
+        """Gives the working memory that the context keeps unused between calls back to the device."""
+        self._check(self._lib.ptbgpu_trim(self._h))
 
     def __enter__(self):
         return self

@@ -33,9 +33,14 @@ struct Error {
                         cudaGetErrorString(e_));                                           \
     } while (0)
 
+// (a library that finds no memory gets a second try without the blocks kept between calls)
 #define PTB_CUBLAS(call)                                                                   \
     do {                                                                                   \
         cublasStatus_t s_ = (call);                                                        \
+        if (s_ == CUBLAS_STATUS_ALLOC_FAILED) {                                            \
+            ::ptb::WorkPool::trim_all();                                                   \
+            s_ = (call);                                                                   \
+        }                                                                                  \
         if (s_ != CUBLAS_STATUS_SUCCESS)                                                   \
             ::ptb::fail(PTBGPU_ECUDA, "%s:%d %s: cublas status %d", __FILE__, __LINE__,     \
                         #call, (int)s_);                                                   \
@@ -44,6 +49,10 @@ struct Error {
 #define PTB_CUSOLVER(call)                                                                 \
     do {                                                                                   \
         cusolverStatus_t s_ = (call);                                                      \
+        if (s_ == CUSOLVER_STATUS_ALLOC_FAILED) {                                          \
+            ::ptb::WorkPool::trim_all();                                                   \
+            s_ = (call);                                                                   \
+        }                                                                                  \
         if (s_ != CUSOLVER_STATUS_SUCCESS)                                                 \
             ::ptb::fail(PTBGPU_ECUDA, "%s:%d %s: cusolver status %d", __FILE__, __LINE__,   \
                         #call, (int)s_);                                                   \
@@ -70,8 +79,8 @@ struct DevBuf {
 // Blocks are handed out by best fit; their users run on the context's stream or on
 // side streams ordered after it, so a block given back may be taken again at once.
 // The blocks kept unused are bounded (1/16 of the device's memory per context) and
-// freed by ptbgpu_finalize, by trim(), or when any allocation of the library on any
-// context of the process finds no memory (trim_all()).
+// freed by ptbgpu_finalize, by ptbgpu_trim, or when any allocation of the library, its
+// graphs, cuBLAS or cuSOLVER on any context of the process finds no memory (trim_all()).
 class WorkPool {
 public:
     WorkPool();

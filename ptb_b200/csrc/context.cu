@@ -282,6 +282,13 @@ int ptbgpu_finalize(ptbgpu_ctx* c) {
     return PTBGPU_OK;
 }
 
+int ptbgpu_trim(ptbgpu_ctx* c) {
+    if (!c) return PTBGPU_EINVAL;
+    c->work->trim();
+    for (ptbgpu_ctx* w : c->workers) w->work->trim();
+    return PTBGPU_OK;
+}
+
 int ptbgpu_last_error(const ptbgpu_ctx* c, char* buf, size_t len) {
     if (!c || !buf || len == 0) return PTBGPU_EINVAL;
     strncpy(buf, c->last_error.c_str(), len - 1);

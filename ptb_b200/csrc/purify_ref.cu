@@ -187,7 +187,15 @@ struct Ctx {
             launch_counter() = l0;   // counted per executed iteration after the launch
             gemm_flops = f0;
         }
-        if (ok) ok = cudaGraphInstantiate(&lg.exec, lg.graph, 0) == cudaSuccess;
+        if (ok) {
+            cudaError_t e = cudaGraphInstantiate(&lg.exec, lg.graph, 0);
+            if (e == cudaErrorMemoryAllocation) {   // the blocks kept between calls make room
+                (void)cudaGetLastError();
+                WorkPool::trim_all();
+                e = cudaGraphInstantiate(&lg.exec, lg.graph, 0);
+            }
+            ok = e == cudaSuccess;
+        }
         if (!ok) {
             cudaGetLastError();
             if (lg.exec) cudaGraphExecDestroy(lg.exec);
