@@ -66,12 +66,19 @@ PoolRegistry& pool_registry() {
     return *r;
 }
 
-// Sizes are rounded up to eighths of a power of two, so that calls on systems of
-// about the same size find each other's blocks.
-size_t work_class(size_t nbytes) {
+// Sizes are rounded up by up to 1/16, so that calls on systems of about the same size find
+// each other's blocks; large ones only while more than half of the device is free, beyond
+// which a block has the size asked for (multiples of 256 bytes), as the largest calls
+// need it.
+constexpr size_t kLargeBlock = size_t(64) << 20;
+size_t work_class(size_t nbytes, bool scarce) {
     size_t step = 256;
-    while (step * 16 < nbytes) step *= 2;
+    while (!scarce && step * 32 < nbytes) step *= 2;
     return (nbytes + step - 1) / step * step;
+}
+bool scarce_for(size_t nbytes) {
+    size_t free_b = 0, total_b = 0;
+    return nbytes >= kLargeBlock && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < total_b / 2;
 }
 
 }  // namespace
@@ -108,7 +115,7 @@ void WorkPool::trim_all() {
 }
 
 void* WorkPool::take(size_t nbytes, size_t* got) {
-    const size_t want = work_class(std::max<size_t>(nbytes, 1));
+    const size_t want = work_class(std::max<size_t>(nbytes, 1), true);
     {
         std::lock_guard<std::mutex> lock(im_->mu);
         size_t best = im_->free_blocks.size();
@@ -118,7 +125,9 @@ void* WorkPool::take(size_t nbytes, size_t* got) {
                 (best == im_->free_blocks.size() || b < im_->free_blocks[best].bytes))
                 best = i;
         }
-        if (best < im_->free_blocks.size()) {
+        // a large block for a much smaller array only while memory is plenty
+        if (best < im_->free_blocks.size() &&
+            (im_->free_blocks[best].bytes <= want + want / 16 || !scarce_for(want))) {
             const Impl::Block b = im_->free_blocks[best];
             im_->free_blocks.erase(im_->free_blocks.begin() + best);
             im_->kept -= b.bytes;
@@ -130,18 +139,20 @@ void* WorkPool::take(size_t nbytes, size_t* got) {
             if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) im_->limit = total_b / 16;
         }
     }
+    size_t size = work_class(want, scarce_for(want));
     void* ptr = nullptr;
-    cudaError_t e = cudaMalloc(&ptr, want);
+    cudaError_t e = cudaMalloc(&ptr, size);
     if (e == cudaErrorMemoryAllocation) {
         (void)cudaGetLastError();
         trim_all();
-        e = cudaMalloc(&ptr, want);
+        size = want;
+        e = cudaMalloc(&ptr, size);
     }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        fail(PTBGPU_ENOMEM, "cudaMalloc(%zu) failed: %s", want, cudaGetErrorString(e));
+        fail(PTBGPU_ENOMEM, "cudaMalloc(%zu) failed: %s", size, cudaGetErrorString(e));
     }
-    *got = want;
+    *got = size;
     return ptr;
 }
 

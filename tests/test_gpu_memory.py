@@ -113,6 +113,23 @@ def test_kept_blocks_make_room_for_another_context(medium):
             torch.cuda.empty_cache()
 
 
+def test_a_call_takes_what_its_arrays_need(medium):
+    """419 systems of order 801: nine arrays of 2.15 GB and 0.5 GB of smaller ones, 19.9 GB in
+    all, with 20.6 GB free.  (Just above a power of two: blocks rounded up by an eighth
+    would come to 22.)"""
+    import torch
+
+    with Context(0) as c:
+        _solve(c, medium, 2)
+        c.trim()
+        hold = torch.empty(_free() - int(20.6e9), dtype=torch.uint8, device="cuda")
+        try:
+            _solve(c, medium, 419)
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+
+
 def test_trim_after_purification():
     s = synth.water_cluster(8, seed=5)
     pur = PurificationSettings(type=1, metric_type=1, cycles=100, prlvl=0, nel=s.nel)
