@@ -1237,8 +1237,16 @@ struct EigBatch {
     std::vector<int2> lists;
     std::vector<DcMerge> merges;
     std::vector<Level> levels;
-    bool timed = false;   // stage times wanted (PTBGPU_EIG_STAGES)
+    bool timed = false;   // stage times wanted (print level 2, PTBGPU_EIG_STAGES)
     std::vector<std::pair<const char*, cudaEvent_t>> marks;   // what ended, and when
+    template <class F>
+    void stage_times(F&& f) const {   // of a batch that has ended
+        for (size_t i = 1; i < marks.size(); ++i) {
+            float ms = 0.f;
+            PTB_CUDA(cudaEventElapsedTime(&ms, marks[i - 1].second, marks[i].second));
+            f(marks[i].first, (double)ms);
+        }
+    }
     std::vector<unsigned> deep;   // tasks of `blocks` that block column j of the Cholesky factor launches
     Seg blocks, leaves, panels, rows, rq, back, density, fblocks, frq, fcols;
     WorkBuf probs, order_d, lists_d, merges_d, cnt, dc, Ca, La, Za, Qa, Va, Da, Ea, Ta, Ba, Xa, Ka, Ia, status;
@@ -1757,6 +1765,7 @@ std::shared_ptr<EigBatch> eig_batch_launch(ptbgpu_ctx* c, int64_t n, const doubl
     if (probs.empty()) return nullptr;
     auto eb = std::make_shared<EigBatch>();
     eb->prl = prl;
+    eb->timed = prl >= 2;
     for (const EigProbHost& q : probs) {
         PTB_CHECK(q.m >= 1 && q.m <= kLargeMax, PTBGPU_EINVAL, "submatrix %d of order %d outside the eigensolver (1..%d)",
                   q.k + 1, q.m, kLargeMax);
@@ -1811,6 +1820,10 @@ EigFault eig_batch_fault(ptbgpu_ctx* c, EigBatch& eb) {
     PTB_CUDA(cudaMemcpyAsync(hst.data(), eb.status.ptr, sizeof(int) * (np + 3), cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
     PTB_CHECK(hst[np + 2] == 0, PTBGPU_ETIMEOUT, "eigensolver: a grid barrier gave up waiting");
+    if (eb.timed)
+        eb.stage_times([&](const char* what, double ms) {
+            log_line(eb.prl, 2, " *   eigensolver stage %-20s %10.3f ms", what, ms);
+        });
     EigFault f;
     for (int q = 0; q < np; ++q)
         if (hst[q] != kStOk) f.merge({eb.hp[q].k, hst[q]});
@@ -1938,13 +1951,9 @@ void eig_full(ptbgpu_ctx* c, int64_t n, const double* H, const double* S, double
     int hs[4];
     PTB_CUDA(cudaMemcpyAsync(hs, eb.status.ptr, sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
     PTB_CUDA(cudaStreamSynchronize(s));
-    if (!eb.marks.empty()) {
+    if (eb.timed) {
         fprintf(stderr, "eig_full n=%d:", m);
-        for (size_t i = 1; i < eb.marks.size(); ++i) {
-            float ms = 0.f;
-            PTB_CUDA(cudaEventElapsedTime(&ms, eb.marks[i - 1].second, eb.marks[i].second));
-            fprintf(stderr, " %s %.3f", eb.marks[i].first, ms);
-        }
+        eb.stage_times([](const char* what, double ms) { fprintf(stderr, " %s %.3f", what, ms); });
         fprintf(stderr, " ms\n");
     }
     PTB_CHECK(hs[3] == 0, PTBGPU_ETIMEOUT, "eigensolver: a grid barrier gave up waiting");
