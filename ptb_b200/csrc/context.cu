@@ -53,6 +53,7 @@ struct WorkPool::Impl {
     std::vector<Block> free_blocks;   // in the order they were given back
     size_t kept = 0;
     size_t limit = 0;                 // bytes kept unused at most (set at the first block)
+    bool scarce = false;              // less than half of the device was free at the last large allocation
 };
 
 namespace {
@@ -76,9 +77,9 @@ size_t work_class(size_t nbytes, bool scarce) {
     while (!scarce && step * 32 < nbytes) step *= 2;
     return (nbytes + step - 1) / step * step;
 }
-bool scarce_for(size_t nbytes) {
+bool memory_scarce() {
     size_t free_b = 0, total_b = 0;
-    return nbytes >= kLargeBlock && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < total_b / 2;
+    return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < total_b / 2;
 }
 
 }  // namespace
@@ -125,9 +126,10 @@ void* WorkPool::take(size_t nbytes, size_t* got) {
                 (best == im_->free_blocks.size() || b < im_->free_blocks[best].bytes))
                 best = i;
         }
-        // a large block for a much smaller array only while memory is plenty
+        // a large block for a much smaller array only while memory is plenty (as the last
+        // allocation of a large one found it: asking takes 70 us)
         if (best < im_->free_blocks.size() &&
-            (im_->free_blocks[best].bytes <= want + want / 16 || !scarce_for(want))) {
+            (im_->free_blocks[best].bytes <= want + want / 16 || want < kLargeBlock || !im_->scarce)) {
             const Impl::Block b = im_->free_blocks[best];
             im_->free_blocks.erase(im_->free_blocks.begin() + best);
             im_->kept -= b.bytes;
@@ -139,7 +141,13 @@ void* WorkPool::take(size_t nbytes, size_t* got) {
             if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) im_->limit = total_b / 16;
         }
     }
-    size_t size = work_class(want, scarce_for(want));
+    bool scarce = false;
+    if (want >= kLargeBlock) {
+        scarce = memory_scarce();
+        std::lock_guard<std::mutex> lock(im_->mu);
+        im_->scarce = scarce;
+    }
+    size_t size = work_class(want, scarce);
     void* ptr = nullptr;
     cudaError_t e = cudaMalloc(&ptr, size);
     if (e == cudaErrorMemoryAllocation) {
