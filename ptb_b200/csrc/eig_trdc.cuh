@@ -6,19 +6,18 @@
 //   * Rows are owned in 32-row chunks (chunk index modulo G, relative to the panel's
 //     first row).  V, W and the partial sums of the owned rows live in the owner's
 //     shared memory; nb is the widest of 16, 12, 8, 4 columns that fits.
-//   * A v: the lower triangle in strips of 64 or 128 rows (short strips read less above
-//     the diagonal, tall ones exchange less), cut into units of 64 x 16 or 128 x 8
-//     elements; every warp of the group takes a contiguous run of units (equal up to
-//     one), half a unit's loads in flight while the other half is multiplied.  A lane
-//     holds two rows of every 32 and every other column of a unit (16-byte loads, 256
-//     bytes of two columns per instruction), so row sums add up in its registers
-//     along the strip and column sums over the strip's rows; 5 to 8 exchanges per
-//     unit remain.  Alone, the pass runs at 63 (64 rows) to 76 bytes per clock and SM
-//     out of L2; with the column sums exchanged for every 32 rows at 52 (the
-//     exchanges), with 32 bytes of four columns per 8 lanes at 31 (the L1 lines per
-//     instruction).  Row sums go to a
-//     slot per (warp of the strip, row), column sums to a slot per strip, both in
-//     the owner's shared memory; they are added in a fixed order.
+//   * A v: the lower triangle in strips of 128 rows, cut into units of 128 x 8 elements;
+//     every warp of the group takes a contiguous run of units (equal up to one), the next
+//     32 rows' loads in flight while 32 rows of a unit are multiplied.  A lane holds two
+//     rows of every 32 and every other column of a unit (16-byte loads, 256 bytes of two
+//     columns per instruction), so row sums add up in its registers along the strip and
+//     column sums over the strip's rows; 5 exchanges per unit remain.  Alone, the pass
+//     runs at 76 bytes per clock and SM out of L2; with strips of 64 rows and units of
+//     64 x 16 (less read above the diagonal, more exchanged) at 63, with the column sums
+//     exchanged for every 32 rows at 52, with 32 bytes of four columns per 8 lanes at 31
+//     (the L1 lines per instruction).  Row sums go to a slot per (warp of the strip,
+//     row), column sums to a slot per strip, both in the owner's shared memory; they are
+//     added in a fixed order.
 //   * The updated column, the partial dot products and the panel's next row are
 //     stored straight into every CTA's shared memory: two cluster barriers per column.
 //   * The update after the panel runs on the FP64 tensor cores (DMMA), a 32 x 32
@@ -26,47 +25,47 @@
 constexpr int kTcFixed = 1024;      // doubles of the scalars in front of the panel's arrays
 constexpr int kTcRed = 34;          // doubles of one CTA's partial sums: |x|^2, V^T x (16), W^T x (16)
 constexpr int kTcNoRow = 1 << 30;
-// Strips of 32 SR rows, units of 32 / SR columns (SR^2 per strip's width): unit q of strip I
-// is number tc_start(I) + q of the lower triangle.
-__host__ __device__ constexpr int tc_strips(int s, int sr) { return (s + 32 * sr - 1) / (32 * sr); }
-__host__ __device__ constexpr int tc_start(int I, int sr) { return sr * sr * (I * (I + 1) / 2); }
-__host__ __device__ constexpr int tc_units(int s, int sr) {
-    return tc_start(tc_strips(s, sr) - 1, sr) + (s * sr + 31) / 32;
-}
-// Warps that take part (on a cluster runs of two units or more: more warps mean more row
-// slots to add) and the row slots of a strip: the most warps that its units are spread over.
-__host__ __device__ constexpr int tc_warps(int s, int sr, int nw) {
-    const int n = tc_units(s, sr), w = nw > 16 ? n / 2 : n;
+constexpr int kTcSr = 4;             // 32-row steps of a strip
+constexpr int kTcRows = 32 * kTcSr;  // rows of a strip and of a unit
+constexpr int kTcCols = 32 / kTcSr;  // columns of a unit
+// Unit q of strip I is number tc_start(I) + q of the lower triangle.
+__host__ __device__ constexpr int tc_strips(int s) { return (s + kTcRows - 1) / kTcRows; }
+__host__ __device__ constexpr int tc_start(int I) { return kTcSr * kTcSr * (I * (I + 1) / 2); }
+__host__ __device__ constexpr int tc_strip_units(int s) { return (s + kTcCols - 1) / kTcCols; }   // of the last strip
+__host__ __device__ constexpr int tc_units(int s) { return tc_start(tc_strips(s) - 1) + tc_strip_units(s); }
+// Warps that take part (runs of two units or more: more warps mean more row slots to add)
+// and the row slots of a strip: the most warps that its units are spread over.
+__host__ __device__ constexpr int tc_warps(int s, int nw) {
+    const int w = tc_units(s) / 2;
     return w >= nw ? nw : w > 1 ? w : 1;
 }
-__host__ __device__ constexpr int tc_row_slots(int s, int sr, int nw) {
-    const int U = (s * sr + 31) / 32, run = tc_units(s, sr) / tc_warps(s, sr, nw);
-    return (U - 1 + run - 1) / run + 1;
+__host__ __device__ constexpr int tc_row_slots(int s, int nw) {
+    const int run = tc_units(s) / tc_warps(s, nw);
+    return (tc_strip_units(s) - 1 + run - 1) / run + 1;
 }
 __host__ __device__ constexpr int tc_own(int s, int G) { return ((s + 31) / 32 + G - 1) / G; }   // chunks per CTA
-// Doubles of shared memory per CTA of a panel of nb columns at trailing order s, G CTAs
-// of nwc warps.
-__host__ __device__ constexpr int tc_panel_doubles(int s, int nb, int sr, int G, int nwc) {
-    const int nown = tc_own(s, G), ldo = nown * 32 + 4, Ts = tc_strips(s, sr);
-    return (2 * nb + 1 + tc_row_slots(s, sr, G * nwc)) * ldo + Ts * 32 * sr + nown * Ts * 32;
+// Doubles of shared memory per CTA of a panel of nb columns at trailing order s, G CTAs.
+constexpr int kTcWarps = kT / 32;
+__host__ __device__ constexpr int tc_panel_doubles(int s, int nb, int G) {
+    const int nown = tc_own(s, G), ldo = nown * 32 + 4, Ts = tc_strips(s);
+    return (2 * nb + 1 + tc_row_slots(s, G * kTcWarps)) * ldo + Ts * kTcRows + nown * Ts * 32;
 }
-__host__ __device__ constexpr int tc_panel_width(int s, int sr, int G, int nwc, int cap) {
-    return tc_panel_doubles(s, 16, sr, G, nwc) + kTcFixed <= cap   ? 16
-           : tc_panel_doubles(s, 12, sr, G, nwc) + kTcFixed <= cap ? 12
-           : tc_panel_doubles(s, 8, sr, G, nwc) + kTcFixed <= cap  ? 8
-           : tc_panel_doubles(s, 4, sr, G, nwc) + kTcFixed <= cap  ? 4
-                                                                 : 0;
+__host__ __device__ constexpr int tc_panel_width(int s, int G, int cap) {
+    return tc_panel_doubles(s, 16, G) + kTcFixed <= cap   ? 16
+           : tc_panel_doubles(s, 12, G) + kTcFixed <= cap ? 12
+           : tc_panel_doubles(s, 8, G) + kTcFixed <= cap  ? 8
+           : tc_panel_doubles(s, 4, G) + kTcFixed <= cap  ? 4
+                                                          : 0;
 }
 // Shared memory per SM that a launch asks for (what is not shared memory is L1, and the
-// loads in flight need L1 lines), in doubles per CTA of nt threads (512 / nt CTAs per
-// SM): the smallest with panels of kTcMinWidth columns or more, 0: too large for G CTAs.
+// loads in flight need L1 lines), in doubles per CTA: the smallest with panels of
+// kTcMinWidth columns or more, 0: too large for G CTAs.
 constexpr int kTcMinWidth = 8;
-constexpr int kTcOwnMax = 1;        // owned rows per thread
-constexpr int tc_cap(int m, int sr, int G, int nt) {
-    if (tc_own(m, G) * 32 > kTcOwnMax * nt) return 0;
+constexpr int tc_cap(int m, int G) {
+    if (tc_own(m, G) > kTcWarps) return 0;   // a warp owns one chunk at most
     for (int i = 0; i < 4; ++i) {
-        const int cap = (kTrdCaps[i] * (nt / 32) / 16 - 1024) / 8;
-        if (tc_panel_width(m, sr, G, nt / 32, cap) >= kTcMinWidth) return cap;
+        const int cap = (kTrdCaps[i] - 1024) / 8;
+        if (tc_panel_width(m, G, cap) >= kTcMinWidth) return cap;
     }
     return 0;
 }
@@ -74,10 +73,10 @@ constexpr int kTcPadCols = 16;      // zeroed columns after a problem's C, and 1
 constexpr int kTcPadRows = 128;
 // Pg: the panel's V and W rows for the update, m x 32 doubles of global scratch (row r: V
 // 16, W 16).
-template <int SR>
-__device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, double* __restrict__ Da, double* __restrict__ Ea,
-                          double* __restrict__ Ta, double* __restrict__ Pg, double* smem, int cap) {
-    constexpr int NT = kT, NW = NT / 32, RPT = kTcOwnMax, H = 32 * SR, UC = SR * SR, NC = 16 / SR;
+__device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, double* __restrict__ Da,
+                                  double* __restrict__ Ea, double* __restrict__ Ta, double* __restrict__ Pg,
+                                  double* smem, int cap) {
+    constexpr int NT = kT, NW = kTcWarps, SR = kTcSr, H = kTcRows, UC = SR * SR, NC = kTcCols / 2;
     cg::cluster_group cl = cg::this_cluster();
     const int G = (int)cl.num_blocks(), rk = (int)cl.block_rank(), gsh = 31 - __clz(G);   // G: a power of two
     const int m = p.m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gw = rk * NW + warp;
@@ -100,40 +99,32 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
     for (int64_t i = rk * NT + tid; i < kTcPadCols * lda + kTcPadRows; i += G * NT) A[m * lda + i] = 0.0;
     cl.sync();
     for (int j0 = 0; j0 < m - 1;) {
-        const int s = m - j0, Ts = tc_strips(s, SR), nun = tc_units(s, SR);
+        const int s = m - j0, Ts = tc_strips(s), nun = tc_units(s);
         const int nown = tc_own(s, G), ldo = nown * 32 + 4;
-        const int width = tc_panel_width(s, SR, G, NW, cap), nb = min(width, m - 1 - j0);
-        const int nwe = tc_warps(s, SR, NW * G);
+        const int width = tc_panel_width(s, G, cap), nb = min(width, m - 1 - j0);
+        const int nwe = tc_warps(s, NW * G);
         double* V = arr;                       // [q][owned row]
         double* W = V + width * ldo;
         double* yl = W + width * ldo;          // owned rows of the updated column
         double* rowp = yl + ldo;               // [slot][owned row]
-        double* vb = rowp + tc_row_slots(s, SR, NW * G) * ldo;   // the column, then the reflector (Ts H)
+        double* vb = rowp + tc_row_slots(s, NW * G) * ldo;   // the column, then the reflector (Ts H)
         double* colp = vb + Ts * H;            // [owned chunk][strip][32]
         double* Aj = A + j0 + j0 * lda;        // element (r, c) of the trailing block at Aj[r + c lda]
-        int row[RPT], pos[RPT];
-        double nxt[RPT];
-#pragma unroll
-        for (int k = 0; k < RPT; ++k) {
-            const int i = warp + NW * k, ch = rk + G * i;
-            row[k] = i < nown ? ch * 32 + lane : kTcNoRow;   // (rows past s: the owned arrays hold zeros)
-            pos[k] = i * 32 + lane;
-            nxt[k] = row[k] < s ? Aj[row[k]] : 0.0;
-        }
+        // this thread's row (rows past s: the owned arrays hold zeros) and its place there
+        const int r = warp < nown ? (rk + G * warp) * 32 + lane : kTcNoRow, o = warp * 32 + lane;
+        double nxt = r < s ? Aj[r] : 0.0;
         // slots of strip I: from the warp of its first unit to the warp of its last
-        auto first_warp = [&](int I) { return ((tc_start(I, SR) + 1) * nwe - 1) / nun; };
+        auto first_warp = [&](int I) { return ((tc_start(I) + 1) * nwe - 1) / nun; };
         auto slots = [&](int I) {
-            const int end = I + 1 == Ts ? nun : tc_start(I + 1, SR);
+            const int end = I + 1 == Ts ? nun : tc_start(I + 1);
             return (end * nwe - 1) / nun - first_warp(I) + 1;
         };
-        int nsl[RPT];
-#pragma unroll
-        for (int k = 0; k < RPT; ++k) nsl[k] = row[k] < s ? slots(row[k] / H) : 0;
+        const int nsl = r < s ? slots(r / H) : 0;
         const int nsl0 = slots(0);
         // this warp's run of units
         const int ubeg = gw < nwe ? nun * gw / nwe : 0, uend = gw < nwe ? nun * (gw + 1) / nwe : 0;
         int Ibeg = 0;
-        while (tc_start(Ibeg + 1, SR) <= ubeg) ++Ibeg;
+        while (tc_start(Ibeg + 1) <= ubeg) ++Ibeg;
         double tq = 0.0;   // tau of the panel's last reflector
         // w of reflector q on the owned rows; on a cluster also V and W at row q + 1 (the
         // next column's) for every CTA: that row is in chunk 0, owned by CTA 0
@@ -154,24 +145,20 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
                     rows[((q + 1) & 1) * 32 + 16 + q] = tq * (y - hc);
                 }
             }
-#pragma unroll
-            for (int k = 0; k < RPT; ++k) {
-                const int r = row[k], o = pos[k];
-                if (r >= kTcNoRow) continue;
-                double w = 0.0;
-                if (r > q && r < s) {
-                    double y = 0.0;
+            if (r >= kTcNoRow) return;
+            double w = 0.0;
+            if (r > q && r < s) {
+                double y = 0.0;
 #pragma unroll 4
-                    for (int t = 0; t < nsl[k]; ++t) y += rowp[t * ldo + o];
-                    const double* cp = colp + (o >> 5) * Ts * 32 + lane;
+                for (int t = 0; t < nsl; ++t) y += rowp[t * ldo + o];
+                const double* cp = colp + warp * Ts * 32 + lane;
 #pragma unroll 4
-                    for (int I = r / H; I < Ts; ++I) y += cp[I * 32];
+                for (int I = r / H; I < Ts; ++I) y += cp[I * 32];
 #pragma unroll 4
-                    for (int i = 0; i < q; ++i) y -= V[i * ldo + o] * wtv[i] + W[i * ldo + o] * vtv[i];
-                    w = tq * (y - hc * V[q * ldo + o]);
-                }
-                W[q * ldo + o] = w;
+                for (int i = 0; i < q; ++i) y -= V[i * ldo + o] * wtv[i] + W[i * ldo + o] * vtv[i];
+                w = tq * (y - hc * V[q * ldo + o]);
             }
+            W[q * ldo + o] = w;
         };
         for (int jj = 0; jj < nb; ++jj) {
             const int j = j0 + jj;
@@ -180,22 +167,18 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
             __syncthreads();
             // ---- column j with the panel's updates, to every CTA; |x|^2, V^T x, W^T x
             double part = 0.0;
-#pragma unroll
-            for (int k = 0; k < RPT; ++k) {
-                const int r = row[k], o = pos[k];
-                if (r >= jj && r < s) {
-                    double a = nxt[k];
+            if (r >= jj && r < s) {
+                double a = nxt;
 #pragma unroll 4
-                    for (int q = 0; q < jj; ++q) a -= V[q * ldo + o] * rw[q] + W[q * ldo + o] * rv[q];
-                    nxt[k] = a;
-                    yl[o] = r >= jj + 2 ? a : 0.0;
-                    if (r >= jj + 2) part = fma(a, a, part);
-                    for (int g = 0; g < G; ++g) at(vb, g)[r] = a;
-                    if (r <= jj + 1)
-                        for (int g = 0; g < G; ++g) at(scal, g)[r - jj] = a;
-                } else if (r < kTcNoRow) {
-                    yl[o] = 0.0;
-                }
+                for (int q = 0; q < jj; ++q) a -= V[q * ldo + o] * rw[q] + W[q * ldo + o] * rv[q];
+                nxt = a;
+                yl[o] = r >= jj + 2 ? a : 0.0;
+                if (r >= jj + 2) part = fma(a, a, part);
+                for (int g = 0; g < G; ++g) at(vb, g)[r] = a;
+                if (r <= jj + 1)
+                    for (int g = 0; g < G; ++g) at(scal, g)[r - jj] = a;
+            } else if (r < kTcNoRow) {
+                yl[o] = 0.0;
             }
             part = warp_sum(part);
             if (lane == 0) rva[warp] = part;   // (rva is free between its reads above and the next A v)
@@ -207,7 +190,7 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
                 } else {
                     const double* col = t < jj ? V + t * ldo : W + (t - jj) * ldo;
 #pragma unroll 4
-                    for (int o = lane; o < nown * 32; o += 32) acc = fma(col[o], yl[o], acc);
+                    for (int i = lane; i < nown * 32; i += 32) acc = fma(col[i], yl[i], acc);
                 }
                 acc = warp_sum(acc);
                 const int slot = t == 2 * jj ? 0 : t < jj ? 1 + t : 17 + t - jj;
@@ -237,19 +220,15 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
                 for (int g = 0; g < G; ++g) acc += red[g * kTcRed + 1 + i];
                 (tid < jj ? vtv : wtv)[q] = fma(sc, acc, rows[((jj + 1) & 1) * 32 + i]);
             }
-            for (int r = tid; r < Ts * H; r += NT)
-                vb[r] = (r > jj && r < s) ? (r == jj + 1 ? 1.0 : vb[r] * sc) : 0.0;
-#pragma unroll
-            for (int k = 0; k < RPT; ++k) {
-                const int r = row[k];
-                if (r < kTcNoRow) {
-                    const double v = (r < s && r > jj) ? (r == jj + 1 ? 1.0 : nxt[k] * sc) : 0.0;
-                    V[jj * ldo + pos[k]] = v;
-                    if (r > jj + 1 && r < s) Aj[r + jj * lda] = v;
-                }
-                // the next column, as it was at the panel's start
-                if (jj + 1 < nb) nxt[k] = (r > jj && r < s) ? Aj[r + (jj + 1) * lda] : 0.0;
+            for (int i = tid; i < Ts * H; i += NT)
+                vb[i] = (i > jj && i < s) ? (i == jj + 1 ? 1.0 : vb[i] * sc) : 0.0;
+            if (r < kTcNoRow) {
+                const double v = (r < s && r > jj) ? (r == jj + 1 ? 1.0 : nxt * sc) : 0.0;
+                V[jj * ldo + o] = v;
+                if (r > jj + 1 && r < s) Aj[r + jj * lda] = v;
             }
+            // the next column, as it was at the panel's start
+            if (jj + 1 < nb) nxt = (r > jj && r < s) ? Aj[r + (jj + 1) * lda] : 0.0;
             if (rk == 0 && tid == 0) {
                 d[j] = scal[0];
                 e[j] = beta;
@@ -263,7 +242,7 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
             double vav = 0.0;
             if (ubeg < uend) {
                 const int l = lane & 15, h = lane >> 4;
-                int I = Ibeg, q = ubeg - tc_start(Ibeg, SR);
+                int I = Ibeg, q = ubeg - tc_start(Ibeg);
                 double2 buf[2][NC];
                 auto load = [&](int k, const double* pa) {
 #pragma unroll
@@ -352,18 +331,14 @@ __device__ void stage_trd_cluster(const EigProb& p, double* __restrict__ Ca, dou
             cl.sync();
         }
         finish_w(nb - 1);
-        {   // the panel's rows to global memory, row r: V 16, W 16
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < RPT; ++k)
-                if (row[k] < s) {
-                    double2* pr = reinterpret_cast<double2*>(Pg + (int64_t)row[k] * 32);
-                    for (int q = 0; q < 8; ++q) {
-                        const int a = 2 * q, b = 2 * q + 1, o = pos[k];
-                        pr[q] = make_double2(a < nb ? V[a * ldo + o] : 0.0, b < nb ? V[b * ldo + o] : 0.0);
-                        pr[8 + q] = make_double2(a < nb ? W[a * ldo + o] : 0.0, b < nb ? W[b * ldo + o] : 0.0);
-                    }
-                }
+        __syncthreads();
+        if (r < s) {   // the panel's rows to global memory, row r: V 16, W 16
+            double2* pr = reinterpret_cast<double2*>(Pg + (int64_t)r * 32);
+            for (int q = 0; q < 8; ++q) {
+                const int a = 2 * q, b = 2 * q + 1;
+                pr[q] = make_double2(a < nb ? V[a * ldo + o] : 0.0, b < nb ? V[b * ldo + o] : 0.0);
+                pr[8 + q] = make_double2(a < nb ? W[a * ldo + o] : 0.0, b < nb ? W[b * ldo + o] : 0.0);
+            }
         }
         cl.sync();
         // ---- trailing block A -= V W^T + W V^T (lower 32 x 32 blocks, one per warp, 16

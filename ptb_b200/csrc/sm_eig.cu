@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <numeric>
 #include <vector>
 
 #include "sm_eig.cuh"
@@ -740,19 +741,13 @@ __host__ __device__ inline LgLayout lg_layout(int m, int G) {
 
 struct LgSmem {
     double *sA, *sB;           // tile staging
-    double* sD;                // diagonal blocks (TS x (TS+1)), union with the vectors below
     double *v, *y;             // tridiagonalisation: reflector and updated column (M each)
     double *pw, *pv, *wtv, *vtv, *wj, *vj;   // NB each
     double* red;               // kT / 32 + 2
-    double* dsc;               // scalars
-    int* ints;                 // 16
+    double* dsc;               // scalars (8)
 };
-__host__ __device__ constexpr size_t lg_union_doubles(int M) {
-    return (size_t)2 * M + 6 * NB + kT / 32 + 2 + 8 > (size_t)TS * (TS + 1) ? (size_t)2 * M + 6 * NB + kT / 32 + 2 + 8
-                                                                            : (size_t)TS * (TS + 1);
-}
 __host__ __device__ constexpr size_t lg_smem_bytes(int M) {
-    return sizeof(double) * (2 * kStageOp + lg_union_doubles(M)) + sizeof(int) * 16;
+    return sizeof(double) * (2 * kStageOp + 2 * (size_t)M + 6 * NB + kT / 32 + 2 + 8);
 }
 static_assert(lg_smem_bytes(kLargeMax) <= 232448, "cluster solver shared memory within the per-CTA limit");
 __device__ LgSmem lg_smem(unsigned char* base, int M) {
@@ -760,10 +755,8 @@ __device__ LgSmem lg_smem(unsigned char* base, int M) {
     double* d = reinterpret_cast<double*>(base);
     s.sA = d;
     s.sB = d + kStageOp;
-    double* u = d + 2 * kStageOp;
-    s.sD = u;
-    s.v = u;
-    s.y = u + M;
+    s.v = d + 2 * kStageOp;
+    s.y = s.v + M;
     s.pw = s.y + M;
     s.pv = s.pw + NB;
     s.wtv = s.pv + NB;
@@ -772,7 +765,6 @@ __device__ LgSmem lg_smem(unsigned char* base, int M) {
     s.vj = s.wj + NB;
     s.red = s.vj + NB;
     s.dsc = s.red + kT / 32 + 2;
-    s.ints = reinterpret_cast<int*>(u + lg_union_doubles(M));
     return s;
 }
 
@@ -785,10 +777,6 @@ __device__ __forceinline__ void tri_decode(int64_t idx, int& rb, int& cb) {
     cb = (int)(idx - (int64_t)r * (r + 1) / 2);
 }
 
-// w of reflector jp (column j - 1 of the panel's first column j0 = j - 1 - jp)
-// on this CTA's rows r >= j, from the summed partial products; the reflector
-// itself goes into column j - 1 below its leading 1.  Returns w at row j
-// (every CTA computes it).
 // Units of the A v pass for the trailing block from row/column s: tile rows
 // I in [s/64, nT), each cut into kSegW-column segments from column 64 (s/64).
 __device__ __forceinline__ int av_nseg(int I, int cstart) {
@@ -1040,9 +1028,8 @@ __device__ void lg_sytrd(const Grp& g, const EigProb& p, double* __restrict__ Ca
     }
 }
 
-
-// Gather and Cholesky, tridiagonalisation: a cluster per problem (order[]: largest
-// first), or with bar non-null one problem on the whole cooperative grid.
+// A cluster per problem (order[]: largest first), or with bar non-null one problem on the
+// whole cooperative grid.
 __device__ __forceinline__ Grp lg_group(unsigned* bar, int* err) {
     if (bar) return Grp{(int)blockIdx.x, (int)gridDim.x, bar, err};
     cg::cluster_group cl = cg::this_cluster();
@@ -1071,7 +1058,7 @@ __global__ void __launch_bounds__(kT, 1) k_trd_cluster(const EigProb* __restrict
     const int pi = order[blockIdx.x / cg::this_cluster().num_blocks()];
     if (status[pi] != kStOk) return;
     const EigProb p = probs[pi];
-    stage_trd_cluster<4>(p, Ca, Da, Ea, Ta, Xa + p.xoff, reinterpret_cast<double*>(smraw), cap);
+    stage_trd_cluster(p, Ca, Da, Ea, Ta, Xa + p.xoff, reinterpret_cast<double*>(smraw), cap);
 }
 
 // ---- inverse of a lower triangle, in place, and the products with it (of the strict
@@ -1228,12 +1215,12 @@ struct EigBatch {
         int off = 0, n = 0, cap = 0;
     };
     int nprob = 0;
-    int G = 1;                    // CTAs per cluster of the large problems' Cholesky
-    int nsmall = 0, nlarge = 0;
+    int G = 1;                    // CTAs per problem of k_lg_trd
+    int nlarge = 0;
     bool grid = false;            // one problem on a cooperative grid
     std::vector<Trd> trd;
     std::vector<EigProb> hp;
-    std::vector<int> order;       // small problems first, each part largest first; then by tridiagonalisation group
+    std::vector<int> order;       // by tridiagonalisation group, largest first in each
     std::vector<int2> lists;
     std::vector<DcMerge> merges;
     std::vector<Level> levels;
@@ -1372,7 +1359,7 @@ std::vector<int> trd_groups(ptbgpu_ctx* c, const std::vector<int>& m, int small_
         // clusters of 2 to 16 took 155 ms on 48 problems up to 2773, 8 for all of them 144)
         if (mm > small_max && G < 8) return false;
         if (forced > 0 && mm > small_max && G != forced) return false;
-        return tc_cap(mm, 4, G, kT) > 0 && eig_active_cached(c, G) > 0;
+        return tc_cap(mm, G) > 0 && eig_active_cached(c, G) > 0;
     };
     std::vector<int> pick(m.size(), 0);
     auto fill = [&](double T) {
@@ -1420,7 +1407,6 @@ void launch_clustered(K kern, int nclusters, int G, size_t smem, cudaStream_t s,
     PTB_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
-
 EigStreams& eig_streams(ptbgpu_ctx* c, EigBatch& eb) {
     if (!c->eig_streams) c->eig_streams = std::make_shared<EigStreams>();
     eb.st = std::static_pointer_cast<EigStreams>(c->eig_streams);
@@ -1433,13 +1419,10 @@ EigStreams& eig_streams(ptbgpu_ctx* c, EigBatch& eb) {
 void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double* Uout) {
     eig_setup_attrs();
     const int np = eb.nprob = (int)eb.hp.size();
-    std::vector<int> large;
-    for (int q = 0; q < np; ++q) (eb.hp[q].m > small_max ? large : eb.order).push_back(q);
-    auto by_size = [&](int a, int b) { return eb.hp[a].m > eb.hp[b].m; };
-    std::stable_sort(eb.order.begin(), eb.order.end(), by_size);
-    std::stable_sort(large.begin(), large.end(), by_size);
-    eb.nsmall = (int)eb.order.size();
-    eb.nlarge = (int)large.size();
+    std::vector<int> all(np);   // largest first
+    std::iota(all.begin(), all.end(), 0);
+    std::stable_sort(all.begin(), all.end(), [&](int a, int b) { return eb.hp[a].m > eb.hp[b].m; });
+    while (eb.nlarge < np && eb.hp[all[eb.nlarge]].m > small_max) ++eb.nlarge;
     if (eb.nlarge > 0 && !eb.grid) eb.G = eig_cluster_size(c, eb.nlarge);
     const int nsm = c->num_sms > 0 ? c->num_sms : 148;
     int64_t asz = 0, csz = 0, vsz = 0, bsz = 0, psz = 0, xsz = 0, ksz = 0, isz = 0;
@@ -1463,9 +1446,6 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
         bsz += p.mode == 2 ? (int64_t)p.m * p.m : 4 * (int64_t)p.nown * p.m;
     }
     // task lists, largest problems first in each
-    std::vector<int> all(large);
-    all.insert(all.end(), eb.order.begin(), eb.order.end());
-    eb.order.insert(eb.order.end(), large.begin(), large.end());
     {
         std::vector<int> ms, pick;
         for (int q : all) ms.push_back(eb.hp[q].m);
@@ -1485,7 +1465,7 @@ void eig_plan(ptbgpu_ctx* c, EigBatch& eb, cudaStream_t s, int small_max, double
                 p.xoff = xsz;
                 xsz += G == 0 ? lg_layout(p.m, eb.G).total : G == 1 ? 0 : (int64_t)32 * p.m;
                 if (t.n++ == 0) t.cap = G == 0 ? (p.m + 1) & ~1 : 0;
-                t.cap = std::max(t.cap, G == 0 ? 0 : G == 1 ? trd_cap(p.m, nt) : tc_cap(p.m, 4, G, kT));
+                t.cap = std::max(t.cap, G == 0 ? 0 : G == 1 ? trd_cap(p.m, nt) : tc_cap(p.m, G));
                 eb.order.push_back(all[i]);
             }
             if (t.n > 0) eb.trd.push_back(t);
@@ -1838,9 +1818,8 @@ void eig_fault_raise(const EigFault& f, const char* what) {
 
 void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb) { eig_fault_raise(eig_batch_fault(c, eb), "submatrix"); }
 
-void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, int64_t n, const int* d_maps, const int* d_own_cols,
-                     double* dP, double* dPdense) {
-    (void)n;
+void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, const int* d_maps, const int* d_own_cols, double* dP,
+                     double* dPdense) {
     if (eb.nprob == 0 || eb.fcols.n == 0) return;
     cudaStream_t s = c->stream;
     const EigProb* dp = eb.probs.as<EigProb>();
@@ -2181,7 +2160,7 @@ void sygv_batched_entry(ptbgpu_ctx* c, int64_t np, const int64_t* dims, const do
     PTB_CUDA(cudaMemcpyAsync(fe, b.fe.ptr, sizeof(double) * nsum, cudaMemcpyDeviceToHost, st));
     if (Pcols) {
         b.p.reserve(c, sizeof(double) * psz);
-        eig_batch_final(c, *eb, mu, 0, b.maps.as<int>(), b.own.as<int>(), nullptr, b.p.as<double>());
+        eig_batch_final(c, *eb, mu, b.maps.as<int>(), b.own.as<int>(), nullptr, b.p.as<double>());
         PTB_CUDA(cudaMemcpyAsync(Pcols, b.p.ptr, sizeof(double) * psz, cudaMemcpyDeviceToHost, st));
     }
     PTB_CUDA(cudaStreamSynchronize(st));

@@ -52,7 +52,7 @@ void eig_batch_check(ptbgpu_ctx* c, EigBatch& eb);
 // The owned columns of P_k = U occ U^T at mu for every prepared problem,
 // written into the packed result (rows map(i) <= c of column c), or with
 // dPdense non-null as m x nown column-major blocks, one after another.
-void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, int64_t n, const int* d_maps,
+void eig_batch_final(ptbgpu_ctx* c, EigBatch& eb, double mu, const int* d_maps,
                      const int* d_own_cols, double* dP, double* dPdense = nullptr);
 
 // All eigenpairs of a dense problem on the device with the same solver on the

@@ -914,8 +914,8 @@ void sm_prepare(ptbgpu_ctx* c, SmPlan& pl, const std::vector<int>& ids) {
         const char* v = getenv("PTBGPU_SM_EIG");
         return v != nullptr && std::string(v) == "library";
     }();
-    // launched on the context's stream after the side streams' start event, so
-    // that it runs while the large submatrices are solved on the side streams
+    // launched on the context's stream; what is left to cuSOLVER above kBatchMax runs on side
+    // streams beside it
     std::vector<EigProbHost> own_probs;
     if (!use_library) {
         own_probs.reserve(small.size() + large.size());
@@ -1182,7 +1182,7 @@ void sm_finish(ptbgpu_ctx* c, SmPlan& pl, double mu, double* dP) {
     const int* d_ipos = c->buf(B_SM7).as<int>();
     const double one = 1.0, zero = 0.0;
     PTB_CUDA(cudaMemsetAsync(dP, 0, sizeof(double) * (size_t)npacked(n), s));
-    if (pl.eig) eig_batch_final(c, *pl.eig, mu, n, d_maps, d_own_cols, dP);
+    if (pl.eig) eig_batch_final(c, *pl.eig, mu, d_maps, d_own_cols, dP);
     DevBuf tbuf;
     try {
         for (Bucket& bk : pl.bks) {
