@@ -1072,7 +1072,16 @@ void tc_purify_device(ptbgpu_ctx* c, int64_t n, int64_t nel, const double* dH, c
                             : orthogonalise(c, n, dH, dS, o->filter);
     phase("Gershgorin bounds");
     if (st) st->flops += (1.0 / 3.0 + 4.0) * (double)n * n * n;   // potrf + 4 trsm
-    if (o->precision == PTBGPU_PREC_FP64) {
+    if (nel == 2 * n) {
+        // every state occupied: nothing to purify (and X_0 has the eigenvalue 0, which no step
+        // raises, where the upper bound is exact)
+        double* X = c->buf(B_H).as<double>();
+        DevBuf& bw = c->buf(B_W0);
+        bw.reserve(sizeof(double) * n * n);
+        set_identity(c->stream, n, n, X, 1.0);
+        if (Suse > 0) back_transform_oz(c, n, X, bw.as<double>(), dP, Suse);
+        else back_transform(c, n, X, bw.as<double>(), dP);
+    } else if (o->precision == PTBGPU_PREC_FP64) {
         sp2_fp64(c, n, nel, pro, maxit, 0, dP, st, prl);
     } else if (!sp2_mixed(c, n, nel, pro, maxit, o->precision != 2, rounds, rtol, o->split3_iters, Suse, dP, st,
                           prl)) {

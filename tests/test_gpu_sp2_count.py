@@ -64,6 +64,34 @@ def test_too_few_iterations_are_refused(ctx, precision):
     assert ei.value.code == api.EITER
 
 
+@pytest.mark.parametrize("precision,tol", [(PREC_MIXED, 1e-6), (PREC_FP64, 1e-9)])
+@pytest.mark.parametrize("pairs", [1, 2, -1, 0])
+def test_few_electrons_and_few_holes(ctx, water8, pairs, precision, tol):
+    """One or two occupied states, one empty one, none: the neighbours in energy are in the
+    middle of a band there."""
+    s = water8
+    n = s.ndim
+    nel = 2 * (pairs if pairs > 0 else n + pairs)
+    H, S = O.blowsym(n, s.Hvec), O.blowsym(n, s.Svec)
+    U = sl.eigh(H, S)[1][:, : nel // 2]
+    opts = Options(filter=0.0, precision=precision)
+    _check(n, nel, ctx.tc_purify(n, nel, s.Hvec, s.Svec, opts)[0], 2.0 * U @ U.T, S, tol)
+    _check(n, nel, ctx.tc_purify_grouped([(n, nel, s.Hvec, s.Svec)], opts)[0][0], 2.0 * U @ U.T, S, tol)
+
+
+@pytest.mark.parametrize("precision", [PREC_MIXED, PREC_FP64])
+@pytest.mark.parametrize("nel", [2, 78, 80])
+def test_exact_spectral_bounds(ctx, nel, precision):
+    """Uncoupled states, for which the bounds of the spectrum are its ends."""
+    n = 40
+    e = np.sort(np.random.default_rng(1).random(n))
+    H, S = O.packsym(np.diag(e)), O.packsym(np.eye(n))
+    opts = Options(filter=0.0, precision=precision)
+    ref = np.diag(2.0 * (np.arange(n) < nel // 2))
+    _check(n, nel, ctx.tc_purify(n, nel, H, S, opts)[0], ref, np.eye(n), 1e-9)
+    _check(n, nel, ctx.tc_purify_grouped([(n, nel, H, S)], opts)[0][0], ref, np.eye(n), 1e-9)
+
+
 @pytest.mark.parametrize("nmol,seed", [(130, 31), (190, 27)])
 def test_frontier_state_below_the_floor_of_pass_1(ctx, nmol, seed):
     """Boxes whose pass 1 ends with a frontier state a percent away from 0 or 1, under the
