@@ -175,13 +175,14 @@ int ptbgpu_purify(ptbgpu_ctx* ctx, const ptbgpu_pur_settings* pur, int64_t ndim,
 /* Trace-correcting (SP2) purification, the B200 fast path for the dense
  * density step; replaces the mu search of purification_search
  * (source/purification.f90:232-353) with trace correction.  nel must be even.
- * opts->precision selects FP64 or bf16x3 + FP64 refinement. */
+ * opts->precision selects FP64 or bf16x3 + FP64 refinement; where the latter cannot
+ * reach opts->refine_tol the call is redone in FP64 (stats.fp64_fallback).  EITER: the
+ * FP64 iteration did not settle within opts->max_iter steps. */
 int ptbgpu_tc_purify(ptbgpu_ctx* ctx, int64_t ndim, int64_t nel,
                      const double* Hpk, const double* Spk, double* Ppk,
                      const ptbgpu_opts* opts, ptbgpu_stats* st);
 
-/* Same with device-resident packed arrays (no host copies); stream is a
- * cudaStream_t or NULL for the context's own stream. */
+/* Same with device-resident packed arrays (no host copies), on the context's own stream. */
 int ptbgpu_tc_purify_device(ptbgpu_ctx* ctx, int64_t ndim, int64_t nel,
                             const double* dHpk, const double* dSpk, double* dPpk,
                             const ptbgpu_opts* opts, ptbgpu_stats* st);
@@ -362,7 +363,7 @@ int ptbgpu_oz_gemm(ptbgpu_ctx* ctx, int64_t n, int64_t slices, int64_t kblock, i
  * host problems (kernel-level entry for tests and measurements; it replaces the
  * per-submatrix la_sygvd and the S_k U product of source/sm.f90:296-310).
  * Every stage is launched over all problems of the call.  nprob problems of orders dims[k]
- * (1..10240): H and S hold their column-major dims[k]^2 blocks one after
+ * (1..12032): H and S hold their column-major dims[k]^2 blocks one after
  * another; owned holds nown[k] (0-based, local) owned indices per problem, one
  * list after another.  Out: e and fe (sum of dims each, per problem in the
  * solver's order, not sorted): the eigenvalues of H c = e S c and the weights

@@ -79,8 +79,10 @@ __host__ __device__ inline int dc_levels(int m) {
 }
 __host__ __device__ inline int dc_start(int m, int q, int lev) { return (int)(((int64_t)q * m) >> lev); }
 
-// Leaf: implicit QL on d[0..s), e[0..s-1) with Z = I accumulated.  Every
-// lane runs the same scalar iteration on its own copies of d and e and rotates
+// Leaf: the implicit QL iteration on d[0..s), e[0..s-1) with Z = I accumulated, in the steps
+// of EISPACK's imtql2 (Martin and Wilkinson, Numer. Math. 12, 377 (1968); Dubrulle, Numer.
+// Math. 15, 450 (1970)): the shift from the leading 2 x 2 block, the chase of the bulge by
+// plane rotations and the restart where a rotation vanishes.  Every lane runs the same scalar iteration on its own copies of d and e and rotates
 // its own row z of Z (lane r holds row r), so no lane reads another's data.
 __device__ bool dc_leaf(int s, double* d, double* e, double* z, int lane) {
     const double eps = 2.220446049250313e-16;

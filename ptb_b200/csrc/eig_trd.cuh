@@ -20,9 +20,9 @@
 //   * The update after the panel runs on the FP64 tensor cores (DMMA) straight from
 //     the shared V and W, a 32 x 32 block per warp and no barrier.
 // NT = 512 threads (one CTA per SM) or 256 (two CTAs per SM, smaller orders).
-// Measured: 96 problems of order 218-595, one CTA each: 9.5 ms (29 ms with the
-// unblocked reduction that read and wrote the whole trailing square per column);
-// 602 problems of order <= 253, two CTAs per SM: 4.9 ms.
+// Measured: 96 problems of order 218-595, one CTA each: 7.0 ms (9.2 with 32
+// bytes of four columns per 8 lanes, 29 with the unblocked reduction that read and wrote
+// the whole trailing square per column); 602 problems of order <= 253, two CTAs per SM: 3.7 ms.
 
 __host__ __device__ constexpr int trd_ld(int s) { return ((s + 11) / 16) * 16 + 4; }   // >= s, = 4 mod 16
 __host__ __device__ constexpr int trd_strips(int s) { return (s + 31) / 32; }

@@ -38,7 +38,7 @@ using namespace tc::ptx;
 constexpr int THREADS = 256;
 constexpr int kSmemBudget = 196608;
 constexpr int kTmemCols = 512;
-constexpr int kSms = 148;
+constexpr int kSms = 148;   // of a whole B200: on a partition variant_for's choice costs time, not results
 // Dynamic shared memory that keeps a kernel at one resident CTA per SM (more
 // than half of the 227 KB a block may use).  The CTA-pair kernels hold all 512
 // TMEM columns of both SMs of a pair: two pair CTAs resident on the same SMs

@@ -1338,7 +1338,9 @@ int eig_cluster_size(ptbgpu_ctx* c, int nlarge) {
 }
 
 // Clocks of one tridiagonalisation on G CTAs: a chain of short steps per column and the
-// passes over the triangle (fitted to orders 576 on one CTA and 900 to 2100 on 8 and 16).
+// passes over the triangle.  Fitted to order 576 on one CTA and 900 to 2100 on 8 and 16;
+// used for all orders, where only the ratio between the sizes matters (one problem
+// alone goes from one CTA to 16 at order 360).
 double trd_clocks(int m, int G) {
     const double n = m, n3 = n * n * n;
     return G == 1 ? 7.0e3 * n + 0.058 * n3 : 14.0e3 * n + 0.05 * n3 / G;
@@ -1979,10 +1981,12 @@ void eig_density_batch(ptbgpu_ctx* c, int64_t ninst, const int64_t* ndim, const 
     // The systems above kEigBatchMax go first, in up to kEigSlots parts of the input
     // order, each a batch on a stream of its own: a part is copied in while the one
     // before it is solved, and copied out while the next is.  The small systems are
-    // copied in after them and solved and copied out beside them.  Parts smaller than
-    // kPartMin systems leave a wave of clusters short (64 systems in four parts 590 ms, in
-    // two 550, in one 659), but two parts pay from kPartMin on: 32 systems 368 -> 336 ms,
-    // 100 862 -> 782, 256 1.79 -> 1.65 s (pageable host arrays, copies inside).
+    // copied in after them and solved and copied out beside them.  A part of few systems
+    // leaves SMs idle, so that two parts lose against one below 20 large systems and pay
+    // above (ndim 1000 to 3060, pageable host arrays, copies inside; two parts against one:
+    // 8 systems 217 / 168 ms, 16 272 / 262, 20 305 / 304, 24 325 / 343, 28 375 / 412, 32
+    // 401 / 468), and more than two need parts of 24 each (64 systems in two parts 550 ms, in
+    // four 590, in one 659; 100 862 -> 782, 256 1.79 -> 1.65 s).
     constexpr size_t kPartMin = 24;
     std::vector<int64_t> large, small;
     std::vector<int64_t> pkoff((size_t)ninst + 1, 0);

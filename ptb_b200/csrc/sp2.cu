@@ -24,7 +24,10 @@
 //            its response is propagated through the recorded branch sequence
 //            over the stored trajectory, X1 <- X0_k X1 + X1 X0_k (or
 //            2 X1 - (...)), again with bf16x3 products; P = P~ + X1.
-//            The error left is second order in the pass-1 error.
+//            The error left is second order in the pass-1 error; rounds repeat
+//            until the predicted one is below refine_tol.
+//   A pass 1 that does not settle, a cleanup that leaves no projector onto N
+//   states, and rounds that cannot reach refine_tol are redone in FP64.
 //
 // The FP64 products of the mixed path (A = L^-1 H L^-T through the explicit
 // triangular inverse, the cleanup squares, the commutator and the
@@ -195,7 +198,8 @@ __global__ void k_split2(int64_t count, const float* __restrict__ x, __nv_bfloat
 }
 
 // Per-block partials of ||Y - X||_F^2: X an FP32 plane (ldp), Y FP64 column-major, both
-// symmetric n x n.
+// symmetric n x n.  One pass over both, 0.58 ms at order 11776 (with eight loads a thread
+// in flight 0.92) and 10 us at 1495.
 constexpr int kParts = 296;
 __global__ void k_moved(int64_t n, int64_t ldp, const float* __restrict__ x, const double* __restrict__ y,
                         double* __restrict__ out) {

@@ -18,7 +18,8 @@ constexpr int kPairKernel = 1000;
 // tiles fit one wave.  The accumulation order over K and the plane products is
 // that of every other kernel: the results are the same bits.
 constexpr int kNarrowKernel = 2064;
-// Whether they do, with `tiles` tiles of 128 x 128: 256 x 256 tiles on CTA pairs
+// Whether they do, with `tiles` tiles of 128 x 128 on the 148 SMs of a whole B200 (on a
+// partition the choice costs time, not results): 256 x 256 tiles on CTA pairs
 // then occupy less than half of the 148 SMs for twice the time (order 1495, padded
 // to 1536: the symmetric product 42 CTAs 73 us, 78 narrow ones 58; the general one
 // 72 CTAs 43 us, 144 narrow ones 38).
